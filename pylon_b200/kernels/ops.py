@@ -243,6 +243,7 @@ _SIGNATURES = {
         "pylon_gemm_f32_nt": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p],
         "pylon_gemm_f32_nt_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_longlong,
                                       c_longlong, c_longlong, c_void_p],
+        "pylon_gemm_f32_nt_forced": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
     },
     "attention_latent.cu": {
         "pylon_latent_attention": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
@@ -671,7 +672,7 @@ SKINNY_MAX_ROWS = 8   # up to this many rows the weight-streaming kernel runs (i
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``x [M, K] @ w [N, K].T`` with float32 accumulation.
 
-    float32 operands use the plain-FMA kernel (true 32-bit, no tensor cores).  bfloat16
+    float32 operands use the plain-FMA kernels (true 32-bit, no tensor cores; a row's bits do not depend on the others).  bfloat16
     operands with up to ``SKINNY_MAX_ROWS`` rows use the weight-streaming kernel; many rows
     whose 128 x 256 tiles fill whole rounds over the SMs use our tcgen05 kernel; the rest go to
     the library matrix product, as raun6k/Pylon's ``nn.Linear`` layers do

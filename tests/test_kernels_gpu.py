@@ -91,6 +91,29 @@ def test_gemm_f32_is_true_32_bit(m, n, k):
     assert torch.equal(alone[0], y[0])
 
 
+@pytest.mark.parametrize("n, k", [(64, 64), (130, 33), (97, 515), (300, 20), (517, 1000), (2560, 4096), (1000, 9728), (70_000, 64)])
+def test_gemm_f32_gives_a_row_the_same_bits_in_every_kernel(n, k):
+    """Around every edge of the dispatch and in every tile and cluster size: the sum's order is a function of k alone."""
+    from pylon_b200.kernels import ops
+
+    x = torch.randn(300, k + 4, device=DEVICE)[:, :k]
+    w = torch.randn(n, k, device=DEVICE) * 0.05
+    full = ops.linear(x, w)
+    expected = x.double() @ w.double().T
+    # chains of at most k / 32 + 16 terms, 32 of them added up: a random walk of half an ulp a step
+    bound = 0.5 * 2.0**-23 * ((k / 32 + 16) ** 0.5 + 32**0.5)
+    assert float((full.double() - expected).norm() / expected.norm()) < bound
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 129):
+        assert torch.equal(ops.linear(x[:m].contiguous(), w), full[:m]), m
+    library = ops._library("gemm_f32.cu")
+    tiles = [(2, 8), (3, 5), (3, 6), (4, 5), (4, 6), (4, 7), (5, 5), (6, 5), (7, 4), (7, 5)] if k % 4 == 0 else [(4, 4)]
+    for m, forms in ((11, (-1, -2)), (129, [100 * tm + 10 * tn + blocks for tm, tn in tiles for blocks in (1, 2, 4, 8)])):
+        for form in forms:
+            y = torch.full((m, n), float("nan"), device=DEVICE)
+            ops._check(library, library.pylon_gemm_f32_nt_forced(ops._ptr(x), ops._ptr(w), ops._ptr(y), m, n, k, x.stride(0), k, n, form, ops._stream()))
+            assert torch.equal(y, full[:m]), (m, form)
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 256, 128), (8, 6144, 2560), (40, 1000, 96), (300, 320, 224)])
 def test_linear_bf16(m, n, k):
     from pylon_b200.kernels import ops

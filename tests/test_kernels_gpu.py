@@ -522,6 +522,37 @@ def test_paged_attention(case, mode):
     assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0   # no wait for a TMA copy ran out
 
 
+@pytest.mark.parametrize("nq, nkv, d, dv", [(4, 1, 64, 64), (6, 3, 20, 36), (3, 3, 128, 192), (8, 1, 132, 512), (5, 1, 8, 4)])
+@pytest.mark.parametrize("options", ["plain", "window", "kept", "chunk", "softcap", "bias", "slopes", "sinks", "sigmoid", "gate", "elements"])
+def test_float32_attention_with_shared_reads(nq, nkv, d, dv, options):
+    """The float32 kernel that shares its reads between heads against the plain one, which rows that start off a 16-byte
+    boundary go to: every option, groups of 1 to 8 heads, contexts around the chunks of 128 keys."""
+    from pylon_b200.kernels import ops
+
+    kv_lens, q_lens = [1, 128, 129, 300, 257], [1, 2, 129, 3, 1]
+    cache = Paged(kv_lens, q_lens, nkv, d, 16, torch.float32, seed=3)
+    v_pages = torch.randn((*cache.k_pages.shape[:3], dv), device=DEVICE)
+    tokens = cache.tokens
+    q = torch.randn(tokens, nq * d, device=DEVICE)
+    head, element = torch.randn(tokens, nq, device=DEVICE), torch.randn(tokens, nq * dv, device=DEVICE)
+    keywords = {"plain": {}, "window": dict(window=130), "kept": dict(window=40, keep_first=5), "chunk": dict(chunk=100), "softcap": dict(softcap=3.0),
+                "bias": dict(distance_bias=torch.randn(150, nq, device=DEVICE)), "slopes": dict(distance_slopes=torch.rand(nq, device=DEVICE) * 0.1),
+                "sinks": dict(sinks=torch.randn(nq, device=DEVICE)), "sigmoid": dict(weighting="sigmoid", score_bias=torch.randn(nq, device=DEVICE) - 5),
+                "gate": dict(head_gate=head, out_factor=0.5), "elements": dict(head_gate=element)}[options]
+
+    def run(k_pages, v_pages):
+        return ops.paged_attention(q, k_pages, v_pages, cache.positions, cache.token_row, cache.q_start, cache.kv_len, cache.table, nq, max(q_lens),
+                                   max(kv_lens), **keywords)
+
+    def shifted(pages):
+        flat = torch.empty(pages.numel() + 1, device=DEVICE)
+        flat[1:] = pages.reshape(-1)
+        return flat[1:].view(pages.shape)
+
+    # sums of at most 300 products in another order: some ulps of the largest term
+    torch.testing.assert_close(run(cache.k_pages, v_pages), run(shifted(cache.k_pages), shifted(v_pages)), rtol=2e-5, atol=2e-6)
+
+
 @pytest.mark.parametrize("d, nq, nkv", [(128, 32, 8), (64, 12, 4)])
 def test_tcgen05_attention_gives_the_same_bits_every_time(d, nq, nkv):
     """Eight prompt portions of some 500 tokens: several waves of blocks, each with eight key tiles and more in flight.  A

@@ -4,7 +4,8 @@
 // tcgen05.ld for the epilogue.  For the products of prompt portions (many rows).
 //
 // One persistent block per SM walks 128 x BN output tiles.  Six warps with fixed roles:
-//   warp 0      TMA producer: fills a ring of STAGES shared-memory stages (A 128 x 64, B BN x 64)
+//   warp 0      TMA producer: fills a ring of STAGES shared-memory stages (A 128 x 64, B BN x 64), the first boxes of B
+//               before the kernel ahead has finished
 //   warp 1      MMA issuer: four tcgen05.mma (K = 16 each) per stage into one of two
 //               accumulator buffers in tensor memory; tcgen05.commit frees the stage and, after
 //               the last stage of a tile, hands the accumulator to the epilogue
@@ -130,16 +131,21 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 
 constexpr int TC_STAGING_BYTES = 4 * 2 * 32 * 128;   // four epilogue warps x two buffers x 32 rows x up to 128 bytes
 
-template <int BN>
+// R: row tiles of 128 that a block multiplies by the same tile of B.  With R = 2 (the product's only rows, 129 to 256) a stage's A holds the
+// rows there are, rounded up to 32, and no more: the second product reads on into what lies behind them, for rows that are not stored;
+// the smaller stages are then more (160 rows: four of 44 KB where two whole tiles of A left room for three).
+template <int BN, int R = 1>
 struct TcShared {
-  static constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
+  static constexpr int A_BYTES = R * TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
   static constexpr int PIECES = BN > 256 ? 2 : 1;            // products (and boxes of B) per step of k: the tensor core's N and a TMA box end at 256
   static constexpr int PIECE_ROWS = BN / PIECES;
-  static constexpr int ACCUMULATORS = 2 * BN <= 512 ? 2 : 1;  // buffers in tensor memory (512 columns)
+  static constexpr int ACCUMULATORS = 2 * R * BN <= 512 ? 2 : 1;  // buffers in tensor memory (512 columns)
+  static_assert(R == 1 || PIECES == 1, "several row tiles go with a B tile of one piece");
   static_assert(PIECE_ROWS % 16 == 0 && PIECE_ROWS <= 256 && (PIECE_ROWS * 128) % 1024 == 0, "a piece of B must be a valid N and start on a swizzle group");
   static constexpr int FIT = (227 * 1024 - 1024 /* alignment slack */ - 256 /* barriers */ - TC_STAGING_BYTES) / (A_BYTES + B_BYTES);
   static constexpr int STAGES = FIT > 6 ? 6 : FIT;
-  static constexpr size_t BYTES = (size_t)STAGES * (A_BYTES + B_BYTES) + TC_STAGING_BYTES + 1024 + 256;
+  static constexpr size_t RING = 227 * 1024 - 1024 - 256 - TC_STAGING_BYTES;   // with R = 2: what the stages, however many, share
+  static constexpr size_t BYTES = R > 1 ? RING + TC_STAGING_BYTES + 1024 + 256 : (size_t)STAGES * (A_BYTES + B_BYTES) + TC_STAGING_BYTES + 1024 + 256;
 };
 
 // Columns of the output that one TMA store writes: 64 (128-byte rows, 128-byte swizzle) where the tile's width divides
@@ -301,38 +307,40 @@ __device__ __forceinline__ void rotate_epilogue(const RotateArgs& rot, uint32_t 
 }
 
 // error: 0 = fine; otherwise 1 producer, 2 MMA issuer, 3 epilogue gave up waiting.
-template <int BN, int MODE, int D>
+template <int BN, int MODE, int D, int R = 1>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                       const __grid_constant__ CUtensorMap map_b,
                                                                       const __grid_constant__ CUtensorMap map_c, int M, int N, int K,
                                                                       int* __restrict__ error, const RotateArgs rot,
                                                                       const int* __restrict__ tile_group, int group_rows) {
   constexpr bool SWIGLU = MODE == TC_SWIGLU;
-  using S = TcShared<BN>;
-  constexpr int STAGES = S::STAGES;
+  using S = TcShared<BN, R>;
+  constexpr int MOST_STAGES = R > 1 ? 6 : S::STAGES;
+  const int a_rows = R > 1 ? (M + 31) & ~31 : TC_BM, a_bytes = a_rows * TC_BK * 2;
+  const int stages = R > 1 ? min(MOST_STAGES, (int)S::RING / (a_bytes + S::B_BYTES)) : S::STAGES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* a_tiles = smem;
-  unsigned char* b_tiles = smem + (size_t)STAGES * S::A_BYTES;
-  unsigned char* staging = b_tiles + (size_t)STAGES * S::B_BYTES;   // 1024-byte aligned: every stage is a multiple of that
+  unsigned char* b_tiles = smem + (size_t)stages * a_bytes;
+  unsigned char* staging = b_tiles + (size_t)stages * S::B_BYTES;   // 1024-byte aligned: every stage is a multiple of that
   uint64_t* full = reinterpret_cast<uint64_t*>(staging + TC_STAGING_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* acc_full = empty + STAGES;      // [2]
+  uint64_t* empty = full + MOST_STAGES;
+  uint64_t* acc_full = empty + MOST_STAGES;      // [2]
   uint64_t* acc_empty = acc_full + 2;       // [2]
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + BN - 1) / BN;
+  const int tiles_m = (M + R * TC_BM - 1) / (R * TC_BM), tiles_n = (N + BN - 1) / BN;
   const int total_tiles = tiles_m * tiles_n;
   const int k_blocks = (K + TC_BK - 1) / TC_BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   constexpr int ACCUMULATORS = S::ACCUMULATORS;
-  constexpr int TMEM_COLUMNS = ACCUMULATORS * BN <= 256 ? 256 : 512;   // the accumulator buffers; allocations are powers of two
+  constexpr int TMEM_COLUMNS = ACCUMULATORS * R * BN <= 256 ? 256 : 512;   // the accumulator buffers; allocations are powers of two
   if (warp == 1) {   // the whole warp allocates
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_base_slot)), "r"(TMEM_COLUMNS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
@@ -341,8 +349,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
-  // Barriers and tensor memory are set up while the kernel before this one finishes (dependent launch); its output is
-  // read, and anything written, only from here on.
+  // Barriers and tensor memory are set up while the kernel before this one finishes (dependent launch).  So are the first boxes of the
+  // weights asked for, which do not depend on it (which of several stacked matrices a tile multiplies by may): the activations'
+  // boxes follow on the same barriers.
+  const int ahead = tile_group || (int)blockIdx.x >= total_tiles ? 0 : (k_blocks < stages ? k_blocks : stages);
+  if (warp == 0 && lane == 0) {
+    for (int kb = 0; kb < ahead; ++kb) {
+      mbar_expect_tx(&full[kb], a_bytes + S::B_BYTES);
+#pragma unroll
+      for (int piece = 0; piece < S::PIECES; ++piece)
+        tma_load_2d(b_tiles + (size_t)kb * S::B_BYTES + (size_t)piece * S::PIECE_ROWS * 128, &map_b, &full[kb], kb * TC_BK,
+                    (int)(blockIdx.x / tiles_m) * BN + piece * S::PIECE_ROWS);
+    }
+  }
+  // That kernel's output is read, and anything written, only from here on.
   grid_dependency_wait();
   allow_dependents();
 
@@ -351,18 +371,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
       uint32_t stage = 0, phase = 0;
       bool alive = true;
       for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x) {
-        const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BN;   // neighbours in the grid share their B tile
+        const int m0 = (tile % tiles_m) * (R * TC_BM), n0 = (tile / tiles_m) * BN;   // neighbours in the grid share their B tile
         const int group = tile_group ? tile_group[tile % tiles_m] : 0;
         if (group < 0) continue;                                               // a row tile that holds nothing: all three roles pass over it
         const int b_row = group * group_rows + n0;
         for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1)) { atomicExch(error, 1); alive = false; break; }
-          mbar_expect_tx(&full[stage], S::A_BYTES + S::B_BYTES);
-          tma_load_2d(a_tiles + (size_t)stage * S::A_BYTES, &map_a, &full[stage], kb * TC_BK, m0);
+          const bool asked = tile == (int)blockIdx.x && kb < ahead;   // the weights' box of this stage is on its way already
+          if (!asked) {
+            if (!mbar_wait(&empty[stage], phase ^ 1)) { atomicExch(error, 1); alive = false; break; }
+            mbar_expect_tx(&full[stage], a_bytes + S::B_BYTES);
+          }
+          tma_load_2d(a_tiles + (size_t)stage * a_bytes, &map_a, &full[stage], kb * TC_BK, m0);
 #pragma unroll
-          for (int piece = 0; piece < S::PIECES; ++piece)
+          for (int piece = 0; piece < (asked ? 0 : S::PIECES); ++piece)
             tma_load_2d(b_tiles + (size_t)stage * S::B_BYTES + (size_t)piece * S::PIECE_ROWS * 128, &map_b, &full[stage], kb * TC_BK, b_row + piece * S::PIECE_ROWS);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if ((int)++stage == stages) { stage = 0; phase ^= 1; }
         }
       }
     }
@@ -378,19 +401,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
         ++round;
         if (!mbar_wait(&acc_empty[buffer], buffer_phase ^ 1)) { atomicExch(error, 2); break; }
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + buffer * BN;
+        const uint32_t tmem_d = tmem_base + buffer * (R * BN);
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!mbar_wait(&full[stage], phase)) { atomicExch(error, 2); alive = false; break; }
           tc_fence_after();
-          const uint64_t a_desc = tc_smem_desc(a_tiles + (size_t)stage * S::A_BYTES);
+          const uint64_t a_desc = tc_smem_desc(a_tiles + (size_t)stage * a_bytes);
           const uint64_t b_desc = tc_smem_desc(b_tiles + (size_t)stage * S::B_BYTES);
 #pragma unroll
           for (int k = 0; k < TC_BK / 16; ++k)   // 16 k-values = 32 bytes further along the swizzled row: +2 in 16-byte units
 #pragma unroll
             for (int piece = 0; piece < S::PIECES; ++piece)   // a piece of B lies PIECE_ROWS rows of 128 bytes further on, its columns of the accumulator likewise
-              tc_mma(tmem_d + piece * S::PIECE_ROWS, a_desc + 2 * k, b_desc + 2 * k + (uint64_t)((piece * S::PIECE_ROWS * 128) >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
+#pragma unroll
+              for (int r = 0; r < R; ++r)                       // and so does a row tile of A
+                tc_mma(tmem_d + piece * S::PIECE_ROWS + r * BN, a_desc + 2 * k + (uint64_t)((r * TC_BM * 128) >> 4),
+                       b_desc + 2 * k + (uint64_t)((piece * S::PIECE_ROWS * 128) >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
           tc_commit(&empty[stage]);   // the stage is free once these products have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if ((int)++stage == stages) { stage = 0; phase ^= 1; }
         }
         if (alive) tc_commit(&acc_full[buffer]);   // the accumulator is complete once all products are
       }
@@ -404,58 +430,61 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
     uint32_t round = 0, staged = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
       if (tile_group && tile_group[tile % tiles_m] < 0) continue;
-      const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BN;
+      const int m0 = (tile % tiles_m) * (R * TC_BM), n0 = (tile / tiles_m) * BN;
       const uint32_t buffer = round % ACCUMULATORS, buffer_phase = (round / ACCUMULATORS) & 1;
       ++round;
       if (!mbar_wait(&acc_full[buffer], buffer_phase)) { atomicExch(error, 3); break; }
       tc_fence_after();
-      const int row0 = m0 + quarter * 32;
-      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * BN;
-      const float row_scale = SWIGLU && rot.unit_row_scale && row0 + lane < M ? rot.unit_row_scale[row0 + lane] : 1.f;
       if constexpr (MODE == TC_ROTATE) {
-        rotate_epilogue<BN, D>(rot, taddr, my_staging, row0, n0, M, lane);
+        rotate_epilogue<BN, D>(rot, tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * BN, my_staging, m0 + quarter * 32, n0, M, lane);
       } else
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += Store::ACCUMULATOR_COLUMNS, ++staged) {
-        unsigned char* stage_rows = my_staging + (staged & 1) * (32 * 128);
-        if (lane == 0) tma_store_wait_read<1>();   // the store that last read this buffer is two stores back
-        __syncwarp();
+      for (int r = 0; r < R; ++r) {
+        const int row0 = m0 + r * TC_BM + quarter * 32;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * (R * BN) + r * BN;
+        const float row_scale = SWIGLU && rot.unit_row_scale && row0 + lane < M ? rot.unit_row_scale[row0 + lane] : 1.f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += Store::ACCUMULATOR_COLUMNS, ++staged) {
+          unsigned char* stage_rows = my_staging + (staged & 1) * (32 * 128);
+          if (lane == 0) tma_store_wait_read<1>();   // the store that last read this buffer is two stores back
+          __syncwarp();
 #pragma unroll
-        for (int part = 0; part < Store::ACCUMULATOR_COLUMNS / 32; ++part) {
-          uint32_t raw[32];
-          tc_load_32(taddr + c0 + part * 32, raw);
-          uint32_t packed[16];
-          if (SWIGLU) {   // [g0..g7 u0..u7 g8..g15 u8..u15] -> 16 outputs
+          for (int part = 0; part < Store::ACCUMULATOR_COLUMNS / 32; ++part) {
+            uint32_t raw[32];
+            tc_load_32(taddr + c0 + part * 32, raw);
+            uint32_t packed[16];
+            if (SWIGLU) {   // [g0..g7 u0..u7 g8..g15 u8..u15] -> 16 outputs
 #pragma unroll
-            for (int group = 0; group < 2; ++group)
+              for (int group = 0; group < 2; ++group)
 #pragma unroll
-              for (int j = 0; j < 8; j += 2) {
-                const float g0 = row_scale * __uint_as_float(raw[group * 16 + j]), g1 = row_scale * __uint_as_float(raw[group * 16 + j + 1]);
-                const float u0 = row_scale * __uint_as_float(raw[group * 16 + 8 + j]), u1 = row_scale * __uint_as_float(raw[group * 16 + 8 + j + 1]);
-                packed[group * 4 + j / 2] = pack2(gated_unit_fast(g0, u0, rot.unit_limit, rot.unit_alpha), gated_unit_fast(g1, u1, rot.unit_limit, rot.unit_alpha));
-              }
-          } else {
+                for (int j = 0; j < 8; j += 2) {
+                  const float g0 = row_scale * __uint_as_float(raw[group * 16 + j]), g1 = row_scale * __uint_as_float(raw[group * 16 + j + 1]);
+                  const float u0 = row_scale * __uint_as_float(raw[group * 16 + 8 + j]), u1 = row_scale * __uint_as_float(raw[group * 16 + 8 + j + 1]);
+                  packed[group * 4 + j / 2] = pack2(gated_unit_fast(g0, u0, rot.unit_limit, rot.unit_alpha), gated_unit_fast(g1, u1, rot.unit_limit, rot.unit_alpha));
+                }
+            } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) packed[j] = pack2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
+              for (int j = 0; j < 16; ++j) packed[j] = pack2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
+            }
+            constexpr int UNITS = SWIGLU ? 2 : 4;   // 16-byte units this part adds to the row
+#pragma unroll
+            for (int unit = 0; unit < UNITS; ++unit) {
+              uint32_t offset = (uint32_t)lane * Store::ROW_BYTES + (uint32_t)(part * UNITS + unit) * 16;
+              offset ^= ((offset >> 7) & Store::SWIZZLE_MASK) << 4;
+              *reinterpret_cast<uint4*>(stage_rows + offset) = make_uint4(packed[unit * 4], packed[unit * 4 + 1], packed[unit * 4 + 2], packed[unit * 4 + 3]);
+            }
           }
-          constexpr int UNITS = SWIGLU ? 2 : 4;   // 16-byte units this part adds to the row
-#pragma unroll
-          for (int unit = 0; unit < UNITS; ++unit) {
-            uint32_t offset = (uint32_t)lane * Store::ROW_BYTES + (uint32_t)(part * UNITS + unit) * 16;
-            offset ^= ((offset >> 7) & Store::SWIZZLE_MASK) << 4;
-            *reinterpret_cast<uint4*>(stage_rows + offset) = make_uint4(packed[unit * 4], packed[unit * 4 + 1], packed[unit * 4 + 2], packed[unit * 4 + 3]);
+          fence_async_shared();   // the writes above, before the TMA engine reads them
+          __syncwarp();
+          const int out_column = (n0 + c0) / (SWIGLU ? 2 : 1);
+          if (lane == 0) {
+            if (row0 < M && out_column < out_columns) tma_store_2d(&map_c, stage_rows, out_column, row0);
+            // A group for every turn of this loop, empty where the rows lie outside the matrix and nothing is stored: the wait
+            // at the loop's head counts groups ("all but the newest have read their buffer"), and a turn without one would let
+            // the turn after it write the buffer that the last real store is still reading.  (Seen with a last row tile
+            // whose lower quarters lie outside the matrix: the tile a block had stored just before it came out wrong in places.)
+            tma_store_commit();
           }
-        }
-        fence_async_shared();   // the writes above, before the TMA engine reads them
-        __syncwarp();
-        const int out_column = (n0 + c0) / (SWIGLU ? 2 : 1);
-        if (lane == 0) {
-          if (row0 < M && out_column < out_columns) tma_store_2d(&map_c, stage_rows, out_column, row0);
-          // A group for every turn of this loop, empty where the rows lie outside the matrix and nothing is stored: the wait
-          // at the loop's head counts groups ("all but the newest have read their buffer"), and a turn without one would let
-          // the turn after it write the buffer that the last real store is still reading.  (Seen with a last row tile
-          // whose lower quarters lie outside the matrix: the tile a block had stored just before it came out wrong in places.)
-          tma_store_commit();
         }
       }
       tc_fence_before();
@@ -506,27 +535,27 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, long lo
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool SWIGLU>
+template <int BN, bool SWIGLU, int R = 1>
 static int launch_tcgen05(const CUtensorMap& map_a, const CUtensorMap& map_b, __nv_bfloat16* c, int M, int N, int K, long long ldc,
                           int* error, int sm_count, cudaStream_t stream, float unit_limit = 0.f, float unit_alpha = 1.f,
                           const int* tile_group = nullptr, int group_rows = 0, const float* unit_row_scale = nullptr) {
-  auto kernel = gemm_tcgen05_kernel<BN, SWIGLU ? TC_SWIGLU : TC_PLAIN, 128>;
+  auto kernel = gemm_tcgen05_kernel<BN, SWIGLU ? TC_SWIGLU : TC_PLAIN, 128, R>;
   static bool configured_on[pylon::MAX_DEVICES] = {};   // function attributes belong to a device
   bool& configured = configured_on[pylon::current_device_slot()];
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcShared<BN>::BYTES);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcShared<BN, R>::BYTES);
     if (err != cudaSuccess) PYLON_REFUSE("gemm_tcgen05: %s", cudaGetErrorString(err));
     configured = true;
   }
   CUtensorMap map_c;
   if (!make_map(&map_c, c, M, SWIGLU ? N / 2 : N, ldc, 32, TcStore<BN, SWIGLU>::COLUMNS)) PYLON_REFUSE("gemm_tcgen05: the output's tensor map could not be made");
-  const int tiles = ((M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
+  const int tiles = ((M + R * TC_BM - 1) / (R * TC_BM)) * ((N + BN - 1) / BN);
   const int blocks = tiles < sm_count ? tiles : sm_count;
   RotateArgs unit{};
   unit.unit_limit = unit_limit;
   unit.unit_alpha = unit_alpha;
   unit.unit_row_scale = unit_row_scale;
-  launch_dependent<LAUNCH_GEMM>(kernel, dim3(blocks), dim3(TC_THREADS), TcShared<BN>::BYTES, stream, map_a, map_b, map_c, M, N, K, error, unit, tile_group, group_rows);
+  launch_dependent<LAUNCH_GEMM>(kernel, dim3(blocks), dim3(TC_THREADS), TcShared<BN, R>::BYTES, stream, map_a, map_b, map_c, M, N, K, error, unit, tile_group, group_rows);
   PYLON_CHECK_LAUNCH("gemm_tcgen05");
 }
 
@@ -552,7 +581,8 @@ static int forced_columns = 0;
 
 }  // namespace pylon
 
-// For measurements: every later product uses tiles of 128 x columns (288, 256, 192, 160 or 128); 0 returns to the choice by size.
+// For measurements: every later product uses tiles of 128 x columns (288, 256, 192, 160 or 128; 1192 or 1128: both row tiles of a gated product of
+// 129 to 256 rows with tiles of 192 or 128 columns); 0 returns to the choice by size.
 extern "C" int pylon_gemm_tcgen05_force_tile(int columns) {
   pylon::forced_columns = columns;
   return 0;
@@ -578,7 +608,7 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
   int bn = 128;
   long long best = -1;
   for (int candidate : {288, 256, 192, 160, 128}) {
-    if (forced_columns && candidate != forced_columns) continue;
+    if (forced_columns && forced_columns < 1000 && candidate != forced_columns) continue;
     if (swiglu && (candidate == 160 || candidate == 288)) continue;   // their accumulator columns do not divide into stores of 32 output columns
     if (tile_group && (candidate == 160 || candidate == 288)) continue;
     const long long tiles = tiles_m * ((N + candidate - 1) / candidate);
@@ -589,8 +619,20 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
     if (candidate > 256) cost += rounds * 100;   // one accumulator buffer: the epilogue of a tile holds up the next (21 us a round)
     if (best < 0 || cost < best) { best = cost; bn = candidate; }
   }
+  // 129 to 256 rows are bound by how often the weights' tiles cross from L2: a block takes both row tiles with one tile of B.  Its operands are
+  // M + width rows of k a step; with 192 columns the accumulators of both fill tensor memory (one buffer).  Gate and up of the Qwen3-4B shape
+  // for 160 rows: 27 us where two rounds of 128 x 192 tiles took 35 (the bytes alone take 15); [24576, 4096]: 57 against 65.  Not beyond 256
+  // rows: with whole tiles of A and rounds of blocks the two products per tile of B measured slower than two accumulators of 256 columns.
+  int row_tiles = 1;
+  if (swiglu && !tile_group && M > TC_BM && M <= 2 * TC_BM && (forced_columns == 0 || forced_columns >= 1000))
+    for (int candidate : {192, 128}) {
+      if (forced_columns && candidate != forced_columns - 1000) continue;
+      const long long rounds = ((N + candidate - 1) / candidate + sm_count - 1) / sm_count;
+      const long long cost = rounds * (candidate + M + 85 + (candidate > 128 ? 100 : 0));
+      if (cost < best || forced_columns) { best = cost; bn = candidate; row_tiles = 2; }
+    }
   CUtensorMap map_a, map_b;
-  if (!make_map(&map_a, x, M, K, ldx, TC_BM) || !make_map(&map_b, w, (long long)groups * N, K, ldw, bn > 256 ? bn / 2 : bn))
+  if (!make_map(&map_a, x, M, K, ldx, row_tiles == 2 ? (M + 31) & ~31 : TC_BM) || !make_map(&map_b, w, (long long)groups * N, K, ldw, bn > 256 ? bn / 2 : bn))
     PYLON_REFUSE("gemm_tcgen05: the tensor maps could not be made");
   __nv_bfloat16* out = (__nv_bfloat16*)y;
 #define PYLON_TC_CASE(BN_)                                                                                          \
@@ -598,6 +640,8 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
     if (swiglu) return launch_tcgen05<BN_, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale); \
     return launch_tcgen05<BN_, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N);                          \
   }
+  if (row_tiles == 2 && bn == 192) return launch_tcgen05<192, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha);
+  if (row_tiles == 2) return launch_tcgen05<128, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha);
   PYLON_TC_CASE(256) PYLON_TC_CASE(192)
 #undef PYLON_TC_CASE
   if (bn == 288) return launch_tcgen05<288, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream);

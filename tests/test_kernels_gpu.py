@@ -127,6 +127,30 @@ def test_linear_bf16(m, n, k):
     torch.testing.assert_close(wide.double(), expected, rtol=1e-3, atol=1e-3)
 
 
+@pytest.mark.parametrize("m", [129, 160, 161, 224, 255, 256])
+@pytest.mark.parametrize("inter, k", [(24, 64), (200, 1000), (9728, 2560)])
+def test_tcgen05_gated_product_with_both_row_tiles(m, inter, k):
+    """129 to 256 rows: a block multiplies both row tiles by one tile of weights, the second one cut off at 32 rows.  The sums of a
+    result are the same products in the same order as with one row tile to a block: the same bits."""
+    from pylon_b200.kernels import ops
+
+    x = torch.randn(m, k, device=DEVICE).to(torch.bfloat16)
+    gate, up = ((torch.randn(inter, k, device=DEVICE) * k**-0.5).to(torch.bfloat16) for _ in range(2))
+    weights = ops.interleave_gate_up(gate, up)
+    g, u = x.double() @ gate.double().T, x.double() @ up.double().T
+    results = []
+    try:
+        for columns in (128, 1128, 1192, 0):
+            ops.tcgen05_force_tile(columns)
+            results.append(ops.linear_tcgen05(x, weights, swiglu=True))
+    finally:
+        ops.tcgen05_force_tile(0)
+    assert int(ops.tcgen05_error_word(torch.device(DEVICE)).item()) == 0
+    torch.testing.assert_close(results[0].double(), g * torch.sigmoid(g) * u, rtol=2e-2, atol=2e-2)
+    for result in results[1:]:
+        assert torch.equal(result, results[0])
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16, 31, 64])
 @pytest.mark.parametrize("n, k", [(100, 64), (2560, 4096), (77, 1000), (333, 264)])
 def test_skinny_gemm_every_row_count(m, n, k):

@@ -328,6 +328,28 @@ def test_streams_update_and_norm(streams, kind):
     torch.testing.assert_close(got.double().cpu(), want, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("kind", ["layernorm", "rmsnorm"])
+@pytest.mark.parametrize("streams, width", [(2, 1024), (2, 4096), (4, 1024), (4, 2048), (4, 4096)])
+@pytest.mark.parametrize("delta_dtype", [torch.bfloat16, torch.float32])
+def test_streams_update_and_norm_of_a_prompt_portion(streams, width, kind, delta_dtype):
+    """The kernel for more than 256 rows, whose sizes the compiler knows, against the one for any (a step of 256 rows goes there)."""
+    from pylon_b200.kernels import ops
+
+    tokens = 257
+    x = torch.randn(tokens, streams, width, device=DEVICE)
+    delta = torch.randn(tokens, width, device=DEVICE).to(delta_dtype)
+    if delta_dtype == torch.float32:
+        delta = delta.unsqueeze(0)
+    routes = [torch.randn(streams, streams, device=DEVICE), torch.randn(streams, device=DEVICE), torch.randn(streams, device=DEVICE)]
+    weight = 1 + 0.2 * torch.randn(width, device=DEVICE)
+    for mix, out_w, read in (routes, (None, None, None)):
+        whole, first = x.clone(), x[:256].clone()
+        got = ops.streams_update_norm(whole, delta, 0.6, mix, out_w, read, weight, 1e-5, kind, torch.bfloat16)
+        want = ops.streams_update_norm(first, delta[..., :256, :].contiguous(), 0.6, mix, out_w, read, weight, 1e-5, kind, torch.bfloat16)
+        torch.testing.assert_close(whole[:256], first, rtol=1e-6, atol=1e-6)
+        torch.testing.assert_close(got[:256].float(), want.float(), rtol=1e-2, atol=1e-3)   # the statistics in another order: now and then the next bfloat16
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_clamped_gated_unit(dtype):
     from pylon_b200.kernels import ops
@@ -366,6 +388,38 @@ def plain_delta_from_projections(proj, conv, a_log, dt_bias, norm, heads, kv_hea
     decay = torch.exp(-torch.exp(a_log.double()) * plain.softplus(a + dt_bias.double()))
     out = plain.delta_recurrence(q, k, v, decay, torch.sigmoid(b))
     return (plain.rms_unit(out, eps) * norm.double() * gate).reshape(count, vs)
+
+
+@pytest.mark.parametrize("heads,kv_heads,vdim,taps", [(4, 2, 128, 4), (1, 1, 16, 1), (3, 3, 48, 2)])
+@pytest.mark.parametrize("lengths", [(64,), (100,), (129, 64, 47), (1, 160, 33)])
+@pytest.mark.parametrize("decay", [0.0, 9.0, -9.0])
+def test_gated_delta_rule_in_chunks(heads, kv_heads, vdim, taps, lengths, decay, monkeypatch):
+    """Rows in chunks of 16 tokens against the same rows token by token: full and partly filled chunks, states that go on, decays
+    near one, near zero and in between."""
+    from pylon_b200.kernels import ops
+
+    dim, eps, tokens = 128, 1e-5, sum(lengths)
+    channels = 2 * kv_heads * dim + heads * vdim
+    proj, conv, a_log, dt_bias, norm = (t.to(DEVICE) for t in delta_inputs(tokens, heads, kv_heads, dim, vdim, taps, 7, torch.bfloat16))
+    proj[:, channels + heads * vdim : channels + heads * vdim + heads] += decay
+    floats = (heads * dim * vdim + (taps - 1) * channels + 3) // 4 * 4
+    start = torch.randn(len(lengths), floats, device=DEVICE) * 0.1
+    step = step_view(list(lengths), [0] * len(lengths), torch.bfloat16)
+    slots = torch.arange(len(lengths), dtype=torch.int32, device=DEVICE).flip(0).contiguous()
+    assert ops.delta_rule_in_chunks(torch.bfloat16, dim, vdim, tokens, len(lengths), floats, False)
+
+    def run():
+        state = start.clone()
+        out = ops.gated_delta_rule(proj, conv.t().contiguous(), state, step.token_row, step.q_start, slots, a_log, dt_bias, norm, heads, kv_heads, dim, vdim,
+                                   len(lengths), eps)
+        return out.float(), state
+
+    out, state = run()
+    monkeypatch.setattr(ops, "delta_rule_in_chunks", lambda *_: False)
+    want, want_state = run()
+    # the same 32-bit sums in another order; the state is a sum of at most 160 terms of size one
+    torch.testing.assert_close(state, want_state, rtol=1e-4, atol=2e-5)
+    torch.testing.assert_close(out, want, rtol=2e-2, atol=2e-2)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -125,6 +125,86 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, long long ld, c
   for (int e = lane; e < size; e += 32) qkv[(long long)t * channels + first + e] *= factor;
 }
 
+// The same for prompt portions of bfloat16 models, heads of up to 128 channels, up to four taps: a warp takes TOKENS tokens of a head, a lane four
+// neighbouring channels, whose taps it reads once; all reads of the tokens' inputs are under way together.  2,048 tokens of 8 + 8 + 16 heads
+// of 128: 27 us, where a channel at a time, with the taps read anew for every token, took 67; what bounds it are the 33 MB it writes
+// and the exponentials.
+__device__ __forceinline__ float4 delta_load4(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <int TOKENS>
+__global__ void __launch_bounds__(128) delta_prepare_wide_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const float* __restrict__ conv_w, int taps,
+                                                                 const float* __restrict__ state, long long slot_floats, long long conv_offset,
+                                                                 const int* __restrict__ token_row, const int* __restrict__ q_start,
+                                                                 const int* __restrict__ slots, float* __restrict__ qkv, float* __restrict__ gates,
+                                                                 const float* __restrict__ a_log, const float* __restrict__ dt_bias, int col_a, int col_b,
+                                                                 int heads, int kv_heads, int dim, int vdim, float unit_eps, int num_tokens) {
+  constexpr int TAPS = 4;
+  grid_dependency_wait();
+  allow_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int units = 2 * kv_heads + heads + 1;
+  const long long item = (long long)blockIdx.x * 4 + warp;
+  const int t0 = (int)(item / units) * TOKENS, unit = (int)(item % units);
+  if (t0 >= num_tokens) return;
+  if (unit == units - 1) {
+    for (int x = lane; x < TOKENS * heads; x += 32) {
+      const int t = t0 + x / heads, h = x % heads;
+      if (t >= num_tokens || token_row[t] < 0) continue;
+      const __nv_bfloat16* mine = proj + (long long)t * ld;
+      gates[(long long)t * 2 * heads + h] = expf(-expf(a_log[h]) * softplus_f(to_float<__nv_bfloat16>(mine[col_a + h]) + dt_bias[h]));
+      gates[(long long)t * 2 * heads + heads + h] = 1.f / (1.f + expf(-to_float<__nv_bfloat16>(mine[col_b + h])));
+    }
+    return;
+  }
+  const int channels = 2 * kv_heads * dim + heads * vdim;
+  const bool is_value = unit >= 2 * kv_heads;
+  const int size = is_value ? vdim : dim;
+  const int c = (is_value ? 2 * kv_heads * dim + (unit - 2 * kv_heads) * vdim : unit * dim) + 4 * lane;
+  const bool live = 4 * lane < size;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // The inputs of the tokens and of the three before them are asked for before it is known whose they are: where a token's row began later, the
+  // slot's inputs take the place of what does not belong to it.
+  float4 weight[TAPS], input[TOKENS + TAPS - 1];
+  int rows[TOKENS + TAPS - 1];
+#pragma unroll
+  for (int n = 0; n < TOKENS + TAPS - 1; ++n) {
+    const int t = t0 + n - (TAPS - 1);
+    const bool there = t >= 0 && t < num_tokens;
+    rows[n] = there ? token_row[t] : -1;
+    input[n] = there && live ? delta_load4(proj + (long long)t * ld + c) : zero;
+  }
+#pragma unroll
+  for (int j = 0; j < TAPS; ++j)   // by how far back they reach
+    weight[j] = live && j < taps ? *reinterpret_cast<const float4*>(conv_w + (long long)(taps - 1 - j) * channels + c) : zero;
+#pragma unroll
+  for (int n = 0; n < TOKENS; ++n) {
+    const int row = rows[n + TAPS - 1];
+    if (row < 0) continue;
+    float4 acc = zero;
+#pragma unroll
+    for (int back = TAPS - 1; back >= 0; --back) {   // the tap `back` tokens before this one; taps that are not there are passed over
+      if (back >= taps) continue;
+      float4 x = input[n + TAPS - 1 - back];
+      if (rows[n + TAPS - 1 - back] != row) {
+        const int index = t0 + n - q_start[row];   // below back: the row's tokens lie side by side
+        x = live ? *reinterpret_cast<const float4*>(state + (long long)slots[row] * slot_floats + conv_offset + (long long)(taps - 1 - (back - index)) * channels + c) : zero;
+      }
+      const float4 k = weight[back];
+      acc.x = fmaf(k.x, x.x, acc.x); acc.y = fmaf(k.y, x.y, acc.y); acc.z = fmaf(k.z, x.z, acc.z); acc.w = fmaf(k.w, x.w, acc.w);
+    }
+    acc = make_float4(silu_f(acc.x), silu_f(acc.y), silu_f(acc.z), silu_f(acc.w));
+    if (!is_value) {
+      float factor = rsqrtf(warp_sum(fmaf(acc.x, acc.x, fmaf(acc.y, acc.y, fmaf(acc.z, acc.z, acc.w * acc.w)))) + unit_eps);
+      if (unit < kv_heads) factor *= rsqrtf((float)dim);
+      acc = make_float4(acc.x * factor, acc.y * factor, acc.z * factor, acc.w * factor);
+    }
+    if (live) *reinterpret_cast<float4*>(qkv + (long long)(t0 + n) * channels + c) = acc;
+  }
+}
+
 // The last (taps - 1) convolution inputs of every row move on by the tokens the row brought.
 template <typename T, int MAX_TAPS>
 __global__ void delta_conv_advance_kernel(const T* __restrict__ proj, long long ld, int taps, float* __restrict__ state,
@@ -424,6 +504,284 @@ __global__ void __launch_bounds__(128) delta_recurrence_exact_kernel(const float
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The rule a chunk of tokens at a time, for prompt portions: the same float32 sums with fewer dependent steps.
+//
+// With S the state before a chunk, G_t the product of the chunk's decays up to token t and D[t, i] that of the decays behind i up to t:
+//
+//     u_t = v_t - G_t S^T k_t;   w = T u;   o_t = G_t S^T q_t + sum_{i <= t} B[t, i] w_i;   S <- G_last S + sum_i D[last, i] k_i w_i^T
+//
+// where B[t, i] = D[t, i] (q_t . k_i), and T = (I + diag(beta) A)^-1 diag(beta) with A[t, i] = D[t, i] (k_t . k_i) below the diagonal is the
+// substitution of the w_i into each other, worked out once.  T and B depend neither on the state nor on the column, so a
+// kernel of its own makes them for all chunks at once; what is left of the walk is three small products a chunk.  (The chunked form of delta
+// rules: Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", 2024.)  D is multiplied up and never
+// divided, so decays that vanish do no harm.  A row's chunks start at the first token it brings.
+constexpr int CHUNK = 16, CHUNK_MATRIX = 2 * CHUNK * CHUNK + 2 * CHUNK;   // T | B | G | D[last]
+
+// Chunk c of row r has the number q_start[r] / CHUNK + r + c: rows' numbers do not meet, and all lie below tokens / CHUNK + rows + 1.
+// grid (those numbers, kv_heads), 128 threads; matrices: float32 [numbers, heads, CHUNK_MATRIX].
+template <int DIM>
+__global__ void __launch_bounds__(128) delta_chunk_matrices_kernel(const float* __restrict__ qkv, const float* __restrict__ gates,
+                                                                   float* __restrict__ matrices, const int* __restrict__ q_start, int num_rows,
+                                                                   int heads, int kv_heads, int vdim) {
+  constexpr int ROW = DIM + 4;
+  __shared__ __align__(16) float ks[CHUNK * ROW], qs[CHUNK * ROW];
+  __shared__ float kk[CHUNK][CHUNK + 1], qk[CHUNK][CHUNK + 1], a[CHUNK][CHUNK + 1], decay[CHUNK], beta[CHUNK];
+  __shared__ int begin_at, tokens_here;
+  grid_dependency_wait();
+  allow_dependents();
+  const int tid = threadIdx.x, number = blockIdx.x, kv = blockIdx.y;
+  if (tid == 0) tokens_here = 0;
+  __syncthreads();
+  for (int r = tid; r < num_rows; r += 128) {
+    const int begin = q_start[r], end = q_start[r + 1], chunk = number - (begin / CHUNK + r);
+    if (chunk >= 0 && begin + chunk * CHUNK < end) {   // one row at most
+      begin_at = begin + chunk * CHUNK;
+      tokens_here = min(CHUNK, end - begin_at);
+    }
+  }
+  __syncthreads();
+  const int count = tokens_here;
+  if (count == 0) return;
+  const int first = begin_at, channels = 2 * kv_heads * DIM + heads * vdim;
+  for (int x = tid; x < CHUNK * DIM / 4; x += 128) {
+    const int t = x / (DIM / 4), e = (x % (DIM / 4)) * 4;
+    const float* src = qkv + (long long)(first + t) * channels + kv * DIM + e;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(qs + t * ROW + e) = t < count ? *reinterpret_cast<const float4*>(src) : zero;
+    *reinterpret_cast<float4*>(ks + t * ROW + e) = t < count ? *reinterpret_cast<const float4*>(src + kv_heads * DIM) : zero;
+  }
+  __syncthreads();
+  {
+    const int t = tid >> 3, i0 = (tid & 7) * 2;
+    float sums[4] = {0.f, 0.f, 0.f, 0.f};   // k_t . k_i, q_t . k_i for i = i0, i0 + 1
+#pragma unroll 4
+    for (int e = 0; e < DIM; e += 4) {
+      const float4 kt = *reinterpret_cast<const float4*>(ks + t * ROW + e), qt = *reinterpret_cast<const float4*>(qs + t * ROW + e);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const float4 ki = *reinterpret_cast<const float4*>(ks + (i0 + n) * ROW + e);
+        sums[n] = fmaf(kt.x, ki.x, fmaf(kt.y, ki.y, fmaf(kt.z, ki.z, fmaf(kt.w, ki.w, sums[n]))));
+        sums[2 + n] = fmaf(qt.x, ki.x, fmaf(qt.y, ki.y, fmaf(qt.z, ki.z, fmaf(qt.w, ki.w, sums[2 + n]))));
+      }
+    }
+    kk[t][i0] = sums[0]; kk[t][i0 + 1] = sums[1];
+    qk[t][i0] = sums[2]; qk[t][i0 + 1] = sums[3];
+  }
+  const int group = heads / kv_heads;
+  for (int h = kv * group; h < (kv + 1) * group; ++h) {
+    float* mine = matrices + ((long long)number * heads + h) * CHUNK_MATRIX;
+    __syncthreads();
+    if (tid < CHUNK) {   // tokens that are not there change nothing
+      decay[tid] = tid < count ? gates[(long long)(first + tid) * 2 * heads + h] : 1.f;
+      beta[tid] = tid < count ? gates[(long long)(first + tid) * 2 * heads + heads + h] : 0.f;
+    }
+    __syncthreads();
+    for (int x = tid; x < CHUNK * CHUNK; x += 128) {
+      const int t = x / CHUNK, i = x % CHUNK;
+      float d = 1.f;
+      for (int j = i + 1; j <= t; ++j) d *= decay[j];
+      a[t][i] = i < t ? d * kk[t][i] : 0.f;
+      mine[CHUNK * CHUNK + x] = i <= t ? d * qk[t][i] : 0.f;
+    }
+    if (tid < CHUNK) {
+      float up_to = 1.f, behind = 1.f;
+      for (int j = 0; j < CHUNK; ++j) {
+        if (j <= tid) up_to *= decay[j]; else behind *= decay[j];
+      }
+      mine[2 * CHUNK * CHUNK + tid] = up_to;
+      mine[2 * CHUNK * CHUNK + CHUNK + tid] = behind;
+    }
+    __syncthreads();
+    if (tid < CHUNK) {   // column tid of T, by substitution
+      float column[CHUNK];
+#pragma unroll
+      for (int t = 0; t < CHUNK; ++t) {
+        float value = t == tid ? 1.f : 0.f;
+#pragma unroll
+        for (int i = 0; i < t; ++i) value = fmaf(-a[t][i], column[i], value);
+        column[t] = beta[t] * value;
+        mine[t * CHUNK + tid] = column[t];
+      }
+    }
+  }
+}
+
+// The walk over the chunks: grid (slices of 16 columns, heads, rows), 128 threads.  Every warp holds the slice of S whole, 64 numbers a
+// thread (16 entries of 4 columns), so that a read of a key or query serves 16 multiply-adds and S is never an operand in shared memory; the warps share
+// the 32 sums over S (16 keys, 16 queries) by rows and the update of S by entries, and give each other what they have updated through
+// shared memory.  Three barriers a chunk.  A lane's entries hang on its bits {0, 3, 4} and its columns on {1, 2}: 16-byte reads that differ in bits
+// {0, 1, 2} take twice as long.  2,048 tokens of 16 heads of 128 x 128, 128 blocks: 193 us (the walk token by token 525): 3,000 cycles a
+// chunk, 1,400 instructions of each of an SM's four warps, which nothing else hides the latencies of.
+template <int DIM>
+__global__ void __launch_bounds__(128) delta_chunk_walk_kernel(const float* __restrict__ qkv, const float* __restrict__ matrices, float* __restrict__ state,
+                                                               long long slot_floats, const int* __restrict__ q_start, const int* __restrict__ slots,
+                                                               float* __restrict__ out, int heads, int kv_heads, int vdim) {
+  static_assert(DIM == 128, "a warp updates a fourth of the entries, eight lanes' four each");
+  constexpr int COLS = 16, STAGE = 2 * CHUNK * DIM + CHUNK * COLS + CHUNK_MATRIX;   // keys | queries | values | matrices
+  extern __shared__ __align__(16) float stages[];
+  float* s_shared = stages + 2 * STAGE;        // [4][4][32 lanes' order][4]
+  float* u = s_shared + DIM * COLS;            // [CHUNK][COLS] each: u, G S^T q, w, w times the decays behind it
+  float* r = u + CHUNK * COLS;
+  float* w = r + CHUNK * COLS;
+  float* wd = w + CHUNK * COLS;
+  grid_dependency_wait();
+  allow_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int dg = (lane & 1) | ((lane >> 2) & 6), cg = (lane >> 1) & 3;
+  const int head = blockIdx.y, row = blockIdx.z, col0 = blockIdx.x * COLS;
+  const int begin = q_start[row], end = q_start[row + 1];
+  if (end <= begin) return;
+  const int kv = head / (heads / kv_heads), channels = 2 * kv_heads * DIM + heads * vdim;
+  const int q_col = kv * DIM, k_col = kv_heads * DIM + kv * DIM, v_col = 2 * kv_heads * DIM + head * vdim + col0;
+  const long long number0 = begin / CHUNK + row;
+  float* mine = state + (long long)slots[row] * slot_floats + (long long)head * DIM * vdim + col0 + 4 * cg;   // S[d, columns] at mine[d * vdim]
+
+  auto fetch = [&](int chunk, int buffer) {
+    float* dst = stages + buffer * STAGE;
+    const int first = begin + chunk * CHUNK, count = min(CHUNK, end - first);
+    auto copy = [](float* to, const float* from, bool there) {
+      const int bytes = there ? 16 : 0;   // zeros for tokens that are not there
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from), "r"(bytes) : "memory");
+    };
+    for (int x = tid; x < CHUNK * DIM / 4; x += 128) {
+      const int t = x / (DIM / 4), e = (x % (DIM / 4)) * 4;
+      const float* src = qkv + (long long)(first + min(t, count - 1)) * channels + e;
+      copy(dst + t * DIM + e, src + k_col, t < count);
+      copy(dst + CHUNK * DIM + t * DIM + e, src + q_col, t < count);
+    }
+    if (tid < CHUNK * COLS / 4) {
+      const int t = tid >> 2, e = (tid & 3) * 4;
+      copy(dst + 2 * CHUNK * DIM + t * COLS + e, qkv + (long long)(first + min(t, count - 1)) * channels + v_col + e, t < count);
+    }
+    const float* from = matrices + ((number0 + chunk) * heads + head) * CHUNK_MATRIX;
+    for (int x = tid; x < CHUNK_MATRIX / 4; x += 128) copy(dst + 2 * CHUNK * DIM + CHUNK * COLS + 4 * x, from + 4 * x, true);
+    delta_copy_commit();
+  };
+
+  // s[n][j]: entry 4 (m 8 + dg) + j, columns 4 cg .. + 3, with m = (warp + n) % 4: s[0] is what this warp updates
+  float4 s[4][4];
+  fetch(0, 0);
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[n][j] = *reinterpret_cast<const float4*>(mine + (long long)(4 * ((((warp + n) & 3) << 3) + dg) + j) * vdim);
+
+  const int chunks = (end - begin + CHUNK - 1) / CHUNK;
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    delta_copy_wait<0>();
+    __syncthreads();   // the chunk's operands and the other warps' entries of S are here; the other stage is free
+    if (chunk + 1 < chunks) fetch(chunk + 1, (chunk + 1) & 1);
+    const float* keys = stages + (chunk & 1) * STAGE;
+    const float* values = keys + 2 * CHUNK * DIM;
+    const float* t_matrix = values + CHUNK * COLS;
+    const float* b_matrix = t_matrix + CHUNK * CHUNK;
+    const float* up_to = b_matrix + CHUNK * CHUNK;
+    const float* behind = up_to + CHUNK;
+    if (chunk > 0) {
+#pragma unroll
+      for (int n = 1; n < 4; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          s[n][j] = *reinterpret_cast<const float4*>(s_shared + (((((warp + n) & 3) << 2) + j) * 32 + dg * 4 + cg) * 4);
+    }
+    // this warp's rows: keys 4 warp .. + 3, then queries 4 warp .. + 3
+    float4 part[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(keys + ((i >> 2) * CHUNK + 4 * warp + (i & 3)) * DIM + 4 * ((((warp + n) & 3) << 3) + dg));
+        const float each[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          part[i].x = fmaf(each[j], s[n][j].x, part[i].x); part[i].y = fmaf(each[j], s[n][j].y, part[i].y);
+          part[i].z = fmaf(each[j], s[n][j].z, part[i].z); part[i].w = fmaf(each[j], s[n][j].w, part[i].w);
+        }
+      }
+    // over the eight lanes of a row: each round a lane keeps half of its rows and hands on the others
+    auto halve = [&](auto& rows, int kept, int bit) {
+      const bool upper = lane & bit;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= kept) continue;
+        const float4 give = upper ? rows[i] : rows[i + kept], keep = upper ? rows[i + kept] : rows[i];
+        rows[i] = make_float4(keep.x + __shfl_xor_sync(0xffffffffu, give.x, bit), keep.y + __shfl_xor_sync(0xffffffffu, give.y, bit),
+                              keep.z + __shfl_xor_sync(0xffffffffu, give.z, bit), keep.w + __shfl_xor_sync(0xffffffffu, give.w, bit));
+      }
+    };
+    halve(part, 4, 16);
+    halve(part, 2, 8);
+    halve(part, 1, 1);
+    {
+      const int t = 4 * warp + ((lane >> 2) & 2) + (lane & 1);
+      const float g = up_to[t];
+      if (lane & 16) {
+        *reinterpret_cast<float4*>(r + t * COLS + 4 * cg) = make_float4(g * part[0].x, g * part[0].y, g * part[0].z, g * part[0].w);
+      } else {
+        const float4 v = *reinterpret_cast<const float4*>(values + t * COLS + 4 * cg);
+        *reinterpret_cast<float4*>(u + t * COLS + 4 * cg) = make_float4(fmaf(-g, part[0].x, v.x), fmaf(-g, part[0].y, v.y), fmaf(-g, part[0].z, v.z), fmaf(-g, part[0].w, v.w));
+      }
+    }
+    __syncthreads();
+    const int t = tid >> 3, c = (tid & 7) * 2;
+    {
+      float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < CHUNK; i += 4) {
+        const float4 m = *reinterpret_cast<const float4*>(t_matrix + t * CHUNK + i);
+        const float each[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 x = *reinterpret_cast<const float2*>(u + (i + j) * COLS + c);
+          sum.x = fmaf(each[j], x.x, sum.x); sum.y = fmaf(each[j], x.y, sum.y);
+        }
+      }
+      const float d = behind[t];
+      *reinterpret_cast<float2*>(w + t * COLS + c) = sum;
+      *reinterpret_cast<float2*>(wd + t * COLS + c) = make_float2(d * sum.x, d * sum.y);
+    }
+    __syncthreads();
+    {
+      const float all = up_to[CHUNK - 1];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { s[0][j].x *= all; s[0][j].y *= all; s[0][j].z *= all; s[0][j].w *= all; }
+#pragma unroll
+      for (int i = 0; i < CHUNK; ++i) {
+        const float4 k = *reinterpret_cast<const float4*>(keys + i * DIM + 4 * ((warp << 3) + dg));
+        const float4 x = *reinterpret_cast<const float4*>(wd + i * COLS + 4 * cg);
+        const float each[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[0][j].x = fmaf(each[j], x.x, s[0][j].x); s[0][j].y = fmaf(each[j], x.y, s[0][j].y);
+          s[0][j].z = fmaf(each[j], x.z, s[0][j].z); s[0][j].w = fmaf(each[j], x.w, s[0][j].w);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(s_shared + (((warp << 2) + j) * 32 + dg * 4 + cg) * 4) = s[0][j];
+    }
+    {
+      float2 sum = *reinterpret_cast<const float2*>(r + t * COLS + c);
+#pragma unroll
+      for (int i = 0; i < CHUNK; i += 4) {
+        const float4 m = *reinterpret_cast<const float4*>(b_matrix + t * CHUNK + i);
+        const float each[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 x = *reinterpret_cast<const float2*>(w + (i + j) * COLS + c);
+          sum.x = fmaf(each[j], x.x, sum.x); sum.y = fmaf(each[j], x.y, sum.y);
+        }
+      }
+      const int token = begin + chunk * CHUNK + t;
+      if (token < end) *reinterpret_cast<float2*>(out + ((long long)token * heads + head) * vdim + col0 + c) = sum;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(mine + (long long)(4 * ((warp << 3) + dg) + j) * vdim) = s[0][j];
+}
+
 // o: float32 [T, heads, vdim]; gate: columns of proj from col_gate, [heads, vdim], through silu - or, if given, the float32 tensor
 // gate_own [T, ld_gate] through a sigmoid; out [T, heads * vdim] in T.
 template <typename T>
@@ -464,13 +822,25 @@ static int launch_delta(const void* proj_v, long long ld, const float* conv_w, i
                         const float* a_log, const float* dt_bias, const float* norm_weight, int col_a, int col_b, int col_gate,
                         int heads, int kv_heads, int dim, int vdim, float unit_eps, float norm_eps, int num_tokens, int num_rows,
                         const float* decay_in, long long ld_decay, float* decays, const float* gate_own, long long ld_gate,
-                        cudaStream_t stream) {
+                        float* matrices, cudaStream_t stream) {
   const T* proj = (const T*)proj_v;
   const bool channel = decay_in != nullptr;
   T* out = (T*)out_v;
   const int channels = 2 * kv_heads * dim + heads * vdim;
   const long long conv_offset = (long long)heads * dim * vdim;
-  {
+  bool prepared = false;
+  if constexpr (sizeof(T) == 2) {   // in float32 mode the order of a norm's sum must not depend on how many tokens a step has
+    // short rows: every token would go through its slot's inputs, eight to a warp one behind the other (16 rows of 4 tokens: 5 us slower)
+    if (!channel && taps <= 4 && dim % 4 == 0 && vdim % 4 == 0 && dim <= 128 && vdim <= 128 && ld % 4 == 0 && slot_floats % 4 == 0 && num_tokens >= 64 &&
+        num_tokens >= 16LL * num_rows && (((uintptr_t)conv_w | (uintptr_t)state | (uintptr_t)qkv) & 15) == 0 && (uintptr_t)proj % 8 == 0) {
+      constexpr int TOKENS = 8;
+      const long long items = (long long)((num_tokens + TOKENS - 1) / TOKENS) * (2 * kv_heads + heads + 1);
+      launch_dependent(delta_prepare_wide_kernel<TOKENS>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream, proj, ld, conv_w, taps, state, slot_floats,
+                       conv_offset, token_row, q_start, slots, qkv, gates, a_log, dt_bias, col_a, col_b, heads, kv_heads, dim, vdim, unit_eps, num_tokens);
+      prepared = true;
+    }
+  }
+  if (!prepared) {
     const int warps = 4;
     const long long items = (long long)num_tokens * (2 * kv_heads + heads + 1 + (channel ? heads : 0));
     launch_dependent(delta_prepare_kernel<T, DELTA_MAX_TAPS>, dim3((unsigned)((items + warps - 1) / warps)), dim3(warps * 32), 0, stream,
@@ -483,7 +853,27 @@ static int launch_delta(const void* proj_v, long long ld, const float* conv_w, i
         proj, ld, taps, state, slot_floats, conv_offset, q_start, slots, channels, num_rows);
   }
   bool walked = false;
-  if (dim % 4 == 0 && vdim % 4 == 0 && (uintptr_t)qkv % 16 == 0) {
+  if (matrices != nullptr) {
+    constexpr int DIM = 128, COLS = 16;
+    constexpr size_t smem = (2 * (2 * CHUNK * DIM + CHUNK * COLS + CHUNK_MATRIX) + DIM * COLS + 4 * CHUNK * COLS) * sizeof(float);
+    // A dependent launch places its blocks while the kernel ahead still fills the SMs, several to one that has just become free: with blocks for
+    // every SM at most, each asks for more than half of an SM's shared memory (2,048 tokens of 16 heads: 193 us against 398).
+    const bool alone = (long long)(vdim / COLS) * heads * num_rows <= multiprocessors();
+    constexpr size_t HALF_SM = 116 * 1024;
+    static bool raised_on[MAX_DEVICES] = {};   // function attributes belong to a device
+    bool& raised = raised_on[current_device_slot()];
+    if (!raised) {
+      const cudaError_t err = cudaFuncSetAttribute(delta_chunk_walk_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HALF_SM);
+      if (err != cudaSuccess) PYLON_REFUSE("gated_delta_rule: %s", cudaGetErrorString(err));
+      raised = true;
+    }
+    launch_dependent(delta_chunk_matrices_kernel<DIM>, dim3((unsigned)(num_tokens / CHUNK + num_rows + 1), kv_heads), dim3(128), 0, stream, (const float*)qkv,
+                     (const float*)gates, matrices, q_start, num_rows, heads, kv_heads, vdim);
+    launch_dependent(delta_chunk_walk_kernel<DIM>, dim3(vdim / COLS, heads, num_rows), dim3(128), alone ? HALF_SM : smem, stream, (const float*)qkv, (const float*)matrices, state,
+                     slot_floats, q_start, slots, o, heads, kv_heads, vdim);
+    walked = true;
+  }
+  if (!walked && dim % 4 == 0 && vdim % 4 == 0 && (uintptr_t)qkv % 16 == 0) {
     // the sizes models have: the kernel whose inner loop is fixed when it is compiled
 #define PYLON_DELTA_EXACT(PER_, P_)                                                                                                   \
     if (!walked && dim == PER_ * P_) {                                                                                                 \
@@ -547,14 +937,15 @@ static int launch_delta(const void* proj_v, long long ld, const float* conv_w, i
 // buffers.  out: [T, heads * vdim] in dtype.  Rows without tokens leave their slot as it is.  decay_in (or null): float32 [T, ld_decay],
 // heads * dim columns, the decay's input per head and key channel; dt_bias is then [heads * dim], decays a float32 work buffer
 // [T, heads * dim], and col_a is not read.  gate_own (or null): float32 [T, ld_gate], heads * vdim columns, the output gate's input, through a
-// sigmoid; col_gate is then not read.
+// sigmoid; col_gate is then not read.  matrices (or null: token by token): a float32 work buffer [num_tokens / 16 + num_rows + 1, heads, 544],
+// 16-byte aligned, with which the rows are walked in chunks of 16 tokens; dim 128, vdim a multiple of 16, no decay_in.
 extern "C" int pylon_gated_delta_rule(const void* proj, long long ld, const float* conv_w, int taps, float* state,
                                       long long slot_floats, const int* token_row, const int* q_start, const int* slots, float* qkv,
                                       float* gates, float* o, void* out, const float* a_log, const float* dt_bias,
                                       const float* norm_weight, int col_a, int col_b, int col_gate, int heads, int kv_heads, int dim,
                                       int vdim, float unit_eps, float norm_eps, int num_tokens, int num_rows, int dtype,
                                       const float* decay_in, long long ld_decay, float* decays, const float* gate_own, long long ld_gate,
-                                      cudaStream_t stream) {
+                                      float* matrices, cudaStream_t stream) {
   if (num_tokens <= 0 || num_rows <= 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads) PYLON_REFUSE("gated_delta_rule: %d heads over %d query/key heads", heads, kv_heads);
   if (dim < 1 || dim > 1024 || vdim < 1) PYLON_REFUSE("gated_delta_rule: dim %d (1 to 1024), vdim %d", dim, vdim);
@@ -563,9 +954,11 @@ extern "C" int pylon_gated_delta_rule(const void* proj, long long ld, const floa
   const long long needed = (long long)heads * dim * vdim + (long long)(taps - 1) * (2 * kv_heads * dim + heads * vdim);
   if (decay_in != nullptr && decays == nullptr) PYLON_REFUSE("gated_delta_rule: a decay per channel needs its work buffer");
   if (slot_floats < needed) PYLON_REFUSE("gated_delta_rule: a slot of %lld floats, %lld needed", slot_floats, needed);
+  if (matrices != nullptr && (dim != 128 || vdim % 16 || decay_in != nullptr || slot_floats % 4 || (((uintptr_t)qkv | (uintptr_t)state | (uintptr_t)matrices | (uintptr_t)o) & 15)))
+    PYLON_REFUSE("gated_delta_rule: chunks of tokens take heads of 128 x a multiple of 16 with a decay per head, and rows on 16-byte boundaries");
 #define PYLON_DELTA_ARGS proj, ld, conv_w, taps, state, slot_floats, token_row, q_start, slots, qkv, gates, o, out, a_log, dt_bias, \
     norm_weight, col_a, col_b, col_gate, heads, kv_heads, dim, vdim, unit_eps, norm_eps, num_tokens, num_rows, decay_in, ld_decay, decays, \
-    gate_own, ld_gate, stream
+    gate_own, ld_gate, matrices, stream
   if (dtype == PYLON_DTYPE_F32) return launch_delta<float>(PYLON_DELTA_ARGS);
   if (dtype == PYLON_DTYPE_BF16) return launch_delta<__nv_bfloat16>(PYLON_DELTA_ARGS);
 #undef PYLON_DELTA_ARGS

@@ -679,6 +679,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     the library matrix product, as raun6k/Pylon's ``nn.Linear`` layers do
     (src/pylon/model/layers.py:17-23,95-106).  ``out_dtype=torch.float32`` keeps the 32-bit
     accumulator (used for logits).
+
+    ``w`` holds weights: our kernels ask for its first rows while the kernel ahead of them on the stream is still
+    running, so it must not be what one of this package's own kernels has just been queued to write.
     """
     _need_cuda(x, w)
     _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1], f"linear: shapes {tuple(x.shape)} and {tuple(w.shape)} do not match")

@@ -698,15 +698,23 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         return y
     _need(x.dtype == torch.bfloat16, f"linear: unsupported dtype {x.dtype}")
     _need(out_dtype in (torch.bfloat16, torch.float32), f"linear: unsupported result dtype {out_dtype}")
-    if m <= SKINNY_MAX_ROWS and k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
-            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
-        return linear_skinny(x, w, out_dtype)   # few rows (decode): our weight-streaming kernel
+    aligned = k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+    if m <= SKINNY_MAX_ROWS and aligned:
+        # few rows (decode): our weight-streaming kernels.  A bfloat16 result of many weight rows goes to the TMA-fed one, whose blocks of 64
+        # rows then fill the device by themselves ([8192, 4096] 17.4 against 14.5 us, [16384, 2048] 13.8 against 12.2; but [6144, 4096] 10.2
+        # against 12.1, [12352, 2048] 10.1 against 10.4).
+        if out_dtype == torch.bfloat16 and 0 < m and (n >= 16_384 or (n >= 8_192 and k >= 4_096)) and k >= 1_024 and n <= 1 << 21:
+            return linear_stream(x, w)
+        return linear_skinny(x, w, out_dtype)
+    if out_dtype == torch.float32 and m <= STREAM_MAX_ROWS and aligned and k >= 1_024 and 6 * _multiprocessors(x.device) <= -(-n // 64) <= 1 << 15:
+        # the head of 9 to 32 rows: the TMA-fed kernel over the whole of k, once its blocks (three to an SM) go round twice.  16 rows of
+        # [151936, 5120]: 228 us, the library 258; 32 of [151936, 2560]: 128 and 133; but [32768, 4096]: 52 and 47.  Its sums are also closer to
+        # 64-bit ones (2.1e-6 against 4.4e-6 at k = 4,096); with eight rows or fewer the kernel above is closer still (5e-7) and is kept.
+        return linear_stream_partial(x, w, parts=1)[0]
     if out_dtype == torch.bfloat16:
-        if (m <= STREAM_MAX_ROWS and k >= 1024 and k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
-                and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+        if m <= STREAM_MAX_ROWS and k >= 1024 and aligned:
             return linear_stream(x, w)   # 9 to 32 rows over a long k: the TMA-fed kernel is ahead of the library there
-        if _tcgen05_fills_the_sms(m, n, _multiprocessors(x.device)) and k % 8 == 0 and n % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
-                and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+        if _tcgen05_fills_the_sms(m, n, _multiprocessors(x.device)) and aligned and n % 8 == 0:
             return linear_tcgen05(x, w)
         return torch.mm(x, w.t())
     return torch.mm(x, w.t(), out_dtype=torch.float32)

@@ -127,6 +127,23 @@ def test_linear_bf16(m, n, k):
     torch.testing.assert_close(wide.double(), expected, rtol=1e-3, atol=1e-3)
 
 
+@pytest.mark.parametrize("m, n, k, out_dtype", [(1, 16_384, 1_024, torch.bfloat16), (8, 16_397, 1_032, torch.bfloat16), (5, 8_192, 4_096, torch.bfloat16),
+                                                (8, 8_191, 4_096, torch.bfloat16), (9, 57_001, 1_024, torch.float32), (32, 60_000, 1_160, torch.float32),
+                                                (8, 57_001, 1_024, torch.float32), (33, 57_001, 1_024, torch.float32)])
+def test_linear_of_many_weight_rows(m, n, k, out_dtype):
+    """Either side of the lines behind which few rows go to the TMA-fed kernel."""
+    from pylon_b200.kernels import ops
+
+    x = torch.randn(m, k + 8, device=DEVICE).to(torch.bfloat16)[:, :k]
+    w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
+    expected = x.double() @ w.double().T
+    got = ops.linear(x, w, out_dtype=out_dtype)
+    assert got.shape == (m, n) and got.dtype == out_dtype
+    # float32 sums of k products of size k^-0.5: k / 2 ulps of the largest partial sum at most, and usually their root
+    torch.testing.assert_close(got.double(), expected, **(dict(rtol=1e-5, atol=2e-5) if out_dtype == torch.float32 else dict(rtol=2e-2, atol=2e-2)))
+    assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
+
+
 @pytest.mark.parametrize("m", [129, 160, 161, 224, 255, 256])
 @pytest.mark.parametrize("inter, k", [(24, 64), (200, 1000), (9728, 2560)])
 def test_tcgen05_gated_product_with_both_row_tiles(m, inter, k):

@@ -699,6 +699,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     _need(x.dtype == torch.bfloat16, f"linear: unsupported dtype {x.dtype}")
     _need(out_dtype in (torch.bfloat16, torch.float32), f"linear: unsupported result dtype {out_dtype}")
     aligned = k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+    if (out_dtype == torch.float32 and 0 < m <= STREAM_MAX_ROWS and aligned and k >= (2_560 if m <= SKINNY_MAX_ROWS else 1_024)
+            and 6 * _multiprocessors(x.device) <= -(-n // 64) <= 1 << 15):
+        # the head: the TMA-fed kernel over the whole of k, once its blocks (three to an SM) go round twice.  One row of [151936, 2560]: 109 us
+        # against 118 of the kernel below; 16 rows of [151936, 5120]: 224, the library 258; 32 of [151936, 2560]: 126 and 133; but 16 of
+        # [32768, 4096]: 52 and 47.  Its error against 64-bit sums is 2.4e-7 at any k, the kernel below's 1.3e-7 at k = 1,024, 2.9e-7 at 2,560 and
+        # 4.7e-7 at 4,096 (whence the line for the rows that one takes), the library's 4.4e-6 at 4,096.
+        return linear_stream_partial(x, w, parts=1)[0]
     if m <= SKINNY_MAX_ROWS and aligned:
         # few rows (decode): our weight-streaming kernels.  A bfloat16 result of many weight rows goes to the TMA-fed one, whose blocks of 64
         # rows then fill the device by themselves ([8192, 4096] 17.4 against 14.5 us, [16384, 2048] 13.8 against 12.2; but [6144, 4096] 10.2
@@ -706,11 +713,6 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         if out_dtype == torch.bfloat16 and 0 < m and (n >= 16_384 or (n >= 8_192 and k >= 4_096)) and k >= 1_024 and n <= 1 << 21:
             return linear_stream(x, w)
         return linear_skinny(x, w, out_dtype)
-    if out_dtype == torch.float32 and m <= STREAM_MAX_ROWS and aligned and k >= 1_024 and 6 * _multiprocessors(x.device) <= -(-n // 64) <= 1 << 15:
-        # the head of 9 to 32 rows: the TMA-fed kernel over the whole of k, once its blocks (three to an SM) go round twice.  16 rows of
-        # [151936, 5120]: 228 us, the library 258; 32 of [151936, 2560]: 128 and 133; but [32768, 4096]: 52 and 47.  Its sums are also closer to
-        # 64-bit ones (2.1e-6 against 4.4e-6 at k = 4,096); with eight rows or fewer the kernel above is closer still (5e-7) and is kept.
-        return linear_stream_partial(x, w, parts=1)[0]
     if out_dtype == torch.bfloat16:
         if m <= STREAM_MAX_ROWS and k >= 1024 and aligned:
             return linear_stream(x, w)   # 9 to 32 rows over a long k: the TMA-fed kernel is ahead of the library there

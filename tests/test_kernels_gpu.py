@@ -129,7 +129,8 @@ def test_linear_bf16(m, n, k):
 
 @pytest.mark.parametrize("m, n, k, out_dtype", [(1, 16_384, 1_024, torch.bfloat16), (8, 16_397, 1_032, torch.bfloat16), (5, 8_192, 4_096, torch.bfloat16),
                                                 (8, 8_191, 4_096, torch.bfloat16), (9, 57_001, 1_024, torch.float32), (32, 60_000, 1_160, torch.float32),
-                                                (8, 57_001, 1_024, torch.float32), (33, 57_001, 1_024, torch.float32)])
+                                                (8, 57_001, 1_024, torch.float32), (33, 57_001, 1_024, torch.float32),
+                                                (1, 57_001, 2_560, torch.float32), (8, 56_832, 2_568, torch.float32)])
 def test_linear_of_many_weight_rows(m, n, k, out_dtype):
     """Either side of the lines behind which few rows go to the TMA-fed kernel."""
     from pylon_b200.kernels import ops
@@ -142,6 +143,21 @@ def test_linear_of_many_weight_rows(m, n, k, out_dtype):
     # float32 sums of k products of size k^-0.5: k / 2 ulps of the largest partial sum at most, and usually their root
     torch.testing.assert_close(got.double(), expected, **(dict(rtol=1e-5, atol=2e-5) if out_dtype == torch.float32 else dict(rtol=2e-2, atol=2e-2)))
     assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
+
+
+@pytest.mark.parametrize("m", [1, 16, 33])
+@pytest.mark.parametrize("k", [512, 520, 1_032, 9_728])
+@pytest.mark.parametrize("parts", [1, 3])
+def test_stream_gemm_sums_do_not_drift_with_k(m, k, parts):
+    """The tensor core's sums are cut off, not rounded: a chain is ended every 512 k, so that the error does not grow with k."""
+    from pylon_b200.kernels import ops
+
+    x = torch.randn(m, k, device=DEVICE).to(torch.bfloat16)
+    w = torch.randn(200, k, device=DEVICE).to(torch.bfloat16)
+    expected = x.double() @ w.double().T
+    got = ops.linear_stream_partial(x, w, parts=parts).double().sum(dim=0)
+    # 16 truncations of half an ulp on average in a chain of 256 products (16 to an instruction), all the same way, with a few ulps to spare
+    assert float((got - expected).norm() / expected.norm()) < 16 * 2.0**-24
 
 
 @pytest.mark.parametrize("m", [129, 160, 161, 224, 255, 256])

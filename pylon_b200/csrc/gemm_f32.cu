@@ -43,6 +43,7 @@ struct GemmArgs {
   float* y;
   int M, N, K;
   long long ldx, ldw, ldy, batch_x, batch_w, batch_y;
+  int w_static;   // nothing queued on the stream writes w: its first stages are asked for while the kernel ahead still runs
 };
 
 typedef unsigned long long Pair;   // two float32: the element of an even k and that of the next
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
   const int k_begin = unit * leaves * leaf, k_end = min(a.K, k_begin + leaves * leaf);
   const int steps = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
 
-  // The weights do not depend on the kernel before this one: their first stages are asked for before waiting for it.
+  if (!a.w_static) grid_dependency_wait();
 #pragma unroll
   for (int s = 0; s < Ring::STAGES - 1; ++s)
     if (s < steps) stage_copy<VEC, NR * 32, 32, BK, true>(ring + s * Ring::STAGE, w, a.ldw, n0, a.N - 1, k_begin + s * BK, a.K, lane);
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const GemmArgs a)
   const int k_begin = leaf_begin * leaf, k_end = min(a.K, (leaf_begin + LEAVES / blocks) * leaf);
   const int steps = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
 
+  if (!a.w_static) grid_dependency_wait();
 #pragma unroll
   for (int s = 0; s < Shape::STAGES - 1; ++s)
     if (s < steps) stage_copy<VEC, Shape::BN, 256, Shape::ROW, false>(stages + s * Shape::STAGE + Shape::BM * Shape::ROW, w, a.ldw, n0, a.N - 1, k_begin + s * BK, a.K, threadIdx.x);
@@ -527,24 +529,25 @@ static int gemm_f32(const GemmArgs& a, int batch, int force, cudaStream_t stream
 
 }  // namespace pylon
 
+// w_static: 1 where nothing queued on the stream writes w; its first columns are then asked for while the kernel ahead is still running.
 extern "C" int pylon_gemm_f32_nt(const float* x, const float* w, float* y, int M, int N, int K, long long ldx,
-                                 long long ldw, long long ldy, cudaStream_t stream) {
+                                 long long ldw, long long ldy, int w_static, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) PYLON_REFUSE("gemm_f32: K = %d", K);
   if (ldx < K || ldw < K || ldy < N) PYLON_REFUSE("gemm_f32: a leading dimension is shorter than its row");
   if ((M + 63) / 64 > 65535) PYLON_REFUSE("gemm_f32: M = %d is too large", M);
-  return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0}, 1, 0, stream);
+  return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0, w_static}, 1, 0, stream);
 }
 
 // `batch` products of one shape in one launch: y_b[M, N] = x_b[M, K] * W_b[N, K]^T, the operands of product b lying
 // b * batch_x / batch_w / batch_y elements behind the first (a head's slice of a row, say: batch_x = the head's width, ldx = the row's).
 extern "C" int pylon_gemm_f32_nt_batched(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
-                                         int batch, long long batch_x, long long batch_w, long long batch_y, cudaStream_t stream) {
+                                         int batch, long long batch_x, long long batch_w, long long batch_y, int w_static, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (K <= 0) PYLON_REFUSE("gemm_f32_batched: K = %d", K);
   if (ldx < K || ldw < K || ldy < N) PYLON_REFUSE("gemm_f32_batched: a leading dimension is shorter than its row");
   if ((M + 63) / 64 > 65535 || batch > 65535) PYLON_REFUSE("gemm_f32_batched: M = %d, batch = %d", M, batch);
-  return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, batch_x, batch_w, batch_y}, batch, 0, stream);
+  return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, batch_x, batch_w, batch_y, w_static}, batch, 0, stream);
 }
 
 // For measurements and tests: the kernel for few rows (force = -1) or a tile kernel (100 TM + 10 TN + cluster size; 0: the choice by size).
@@ -552,5 +555,5 @@ extern "C" int pylon_gemm_f32_nt_forced(const float* x, const float* w, float* y
                                         long long ldw, long long ldy, int force, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || ldx < K || ldw < K || ldy < N || (M + 15) / 16 > 65535 || (force < 0 && M > pylon::ROWS_MOST)) PYLON_REFUSE("gemm_f32_forced: M = %d, K = %d", M, K);
-  return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0}, 1, force, stream);
+  return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0, 0}, 1, force, stream);
 }

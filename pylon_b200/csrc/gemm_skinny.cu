@@ -17,9 +17,11 @@
 
 namespace pylon {
 
-__device__ __forceinline__ uint4 load_stream_16(const void* p) {   // weights: read once, keep out of L1
+// Weights: read once, keep out of L1.  Not through the non-coherent path: its loads may be moved ahead of the wait for the kernel that
+// writes them (with .nc the matrix that the kernel ahead had just been queued to write was read too early in 197 of 200 calls).
+__device__ __forceinline__ uint4 load_stream_16(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 // Activations: shared by every block, so they may stay in L1; an ordinary (coherent) load, because under a dependent
@@ -45,7 +47,7 @@ __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat16* p, float
 // inside a block.
 template <int MT, int NT, int WARPS, int UNROLL, typename OutT>
 __global__ void __launch_bounds__(WARPS * 32) gemm_skinny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                                                 OutT* __restrict__ y, int M, int N, int K, long long ldx, long long ldw, long long ldy) {
+                                                                 OutT* __restrict__ y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int w_static) {
   extern __shared__ float reduce[];   // [WARPS][NT * 16][MT * 8]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * (NT * 16);
@@ -117,10 +119,11 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_skinny_kernel(const __nv_bflo
     }
   };
 
-  // The weights do not depend on the kernel before this one: the fragments of both register
+  // Weights that the kernel before this one does not write (w_static): the fragments of both register
   // buffers are on their way before this kernel waits for its activations.  (Asking L2 for the block's whole
   // weight slab up front with cp.async.bulk.prefetch.L2 was measured slower: 22 against 18
   // microseconds on the 19456 x 2560 product.)
+  if (!w_static) grid_dependency_wait();
   int ks0 = step_begin + warp;
   load_weights(wa, ks0);
   bool second_loaded = ks0 + STRIDE < k_steps;   // both register buffers are filled before the wait
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_skinny_kernel(const __nv_bflo
 
 template <int MT, int NT, int WARPS, int UNROLL, typename OutT>
 static int launch_skinny(const __nv_bfloat16* x, const __nv_bfloat16* w, OutT* y, int M, int N, int K, long long ldx,
-                         long long ldw, long long ldy, cudaStream_t stream) {
+                         long long ldw, long long ldy, int w_static, cudaStream_t stream) {
   constexpr size_t smem = (size_t)WARPS * NT * 16 * MT * 8 * sizeof(float);
   auto kernel = gemm_skinny_kernel<MT, NT, WARPS, UNROLL, OutT>;
   if (smem > 48 * 1024) {
@@ -179,34 +182,35 @@ static int launch_skinny(const __nv_bfloat16* x, const __nv_bfloat16* w, OutT* y
     }
   }
   const int blocks = (N + NT * 16 - 1) / (NT * 16);
-  launch_dependent<LAUNCH_GEMM>(kernel, dim3(blocks), dim3(WARPS * 32), smem, stream, x, w, y, M, N, K, ldx, ldw, ldy);
+  launch_dependent<LAUNCH_GEMM>(kernel, dim3(blocks), dim3(WARPS * 32), smem, stream, x, w, y, M, N, K, ldx, ldw, ldy, w_static);
   PYLON_CHECK_LAUNCH("gemm_skinny");
 }
 
 template <typename OutT>
 static int dispatch_skinny(const __nv_bfloat16* x, const __nv_bfloat16* w, OutT* y, int M, int N, int K, long long ldx,
-                           long long ldw, long long ldy, cudaStream_t stream) {
-  if (M <= 8) return launch_skinny<1, 1, 8, 2, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-  if (M <= 16) return launch_skinny<2, 1, 8, 2, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-  if (M <= 32) return launch_skinny<4, 1, 8, 1, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
-  return launch_skinny<8, 2, 4, 1, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
+                           long long ldw, long long ldy, int w_static, cudaStream_t stream) {
+  if (M <= 8) return launch_skinny<1, 1, 8, 2, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, w_static, stream);
+  if (M <= 16) return launch_skinny<2, 1, 8, 2, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, w_static, stream);
+  if (M <= 32) return launch_skinny<4, 1, 8, 1, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, w_static, stream);
+  return launch_skinny<8, 2, 4, 1, OutT>(x, w, y, M, N, K, ldx, ldw, ldy, w_static, stream);
 }
 
 }  // namespace pylon
 
 // x: bfloat16 [M, K] (row stride ldx), w: bfloat16 [N, K] (row stride ldw), y: [M, N] (row
 // stride ldy) in bfloat16 (out_dtype 1) or float32 (out_dtype 0).  M <= 64; K and the row
-// strides of x and w multiples of 8; x and w 16-byte aligned.
+// strides of x and w multiples of 8; x and w 16-byte aligned.  w_static: 1 where nothing queued on the stream writes w; its first
+// columns are then asked for while the kernel ahead is still running.
 extern "C" int pylon_gemm_skinny_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx,
-                                      long long ldw, long long ldy, int out_dtype, cudaStream_t stream) {
+                                      long long ldw, long long ldy, int out_dtype, int w_static, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 64) PYLON_REFUSE("gemm_skinny: M = %d is more than 64 rows", M);
   if (K <= 0 || K % 8 || ldx % 8 || ldw % 8) PYLON_REFUSE("gemm_skinny: K = %d and the row strides must be multiples of 8", K);
   if (((uintptr_t)x % 16) || ((uintptr_t)w % 16)) PYLON_REFUSE("gemm_skinny: x and w must be 16-byte aligned");
   if (ldx < K || ldw < K || ldy < N) PYLON_REFUSE("gemm_skinny: a row stride is shorter than its row");
   if (out_dtype == PYLON_DTYPE_BF16)
-    return pylon::dispatch_skinny<__nv_bfloat16>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, M, N, K, ldx, ldw, ldy, stream);
+    return pylon::dispatch_skinny<__nv_bfloat16>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, M, N, K, ldx, ldw, ldy, w_static, stream);
   if (out_dtype == PYLON_DTYPE_F32)
-    return pylon::dispatch_skinny<float>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (float*)y, M, N, K, ldx, ldw, ldy, stream);
+    return pylon::dispatch_skinny<float>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (float*)y, M, N, K, ldx, ldw, ldy, w_static, stream);
   PYLON_REFUSE("gemm_skinny: unknown result dtype %d", out_dtype);
 }

@@ -75,7 +75,7 @@ __device__ __forceinline__ void st_mma(float (&c)[4], const unsigned (&a)[4], un
 template <int MT, int FORM>
 __global__ void __launch_bounds__(ST_THREADS, 3) gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                      void* __restrict__ y, int M, int N, int K, long long ldy, int* __restrict__ error,
-                                                                     float unit_limit, float unit_alpha) {
+                                                                     float unit_limit, float unit_alpha, int w_static) {
   using Ring = StreamRing<MT>;
   constexpr int STAGES = Ring::STAGES, STAGE_BYTES = Ring::STAGE_BYTES;
   extern __shared__ unsigned char smem_raw[];
@@ -96,9 +96,10 @@ __global__ void __launch_bounds__(ST_THREADS, 3) gemm_stream_kernel(const __grid
 
   if (warp == 0) {
     if (lane == 0) {
-      // The weights do not depend on the kernel before this one: the boxes that fit in the ring are asked for before
+      // Weights that the kernel before this one does not write (w_static): the boxes that fit in the ring are asked for before
       // this kernel waits for it (a dependent launch may start while that kernel is still running); the activations'
       // boxes follow after the wait, on the same barriers.
+      if (!w_static) grid_dependency_wait();
       const int ahead = min(STAGES, box_end - box_begin);
       for (int i = 0; i < ahead; ++i) {
         st_mbar_expect_tx(&full[i], STAGE_BYTES);   // rows past N, M or K arrive as zeros and count all the same
@@ -259,7 +260,7 @@ static bool matrix_map(CUtensorMap* map, const void* base, long long rows, long 
 
 template <int MT, int FORM>
 static int launch_stream(const CUtensorMap& map_w, const CUtensorMap& map_x, void* y, int M, int N, int K, long long ldy, int parts, int slabs,
-                         int* error, cudaStream_t stream, float unit_limit, float unit_alpha) {
+                         int* error, cudaStream_t stream, float unit_limit, float unit_alpha, int w_static) {
   auto kernel = gemm_stream_kernel<MT, FORM>;
   static bool configured_on[pylon::MAX_DEVICES] = {};   // function attributes belong to a device
   bool& configured = configured_on[pylon::current_device_slot()];
@@ -268,13 +269,13 @@ static int launch_stream(const CUtensorMap& map_w, const CUtensorMap& map_x, voi
     if (err != cudaSuccess) PYLON_REFUSE("gemm_stream: %s", cudaGetErrorString(err));
     configured = true;
   }
-  launch_dependent<LAUNCH_GEMM>(kernel, dim3(parts, slabs), dim3(ST_THREADS), StreamRing<MT>::SMEM, stream, map_w, map_x, y, M, N, K, ldy, error, unit_limit, unit_alpha);
+  launch_dependent<LAUNCH_GEMM>(kernel, dim3(parts, slabs), dim3(ST_THREADS), StreamRing<MT>::SMEM, stream, map_w, map_x, y, M, N, K, ldy, error, unit_limit, unit_alpha, w_static);
   PYLON_CHECK_LAUNCH("gemm_stream");
 }
 
 template <int FORM>
 static int dispatch_stream(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts,
-                           int* error, cudaStream_t stream, const char* name, float unit_limit = 0.f, float unit_alpha = 1.f) {
+                           int* error, int w_static, cudaStream_t stream, const char* name, float unit_limit = 0.f, float unit_alpha = 1.f) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 64) PYLON_REFUSE("%s: M = %d is more than 64 rows", name, M);
   if (K <= 0 || K % 8 || ldx % 8 || ldw % 8) PYLON_REFUSE("%s: K = %d and the row strides must be multiples of 8", name, K);
@@ -286,10 +287,10 @@ static int dispatch_stream(const void* x, const void* w, void* y, int M, int N, 
   const int tiles = M <= 8 ? 1 : (M <= 16 ? 2 : (M <= 32 ? 4 : 8));
   CUtensorMap map_w, map_x;
   if (!matrix_map(&map_w, w, N, K, ldw, ST_ROWS) || !matrix_map(&map_x, x, M, K, ldx, 8 * tiles)) PYLON_REFUSE("%s: the tensor maps could not be made", name);
-  if (tiles == 1) return launch_stream<1, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha);
-  if (tiles == 2) return launch_stream<2, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha);
-  if (tiles == 4) return launch_stream<4, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha);
-  return launch_stream<8, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha);
+  if (tiles == 1) return launch_stream<1, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha, w_static);
+  if (tiles == 2) return launch_stream<2, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha, w_static);
+  if (tiles == 4) return launch_stream<4, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha, w_static);
+  return launch_stream<8, FORM>(map_w, map_x, y, M, N, K, ldy, parts, slabs, error, stream, unit_limit, unit_alpha, w_static);
 }
 
 }  // namespace pylon
@@ -297,31 +298,32 @@ static int dispatch_stream(const void* x, const void* w, void* y, int M, int N, 
 // x: bfloat16 [M, K] (row stride ldx), M <= 64; w: bfloat16 [N, K] (row stride ldw); y: float32 [parts, M, N] contiguous,
 // whose sum over the first dimension is x @ w.T.  K and the row strides multiples of 8, x and w 16-byte aligned,
 // 1 <= parts <= number of 64-wide slices of k.  error: one int in device memory that the kernel sets non-zero if one of its
-// waits ran out (the result is then void).
+// waits ran out (the result is then void).  w_static: 1 where nothing queued on the stream writes w; its first boxes are then asked for
+// while the kernel ahead is still running.
 extern "C" int pylon_gemm_stream_partial(const void* x, const void* w, float* y, int M, int N, int K, long long ldx, long long ldw,
-                                         int parts, int* error, cudaStream_t stream) {
-  return pylon::dispatch_stream<pylon::ST_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, parts, error, stream, "gemm_stream_partial");
+                                         int parts, int* error, int w_static, cudaStream_t stream) {
+  return pylon::dispatch_stream<pylon::ST_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, parts, error, w_static, stream, "gemm_stream_partial");
 }
 
 // The product itself: y bfloat16 [M, N], row stride ldy.
 extern "C" int pylon_gemm_stream_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
-                                      long long ldy, int* error, cudaStream_t stream) {
+                                      long long ldy, int* error, int w_static, cudaStream_t stream) {
   if (ldy < N) PYLON_REFUSE("gemm_stream_bf16: a row stride is shorter than its row");
-  return pylon::dispatch_stream<pylon::ST_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, 1, error, stream, "gemm_stream_bf16");
+  return pylon::dispatch_stream<pylon::ST_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, 1, error, w_static, stream, "gemm_stream_bf16");
 }
 
 // silu(x gate^T) * (x up^T): w's rows are interleaved in groups of 8 (rows 16b..16b+7 gate rows 8b..8b+7, rows 16b+8..16b+15
 // the matching up rows; N a multiple of 16); y bfloat16 [M, N / 2], row stride ldy.
 extern "C" int pylon_gemm_stream_swiglu(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
-                                        long long ldy, int* error, cudaStream_t stream) {
+                                        long long ldy, int* error, int w_static, cudaStream_t stream) {
   if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_stream_swiglu: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
-  return pylon::dispatch_stream<pylon::ST_SWIGLU>(x, w, y, M, N, K, ldx, ldw, ldy, 1, error, stream, "gemm_stream_swiglu");
+  return pylon::dispatch_stream<pylon::ST_SWIGLU>(x, w, y, M, N, K, ldx, ldw, ldy, 1, error, w_static, stream, "gemm_stream_swiglu");
 }
 
 // The same with the clamped gated unit: g = min(x gate^T, limit), u = clamp(x up^T, -limit, limit), y = g * sigmoid(alpha * g) * (u + 1).
 extern "C" int pylon_gemm_stream_glu_clamped(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
-                                             long long ldy, float limit, float alpha, int* error, cudaStream_t stream) {
+                                             long long ldy, float limit, float alpha, int* error, int w_static, cudaStream_t stream) {
   if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_stream_glu_clamped: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
   if (!(limit > 0.f)) PYLON_REFUSE("gemm_stream_glu_clamped: the limit must be positive");
-  return pylon::dispatch_stream<pylon::ST_SWIGLU>(x, w, y, M, N, K, ldx, ldw, ldy, 1, error, stream, "gemm_stream_glu_clamped", limit, alpha);
+  return pylon::dispatch_stream<pylon::ST_SWIGLU>(x, w, y, M, N, K, ldx, ldw, ldy, 1, error, w_static, stream, "gemm_stream_glu_clamped", limit, alpha);
 }

@@ -181,6 +181,7 @@ struct RotateArgs {
   // the gated unit of a SWIGLU epilogue: limit 0 is silu(gate) * up; limit > 0 the clamped unit,
   // min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1)
   float unit_limit = 0.f, unit_alpha = 1.f;
+  int w_static = 0;   // nothing queued on the stream writes the weights: with R = 2 their first boxes are asked for while the kernel ahead still runs
   const float* unit_row_scale = nullptr;   // not null: a row's sums of gate and up are multiplied by its number before the unit (a row of the operand times it)
 };
 enum TcMode { TC_PLAIN = 0, TC_SWIGLU = 1, TC_ROTATE = 2 };
@@ -349,9 +350,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
   // Barriers and tensor memory are set up while the kernel before this one finishes (dependent launch).  With R = 2, one round of tiles whose
-  // weights come from memory, the first boxes of the weights, which do not depend on that kernel, are asked for as well; the activations' boxes
+  // weights come from memory, the first boxes of weights that nothing queued writes (w_static) are asked for as well; the activations' boxes
   // follow on the same barriers.  (Products of many rows gain nothing: 2,079 rows beside decoded ones 6.81 against 6.70 ms a step.)
-  const int ahead = R == 1 || (int)blockIdx.x >= total_tiles ? 0 : (k_blocks < stages ? k_blocks : stages);
+  const int ahead = R == 1 || !rot.w_static || (int)blockIdx.x >= total_tiles ? 0 : (k_blocks < stages ? k_blocks : stages);
   if (warp == 0 && lane == 0) {
     for (int kb = 0; kb < ahead; ++kb) {
       mbar_expect_tx(&full[kb], a_bytes + S::B_BYTES);
@@ -537,7 +538,7 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, long lo
 template <int BN, bool SWIGLU, int R = 1>
 static int launch_tcgen05(const CUtensorMap& map_a, const CUtensorMap& map_b, __nv_bfloat16* c, int M, int N, int K, long long ldc,
                           int* error, int sm_count, cudaStream_t stream, float unit_limit = 0.f, float unit_alpha = 1.f,
-                          const int* tile_group = nullptr, int group_rows = 0, const float* unit_row_scale = nullptr) {
+                          const int* tile_group = nullptr, int group_rows = 0, const float* unit_row_scale = nullptr, int w_static = 0) {
   auto kernel = gemm_tcgen05_kernel<BN, SWIGLU ? TC_SWIGLU : TC_PLAIN, 128, R>;
   static bool configured_on[pylon::MAX_DEVICES] = {};   // function attributes belong to a device
   bool& configured = configured_on[pylon::current_device_slot()];
@@ -554,6 +555,7 @@ static int launch_tcgen05(const CUtensorMap& map_a, const CUtensorMap& map_b, __
   unit.unit_limit = unit_limit;
   unit.unit_alpha = unit_alpha;
   unit.unit_row_scale = unit_row_scale;
+  unit.w_static = w_static;
   launch_dependent<LAUNCH_GEMM>(kernel, dim3(blocks), dim3(TC_THREADS), TcShared<BN, R>::BYTES, stream, map_a, map_b, map_c, M, N, K, error, unit, tile_group, group_rows);
   PYLON_CHECK_LAUNCH("gemm_tcgen05");
 }
@@ -593,7 +595,7 @@ extern "C" int pylon_gemm_tcgen05_force_tile(int columns) {
 // error: one int in device memory; the kernel sets it non-zero if one of its waits ran out (the result is then void).
 static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
                              long long ldy, int swiglu, float unit_limit, float unit_alpha, int* error, int sm_count, cudaStream_t stream,
-                             const int* tile_group = nullptr, int groups = 1, const float* unit_row_scale = nullptr) {
+                             const int* tile_group = nullptr, int groups = 1, const float* unit_row_scale = nullptr, int w_static = 0) {
   using namespace pylon;
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || K % 8 || ldx % 8 || ldw % 8 || ldy % 8) PYLON_REFUSE("gemm_tcgen05: K = %d and the row strides must be multiples of 8", K);
@@ -639,8 +641,8 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
     if (swiglu) return launch_tcgen05<BN_, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale); \
     return launch_tcgen05<BN_, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N);                          \
   }
-  if (row_tiles == 2 && bn == 192) return launch_tcgen05<192, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha);
-  if (row_tiles == 2) return launch_tcgen05<128, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha);
+  if (row_tiles == 2 && bn == 192) return launch_tcgen05<192, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, nullptr, 0, nullptr, w_static);
+  if (row_tiles == 2) return launch_tcgen05<128, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, nullptr, 0, nullptr, w_static);
   PYLON_TC_CASE(256) PYLON_TC_CASE(192)
 #undef PYLON_TC_CASE
   if (bn == 288) return launch_tcgen05<288, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream);
@@ -663,17 +665,18 @@ extern "C" int pylon_gemm_tcgen05_grouped(const void* x, const void* w, void* y,
   return gemm_tcgen05_entry(x, w, y, M, N, K, ldx, ldw, ldy, swiglu, limit, alpha, error, sm_count, stream, tile_group, groups, row_scale);
 }
 
+// w_static: 1 where nothing queued on the stream writes w; its first boxes may then be asked for while the kernel ahead is still running.
 extern "C" int pylon_gemm_tcgen05_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
-                                       long long ldy, int swiglu, int* error, int sm_count, cudaStream_t stream) {
-  return gemm_tcgen05_entry(x, w, y, M, N, K, ldx, ldw, ldy, swiglu, 0.f, 1.f, error, sm_count, stream);
+                                       long long ldy, int swiglu, int* error, int sm_count, int w_static, cudaStream_t stream) {
+  return gemm_tcgen05_entry(x, w, y, M, N, K, ldx, ldw, ldy, swiglu, 0.f, 1.f, error, sm_count, stream, nullptr, 1, nullptr, w_static);
 }
 
 // The product of interleaved gate and up rows with the clamped gated unit in its epilogue: g = min(gate, limit),
 // u = clamp(up, -limit, limit), y = g * sigmoid(alpha * g) * (u + 1); y bfloat16 [M, N / 2].
 extern "C" int pylon_gemm_tcgen05_glu_clamped(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
-                                              long long ldy, float limit, float alpha, int* error, int sm_count, cudaStream_t stream) {
+                                              long long ldy, float limit, float alpha, int* error, int sm_count, int w_static, cudaStream_t stream) {
   if (!(limit > 0.f)) PYLON_REFUSE("gemm_tcgen05_glu_clamped: the limit must be positive");
-  return gemm_tcgen05_entry(x, w, y, M, N, K, ldx, ldw, ldy, 1, limit, alpha, error, sm_count, stream);
+  return gemm_tcgen05_entry(x, w, y, M, N, K, ldx, ldw, ldy, 1, limit, alpha, error, sm_count, stream, nullptr, 1, nullptr, w_static);
 }
 
 // The fused QKV product with its heads finished in the epilogue: x bfloat16 [M, K], w bfloat16 [(nq + 2 nkv) * d, K] (q rows,

@@ -241,9 +241,9 @@ _SIGNATURES = {
                                  c_longlong, c_void_p, c_void_p],
     },
     "gemm_f32.cu": {
-        "pylon_gemm_f32_nt": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p],
+        "pylon_gemm_f32_nt": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
         "pylon_gemm_f32_nt_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_longlong,
-                                      c_longlong, c_longlong, c_void_p],
+                                      c_longlong, c_longlong, c_int, c_void_p],
         "pylon_gemm_f32_nt_forced": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
     },
     "attention_latent.cu": {
@@ -266,19 +266,19 @@ _SIGNATURES = {
                                c_int, c_int, c_int, c_int, c_void_p],
     },
     "gemm_skinny.cu": {
-        "pylon_gemm_skinny_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
+        "pylon_gemm_skinny_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p],
     },
     "gemm_stream.cu": {
-        "pylon_gemm_stream_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_void_p, c_void_p],
-        "pylon_gemm_stream_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
-        "pylon_gemm_stream_swiglu": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
-        "pylon_gemm_stream_glu_clamped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_void_p],
+        "pylon_gemm_stream_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p],
+        "pylon_gemm_stream_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_int, c_void_p],
+        "pylon_gemm_stream_swiglu": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_int, c_void_p],
+        "pylon_gemm_stream_glu_clamped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_int, c_void_p],
     },
     "gemm_tcgen05.cu": {
         "pylon_gemm_tcgen05_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
-                                    c_void_p, c_int, c_void_p],
+                                    c_void_p, c_int, c_int, c_void_p],
         "pylon_gemm_tcgen05_glu_clamped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float,
-                                           c_void_p, c_int, c_void_p],
+                                           c_void_p, c_int, c_int, c_void_p],
         "pylon_gemm_tcgen05_force_tile": [c_int],
         "pylon_gemm_tcgen05_grouped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_float, c_float, c_void_p, c_void_p, c_int,
                                        c_void_p, c_int, c_void_p],
@@ -670,7 +670,7 @@ def swiglu(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None, interleave
 SKINNY_MAX_ROWS = 8   # up to this many rows the weight-streaming kernel runs (it takes up to 64); above, the library
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, static_weights: bool = False) -> torch.Tensor:
     """``x [M, K] @ w [N, K].T`` with float32 accumulation.
 
     float32 operands use the plain-FMA kernels (true 32-bit, no tensor cores; a row's bits do not depend on the others).  bfloat16
@@ -680,8 +680,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     (src/pylon/model/layers.py:17-23,95-106).  ``out_dtype=torch.float32`` keeps the 32-bit
     accumulator (used for logits).
 
-    ``w`` holds weights: our kernels ask for its first rows while the kernel ahead of them on the stream is still
-    running, so it must not be what one of this package's own kernels has just been queued to write.
+    ``static_weights`` says that nothing queued on the stream writes ``w``: our kernels then ask for its first rows while the
+    kernel ahead of them is still running.  Without it they wait for that kernel first, and ``w`` may be its result.
     """
     _need_cuda(x, w)
     _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1], f"linear: shapes {tuple(x.shape)} and {tuple(w.shape)} do not match")
@@ -694,7 +694,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         _need(out_dtype == torch.float32, "linear: float32 operands give float32 results")
         y = torch.empty((m, n), dtype=torch.float32, device=x.device)
         library = _library("gemm_f32.cu")
-        _check(library, library.pylon_gemm_f32_nt(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), n, _stream()))
+        _check(library, library.pylon_gemm_f32_nt(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), n, int(static_weights), _stream()))
         return y
     _need(x.dtype == torch.bfloat16, f"linear: unsupported dtype {x.dtype}")
     _need(out_dtype in (torch.bfloat16, torch.float32), f"linear: unsupported result dtype {out_dtype}")
@@ -705,24 +705,24 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         # against 118 of the kernel below; 16 rows of [151936, 5120]: 224, the library 258; 32 of [151936, 2560]: 126 and 133; but 16 of
         # [32768, 4096]: 52 and 47.  Its error against 64-bit sums is 2.4e-7 at any k, the kernel below's 1.3e-7 at k = 1,024, 2.9e-7 at 2,560 and
         # 4.7e-7 at 4,096 (whence the line for the rows that one takes), the library's 4.4e-6 at 4,096.
-        return linear_stream_partial(x, w, parts=1)[0]
+        return linear_stream_partial(x, w, 1, static_weights)[0]
     if m <= SKINNY_MAX_ROWS and aligned:
         # few rows (decode): our weight-streaming kernels.  A bfloat16 result of many weight rows goes to the TMA-fed one, whose blocks of 64
         # rows then fill the device by themselves ([8192, 4096] 17.4 against 14.5 us, [16384, 2048] 13.8 against 12.2; but [6144, 4096] 10.2
         # against 12.1, [12352, 2048] 10.1 against 10.4).
         if out_dtype == torch.bfloat16 and 0 < m and (n >= 16_384 or (n >= 8_192 and k >= 4_096)) and k >= 1_024 and n <= 1 << 21:
-            return linear_stream(x, w)
-        return linear_skinny(x, w, out_dtype)
+            return linear_stream(x, w, static_weights=static_weights)
+        return linear_skinny(x, w, out_dtype, static_weights)
     if out_dtype == torch.bfloat16:
         if m <= STREAM_MAX_ROWS and k >= 1024 and aligned:
-            return linear_stream(x, w)   # 9 to 32 rows over a long k: the TMA-fed kernel is ahead of the library there
+            return linear_stream(x, w, static_weights=static_weights)   # 9 to 32 rows over a long k: the TMA-fed kernel is ahead of the library there
         if _tcgen05_fills_the_sms(m, n, _multiprocessors(x.device)) and aligned and n % 8 == 0:
-            return linear_tcgen05(x, w)
+            return linear_tcgen05(x, w, static_weights=static_weights)
         return torch.mm(x, w.t())
     return torch.mm(x, w.t(), out_dtype=torch.float32)
 
 
-def linear_stacked(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear_stacked(x: torch.Tensor, w: torch.Tensor, static_weights: bool = False) -> torch.Tensor:
     """:func:`linear` for many weight rows (projections of several readers stacked): a decode step's few rows go to the TMA-fed kernel, whose
     blocks of 64 weight rows then fill the device by themselves."""
     m, k = x.shape
@@ -730,8 +730,8 @@ def linear_stacked(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     if (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and m <= STREAM_MAX_ROWS and k >= 1024 and k % 8 == 0 and n % 8 == 0
             and 2 * n >= 64 * _multiprocessors(x.device) and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
-        return linear_stream(x, w)
-    return linear(x, w)
+        return linear_stream(x, w, static_weights=static_weights)
+    return linear(x, w, static_weights=static_weights)
 
 
 def _tcgen05_fills_the_sms(m: int, n: int, sms: int) -> bool:
@@ -750,7 +750,7 @@ STREAM_MAX_ROWS = 32   # up to this many rows the TMA-fed kernel beats the libra
 STREAM_MAX_PARTS = 4
 
 
-def linear_for_residual(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear_for_residual(x: torch.Tensor, w: torch.Tensor, static_weights: bool = False) -> torch.Tensor:
     """``x @ w.T`` for a result that goes straight into the residual stream: either the
     product ``[M, N]`` in the activation dtype, or - for the few rows of a decode step -
     float32 partial sums ``[parts, M, N]`` over slices of k, which the stream's next norm adds
@@ -761,11 +761,11 @@ def linear_for_residual(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     if (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and m <= STREAM_MAX_ROWS and k >= 1024 and k % 8 == 0
             and n % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
-        return linear_stream_partial(x, w)
-    return linear(x, w)
+        return linear_stream_partial(x, w, static_weights=static_weights)
+    return linear(x, w, static_weights=static_weights)
 
 
-def linear_for_rotation(x: torch.Tensor, w: torch.Tensor, head_dim: int, rotary_dim: int) -> torch.Tensor:
+def linear_for_rotation(x: torch.Tensor, w: torch.Tensor, head_dim: int, rotary_dim: int, static_weights: bool = False) -> torch.Tensor:
     """The fused QKV product for :func:`qk_norm_rope_kv_write`: the product ``[M, N]`` in the
     activation dtype, or - for the few rows of a decode step, where the TMA-fed kernel with
     its slices of k is the fastest way to read the weights - float32 partial sums
@@ -775,8 +775,8 @@ def linear_for_rotation(x: torch.Tensor, w: torch.Tensor, head_dim: int, rotary_
     if (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and m <= STREAM_MAX_ROWS and k >= 1024 and k % 8 == 0
             and head_dim in (64, 128, 256) and rotary_dim in (0, head_dim) and n % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
             and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
-        return linear_stream_partial(x, w)
-    return linear(x, w)
+        return linear_stream_partial(x, w, static_weights=static_weights)
+    return linear(x, w, static_weights=static_weights)
 
 
 def stream_error_word(device: torch.device) -> torch.Tensor:
@@ -785,7 +785,7 @@ def stream_error_word(device: torch.device) -> torch.Tensor:
     return _error_words(device)[2:3]
 
 
-def linear_stream_partial(x: torch.Tensor, w: torch.Tensor, parts: Optional[int] = None) -> torch.Tensor:
+def linear_stream_partial(x: torch.Tensor, w: torch.Tensor, parts: Optional[int] = None, static_weights: bool = False) -> torch.Tensor:
     """bfloat16 ``x [M <= 64, K] @ w [N, K].T`` as float32 partial sums ``[parts, M, N]`` over
     slices of k, the weights streamed by TMA through a shared-memory ring.  ``parts`` defaults
     to what gives every SM up to three blocks (64 weight rows x one slice each), at most
@@ -803,11 +803,12 @@ def linear_stream_partial(x: torch.Tensor, w: torch.Tensor, parts: Optional[int]
     y = torch.empty((parts, m, n), dtype=torch.float32, device=x.device)
     library = _library("gemm_stream.cu")
     _check(library, library.pylon_gemm_stream_partial(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), parts,
-                                                      _ptr(stream_error_word(x.device)), _stream()))
+                                                      _ptr(stream_error_word(x.device)), int(static_weights), _stream()))
     return y
 
 
-def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit: Optional[float] = None, alpha: float = 1.0) -> torch.Tensor:
+def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit: Optional[float] = None, alpha: float = 1.0,
+                  static_weights: bool = False) -> torch.Tensor:
     """bfloat16 ``x [M <= 64, K] @ w [N, K].T`` on the TMA-fed kernel, one block per 64 weight rows
     over the whole of k; with ``swiglu`` the rows of ``w`` are interleaved gate/up groups (see
     :func:`interleave_gate_up`) and the result is ``silu(gate) * up``, ``[M, N / 2]`` - or, with a
@@ -822,14 +823,14 @@ def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit:
     library = _library("gemm_stream.cu")
     if swiglu and limit is not None:
         _check(library, library.pylon_gemm_stream_glu_clamped(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit),
-                                                              float(alpha), _ptr(stream_error_word(x.device)), _stream()))
+                                                              float(alpha), _ptr(stream_error_word(x.device)), int(static_weights), _stream()))
         return y
     entry = library.pylon_gemm_stream_swiglu if swiglu else library.pylon_gemm_stream_bf16
-    _check(library, entry(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), _ptr(stream_error_word(x.device)), _stream()))
+    _check(library, entry(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), _ptr(stream_error_word(x.device)), int(static_weights), _stream()))
     return y
 
 
-def linear_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
+def linear_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, static_weights: bool = False) -> torch.Tensor:
     """The weight-streaming kernel itself: bfloat16 ``x [M <= 64, K] @ w [N, K].T`` with ``K``
     and the row strides multiples of 8 and 16-byte aligned operands; anything else is refused."""
     _need_cuda(x, w)
@@ -840,7 +841,7 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = tor
     n = w.shape[0]
     y = torch.empty((m, n), dtype=out_dtype, device=x.device)
     library = _library("gemm_skinny.cu")
-    _check(library, library.pylon_gemm_skinny_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), n, _dtype_code(out_dtype), _stream()))
+    _check(library, library.pylon_gemm_skinny_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), n, _dtype_code(out_dtype), int(static_weights), _stream()))
     return y
 
 
@@ -858,7 +859,8 @@ def tcgen05_force_tile(columns: int = 0) -> None:
     _library("gemm_tcgen05.cu").pylon_gemm_tcgen05_force_tile(columns)
 
 
-def linear_tcgen05(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit: Optional[float] = None, alpha: float = 1.0) -> torch.Tensor:
+def linear_tcgen05(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit: Optional[float] = None, alpha: float = 1.0,
+                   static_weights: bool = False) -> torch.Tensor:
     """bfloat16 ``x [M, K] @ w [N, K].T`` on the tcgen05 tensor cores (TMA-fed, accumulators in
     tensor memory).  With ``swiglu`` the rows of ``w`` are interleaved by
     :func:`interleave_gate_up` and the result is ``silu(gate) * up``, ``[M, N / 2]`` - or, with a
@@ -873,10 +875,10 @@ def linear_tcgen05(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit
     library = _library("gemm_tcgen05.cu")
     if swiglu and limit is not None:
         _check(library, library.pylon_gemm_tcgen05_glu_clamped(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit),
-                                                               float(alpha), _ptr(tcgen05_error_word(x.device)), _multiprocessors(x.device), _stream()))
+                                                               float(alpha), _ptr(tcgen05_error_word(x.device)), _multiprocessors(x.device), int(static_weights), _stream()))
         return y
     _check(library, library.pylon_gemm_tcgen05_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), int(swiglu),
-                                                    _ptr(tcgen05_error_word(x.device)), _multiprocessors(x.device), _stream()))
+                                                    _ptr(tcgen05_error_word(x.device)), _multiprocessors(x.device), int(static_weights), _stream()))
     return y
 
 QKV_ROTATION_MIN_ROWS = 3_072
@@ -955,7 +957,7 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return torch.stack((gate.reshape(inter // 8, 8, k), up.reshape(inter // 8, 8, k)), dim=1).reshape(2 * inter, k).contiguous()
 
 
-def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0) -> torch.Tensor:
+def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0, static_weights: bool = False) -> torch.Tensor:
     """``silu(x @ gate.T) * (x @ up.T)`` for weights stacked by :func:`interleave_gate_up`:
     one kernel for few rows (the TMA-fed decode kernel) and for many (the tcgen05 kernel), the
     library product and the SwiGLU kernel in between.  With a ``limit`` the gated unit is the clamped
@@ -966,12 +968,12 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and m <= STREAM_MAX_ROWS and x.shape[1] == k
             and k % 8 == 0 and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0
             and w_interleaved.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
-        return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha)
+        return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and m >= TCGEN05_MIN_ROWS and k % 8 == 0
             and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0 and w_interleaved.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
-        return linear_tcgen05(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha)   # many rows: our tcgen05 kernel with the gated unit in its epilogue
-    return swiglu(linear(x, w_interleaved), interleaved=True, limit=limit, alpha=alpha)
+        return linear_tcgen05(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)   # many rows: our tcgen05 kernel with the gated unit in its epilogue
+    return swiglu(linear(x, w_interleaved, static_weights=static_weights), interleaved=True, limit=limit, alpha=alpha)
 
 
 # ---------------------------------------------------------------------------------------
@@ -1773,7 +1775,7 @@ def expert_mixture(h: torch.Tensor, router: torch.Tensor, router_bias: Optional[
                    correction: Optional[torch.Tensor] = None, groups: int = 0, groups_keep: int = 0, share_eps: float = 0.0,
                    common_up: Optional[torch.Tensor] = None, common_down: Optional[torch.Tensor] = None, share_normalized: bool = True,
                    weigh: str = "output", limit: Optional[float] = None, alpha: float = 1.702, scattered: bool = False, group_score: str = "two",
-                   share_scale: float = 1.0, identity: int = 0, always: int = 0) -> Union[torch.Tensor, "ScatteredRows"]:
+                   share_scale: float = 1.0, identity: int = 0, always: int = 0, static_weights: bool = False) -> Union[torch.Tensor, "ScatteredRows"]:
     """``sum over a token's top experts e of share_e * W_down,e (act(W_gate,e h) * (W_up,e h))`` (``csrc/experts.cu``).
 
     ``h [T, width]``; ``router`` float32 ``[experts, width]`` and ``router_bias`` float32 ``[experts]`` (or None): the logits are
@@ -1796,7 +1798,7 @@ def expert_mixture(h: torch.Tensor, router: torch.Tensor, router_bias: Optional[
     ``routing="softmax_all"``: the scores are the softmax over all of the router's outputs, the rest as with sigmoids.  ``group_score="best"``: a group
     is worth its largest choice score.  ``share_scale`` on the shares.  ``identity`` n: the router has n outputs behind the experts', each handing
     ``h`` itself back times its share; groups, correction and top count them.  ``always`` m: the last m of the stacked experts have no router output,
-    and every token goes through them with a share of one.
+    and every token goes through them with a share of one.  ``static_weights``: as in :func:`linear`, of the common expert's matrices.
 
     The tokens are sorted by expert on the device.  A step of few tokens runs the experts' products from row tiles of 32 slots that
     gather their rows themselves (``mma.sync``, bound by the matrices coming from memory); a bfloat16 step with about half a
@@ -1855,7 +1857,7 @@ def expert_mixture(h: torch.Tensor, router: torch.Tensor, router_bias: Optional[
                                                _ptr(share), _ptr(slot_share), per, always, _stream()))
     common, common_code = None, code if identity else F32
     if extra:   # the expert of every token: two plain products around the activation
-        common = linear(activation_in_place(linear(h, common_up), activation), common_down)
+        common = linear(activation_in_place(linear(h, common_up, static_weights=static_weights), activation), common_down, static_weights=static_weights)
         common_code = _dtype_code(common.dtype)
     if grouped:
         product = _library("gemm_tcgen05.cu")
@@ -1905,13 +1907,14 @@ def _expert_parts(experts: int, columns: int, k: int, sms: int) -> int:
 # ---------------------------------------------------------------------------------------
 # products per head
 # ---------------------------------------------------------------------------------------
-def linear_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+def linear_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
+                 static_weights: bool = False) -> torch.Tensor:
     """One product per head: ``y[t, h] = w[h] @ x[t, h]`` for ``x [T, H, K]``, ``w [H, N, K]`` -> ``[T, H, N]``.
     ``out_dtype=torch.float32`` keeps the 32-bit sums of a bfloat16 product (logits of gates, say).
 
     ``x`` and ``out`` may be views whose heads are slices of wider rows (any token and head strides; the last dimension
     contiguous).  float32 runs the plain-FMA kernel, one grid layer per head; bfloat16 goes to the library's batched
-    product with float32 accumulation, as the large plain products do."""
+    product with float32 accumulation, as the large plain products do.  ``static_weights``: as in :func:`linear`."""
     _need_cuda(x, w, out)
     _need(x.dim() == 3 and w.dim() == 3 and x.shape[1] == w.shape[0] and x.shape[2] == w.shape[2], f"linear_heads: shapes {tuple(x.shape)} and {tuple(w.shape)} do not match")
     _need(x.dtype == w.dtype and x.stride(2) == 1 and w.is_contiguous(), "linear_heads: one dtype, the reduced dimension contiguous, the weights contiguous")
@@ -1930,7 +1933,7 @@ def linear_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] =
     if x.dtype == torch.float32:
         library = _library("gemm_f32.cu")
         _check(library, library.pylon_gemm_f32_nt_batched(_ptr(x), _ptr(w), _ptr(out), tokens, n, k, x.stride(0), k, out.stride(0), heads,
-                                                          x.stride(1), n * k, out.stride(1), _stream()))
+                                                          x.stride(1), n * k, out.stride(1), int(static_weights), _stream()))
         return out
     _need(x.dtype == torch.bfloat16, f"linear_heads: unsupported dtype {x.dtype}")
     torch.bmm(x.transpose(0, 1), w.transpose(1, 2), out=out.transpose(0, 1))

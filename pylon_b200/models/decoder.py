@@ -129,7 +129,7 @@ class DecoderModel:
                 # x <- W [x; x0]: what is pending joins the sum, both halves are laid side by side in the compute dtype, and the
                 # product's 32-bit result is the new sum
                 stream.flush()
-                stream.residual = ops.linear(ops.concat_cast(stream.residual, entered, self.dtype), self.reentry, out_dtype=torch.float32)
+                stream.residual = ops.linear(ops.concat_cast(stream.residual, entered, self.dtype), self.reentry, out_dtype=torch.float32, static_weights=True)
             if run.add_embedding:
                 stream.flush()   # what the run before left pending joins the sum first; then the embedding rows, in 32-bit like the sum itself
                 ops.embed_gather(step.token_ids, self.embedding, out=stream.residual, scale=self.spec.embedding_scale, copies=self.spec.streams,
@@ -140,7 +140,7 @@ class DecoderModel:
         if step.num_logits == 0:
             return None
         hidden = self.final_norm.apply(stream, rows=step.logit_rows)
-        logits = ops.linear(hidden, self.lm_head, out_dtype=torch.float32)
+        logits = ops.linear(hidden, self.lm_head, out_dtype=torch.float32, static_weights=True)
         if self.spec.logit_scale != 1.0 or self.spec.logit_softcap is not None:
             ops.logit_transform(logits, self.spec.logit_scale, self.spec.logit_softcap)
         return logits

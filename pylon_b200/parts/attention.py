@@ -315,7 +315,7 @@ class GroupedQueryAttention(Mixer):
         if self.position is not None and table is None:
             # An encoding that is not a rotation by a table runs as a step of its own, on normalised q and k and
             # before k goes into the cache; the fused kernel below is left with the cache write.
-            qkv = ops.linear(h, self.w_qkv)
+            qkv = ops.linear(h, self.w_qkv, static_weights=True)
             if q_norm is not None:
                 ops.qk_norm(qkv, q_norm, k_norm, self.qk_norm_eps, self.n_heads, self.n_kv_heads, self.head_dim)
                 q_norm = k_norm = None
@@ -323,7 +323,7 @@ class GroupedQueryAttention(Mixer):
         elif cos is not None and ops.qkv_rotation_fuses(h, self.w_qkv, self.head_dim, rotary_dim, cache.k_pages):
             qkv = None   # a long prompt portion: norms, rotation and cache write in the product's epilogue
         else:
-            qkv = ops.linear_for_rotation(h, self.w_qkv, self.head_dim, rotary_dim)   # may be partial sums: the next kernel adds them
+            qkv = ops.linear_for_rotation(h, self.w_qkv, self.head_dim, rotary_dim, static_weights=True)   # may be partial sums: the next kernel adds them
         if qkv is None:
             q = ops.linear_qkv_rotated(
                 h, self.w_qkv, q_norm, k_norm, self.qk_norm_eps or 0.0, cos, sin, step.positions, step.token_row,
@@ -339,14 +339,14 @@ class GroupedQueryAttention(Mixer):
             self.n_heads, step.max_q, step.max_kv, window=self.window, scale=self.scale, row_tokens=step.row_tokens,
             rows_alike=step.rows_alike,
         )
-        return ops.linear_for_residual(context, self.w_o)
+        return ops.linear_for_residual(context, self.w_o, static_weights=True)
 
     def _forward_general(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
         """Values of their own width, value mixing, chunks or a soft cap: the product, one kernel for norms, mixing and
         cache write, attention, the output product."""
         if self.position is not None:
             raise NotImplementedError("a position encoding together with value_dim, chunk, softcap or value_mix is not built")
-        qkv = ops.linear(h, self.w_qkv)
+        qkv = ops.linear(h, self.w_qkv, static_weights=True)
         other, other_width = step.carry.get(self.value_mix_key, (None, None)) if self.value_mix == "mix" else (None, None)
         if self.value_mix == "mix" and other is None:
             raise RuntimeError(f"no earlier layer of this step left values under {self.value_mix_key!r}")
@@ -364,13 +364,13 @@ class GroupedQueryAttention(Mixer):
             rows_alike=step.rows_alike, chunk=self.chunk, softcap=self.softcap, sinks=self.sink, keep_first=self.keep_first,
             distance_bias=self.bias_table,
         )
-        return ops.linear_for_residual(context, self.w_o)
+        return ops.linear_for_residual(context, self.w_o, static_weights=True)
 
     def _forward_rotary_general(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
         """Biases, any rotation by tables, the norm on either side of it, values of any width: the product, one kernel for all of
         that and the cache write, attention, the output product."""
         cos, sin, rotary_dim, layout = self.position.tables(h.device) if self.position is not None else (None, None, 0, "halves")
-        qkv = ops.linear(h, self.w_qkv)
+        qkv = ops.linear(h, self.w_qkv, static_weights=True)
         ops.qkv_rotate_write(
             qkv, self.b_qkv, cos, sin, rotary_dim, layout, None if self.qk_norm_eps is None else self.qk_norm_place, self.q_norm, self.k_norm,
             self.qk_norm_eps or 0.0, step.positions, step.token_row, cache.block_table, cache.page_size, cache.k_pages, cache.v_pages,
@@ -381,14 +381,14 @@ class GroupedQueryAttention(Mixer):
             self.n_heads, step.max_q, step.max_kv, window=self.window, scale=self.scale, row_tokens=step.row_tokens,
             rows_alike=step.rows_alike, chunk=self.chunk, softcap=self.softcap,
         )
-        return ops.linear_for_residual(context, self.w_o)
+        return ops.linear_for_residual(context, self.w_o, static_weights=True)
 
     def forward_unjoined(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> tuple[torch.Tensor, Optional[torch.Tensor]]:
         if not self.stacked:
             return self.forward(h, step, cache), None
         context = torch.empty((h.shape[0], self.output_columns.shape[1]), dtype=h.dtype, device=h.device)
-        self.middle(ops.linear_stacked(h, self.input_rows), step, cache, context, 1.0)
-        return ops.linear_for_residual(context, self.output_columns), self.b_out
+        self.middle(ops.linear_stacked(h, self.input_rows, static_weights=True), step, cache, context, 1.0)
+        return ops.linear_for_residual(context, self.output_columns, static_weights=True), self.b_out
 
     def middle(self, proj: torch.Tensor, step: StepView, cache: LayerCache, out: torch.Tensor, factor: float) -> None:
         """Stacked mixers: one kernel for biases, norms, rotation, factor and cache write on the projections, then the attention, which gates

@@ -138,17 +138,17 @@ class GatedDeltaRule(Mixer):
 
     # -- run -----------------------------------------------------------------------------
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
-        proj = ops.linear(h, self.w_in)
+        proj = ops.linear(h, self.w_in, static_weights=True)
         own = {}
         for key, second in (("gate", self.w_gate), ("decay", self.w_decay)):
             if key in self.extra_columns:
                 first, last = self.extra_columns[key]
                 part = proj[:, first:last]
                 # what enters the decay and the gate is float32 from here on: the second factor's product keeps its 32-bit sums
-                own[key] = ops.linear(part, second, out_dtype=torch.float32) if second is not None else part.to(torch.float32)
+                own[key] = ops.linear(part, second, out_dtype=torch.float32, static_weights=True) if second is not None else part.to(torch.float32)
         mixed = ops.gated_delta_rule(
             proj, self.conv, cache.state, step.token_row, step.q_start, step.slots, self.a_log, self.dt_bias, self.norm,
             self.n_heads, self.n_kv_heads, self.head_dim, self.value_dim, step.num_rows, self.norm_eps, self.unit_eps,
             decay_in=own.get("decay"), gate_in=own.get("gate"),
         )
-        return ops.linear_for_residual(mixed, self.w_o)
+        return ops.linear_for_residual(mixed, self.w_o, static_weights=True)

@@ -91,7 +91,7 @@ class LatentAttention(Mixer):
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
         tokens = h.shape[0]
         cos, sin, rotary_dim, layout = self.position.tables(h.device) if self.position is not None else (None, None, 0, "halves")
-        down = ops.linear(h, self.w_down)
+        down = ops.linear(h, self.w_down, static_weights=True)
         if self.q_rank is None:   # the queries are the product's first columns as they are; the rest is the token's cache row
             q_size = self.n_heads * self.q_head
             ops.latent_norm_rotate_write(
@@ -104,9 +104,9 @@ class LatentAttention(Mixer):
                 down, self.q_norm, self.kv_norm, self.norm_eps, cos, sin, rotary_dim, layout, step.positions, step.token_row, cache.block_table,
                 cache.page_size, cache.k_pages, self.q_rank, self.kv_rank, self.rot_dim,
             )
-            q = ops.linear(cq, self.w_uq).view(tokens, self.n_heads, self.q_head)
+            q = ops.linear(cq, self.w_uq, static_weights=True).view(tokens, self.n_heads, self.q_head)
         query = torch.empty((tokens, self.n_heads, self.row), dtype=h.dtype, device=h.device)
-        ops.linear_heads(q[:, :, : self.head_dim], self.w_uk_t, out=query[:, :, : self.kv_rank])
+        ops.linear_heads(q[:, :, : self.head_dim], self.w_uk_t, out=query[:, :, : self.kv_rank], static_weights=True)
         if self.rot_dim:
             ops.rotate_heads(q[:, :, self.head_dim:], query[:, :, self.kv_rank:], cos, sin, rotary_dim, layout, step.positions)
         context = ops.paged_attention(
@@ -114,5 +114,5 @@ class LatentAttention(Mixer):
             cache.block_table, self.n_heads, step.max_q, step.max_kv, window=self.window, scale=self.scale, row_tokens=step.row_tokens,
             sinks=self.sink, values_in_keys=self.kv_rank, split_weights=self.split_weights,
         )
-        values = ops.linear_heads(context.view(tokens, self.n_heads, self.kv_rank), self.w_uv)
-        return ops.linear_for_residual(values.view(tokens, self.n_heads * self.value_dim), self.w_o)
+        values = ops.linear_heads(context.view(tokens, self.n_heads, self.kv_rank), self.w_uv, static_weights=True)
+        return ops.linear_for_residual(values.view(tokens, self.n_heads * self.value_dim), self.w_o, static_weights=True)

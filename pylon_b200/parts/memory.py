@@ -63,8 +63,8 @@ class MatrixMemory(Mixer):
         return CacheNeed(state=StateNeed((self.n_heads * (self.head_dim * self.value_dim + self.head_dim + 1),)))
 
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
-        proj = ops.linear(h, self.w_in)
-        logits = ops.linear(h, self.w_gates, out_dtype=torch.float32)
+        proj = ops.linear(h, self.w_in, static_weights=True)
+        logits = ops.linear(h, self.w_gates, out_dtype=torch.float32, static_weights=True)
         out = ops.matrix_memory(proj, logits, self.gate_bias, self.norm_weight, cache.state, step.q_start, step.slots, self.n_heads, self.head_dim,
                                 self.value_dim, self.gate_cap, self.norm_eps, self.read_eps, step.num_rows)
-        return ops.linear_for_residual(out, self.w_o)
+        return ops.linear_for_residual(out, self.w_o, static_weights=True)

@@ -55,8 +55,8 @@ class MinGRU(Mixer):
 
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
         read = torch.empty((h.shape[0], self.channels), dtype=h.dtype, device=h.device)
-        self.middle(ops.linear_stacked(h, self.input_rows), step, cache, read, 1.0)
-        return ops.linear_for_residual(read, self.output_columns)
+        self.middle(ops.linear_stacked(h, self.input_rows, static_weights=True), step, cache, read, 1.0)
+        return ops.linear_for_residual(read, self.output_columns, static_weights=True)
 
     def middle(self, proj: torch.Tensor, step: StepView, cache: LayerCache, out: torch.Tensor, factor: float) -> None:
         ops.min_gru(proj, self.bias, cache.state, step.q_start, step.slots, step.num_rows, step.max_q, out, factor)

@@ -52,10 +52,10 @@ class SwiGLU(FeedForward):
 
     def forward(self, h: torch.Tensor, step: StepView) -> torch.Tensor:
         if self.interleaved:
-            activation = ops.linear_swiglu(h, self.w_gate_up, limit=self.limit, alpha=self.alpha)
+            activation = ops.linear_swiglu(h, self.w_gate_up, limit=self.limit, alpha=self.alpha, static_weights=True)
         else:
-            activation = ops.swiglu(ops.linear(h, self.w_gate_up), limit=self.limit, alpha=self.alpha)
-        return ops.linear_for_residual(activation, self.w_down)
+            activation = ops.swiglu(ops.linear(h, self.w_gate_up, static_weights=True), limit=self.limit, alpha=self.alpha)
+        return ops.linear_for_residual(activation, self.w_down, static_weights=True)
 
 
 @FEED_FORWARDS.register("clamped_glu")
@@ -109,11 +109,11 @@ class GatedUnit(FeedForward):
 
     def forward(self, h: torch.Tensor, step: StepView) -> torch.Tensor:
         if self.fused:
-            return ops.linear_for_residual(ops.linear_swiglu(h, self.w_gate_up), self.w_down)
-        activation = ops.gated_unit(ops.linear(h, self.w_gate_up), self.b_gate_up, self.activation)
+            return ops.linear_for_residual(ops.linear_swiglu(h, self.w_gate_up, static_weights=True), self.w_down, static_weights=True)
+        activation = ops.gated_unit(ops.linear(h, self.w_gate_up, static_weights=True), self.b_gate_up, self.activation)
         if not self.bias:
-            return ops.linear_for_residual(activation, self.w_down)
-        out = ops.linear(activation, self.w_down, out_dtype=torch.float32)
+            return ops.linear_for_residual(activation, self.w_down, static_weights=True)
+        out = ops.linear(activation, self.w_down, out_dtype=torch.float32, static_weights=True)
         return ops.add_bias(out, self.b_down).unsqueeze(0)   # float32, in the form of partial sums: the stream takes it in 32-bit
 
 
@@ -244,7 +244,7 @@ class ExpertMixture(FeedForward):
                                   gated=self.gated, routing=self.routing, correction=self.correction, groups=self.groups, groups_keep=self.groups_keep,
                                   share_eps=self.share_eps, common_up=self.w_shared_up, common_down=self.w_shared_down, share_normalized=self.share_normalized,
                                   weigh=self.weigh, limit=self.limit, alpha=self.alpha, scattered=scattered, group_score=self.group_score,
-                                  share_scale=self.share_scale, identity=self.identity, always=self.always)
+                                  share_scale=self.share_scale, identity=self.identity, always=self.always, static_weights=True)
 
     def forward_scattered(self, h: torch.Tensor, step: StepView):
         return self.forward(h, step, scattered=self.shared_intermediate is None)

@@ -113,11 +113,11 @@ class WeightedMixers(ParallelMixers):
 
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
         if self.w_in is not None:
-            proj = ops.linear_stacked(h, self.w_in)
+            proj = ops.linear_stacked(h, self.w_in, static_weights=True)
             # columns between the slices meet zeros of the last product's matrix, so they must hold numbers
             middle = (torch.empty if self.filled else torch.zeros)((h.shape[0], self.w_out.shape[1]), dtype=h.dtype, device=h.device)
             for mixer, scale, into, out_of in zip(self.mixers, self.scales, self.in_slices, self.out_slices):
                 mixer.middle(proj[:, into], step, cache, middle[:, out_of], scale)
-            return ops.linear_for_residual(middle, self.w_out)
+            return ops.linear_for_residual(middle, self.w_out, static_weights=True)
         outputs = [mixer.forward(h, step, cache) for mixer in self.mixers]
         return ops.weighted_sum(outputs, self.scales, self.dtype)

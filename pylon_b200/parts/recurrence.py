@@ -66,7 +66,7 @@ class GatedLinearRecurrence(Mixer):
         return CacheNeed(state=StateNeed((self.channels * self.taps,)))
 
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
-        proj = ops.linear(h, self.w_in)
+        proj = ops.linear(h, self.w_in, static_weights=True)
         out = ops.linear_recurrence(proj, self.bias, self.conv_weight, self.conv_bias, self.w_gates, self.gate_bias, self.lam, self.decay_factor,
                                     cache.state, step.token_row, step.q_start, step.slots, step.num_rows, step.max_q)
-        return ops.linear_for_residual(out, self.w_o)
+        return ops.linear_for_residual(out, self.w_o, static_weights=True)

@@ -71,9 +71,9 @@ class StateSpace(Mixer):
         return CacheNeed(state=StateNeed((self.state_floats(),), torch.float32))
 
     def forward(self, h: torch.Tensor, step: StepView, cache: LayerCache) -> torch.Tensor:
-        proj = ops.linear(h, self.w_in)
+        proj = ops.linear(h, self.w_in, static_weights=True)
         mixed = ops.state_space(
             proj, self.conv, self.conv_bias, cache.state, step.token_row, step.q_start, step.slots, self.a_log, self.dt_bias, self.skip,
             self.norm, self.n_heads, self.groups, self.state_dim, self.value_dim, self.norm_groups, step.num_rows, self.norm_eps,
         )
-        return ops.linear_for_residual(mixed, self.w_o)
+        return ops.linear_for_residual(mixed, self.w_o, static_weights=True)

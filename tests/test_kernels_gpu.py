@@ -145,6 +145,42 @@ def test_linear_of_many_weight_rows(m, n, k, out_dtype):
     assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
 
 
+PRODUCTS_OF_ANY_MATRIX = {   # name: dtype, rows of x, [N, K] of the second operand, the product under test
+    "float32 rows": (torch.float32, 5, (4_096, 2_048), lambda ops, x, w: ops.linear(x, w)),
+    "float32 tiles": (torch.float32, 70, (4_096, 2_048), lambda ops, x, w: ops.linear(x, w)),
+    "float32 heads": (torch.float32, 5, (4_096, 2_048), lambda ops, x, w: ops.linear_heads(x.view(5, 8, 256), w.view(8, 2_048 * 2, 256))),
+    "skinny": (torch.bfloat16, 8, (8_192, 2_048), lambda ops, x, w: ops.linear(x, w)),
+    "stream": (torch.bfloat16, 16, (16_384, 2_048), lambda ops, x, w: ops.linear(x, w)),
+    "head": (torch.bfloat16, 16, (57_344, 1_024), lambda ops, x, w: ops.linear(x, w, out_dtype=torch.float32)),
+    "parts": (torch.bfloat16, 4, (2_560, 4_096), lambda ops, x, w: ops.linear_for_residual(x, w)),
+    "gated, few rows": (torch.bfloat16, 4, (19_456, 2_560), lambda ops, x, w: ops.linear_swiglu(x, w)),
+    "gated, both row tiles": (torch.bfloat16, 160, (19_456, 2_560), lambda ops, x, w: ops.linear_swiglu(x, w)),
+}
+
+
+@pytest.mark.parametrize("name", list(PRODUCTS_OF_ANY_MATRIX))
+def test_second_operand_may_be_the_kernel_ahead_s_result(name):
+    """The matrix that a product takes as its weights is what the kernel ahead on the stream has just been queued to write, into memory that holds
+    other numbers: without ``static_weights`` the product waits for it, and gives the bits of a run in which the device is waited for in between."""
+    from pylon_b200.kernels import ops
+
+    dtype, m, (n, k), product = PRODUCTS_OF_ANY_MATRIX[name]
+    x = torch.randn(m, k, device=DEVICE).to(dtype)
+    sources = [torch.randn(n, 2 * k, device=DEVICE).to(dtype) for _ in range(2)]
+    made = [ops.swiglu(source) for source in sources]
+    torch.cuda.synchronize()
+    want = [product(ops, x, matrix) for matrix in made]
+    torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    matrix = torch.empty(n, k, dtype=dtype, device=DEVICE)
+    wrong = torch.zeros((), dtype=torch.int64, device=DEVICE)
+    for turn in range(200):
+        ops.swiglu(sources[turn % 2], out=matrix)
+        got = product(ops, x, matrix)
+        wrong += (got != want[turn % 2]).any()
+    assert int(wrong) == 0
+
+
 @pytest.mark.parametrize("m", [1, 16, 33])
 @pytest.mark.parametrize("k", [512, 520, 1_032, 9_728])
 @pytest.mark.parametrize("parts", [1, 3])

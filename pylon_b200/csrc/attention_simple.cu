@@ -136,14 +136,16 @@ __global__ void __launch_bounds__(SIMPLE_THREADS) paged_attention_simple_kernel(
 // of every sum is again a function of the token's position.  193 tokens of 32 heads over 8 of size 128: 148 us with the plain
 // kernel, under 31 with this one; 16 tokens over some 90 keys each: 36 and under 8.  What bounds it is the latency of a chunk's three phases at few tokens
 // and the traffic with L2 at many.
+// (Its inputs are not const __restrict__: what the kernel ahead writes must not be read through the non-coherent path, whose loads may be
+// moved ahead of the wait for that kernel.)
 template <int HG, int NC>
 __global__ void __launch_bounds__(SIMPLE_THREADS) paged_attention_f32_kernel(
-    const float* __restrict__ q, long long q_token_stride, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
-    float* __restrict__ out, const int* __restrict__ positions, const int* __restrict__ token_row, const int* __restrict__ block_table,
+    const float* q, long long q_token_stride, const float* k_pages, const float* v_pages,
+    float* __restrict__ out, const int* positions, const int* token_row, const int* block_table,
     int table_width, int page_size, int num_pages, int nq, int nkv, int d, int dv, int window, int chunk, float softcap, float scale,
-    const float* __restrict__ sinks, long long k_row_stride, long long v_row_stride, int keep_first, const float* __restrict__ bias,
-    int bias_rows, int sigmoid, const float* __restrict__ score_bias, const float* __restrict__ gate, long long gate_stride, float factor,
-    long long out_stride, const float* __restrict__ slopes, int gate_elements) {
+    const float* sinks, long long k_row_stride, long long v_row_stride, int keep_first, const float* bias,
+    int bias_rows, int sigmoid, const float* score_bias, const float* gate, long long gate_stride, float factor,
+    long long out_stride, const float* slopes, int gate_elements) {
   extern __shared__ __align__(16) float shared_f32[];
   float* qs = shared_f32;                                        // [HG][d]
   float* probs = qs + HG * d;                                    // [HG][128]: scores, then weights

@@ -134,12 +134,14 @@ __device__ __forceinline__ float4 delta_load4(const __nv_bfloat16* p) {
   const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
+// (Here and in delta_chunk_matrices_kernel the inputs are not const __restrict__: what the kernel ahead writes must not be read through the
+// non-coherent path, whose loads may be moved ahead of the wait for that kernel.)
 template <int TOKENS>
-__global__ void __launch_bounds__(128) delta_prepare_wide_kernel(const __nv_bfloat16* __restrict__ proj, long long ld, const float* __restrict__ conv_w, int taps,
-                                                                 const float* __restrict__ state, long long slot_floats, long long conv_offset,
-                                                                 const int* __restrict__ token_row, const int* __restrict__ q_start,
-                                                                 const int* __restrict__ slots, float* __restrict__ qkv, float* __restrict__ gates,
-                                                                 const float* __restrict__ a_log, const float* __restrict__ dt_bias, int col_a, int col_b,
+__global__ void __launch_bounds__(128) delta_prepare_wide_kernel(const __nv_bfloat16* proj, long long ld, const float* conv_w, int taps,
+                                                                 const float* state, long long slot_floats, long long conv_offset,
+                                                                 const int* token_row, const int* q_start,
+                                                                 const int* slots, float* __restrict__ qkv, float* __restrict__ gates,
+                                                                 const float* a_log, const float* dt_bias, int col_a, int col_b,
                                                                  int heads, int kv_heads, int dim, int vdim, float unit_eps, int num_tokens) {
   constexpr int TAPS = 4;
   grid_dependency_wait();
@@ -521,8 +523,8 @@ constexpr int CHUNK = 16, CHUNK_MATRIX = 2 * CHUNK * CHUNK + 2 * CHUNK;   // T |
 // Chunk c of row r has the number q_start[r] / CHUNK + r + c: rows' numbers do not meet, and all lie below tokens / CHUNK + rows + 1.
 // grid (those numbers, kv_heads), 128 threads; matrices: float32 [numbers, heads, CHUNK_MATRIX].
 template <int DIM>
-__global__ void __launch_bounds__(128) delta_chunk_matrices_kernel(const float* __restrict__ qkv, const float* __restrict__ gates,
-                                                                   float* __restrict__ matrices, const int* __restrict__ q_start, int num_rows,
+__global__ void __launch_bounds__(128) delta_chunk_matrices_kernel(const float* qkv, const float* gates,
+                                                                   float* __restrict__ matrices, const int* q_start, int num_rows,
                                                                    int heads, int kv_heads, int vdim) {
   constexpr int ROW = DIM + 4;
   __shared__ __align__(16) float ks[CHUNK * ROW], qs[CHUNK * ROW];

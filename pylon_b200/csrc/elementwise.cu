@@ -608,7 +608,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out
 
 // Vector form for float32 rows whose width is a multiple of 4: a thread takes four columns, a block row of the grid a row of the
 // input, so nothing is divided (an element at a time, with a division each, 224 rows of 9,728 took 9.7 us).
-__global__ void swiglu_f32x4_kernel(const float4* __restrict__ gate_up, float4* __restrict__ out, int inter4, int interleaved, float limit, float alpha) {
+__global__ void swiglu_f32x4_kernel(const float4* gate_up, float4* __restrict__ out, int inter4, int interleaved, float limit, float alpha) {
   grid_dependency_wait();
   allow_dependents();
   const size_t t = blockIdx.y;

@@ -170,8 +170,9 @@ __global__ void streams_update_norm_kernel(float* __restrict__ x, const TD* __re
 // 1,024 V, are known to the compiler, so all of a thread's reads are under way before the first is used, the combined row stays in
 // registers and a sum over the block takes one barrier.  What bounds it is the streams' way from and to memory: 2,048 rows of four streams of
 // 2,048, 150 MB in 26 us (5.8 TB/s); the kernel above took 38.
+// (Not const __restrict__ for what the kernel ahead writes: reads through the non-coherent path may be moved ahead of the wait for it.)
 template <typename TD, int S, int V>
-__global__ void __launch_bounds__(256) streams_update_norm_rows_kernel(float* __restrict__ x, const TD* __restrict__ delta, float scale,
+__global__ void __launch_bounds__(256) streams_update_norm_rows_kernel(float* __restrict__ x, const TD* delta, float scale,
                                                                        const float* __restrict__ mix, const float* __restrict__ outw,
                                                                        const float* __restrict__ read, const float* __restrict__ weight,
                                                                        __nv_bfloat16* __restrict__ out, float eps, int kind) {

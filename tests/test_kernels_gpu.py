@@ -181,6 +181,56 @@ def test_second_operand_may_be_the_kernel_ahead_s_result(name):
     assert int(wrong) == 0
 
 
+@pytest.mark.parametrize("name", ["gated unit", "attention", "streams", "delta rule"])
+def test_inputs_may_be_the_kernel_ahead_s_result(name):
+    """The float32 gated unit and attention, the streams' update and the delta rule of a prompt portion right behind the kernel that
+    writes their input, into memory that holds other numbers: the bits of a run in which the device is waited for in between."""
+    from pylon_b200.kernels import ops
+
+    as_int = lambda values: torch.tensor(values, device=DEVICE, dtype=torch.int32)
+    if name == "gated unit":
+        dtype, rows, columns = torch.float32, 2_000, 4_096
+        run = lambda x: ops.swiglu(x)
+    elif name == "attention":
+        dtype, rows, columns = torch.float32, 600, 16 * 64
+        cache = Paged([600], [600], 4, 64, 64, torch.float32)
+        run = lambda x: ops.paged_attention(x, cache.k_pages, cache.v_pages, cache.positions, cache.token_row, cache.q_start, cache.kv_len, cache.table, 16, 600, 600)
+    elif name == "streams":
+        dtype, rows, columns = torch.bfloat16, 2_000, 2_048
+        start, weight = torch.randn(rows, 4, columns, device=DEVICE), torch.ones(columns, device=DEVICE)
+        streams = start.clone()
+
+        def run(x):
+            streams.copy_(start)
+            return lambda: ops.streams_update_norm(streams, x, 1.0, None, None, None, weight, 1e-5, "rmsnorm", torch.bfloat16)
+    else:
+        heads, dim, rows, dtype = 4, 128, 1_024, torch.bfloat16
+        channels, columns = 3 * heads * dim, 4 * heads * dim + 64
+        conv, gate = torch.randn(4, channels, device=DEVICE) * 0.5, torch.randn(heads, device=DEVICE)
+        state = torch.zeros(1, heads * dim * dim + 3 * channels, device=DEVICE)
+        norm, starts, slots, token_row = torch.ones(dim, device=DEVICE), as_int([0, rows]), as_int([0]), torch.zeros(rows, dtype=torch.int32, device=DEVICE)
+
+        def run(x):
+            state.zero_()
+            return lambda: ops.gated_delta_rule(x, conv, state, token_row, starts, slots, gate, gate, norm, heads, heads, dim, dim, 1, 1e-5)
+    sources = [torch.randn(rows, 2 * columns, device=DEVICE).to(dtype) for _ in range(2)]
+    inputs = torch.empty(rows, columns, dtype=dtype, device=DEVICE)
+
+    def once(turn, wait):
+        ready = run(inputs) if name in ("streams", "delta rule") else lambda: run(inputs)   # their states are put back ahead of the kernel that writes the inputs
+        ops.swiglu(sources[turn], out=inputs)
+        if wait:
+            torch.cuda.synchronize()
+        return ready()
+
+    want = [once(turn, True) for turn in range(2)]
+    assert not torch.equal(want[0], want[1])
+    wrong = torch.zeros((), dtype=torch.int64, device=DEVICE)
+    for turn in range(100):
+        wrong += (once(turn % 2, False) != want[turn % 2]).any()
+    assert int(wrong) == 0
+
+
 @pytest.mark.parametrize("m", [1, 16, 33])
 @pytest.mark.parametrize("k", [512, 520, 1_032, 9_728])
 @pytest.mark.parametrize("parts", [1, 3])

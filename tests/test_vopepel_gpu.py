@@ -422,6 +422,42 @@ def test_gated_delta_rule_in_chunks(heads, kv_heads, vdim, taps, lengths, decay,
     torch.testing.assert_close(out, want, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("what", ["value", "infinite value", "key", "query", "decay", "beta"])
+@pytest.mark.parametrize("at", [0, 5, 31, 37, 70])
+def test_gated_delta_rule_in_chunks_is_causal_for_values_that_are_not_finite(what, at, monkeypatch):
+    """A token whose projections are not finite changes no bit of the tokens before it, of other rows and of other heads, and reaches the
+    same tokens, heads and state entries as when the rows are walked token by token."""
+    from pylon_b200.kernels import ops
+
+    heads, kv_heads, dim, vdim, eps, lengths = 4, 2, 128, 32, 1e-5, (75, 50, 48)
+    tokens, channels = sum(lengths), 2 * kv_heads * dim + heads * vdim
+    proj, conv, a_log, dt_bias, norm = (t.to(DEVICE) for t in delta_inputs(tokens, heads, kv_heads, dim, vdim, 2, 9, torch.bfloat16))
+    floats = heads * dim * vdim + channels
+    start = torch.randn(len(lengths), floats, device=DEVICE) * 0.1
+    step = step_view(list(lengths), [0] * len(lengths), torch.bfloat16)
+    assert ops.delta_rule_in_chunks(torch.bfloat16, dim, vdim, tokens, len(lengths), floats, False)
+
+    def run(inputs):
+        state = start.clone()
+        out = ops.gated_delta_rule(inputs, conv.t().contiguous(), state, step.token_row, step.q_start, step.slots, a_log, dt_bias, norm, heads, kv_heads, dim,
+                                   vdim, len(lengths), eps)
+        return out.float().view(tokens, heads, vdim), state
+
+    column = {"value": 2 * kv_heads * dim + vdim + 3, "infinite value": 2 * kv_heads * dim + vdim + 3, "key": kv_heads * dim + 7, "query": 7,
+              "decay": channels + heads * vdim + 1, "beta": channels + heads * vdim + heads + 1}[what]
+    marked = proj.clone()
+    marked[at, column] = float("inf") if what == "infinite value" else float("nan")
+    clean, _ = run(proj)
+    got, state = run(marked)
+    monkeypatch.setattr(ops, "delta_rule_in_chunks", lambda *_: False)
+    want, want_state = run(marked)
+    assert torch.isfinite(clean).all() and not torch.isfinite(got[at]).all()
+    assert torch.equal(got[:at], clean[:at]) and torch.equal(got[lengths[0]:], clean[lengths[0]:])
+    # an infinity may meet another (and be NaN) a sum earlier or later: a head's norm then makes zeros of its other columns, or NaN
+    assert torch.equal(torch.isfinite(got).all(-1), torch.isfinite(want).all(-1))
+    assert torch.equal(torch.isfinite(state), torch.isfinite(want_state))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps", [(4, 2, 16, 24, 4), (1, 1, 100, 5, 1), (3, 3, 64, 64, 3), (2, 1, 200, 40, 8), (8, 2, 128, 128, 4),
                                                          (2, 1, 32, 8, 2), (1, 1, 256, 16, 3), (2, 2, 96, 20, 4), (1, 1, 512, 12, 2)])

@@ -18,8 +18,9 @@
 //   tile   more rows: bound by the FMA units (2.2 to 2.5 cycles an instruction and scheduler, whatever the order of the
 //          operands) and by the reads from shared memory, which add to them.  256 threads take 16 TM x 16 TN results, each thread TM x TN
 //          of them with two accumulators apiece; pairs of neighbouring k are the packed operands, so both operands stay
-//          in shared memory the way they lie in memory.  Two blocks to an SM: with one of 8 x 8 results a thread, 740 us for
-//          [224, 2560] x [19456, 2560]; with two of 7 x 4 or 7 x 5, 626 us (36 TFLOP/s).  One multiply-add to an instruction: the same.
+//          in shared memory the way they lie in memory.  Two blocks to an SM (7 x 5: only in clusters of four, whose parking place is one tile): with
+//          one of 8 x 8 results a thread, 740 us for [224, 2560] x [19456, 2560]; with 7 x 4 or 7 x 5, 626 us (36 TFLOP/s).  One multiply-add
+//          to an instruction: the same.
 //
 // In both, the blocks of a thread-block cluster take different leaves of the same results where there are too
 // few results to fill the GPU, and add them up through each other's shared memory.
@@ -294,31 +295,21 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const GemmArgs a)
     }
     const float* xs = stages + (step % Shape::STAGES) * Shape::STAGE + tm * Shape::ROW;
     const float* ws = stages + (step % Shape::STAGES) * Shape::STAGE + (Shape::BM + tn) * Shape::ROW;
-    // The rows of W for the next four k are on their way while these are multiplied, where the registers hold both.
-    constexpr int AHEAD = 1;
-    ulonglong2 wv[AHEAD][TN], xv[2];
-#pragma unroll
-    for (int j = 0; j < TN; ++j) wv[0][j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * Shape::ROW);
+    ulonglong2 wv[TN], xv[2];
     xv[0] = *reinterpret_cast<const ulonglong2*>(xs);
 #pragma unroll
     for (int u = 0; u < BK / 4; ++u) {
 #pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        const int next = u * TM + i + 1;
-        if (next < TM * (BK / 4)) xv[next & 1] = *reinterpret_cast<const ulonglong2*>(xs + (next % TM) * 16 * Shape::ROW + 4 * (next / TM));
-        if (AHEAD == 2 && u + 1 < BK / 4) {
+      for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * Shape::ROW + 4 * u);
 #pragma unroll
-          for (int j = i * TN / TM; j < (i + 1) * TN / TM; ++j) wv[(u + 1) & 1][j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * Shape::ROW + 4 * (u + 1));
-        }
+      for (int i = 0; i < TM; ++i) {
+        const int next = u * TM + i + 1;   // the row of x after this one is on its way while this one is multiplied
+        if (next < TM * (BK / 4)) xv[next & 1] = *reinterpret_cast<const ulonglong2*>(xs + (next % TM) * 16 * Shape::ROW + 4 * (next / TM));
         const ulonglong2 x4 = xv[(next - 1) & 1];
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], x4.x, wv[u % AHEAD][j].x);   // the chains take turns: no multiply-add waits for the one before it
+        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], x4.x, wv[j].x);   // the chains take turns: no multiply-add waits for the one before it
 #pragma unroll
-        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], x4.y, wv[u % AHEAD][j].y);
-      }
-      if (AHEAD == 1 && u + 1 < BK / 4) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) wv[0][j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * Shape::ROW + 4 * (u + 1));
+        for (int j = 0; j < TN; ++j) fma_pair(acc[i][j], x4.y, wv[j].y);
       }
     }
     if (--until_fold == 0 || step == steps - 1) {
@@ -515,6 +506,7 @@ static int launch_tile(const GemmArgs& a, int batch, bool aligned, int force, cu
       if ((a.M + 16 * candidate->tm - 1) / (16 * candidate->tm) > 65535) continue;
       if (least < 0.0 || cost < least) { least = cost; best = candidate; best_blocks = blocks; }
     }
+  if (least < 0.0) PYLON_REFUSE("gemm_f32: no tile %d for these operands", force);
   return best->entry(a, batch, best_blocks, stream, nullptr);
 }
 
@@ -523,6 +515,7 @@ constexpr int ROWS_MOST = 16;
 static int gemm_f32(const GemmArgs& a, int batch, int force, cudaStream_t stream) {
   const bool aligned = a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && a.batch_x % 4 == 0 && a.batch_w % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
+  if (force < -2) PYLON_REFUSE("gemm_f32: no form %d", force);
   if (force > 0 || (force == 0 && a.M > ROWS_MOST)) return launch_tile(a, batch, aligned, force, stream);
   return aligned ? dispatch_rows<4>(a, batch, force < 0 ? -force : 0, stream) : dispatch_rows<1>(a, batch, force < 0 ? -force : 0, stream);
 }
@@ -550,7 +543,8 @@ extern "C" int pylon_gemm_f32_nt_batched(const float* x, const float* w, float* 
   return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, batch_x, batch_w, batch_y, w_static}, batch, 0, stream);
 }
 
-// For measurements and tests: the kernel for few rows (force = -1) or a tile kernel (100 TM + 10 TN + cluster size; 0: the choice by size).
+// For measurements and tests: the kernel for few rows (force = -1: clusters of eight blocks, -2: lone blocks) or a tile kernel
+// (100 TM + 10 TN + cluster size; 0: the choice by size).  What is not there for the operands is refused.
 extern "C" int pylon_gemm_f32_nt_forced(const float* x, const float* w, float* y, int M, int N, int K, long long ldx,
                                         long long ldw, long long ldy, int force, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;

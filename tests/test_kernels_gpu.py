@@ -114,6 +114,33 @@ def test_gemm_f32_gives_a_row_the_same_bits_in_every_kernel(n, k):
             assert torch.equal(y, full[:m]), (m, form)
 
 
+@pytest.mark.parametrize("m", [1, 2, 4, 8])
+@pytest.mark.parametrize("n, k", [(130, 33), (97, 516), (2560, 4096)])
+def test_gemm_f32_rows_kernel_alone_and_in_clusters(m, n, k):
+    """Every row count's form of the kernel for few rows, its blocks alone and in clusters of eight: the bits of the tile kernel."""
+    from pylon_b200.kernels import ops
+
+    x, w = torch.randn(17, k, device=DEVICE), torch.randn(n, k, device=DEVICE) * 0.05
+    want = ops.linear(x, w)
+    library = ops._library("gemm_f32.cu")
+    for form in (-1, -2):
+        y = torch.full((m, n), float("nan"), device=DEVICE)
+        ops._check(library, library.pylon_gemm_f32_nt_forced(ops._ptr(x), ops._ptr(w), ops._ptr(y), m, n, k, k, k, n, form, ops._stream()))
+        assert torch.equal(y, want[:m]), form
+
+
+@pytest.mark.parametrize("k, form", [(64, 991), (64, 753), (64, 441), (33, 281), (33, 448), (64, -9)])
+def test_gemm_f32_refuses_a_form_that_is_not_there(k, form):
+    from pylon_b200.kernels import ops
+
+    x, w, y = torch.randn(9, k, device=DEVICE), torch.randn(40, k, device=DEVICE), torch.empty(9, 40, device=DEVICE)
+    library = ops._library("gemm_f32.cu")
+    if (k, form) == (33, 448):   # the one tile of rows that 16-byte copies do not reach
+        return ops._check(library, library.pylon_gemm_f32_nt_forced(ops._ptr(x), ops._ptr(w), ops._ptr(y), 9, 40, k, k, k, 40, form, ops._stream()))
+    with pytest.raises(ops.KernelError, match="gemm_f32: no"):
+        ops._check(library, library.pylon_gemm_f32_nt_forced(ops._ptr(x), ops._ptr(w), ops._ptr(y), 9, 40, k, k, k, 40, form, ops._stream()))
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 256, 128), (8, 6144, 2560), (40, 1000, 96), (300, 320, 224)])
 def test_linear_bf16(m, n, k):
     from pylon_b200.kernels import ops

@@ -4,7 +4,7 @@
 // (raun6k/Pylon runs its float32 model through nn.Linear, src/pylon/model/layers.py:17-23,95-106).
 //
 // The order of a sum depends on K alone, so a row's result does not depend on which other rows share
-// the launch, nor on which of the two kernels below computed it.  K is cut into LEAVES leaves of
+// the launch, nor on which of the kernels below computed it.  K is cut into LEAVES leaves of
 // equal length (a multiple of 32).  A leaf is two chains in ascending k, one over its even and one
 // over its odd places, added at its end; four neighbouring leaves are added up in order to a quarter,
 // and the quarters in order to the result.  Short chains also keep the rounding error below that of one
@@ -22,13 +22,18 @@
 //          one of 8 x 8 results a thread, 740 us for [224, 2560] x [19456, 2560]; with 7 x 4 or 7 x 5, 626 us (36 TFLOP/s).  One multiply-add
 //          to an instruction: the same.
 //
-// In both, the blocks of a thread-block cluster take different leaves of the same results where there are too
+//   short  k up to 128 and more than a few rows: a start of microseconds, not the sums, is what is left, and neither a ring of copies nor a
+//          cluster pays.  256 threads take 64 x 64 results a leaf at a time.  12 rows of [6144, 64]: 5.0 us, the
+//          streaming kernel 7.5 alone and 16 in clusters, the tile kernel 6.9.
+//
+// In the first two, the blocks of a thread-block cluster take different leaves of the same results where there are too
 // few results to fill the GPU, and add them up through each other's shared memory.
 //
 // What went before, 64 x 64 results to a block and a chain over the whole of k to each: 354 us for 16 rows and 1,093 us for 224 rows of
 // [19456, 2560], 307 us for 16 rows of [2560, 4096] (now 29).
 #include "common.cuh"
 
+#include <algorithm>
 #include <cooperative_groups.h>
 
 namespace pylon {
@@ -383,6 +388,85 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const GemmArgs a)
 }
 
 // ---------------------------------------------------------------------------------------------
+// short k
+// ---------------------------------------------------------------------------------------------
+// Grid (64 rows of W, 64 rows of x, products), 256 threads of 4 x 4 results.  A stage is a leaf of 32 k, and all of k one quarter; operands are
+// read element by element, whatever their alignment.
+constexpr int SHORT_MOST = 32 * LEAVES_PER_QUARTER;
+__global__ void __launch_bounds__(256) gemm_f32_short_kernel(const GemmArgs a) {
+  constexpr int ROWS = 64, T = 4, LEAF = 32;
+  __shared__ __align__(16) float xs[LEAF][ROWS + 4], ws[LEAF][ROWS + 4];
+  const float* x = a.x + (size_t)blockIdx.z * a.batch_x;
+  const float* w = a.w + (size_t)blockIdx.z * a.batch_w;
+  float* y = a.y + (size_t)blockIdx.z * a.batch_y;
+  const int m0 = blockIdx.y * ROWS, n0 = blockIdx.x * ROWS, tm = (threadIdx.x / 16) * T, tn = (threadIdx.x % 16) * T;
+  const int row = threadIdx.x / 4, column = threadIdx.x % 4;   // what this thread copies: every fourth k of a row of each
+  const bool has_x = m0 + row < a.M, has_w = n0 + row < a.N;
+  x += (size_t)(has_x ? m0 + row : 0) * a.ldx + column;
+  w += (size_t)(has_w ? n0 + row : 0) * a.ldw + column;
+  float total[T][T];
+#pragma unroll
+  for (int i = 0; i < T; ++i)
+#pragma unroll
+    for (int j = 0; j < T; ++j) total[i][j] = 0.f;
+  grid_dependency_wait();
+  allow_dependents();
+  for (int k0 = 0; k0 < a.K; k0 += LEAF) {
+    const int here = a.K - k0 - column;   // from this thread's first k on
+    float xr[LEAF / 4], wr[LEAF / 4];
+#pragma unroll
+    for (int j = 0; j < LEAF / 4; ++j) {
+      xr[j] = has_x && 4 * j < here ? x[k0 + 4 * j] : 0.f;
+      wr[j] = has_w && 4 * j < here ? w[k0 + 4 * j] : 0.f;
+    }
+    if (k0 > 0) __syncthreads();   // the leaf before has been read
+#pragma unroll
+    for (int j = 0; j < LEAF / 4; ++j) {
+      xs[column + 4 * j][row] = xr[j];
+      ws[column + 4 * j][row] = wr[j];
+    }
+    __syncthreads();
+    float even[T][T], odd[T][T];
+#pragma unroll
+    for (int i = 0; i < T; ++i)
+#pragma unroll
+      for (int j = 0; j < T; ++j) even[i][j] = odd[i][j] = 0.f;
+    const int halves = k0 + LEAF / 2 < a.K ? 2 : 1;
+#pragma unroll 1
+    for (int half = 0; half < halves; ++half)
+#pragma unroll
+      for (int k = 0; k < LEAF / 2; ++k) {
+        const float4 x4 = *reinterpret_cast<const float4*>(&xs[half * (LEAF / 2) + k][tm]), w4 = *reinterpret_cast<const float4*>(&ws[half * (LEAF / 2) + k][tn]);
+        const float xv[T] = {x4.x, x4.y, x4.z, x4.w}, wv[T] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+        for (int i = 0; i < T; ++i)
+#pragma unroll
+          for (int j = 0; j < T; ++j) {
+            if (k % 2 == 0) even[i][j] = fmaf(xv[i], wv[j], even[i][j]);
+            else odd[i][j] = fmaf(xv[i], wv[j], odd[i][j]);
+          }
+      }
+#pragma unroll
+    for (int i = 0; i < T; ++i)
+#pragma unroll
+      for (int j = 0; j < T; ++j) total[i][j] = k0 == 0 ? even[i][j] + odd[i][j] : total[i][j] + (even[i][j] + odd[i][j]);
+  }
+  const bool wide = n0 + tn + T <= a.N && a.ldy % 4 == 0 && a.batch_y % 4 == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
+#pragma unroll
+  for (int i = 0; i < T; ++i) {
+    if (m0 + tm + i >= a.M) continue;
+    float* out = y + (size_t)(m0 + tm + i) * a.ldy + n0 + tn;
+    if (wide) {
+      *reinterpret_cast<float4*>(out) = make_float4(total[i][0], total[i][1], total[i][2], total[i][3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < T; ++j)
+        if (n0 + tn + j < a.N) out[j] = total[i][j];
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
 typedef void (*GemmKernel)(const GemmArgs);
@@ -425,7 +509,8 @@ static cudaError_t configure(GemmKernel kernel, KernelState& state, size_t smem)
 // Rows kernel: 16 warps of a cluster (eight blocks of two) take a leaf each, so that 40 slabs (a matrix of 2,560 rows) are 640 warps.
 // From LONE_WORK results in groups of 64 on, four warps of a lone block take a quarter each: no cluster to place and no shared memory to
 // cross, and a warp's ring runs four times as long (16 rows of x, 304 slabs: 79 against 92 us; 2,374 slabs: 399 against 577 us; 96
-// slabs 34 against 36; 40 slabs 50 against 28).  With four rows of x or fewer the loads bound it and more, smaller blocks keep more
+// slabs 34 against 36; 40 slabs 50 against 28).  The same with a short k, of which most of a cluster's warps have nothing (one row of
+// [2560, 64]: 2.9 against 3.9 us; 12 of [9728, 300] 16.6 against 27.8; but one of [512, 128] 3.7 against 3.4).  With four rows of x or fewer the loads bound it and more, smaller blocks keep more
 // of them in flight (one row, 2,374 slabs: 243 against 268 us).
 constexpr long long LONE_WORK = 4096;
 
@@ -436,7 +521,8 @@ static int launch_rows(const GemmArgs& a, int batch, int force, cudaStream_t str
   static KernelState states[MAX_DEVICES];
   KernelState& state = states[current_device_slot()];
   const long long slabs = (a.N + NR * 32 - 1) / (NR * 32);
-  const bool lone = force ? (force & 2) : (a.M > 4 && slabs * batch * a.M >= LONE_WORK);
+  const long long all = slabs * batch;
+  const bool lone = force ? (force & 2) : a.K <= 64 || (a.K < 512 && all >= (a.K <= 256 ? 32 : 64)) || (a.M > 4 && all * a.M >= LONE_WORK);
   const int blocks = lone ? 1 : 8, warps = lone ? 4 : 2, units = blocks * warps;
   const auto bytes = [](int units_, int blocks_, int warps_) {
     return ((size_t)units_ * (MT * NR * 32 / blocks_) + (size_t)warps_ * Ring::STAGES * Ring::STAGE) * sizeof(float);
@@ -473,7 +559,7 @@ static int tile_kernel(const GemmArgs& a, int batch, int blocks, cudaStream_t st
     const long long tiles = tiles_n * tiles_m * batch, at_once = clusters_at_once(kernel, state, blocks, 256, Shape::smem(blocks));
     const long long resident = at_once * blocks > sms ? 2 : 1, full = tiles / at_once, rest = (tiles % at_once) * blocks;   // blocks to an SM; rounds; blocks of the last, partial one
     const long long last = rest == 0 ? 0 : rest > sms * (resident - 1) ? resident : 1;
-    const double k = (double)a.K / blocks / 1000.0, results = TM * TN;
+    const double k = std::min(a.K, leaf_length(a.K) * (LEAVES / blocks)) / 1000.0, results = TM * TN;   // a short k is not shared by all blocks
     *cost = (double)(full * resident + last) * (1.4 * results + 0.78 * (TM + TN) + 5.9) * k + (double)(full + (rest ? 1 : 0)) * (0.31 * results - 2.7) +
             (last == 1 ? 0.25 * results * k : 0.0) + 7.3;
     return 0;
@@ -484,7 +570,8 @@ static int tile_kernel(const GemmArgs& a, int batch, int blocks, cudaStream_t st
 }
 
 // The estimate is a least-squares fit to 580 timed launches (32 to 320 rows of the four matrices of the Qwen3-4B shape, all tiles and
-// cluster sizes): within 6 % of them, and the tile it picks within 2 % of the fastest on average, 10 % at worst.  What it weighs: results
+// cluster sizes): within 6 % of them, and the tile it picks within 2 % of the fastest on average, 10 % at worst.  Over 1,663 other sizes (17 to
+// 2,048 rows, 64 to 32,000 weight rows, k from 16 to 2,561) the tile is 8 % behind the fastest on average.  What it weighs: results
 // and reads per four k, rounds of blocks (a lone block in the last round runs faster than two that share an SM), the sum across blocks.
 typedef int (*TileEntry)(const GemmArgs&, int, int, cudaStream_t, double*);
 
@@ -512,11 +599,30 @@ static int launch_tile(const GemmArgs& a, int batch, bool aligned, int force, cu
 
 constexpr int ROWS_MOST = 16;
 
+static int launch_short(const GemmArgs& a, int batch, cudaStream_t stream) {
+  launch_dependent<LAUNCH_GEMM>(gemm_f32_short_kernel, dim3((a.N + 63) / 64, (a.M + 63) / 64, batch), dim3(256), 0, stream, a);
+  PYLON_CHECK_LAUNCH("gemm_f32");
+}
+
 static int gemm_f32(const GemmArgs& a, int batch, int force, cudaStream_t stream) {
   const bool aligned = a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && a.batch_x % 4 == 0 && a.batch_w % 4 == 0 &&
                        (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.w) & 15) == 0;
+  if (force == -4 && a.K <= SHORT_MOST) return launch_short(a, batch, stream);
   if (force < -2) PYLON_REFUSE("gemm_f32: no form %d", force);
-  if (force > 0 || (force == 0 && a.M > ROWS_MOST)) return launch_tile(a, batch, aligned, force, stream);
+  if (force > 0) return launch_tile(a, batch, aligned, force, stream);
+  if (force == 0) {
+    const long long slabs = (long long)((a.N + 63) / 64) * batch;
+    // Few rows stream the weights whatever k is (one row of [6144, 128]: 4.0 us, the short kernel 8.2), up to 8 of them, or 4 where k is so
+    // short or so placed that a lane's copies are more than its sums (5 rows of [512, 32]: 3.7 and 3.1; of [512, 64]: 4.5 and 4.6).
+    const bool few = a.M <= (aligned && a.K > 32 ? 8 : 4);
+    // Short k: always up to 64 (64 rows of [6144, 64] 5.7 us, tile kernel 6.2; 16 of [1000, 64] 4.9 and 5.7); up to 128 where 16-byte copies do not reach
+    // (300 rows of [1000, 65] 6.3 and 6.9) or a grid of few rows is many blocks (64 rows of [2560, 128] level at 9.2, but of [512, 128] 9.2 and 6.7).
+    if (!few && (a.K <= 64 || (a.K <= SHORT_MOST && (!aligned || (a.M <= 64 && slabs >= 64))))) return launch_short(a, batch, stream);
+    // 9 to 16 rows stream the weights where there are enough of them for lone blocks (12 rows of [9728, 256] 14.9 us, tile kernel 18.0) or a long
+    // k over a large matrix (12 of [2560, 2560] 20 and 28); else the tile kernel's clusters end sooner (16 of [1000, 512] 9.1 and 7.3).
+    const bool streams = a.M <= ROWS_MOST && (slabs * a.M >= LONE_WORK || (aligned && a.K < 512 && slabs >= 64) || (a.K >= 512 && slabs * 64 * a.K >= 1 << 20));
+    if (!few && !streams) return launch_tile(a, batch, aligned, 0, stream);
+  }
   return aligned ? dispatch_rows<4>(a, batch, force < 0 ? -force : 0, stream) : dispatch_rows<1>(a, batch, force < 0 ? -force : 0, stream);
 }
 
@@ -548,6 +654,6 @@ extern "C" int pylon_gemm_f32_nt_batched(const float* x, const float* w, float* 
 extern "C" int pylon_gemm_f32_nt_forced(const float* x, const float* w, float* y, int M, int N, int K, long long ldx,
                                         long long ldw, long long ldy, int force, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K <= 0 || ldx < K || ldw < K || ldy < N || (M + 15) / 16 > 65535 || (force < 0 && M > pylon::ROWS_MOST)) PYLON_REFUSE("gemm_f32_forced: M = %d, K = %d", M, K);
+  if (K <= 0 || ldx < K || ldw < K || ldy < N || (M + 15) / 16 > 65535 || (force < 0 && force != -4 && M > pylon::ROWS_MOST)) PYLON_REFUSE("gemm_f32_forced: M = %d, K = %d", M, K);
   return pylon::gemm_f32({x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0, 0}, 1, force, stream);
 }

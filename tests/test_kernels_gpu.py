@@ -129,6 +129,35 @@ def test_gemm_f32_rows_kernel_alone_and_in_clusters(m, n, k):
         assert torch.equal(y, want[:m]), form
 
 
+@pytest.mark.parametrize("m", [1, 5, 9, 17, 64, 65, 130])
+@pytest.mark.parametrize("k", [1, 15, 16, 17, 31, 32, 33, 48, 64, 65, 96, 100, 127, 128, 129])
+def test_gemm_f32_of_a_short_k(m, k):
+    """Around the edges of the kernel for a short k (stages of 16 and 32, all of k one quarter): the bits of the tile kernel, and its rows and
+    columns alone; as one product and as one of three with strides of their own."""
+    from pylon_b200.kernels import ops
+
+    n = 70
+    x, w = torch.randn(m, 3, k + 3, device=DEVICE)[:, :, :k], torch.randn(3, n, k, device=DEVICE)
+    library = ops._library("gemm_f32.cu")
+
+    def forced(form):
+        y = torch.full((m, n), float("nan"), device=DEVICE)
+        ops._check(library, library.pylon_gemm_f32_nt_forced(ops._ptr(x), ops._ptr(w), ops._ptr(y), m, n, k, x.stride(0), k, n, form, ops._stream()))
+        return y
+
+    aligned = k % 4 == 0 and (3 * (k + 3)) % 4 == 0
+    want = forced(281 if aligned else 441)
+    expected = x[:, 0].double() @ w[0].double().T
+    # at most 4 leaves of two chains of 16 products: a few half ulps each
+    torch.testing.assert_close(want.double(), expected, rtol=1e-5, atol=16 * 2.0**-24 * k**0.5)
+    if k <= 128:
+        assert torch.equal(forced(-4), want)
+    assert torch.equal(ops.linear(x[:, 0], w[0]), want)
+    heads = ops.linear_heads(x, w)
+    for h in range(3):
+        assert torch.equal(heads[:, h], ops.linear(x[:, h].contiguous(), w[h])), h
+
+
 @pytest.mark.parametrize("k, form", [(64, 991), (64, 753), (64, 441), (33, 281), (33, 448), (64, -9)])
 def test_gemm_f32_refuses_a_form_that_is_not_there(k, form):
     from pylon_b200.kernels import ops

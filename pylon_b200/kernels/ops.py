@@ -699,7 +699,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     _need(x.dtype == torch.bfloat16, f"linear: unsupported dtype {x.dtype}")
     _need(out_dtype in (torch.bfloat16, torch.float32), f"linear: unsupported result dtype {out_dtype}")
     aligned = k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-    if (out_dtype == torch.float32 and 0 < m <= STREAM_MAX_ROWS and aligned and k >= (2_560 if m <= SKINNY_MAX_ROWS else 1_024)
+    apart = x.stride(0) >= k and w.stride(0) >= k   # rows that share memory are the library's; the kernels of few rows refuse them
+    if (out_dtype == torch.float32 and 0 < m <= STREAM_MAX_ROWS and aligned and (apart or m <= SKINNY_MAX_ROWS) and k >= (2_560 if m <= SKINNY_MAX_ROWS else 1_024)
             and 6 * _multiprocessors(x.device) <= -(-n // 64) <= 1 << 15):
         # the head: the TMA-fed kernel over the whole of k, once its blocks (three to an SM) go round twice.  One row of [151936, 2560]: 109 us
         # against 118 of the kernel below; 16 rows of [151936, 5120]: 224, the library 258; 32 of [151936, 2560]: 126 and 133; but 16 of

@@ -201,6 +201,26 @@ def test_linear_of_many_weight_rows(m, n, k, out_dtype):
     assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
 
 
+@pytest.mark.parametrize("m", [8, 9, 32, 33])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_linear_of_rows_that_overlap(m, out_dtype):
+    """Rows of x or w that share memory (one row for all, windows over one vector) where the library takes them keep going there."""
+    from pylon_b200.kernels import ops
+
+    n, k = 57_001, 1_024
+    w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
+    long = torch.randn(n * 8 + k, device=DEVICE).to(torch.bfloat16)
+    pairs = [(torch.randn(1, k, device=DEVICE).to(torch.bfloat16).expand(m, k), w), (long.as_strided((m, k), (8, 1)), w),
+             (torch.randn(m, k, device=DEVICE).to(torch.bfloat16), (long * k**-0.5).as_strided((n, k), (8, 1)))]
+    for x, weights in pairs:
+        if m <= ops.SKINNY_MAX_ROWS or (m <= ops.STREAM_MAX_ROWS and out_dtype == torch.bfloat16):
+            with pytest.raises(ops.KernelError, match="shorter than its row"):   # the kernels of few rows refuse them
+                ops.linear(x, weights, out_dtype=out_dtype)
+        else:
+            want = x.double() @ weights.double().T
+            torch.testing.assert_close(ops.linear(x, weights, out_dtype=out_dtype).double(), want, rtol=2e-2, atol=2e-2)
+
+
 PRODUCTS_OF_ANY_MATRIX = {   # name: dtype, rows of x, [N, K] of the second operand, the product under test
     "float32 rows": (torch.float32, 5, (4_096, 2_048), lambda ops, x, w: ops.linear(x, w)),
     "float32 tiles": (torch.float32, 70, (4_096, 2_048), lambda ops, x, w: ops.linear(x, w)),

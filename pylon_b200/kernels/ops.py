@@ -709,9 +709,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
         return linear_stream_partial(x, w, 1, static_weights)[0]
     if m <= SKINNY_MAX_ROWS and aligned:
         # few rows (decode): our weight-streaming kernels.  A bfloat16 result of many weight rows goes to the TMA-fed one, whose blocks of 64
-        # rows then fill the device by themselves ([8192, 4096] 17.4 against 14.5 us, [16384, 2048] 13.8 against 12.2; but [6144, 4096] 10.2
-        # against 12.1, [12352, 2048] 10.1 against 10.4).
-        if out_dtype == torch.bfloat16 and 0 < m and (n >= 16_384 or (n >= 8_192 and k >= 4_096)) and k >= 1_024 and n <= 1 << 21:
+        # rows then fill the device by themselves ([8192, 4096] 17.4 against 14.5 us, eight rows of [16384, 2560] 13.7 against 10.6; but
+        # [6144, 4096] 10.2 against 12.1), from the k on at which its sums are as near to 64-bit ones as the other's (2.3e-7 at any k; the
+        # other's 1.3e-7 at k = 1,024, 2.3e-7 at 2,048 and 2.9e-7 at 2,560).
+        if out_dtype == torch.bfloat16 and 0 < m and (n >= 16_384 or (n >= 8_192 and k >= 4_096)) and k >= 2_560 and n <= 1 << 21:
             return linear_stream(x, w, static_weights=static_weights)
         return linear_skinny(x, w, out_dtype, static_weights)
     if out_dtype == torch.bfloat16:

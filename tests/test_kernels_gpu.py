@@ -221,6 +221,25 @@ def test_linear_of_rows_that_overlap(m, out_dtype):
             torch.testing.assert_close(ops.linear(x, weights, out_dtype=out_dtype).double(), want, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("k", [1_024, 2_048, 2_552, 2_560, 4_096])
+@pytest.mark.parametrize("m", [1, 8])
+def test_few_rows_of_many_weight_rows_keep_their_error(m, k):
+    """Whichever kernel :func:`linear` takes, the 32-bit sums behind its bfloat16 results are no further from 64-bit ones than the weight-streaming
+    kernel's.  (The sums are seen in the roundings: a sum that lies near the middle between two bfloat16 numbers rounds to the wrong one.)"""
+    from pylon_b200.kernels import ops
+
+    n = 16_384
+    x, w = torch.randn(m, k, device=DEVICE).to(torch.bfloat16), torch.randn(n, k, device=DEVICE).to(torch.bfloat16)
+    sums = {kernel: (kernel(x, w, torch.float32) if kernel is ops.linear_skinny else kernel(x, w, 1)[0]) for kernel in (ops.linear_skinny, ops.linear_stream_partial)}
+    expected = x.double() @ w.double().T
+    error = {kernel: float((value.double() - expected).norm()) for kernel, value in sums.items()}
+    rounded = {kernel: value.to(torch.bfloat16) for kernel, value in sums.items()}
+    assert not torch.equal(*rounded.values())   # so that the results tell which kernel ran
+    got = ops.linear(x, w)
+    taken = [kernel for kernel, value in rounded.items() if torch.equal(got, value)]
+    assert len(taken) == 1 and error[taken[0]] <= 1.02 * error[ops.linear_skinny]
+
+
 PRODUCTS_OF_ANY_MATRIX = {   # name: dtype, rows of x, [N, K] of the second operand, the product under test
     "float32 rows": (torch.float32, 5, (4_096, 2_048), lambda ops, x, w: ops.linear(x, w)),
     "float32 tiles": (torch.float32, 70, (4_096, 2_048), lambda ops, x, w: ops.linear(x, w)),

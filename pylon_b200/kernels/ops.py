@@ -700,12 +700,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     _need(out_dtype in (torch.bfloat16, torch.float32), f"linear: unsupported result dtype {out_dtype}")
     aligned = k % 8 == 0 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
     apart = x.stride(0) >= k and w.stride(0) >= k   # rows that share memory are the library's; the kernels of few rows refuse them
-    if (out_dtype == torch.float32 and 0 < m <= STREAM_MAX_ROWS and aligned and (apart or m <= SKINNY_MAX_ROWS) and k >= (2_560 if m <= SKINNY_MAX_ROWS else 1_024)
-            and 6 * _multiprocessors(x.device) <= -(-n // 64) <= 1 << 15):
-        # the head: the TMA-fed kernel over the whole of k, once its blocks (three to an SM) go round twice.  One row of [151936, 2560]: 109 us
-        # against 118 of the kernel below; 16 rows of [151936, 5120]: 224, the library 258; 32 of [151936, 2560]: 126 and 133; but 16 of
-        # [32768, 4096]: 52 and 47.  Its error against 64-bit sums is 2.4e-7 at any k, the kernel below's 1.3e-7 at k = 1,024, 2.9e-7 at 2,560 and
-        # 4.7e-7 at 4,096 (whence the line for the rows that one takes), the library's 4.4e-6 at 4,096.
+    if out_dtype == torch.float32 and aligned and _head_streams(m, n, k, _multiprocessors(x.device)) and (apart or m <= SKINNY_MAX_ROWS):
         return linear_stream_partial(x, w, 1, static_weights)[0]
     if m <= SKINNY_MAX_ROWS and aligned:
         # few rows (decode): our weight-streaming kernels.  A bfloat16 result of many weight rows goes to the TMA-fed one, whose blocks of 64
@@ -722,6 +717,23 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
             return linear_tcgen05(x, w, static_weights=static_weights)
         return torch.mm(x, w.t())
     return torch.mm(x, w.t(), out_dtype=torch.float32)
+
+
+def _head_streams(m: int, n: int, k: int, sms: int) -> bool:
+    """Whether float32 results of few rows and very many weight rows (the head) go to the TMA-fed kernel over the whole of k.
+
+    Up to 8 rows once its blocks (64 weight rows, three to an SM) go round twice and its sums are as near to 64-bit ones as the weight-streaming
+    kernel's (2.4e-7 at any k; the other's 1.3e-7 at k = 1,024, 2.9e-7 at 2,560, 4.7e-7 at 4,096): one row of [151936, 2560] 111 us, the other 118; of
+    [60000, 4096] 78 and 84.  9 to 32 rows go there instead of the library where the library's 128-row tiles leave a tenth or more of their rounds over the
+    SMs empty: 16 rows of [151936, 2560] 117 us, the library 130; 32 of [100352, 4096] 132 and 141; but 16 of [128256, 4096] 157 and 158, 32 165
+    and 162; and below some 76,000 rows the library has tiles of other sizes (16 rows of [65536, 4096] 86 and 82 us, of [57344, 1024] 22.3 and 20.8).
+    (Errors there: the library 1e-6 at k = 1,024, 4.4e-6 at 4,096.)"""
+    if not (0 < m <= STREAM_MAX_ROWS and -(-n // 64) <= 1 << 15):
+        return False
+    if m <= SKINNY_MAX_ROWS:
+        return k >= 2_560 and -(-n // 64) >= 6 * sms
+    tiles = -(-n // 128)
+    return k >= (1_024 if m <= 16 else 2_048) and tiles >= 4 * sms and tiles <= 0.9 * -(-tiles // sms) * sms
 
 
 def linear_stacked(x: torch.Tensor, w: torch.Tensor, static_weights: bool = False) -> torch.Tensor:

@@ -186,7 +186,9 @@ def test_linear_bf16(m, n, k):
 @pytest.mark.parametrize("m, n, k, out_dtype", [(1, 16_384, 1_024, torch.bfloat16), (8, 16_397, 1_032, torch.bfloat16), (5, 8_192, 4_096, torch.bfloat16),
                                                 (8, 8_191, 4_096, torch.bfloat16), (9, 57_001, 1_024, torch.float32), (32, 60_000, 1_160, torch.float32),
                                                 (8, 57_001, 1_024, torch.float32), (33, 57_001, 1_024, torch.float32),
-                                                (1, 57_001, 2_560, torch.float32), (8, 56_832, 2_568, torch.float32)])
+                                                (1, 57_001, 2_560, torch.float32), (8, 56_832, 2_568, torch.float32),
+                                                (9, 80_001, 1_024, torch.float32), (17, 80_001, 1_024, torch.float32), (32, 80_001, 2_056, torch.float32),
+                                                (16, 75_777, 2_048, torch.float32), (16, 85_248, 1_032, torch.float32)])
 def test_linear_of_many_weight_rows(m, n, k, out_dtype):
     """Either side of the lines behind which few rows go to the TMA-fed kernel."""
     from pylon_b200.kernels import ops
@@ -207,7 +209,7 @@ def test_linear_of_rows_that_overlap(m, out_dtype):
     """Rows of x or w that share memory (one row for all, windows over one vector) where the library takes them keep going there."""
     from pylon_b200.kernels import ops
 
-    n, k = 57_001, 1_024
+    n, k = 80_001, 2_048
     w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
     long = torch.randn(n * 8 + k, device=DEVICE).to(torch.bfloat16)
     pairs = [(torch.randn(1, k, device=DEVICE).to(torch.bfloat16).expand(m, k), w), (long.as_strided((m, k), (8, 1)), w),
@@ -246,7 +248,7 @@ PRODUCTS_OF_ANY_MATRIX = {   # name: dtype, rows of x, [N, K] of the second oper
     "float32 heads": (torch.float32, 5, (4_096, 2_048), lambda ops, x, w: ops.linear_heads(x.view(5, 8, 256), w.view(8, 2_048 * 2, 256))),
     "skinny": (torch.bfloat16, 8, (8_192, 2_048), lambda ops, x, w: ops.linear(x, w)),
     "stream": (torch.bfloat16, 16, (16_384, 2_048), lambda ops, x, w: ops.linear(x, w)),
-    "head": (torch.bfloat16, 16, (57_344, 1_024), lambda ops, x, w: ops.linear(x, w, out_dtype=torch.float32)),
+    "head": (torch.bfloat16, 16, (80_000, 1_024), lambda ops, x, w: ops.linear(x, w, out_dtype=torch.float32)),
     "parts": (torch.bfloat16, 4, (2_560, 4_096), lambda ops, x, w: ops.linear_for_residual(x, w)),
     "gated, few rows": (torch.bfloat16, 4, (19_456, 2_560), lambda ops, x, w: ops.linear_swiglu(x, w)),
     "gated, both row tiles": (torch.bfloat16, 160, (19_456, 2_560), lambda ops, x, w: ops.linear_swiglu(x, w)),

@@ -606,12 +606,15 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out
   }
 }
 
-// Vector form for float32 rows whose width is a multiple of 4: a thread takes four columns, a block row of the grid a row of the
-// input, so nothing is divided (an element at a time, with a division each, 224 rows of 9,728 took 9.7 us).
-__global__ void swiglu_f32x4_kernel(const float4* gate_up, float4* __restrict__ out, int inter4, int interleaved, float limit, float alpha) {
+// Vector form for float32 rows whose width is a multiple of 4: a thread takes four columns, a row of a block's threads a row of the
+// input, so nothing is divided (an element at a time, with a division each, 224 rows of 9,728 took 9.7 us).  Narrow rows share a block: with one
+// each, 4,096 rows of 36 took 5.0 us where an element at a time takes 2.3.
+__global__ void __launch_bounds__(256) swiglu_f32x4_kernel(const float4* gate_up, float4* __restrict__ out, int rows, int inter4, int interleaved, float limit,
+                                                           float alpha) {
   grid_dependency_wait();
   allow_dependents();
-  const size_t t = blockIdx.y;
+  const size_t t = (size_t)blockIdx.y * blockDim.y + threadIdx.y;
+  if (t >= rows) return;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < inter4; c += gridDim.x * blockDim.x) {
     const int gate_column = interleaved ? (c >> 1) * 4 + (c & 1) : c;
     const float4 g = gate_up[t * 2 * inter4 + gate_column], u = gate_up[t * 2 * inter4 + (interleaved ? gate_column + 2 : inter4 + c)];
@@ -1008,9 +1011,12 @@ extern "C" int pylon_swiglu(const void* gate_up, void* out, int num_tokens, int 
     launch_dependent(swiglu_bf16x8_kernel, dim3(grid(total / 8)), dim3(threads), 0, stream, (const uint4*)gate_up, (uint4*)out, inter / 8, total / 8, interleaved, limit, alpha);
   } else if (dtype == PYLON_DTYPE_BF16) {
     swiglu_kernel<__nv_bfloat16><<<grid(total), threads, 0, stream>>>((const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, inter, total, interleaved, limit, alpha);
-  } else if (dtype == PYLON_DTYPE_F32 && inter % 4 == 0 && total / inter <= 65535 && ((uintptr_t)gate_up % 16 == 0) && ((uintptr_t)out % 16 == 0)) {
-    launch_dependent(swiglu_f32x4_kernel, dim3((inter / 4 + threads - 1) / threads, (unsigned)(total / inter)), dim3(threads), 0, stream,
-                     (const float4*)gate_up, (float4*)out, inter / 4, interleaved, limit, alpha);
+  } else if (dtype == PYLON_DTYPE_F32 && inter % 4 == 0 && num_tokens <= 65535 && ((uintptr_t)gate_up % 16 == 0) && ((uintptr_t)out % 16 == 0)) {
+    int across = 8;   // threads to a row
+    while (across < threads && across < inter / 4) across *= 2;
+    const int down = threads / across;
+    launch_dependent(swiglu_f32x4_kernel, dim3((inter / 4 + across - 1) / across, (num_tokens + down - 1) / down), dim3(across, down), 0, stream,
+                     (const float4*)gate_up, (float4*)out, num_tokens, inter / 4, interleaved, limit, alpha);
   } else if (dtype == PYLON_DTYPE_F32) {
     swiglu_kernel<float><<<grid(total), threads, 0, stream>>>((const float*)gate_up, (float*)out, inter, total, interleaved, limit, alpha);
   } else {

@@ -75,6 +75,25 @@ def test_swiglu(dtype, tokens, inter):
     torch.testing.assert_close(out.double(), g * torch.sigmoid(g) * u, **tolerance(dtype))
 
 
+@pytest.mark.parametrize("tokens, inter", [(1, 4), (33, 8), (31, 28), (65, 36), (9, 128), (7, 1024), (5, 1032), (65_535, 8), (65_536, 8)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_float32_swiglu_of_rows_that_share_a_block(tokens, inter, interleaved):
+    """Widths around the powers of two of threads to a row, and counts of rows that a block's last rows do not have: the bits of rows one by one."""
+    from pylon_b200.kernels import ops
+
+    if interleaved and inter % 8:
+        return
+    gate_up = torch.randn(tokens, 2 * inter, device=DEVICE) * 2
+    out = torch.full((tokens + 1, inter), float("nan"), device=DEVICE)
+    ops.swiglu(gate_up, out[:tokens], interleaved=interleaved)
+    halves = gate_up.view(tokens, inter // 8, 2, 8).transpose(1, 2).reshape(tokens, 2 * inter) if interleaved else gate_up
+    g, u = halves[:, :inter].double(), halves[:, inter:].double()
+    torch.testing.assert_close(out[:tokens].double(), g * torch.sigmoid(g) * u, rtol=1e-6, atol=1e-6)
+    assert torch.isnan(out[tokens]).all()
+    for t in (0, tokens // 2, tokens - 1):
+        assert torch.equal(ops.swiglu(gate_up[t : t + 1].clone(), interleaved=interleaved)[0], out[t])
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 300, 77), (5, 64, 64), (70, 130, 2560), (129, 1000, 33), (3, 151_936 // 8, 96)])
 def test_gemm_f32_is_true_32_bit(m, n, k):
     from pylon_b200.kernels import ops

@@ -582,8 +582,8 @@ static int forced_columns = 0;
 
 }  // namespace pylon
 
-// For measurements: every later product uses tiles of 128 x columns (288, 256, 192, 160 or 128; 1192 or 1128: both row tiles of a gated product of
-// 129 to 256 rows with tiles of 192 or 128 columns); 0 returns to the choice by size.
+// For measurements: every later product uses tiles of 128 x columns (288, 256, 192, 160 or 128; 1192: both row tiles of a gated product of
+// 129 to 256 rows with tiles of 192 columns); 0 returns to the choice by size.
 extern "C" int pylon_gemm_tcgen05_force_tile(int columns) {
   pylon::forced_columns = columns;
   return 0;
@@ -622,16 +622,15 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
   }
   // 129 to 256 rows are bound by how often the weights' tiles cross from L2: a block takes both row tiles with one tile of B.  Its operands are
   // M + width rows of k a step; with 192 columns the accumulators of both fill tensor memory (one buffer).  Gate and up of the Qwen3-4B shape
-  // for 160 rows: 27 us where two rounds of 128 x 192 tiles took 35 (the bytes alone take 15); [24576, 4096]: 57 against 65.  Not beyond 256
+  // for 160 rows: 28 us where two rounds of 128 x 192 tiles take 34 (the bytes alone take 15); [24576, 4096]: 45 against 56.  Not beyond 256
   // rows: with whole tiles of A and rounds of blocks the two products per tile of B measured slower than two accumulators of 256 columns.
+  // With 128 columns it never paid (160 rows of [16384, 2048] 21.6 us, one row tile with 256 columns 20.0; [34816, 5120] 83 and 77), so the one form is
+  // weighed against the tiles above by rounds: [12288, 2048] is one round of either, 21.4 us and with one row tile of 192 columns 17.0.
   int row_tiles = 1;
-  if (swiglu && !tile_group && M > TC_BM && M <= 2 * TC_BM && (forced_columns == 0 || forced_columns >= 1000))
-    for (int candidate : {192, 128}) {
-      if (forced_columns && candidate != forced_columns - 1000) continue;
-      const long long rounds = ((N + candidate - 1) / candidate + sm_count - 1) / sm_count;
-      const long long cost = rounds * (candidate + M + 85 + (candidate > 128 ? 100 : 0));
-      if (cost < best || forced_columns) { best = cost; bn = candidate; row_tiles = 2; }
-    }
+  if (swiglu && !tile_group && M > TC_BM && M <= 2 * TC_BM && (forced_columns == 0 || forced_columns == 1192)) {
+    const long long rounds = ((N + 191) / 192 + sm_count - 1) / sm_count, cost = rounds * (192 + M + 185);
+    if (cost < best || forced_columns) { bn = 192; row_tiles = 2; }
+  }
   CUtensorMap map_a, map_b;
   if (!make_map(&map_a, x, M, K, ldx, row_tiles == 2 ? (M + 31) & ~31 : TC_BM) || !make_map(&map_b, w, (long long)groups * N, K, ldw, bn > 256 ? bn / 2 : bn))
     PYLON_REFUSE("gemm_tcgen05: the tensor maps could not be made");
@@ -641,8 +640,7 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
     if (swiglu) return launch_tcgen05<BN_, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale); \
     return launch_tcgen05<BN_, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N);                          \
   }
-  if (row_tiles == 2 && bn == 192) return launch_tcgen05<192, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, nullptr, 0, nullptr, w_static);
-  if (row_tiles == 2) return launch_tcgen05<128, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, nullptr, 0, nullptr, w_static);
+  if (row_tiles == 2) return launch_tcgen05<192, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, nullptr, 0, nullptr, w_static);
   PYLON_TC_CASE(256) PYLON_TC_CASE(192)
 #undef PYLON_TC_CASE
   if (bn == 288) return launch_tcgen05<288, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream);

@@ -332,7 +332,14 @@ extern "C" int pylon_paged_attention_simple(const void* q, long long q_token_str
   dim3 grid(num_tokens, nq);
   // float32 rows on 16-byte boundaries: the kernel that shares its reads between the heads of a group (4, 2 or 1 of them).  The rest - odd
   // widths, rows that start in between, more shared memory than a block has without asking - stays with the plain one.
-  const int group = nq / nkv, heads = group % 4 == 0 ? 4 : (group % 2 == 0 ? 2 : 1);
+  // How many heads go together changes no sum, so it may hang on the step: shared reads pay once there are more blocks than the SMs hold at once (32 heads over 8
+  // of 128: 193 tokens 51 us with four, 61 with one), and before that each block's own time counts (one token over 8,000 keys 606 us with one,
+  // 1,137 with four; 16 tokens over 90 keys 10.7 and 14.7).  Wide values (latent rows) always take two: 16 tokens of 16 heads over 500 keys 111, one 132, four 234.
+  const int group = nq / nkv;
+  const long long at_once = 8LL * multiprocessors();
+  int heads = group % 4 == 0 ? 4 : (group % 2 == 0 ? 2 : 1);
+  if (dv > 128 && heads > 2) heads = 2;
+  while (heads > (dv > 128 ? 2 : 1) && (long long)num_tokens * nq * 2 / heads <= at_once) heads /= 2;
   const size_t wide_smem = ((size_t)heads * (d + SIMPLE_THREADS + 4 * dv) + 8) * sizeof(float) + SIMPLE_THREADS * sizeof(long long);
   if (dtype == PYLON_DTYPE_F32 && d % 4 == 0 && dv % 4 == 0 && k_row_stride % 4 == 0 && v_row_stride % 4 == 0 && wide_smem <= 48 * 1024 &&
       (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
@@ -346,7 +353,7 @@ extern "C" int pylon_paged_attention_simple(const void* q, long long q_token_str
     if (dv <= 128) {
       if (heads == 4) launch(paged_attention_f32_kernel<4, 1>); else if (heads == 2) launch(paged_attention_f32_kernel<2, 1>); else launch(paged_attention_f32_kernel<1, 1>);
     } else {
-      if (heads == 4) launch(paged_attention_f32_kernel<4, 4>); else if (heads == 2) launch(paged_attention_f32_kernel<2, 4>); else launch(paged_attention_f32_kernel<1, 4>);
+      if (heads == 2) launch(paged_attention_f32_kernel<2, 4>); else launch(paged_attention_f32_kernel<1, 4>);
     }
   } else if (dtype == PYLON_DTYPE_F32)
     paged_attention_simple_kernel<float><<<grid, SIMPLE_THREADS, smem, stream>>>(

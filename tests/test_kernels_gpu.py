@@ -812,6 +812,26 @@ def test_float32_attention_with_shared_reads(nq, nkv, d, dv, options):
     torch.testing.assert_close(run(cache.k_pages, v_pages), run(shifted(cache.k_pages), shifted(v_pages)), rtol=2e-5, atol=2e-6)
 
 
+@pytest.mark.parametrize("nq, nkv, d, dv", [(16, 2, 64, 64), (8, 4, 36, 20), (16, 1, 68, 256)])
+def test_float32_attention_of_a_token_does_not_depend_on_the_others(nq, nkv, d, dv):
+    """However many heads a block takes - by the number of the step's tokens - a token's result has the same bits."""
+    from pylon_b200.kernels import ops
+
+    tokens, length = 700, 700
+    cache = Paged([length], [tokens], nkv, d, 64, torch.float32)
+    v_pages, q = torch.randn((*cache.k_pages.shape[:3], dv), device=DEVICE), torch.randn(tokens, nq * d, device=DEVICE)
+
+    def run(first, count):
+        starts = torch.tensor([0, count], device=DEVICE, dtype=torch.int32)
+        return ops.paged_attention(q[first : first + count].contiguous(), cache.k_pages, v_pages, cache.positions[first : first + count].contiguous(),
+                                   cache.token_row[:count].contiguous(), starts, torch.tensor([first + count], device=DEVICE, dtype=torch.int32), cache.table, nq, count,
+                                   first + count)
+
+    whole = run(0, tokens)
+    for first, count in ((0, 1), (699, 1), (130, 40), (300, 100), (511, 160)):
+        assert torch.equal(run(first, count), whole[first : first + count]), (first, count)
+
+
 @pytest.mark.parametrize("d, nq, nkv", [(128, 32, 8), (64, 12, 4)])
 def test_tcgen05_attention_gives_the_same_bits_every_time(d, nq, nkv):
     """Eight prompt portions of some 500 tokens: several waves of blocks, each with eight key tiles and more in flight.  A

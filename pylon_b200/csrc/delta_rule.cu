@@ -835,8 +835,10 @@ static int launch_delta(const void* proj_v, long long ld, const float* conv_w, i
   const long long conv_offset = (long long)heads * dim * vdim;
   bool prepared = false;
   if constexpr (sizeof(T) == 2) {   // in float32 mode the order of a norm's sum must not depend on how many tokens a step has
-    // short rows: every token would go through its slot's inputs, eight to a warp one behind the other (16 rows of 4 tokens: 5 us slower)
-    if (!channel && taps <= 4 && dim % 4 == 0 && vdim % 4 == 0 && dim <= 128 && vdim <= 128 && ld % 4 == 0 && slot_floats % 4 == 0 && num_tokens >= 64 &&
+    // Not for short rows, whose tokens would all go through their slot's inputs, eight to a warp one behind the other (16 rows of 4 tokens: 5 us slower),
+    // nor where a token a warp finds all its warps a place: level at some 7,000 units of a token (16 heads over 8: 128 tokens 1 us slower, 300 3 us
+    // faster; four heads of 64: 100 tokens 6 us slower, 1,024 2 us faster).
+    if (!channel && taps <= 4 && dim % 4 == 0 && vdim % 4 == 0 && dim <= 128 && vdim <= 128 && ld % 4 == 0 && slot_floats % 4 == 0 && (long long)num_tokens * (2 * kv_heads + heads + 1) >= 7000 &&
         num_tokens >= 16LL * num_rows && (((uintptr_t)conv_w | (uintptr_t)state | (uintptr_t)qkv) & 15) == 0 && (uintptr_t)proj % 8 == 0) {
       constexpr int TOKENS = 8;
       const long long items = (long long)((num_tokens + TOKENS - 1) / TOKENS) * (2 * kv_heads + heads + 1);

@@ -1433,11 +1433,11 @@ def streams_update_norm(
 # ---------------------------------------------------------------------------------------
 def delta_rule_in_chunks(dtype: torch.dtype, dim: int, vdim: int, tokens: int, num_rows: int, slot_floats: int, channel_decay: bool) -> bool:
     """Whether :func:`gated_delta_rule` walks a step's rows 16 tokens at a time: prompt portions of bfloat16 models with heads of 128 keys.
-    A chunk costs what seven tokens one by one do, full or not, and its matrices are a kernel of their own: 16 heads of 128 x 128, 266 against
-    577 us for one row of 2,048 tokens (the whole call), 57 against 98 for 300, level at one row of 64 or two of 32, 33 against 28
-    for four of 16.  Not in float32 mode: there a sum's order depends on the token's position only, and chunks start where a portion does."""
+    A chunk costs what seven tokens one by one do, full or not, and its matrices are a kernel of their own: 16 heads of 128 x 128, 267 against
+    577 us for one row of 2,048 tokens (the whole call), 58 against 98 for 300, 26 against 30 for one of 64, level at four rows of 64 (47 and 46), 41 against
+    39 for four of 48.  Not in float32 mode: there a sum's order depends on the token's position only, and chunks start where a portion does."""
     return (dtype == torch.bfloat16 and dim == 128 and vdim % 16 == 0 and slot_floats % 4 == 0 and not channel_decay
-            and tokens >= 64 and tokens >= 48 * num_rows)
+            and tokens >= 64 * max(1, num_rows))
 
 
 def gated_delta_rule(

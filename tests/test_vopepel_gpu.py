@@ -429,7 +429,7 @@ def test_gated_delta_rule_in_chunks_is_causal_for_values_that_are_not_finite(wha
     same tokens, heads and state entries as when the rows are walked token by token."""
     from pylon_b200.kernels import ops
 
-    heads, kv_heads, dim, vdim, eps, lengths = 4, 2, 128, 32, 1e-5, (75, 50, 48)
+    heads, kv_heads, dim, vdim, eps, lengths = 4, 2, 128, 32, 1e-5, (95, 50, 48)
     tokens, channels = sum(lengths), 2 * kv_heads * dim + heads * vdim
     proj, conv, a_log, dt_bias, norm = (t.to(DEVICE) for t in delta_inputs(tokens, heads, kv_heads, dim, vdim, 2, 9, torch.bfloat16))
     floats = heads * dim * vdim + channels

@@ -297,7 +297,8 @@ extern "C" int pylon_streams_update_norm(float* x, const void* delta, int delta_
   const size_t smem = (size_t)(width + 34 + streams * streams + 2 * streams) * sizeof(float);
   const long long part_stride = (long long)tokens * width;
   const bool vector = width % 4 == 0 && ((uintptr_t)x % 16 == 0) && (!delta || (uintptr_t)delta % 16 == 0) && (!out || (uintptr_t)out % 16 == 0);
-  // Several streams over more rows than the SMs hold at once, of a width that 256 threads divide: the kernel that knows its sizes.
+  // Two or four streams of 1,024, 2,048 or 4,096 over more rows than the SMs hold at once: the kernel that knows its sizes, compiled for each of the
+  // six pairs.  Other counts and widths keep the kernel that takes any.
   if (vector && delta && delta_parts == 1 && out && !rows && n_rows > 256 && out_dtype == PYLON_DTYPE_BF16 && kind != 2 && (uintptr_t)weight % 16 == 0) {
     const bool launched = delta_dtype == PYLON_DTYPE_F32
         ? launch_streams_rows<float>(x, delta, scale, mix, outw, read, weight, out, n_rows, streams, width, eps, kind, stream)

@@ -343,11 +343,13 @@ def test_streams_update_and_norm_of_a_prompt_portion(streams, width, kind, delta
     routes = [torch.randn(streams, streams, device=DEVICE), torch.randn(streams, device=DEVICE), torch.randn(streams, device=DEVICE)]
     weight = 1 + 0.2 * torch.randn(width, device=DEVICE)
     for mix, out_w, read in (routes, (None, None, None)):
-        whole, first = x.clone(), x[:256].clone()
+        whole = x.clone()
         got = ops.streams_update_norm(whole, delta, 0.6, mix, out_w, read, weight, 1e-5, kind, torch.bfloat16)
-        want = ops.streams_update_norm(first, delta[..., :256, :].contiguous(), 0.6, mix, out_w, read, weight, 1e-5, kind, torch.bfloat16)
-        torch.testing.assert_close(whole[:256], first, rtol=1e-6, atol=1e-6)
-        torch.testing.assert_close(got[:256].float(), want.float(), rtol=1e-2, atol=1e-3)   # the statistics in another order: now and then the next bfloat16
+        for rows in (slice(0, 256), slice(1, 257)):   # between them all rows, the last one too
+            part = x[rows].clone()
+            want = ops.streams_update_norm(part, delta[..., rows, :].contiguous(), 0.6, mix, out_w, read, weight, 1e-5, kind, torch.bfloat16)
+            torch.testing.assert_close(whole[rows], part, rtol=1e-6, atol=1e-6)
+            torch.testing.assert_close(got[rows].float(), want.float(), rtol=1e-2, atol=1e-3)   # the statistics in another order: now and then the next bfloat16
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -420,6 +422,36 @@ def test_gated_delta_rule_in_chunks(heads, kv_heads, vdim, taps, lengths, decay,
     # the same 32-bit sums in another order; the state is a sum of at most 160 terms of size one
     torch.testing.assert_close(state, want_state, rtol=1e-4, atol=2e-5)
     torch.testing.assert_close(out, want, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(8, 8, 64, 32), (16, 4, 100, 20), (8, 8, 128, 48)])
+def test_gated_delta_rule_of_prompt_portions_behind_others(heads, kv_heads, dim, vdim, taps):
+    """Rows that go on from their slots' convolution inputs and states in a step large enough for the preparation of eight tokens a warp: rows that begin inside
+    such a group, a row of one token, a first portion shorter than the taps.  Against the plain statement of the whole sequences."""
+    from pylon_b200.kernels import ops
+
+    eps, first, rest = 1e-5, (5, 2, 1, 9), (1, 97, 30, 160)
+    channels = 2 * kv_heads * dim + heads * vdim
+    floats = (heads * dim * vdim + (taps - 1) * channels + 3) // 4 * 4
+    inputs = [delta_inputs(a + b, heads, kv_heads, dim, vdim, taps, 90 + i, torch.bfloat16)[0] for i, (a, b) in enumerate(zip(first, rest))]
+    _, conv, a_log, dt_bias, norm = delta_inputs(1, heads, kv_heads, dim, vdim, taps, 90, torch.bfloat16)
+    want = [plain_delta_from_projections(p, conv, a_log, dt_bias, norm, heads, kv_heads, dim, vdim, eps) for p in inputs]
+    on = lambda t: t.to(DEVICE)
+    slots = torch.tensor([2, 4, 0, 3], dtype=torch.int32, device=DEVICE)
+    state = torch.zeros(5, floats, device=DEVICE)
+
+    def run(pieces):
+        step = step_view([p.shape[0] for p in pieces], [0] * len(pieces), torch.bfloat16)
+        out = ops.gated_delta_rule(on(torch.cat(pieces)), on(conv.t().contiguous()), state, step.token_row, step.q_start, slots, on(a_log), on(dt_bias), on(norm), heads,
+                                   kv_heads, dim, vdim, len(pieces), eps)
+        return torch.split(out.double().cpu(), [p.shape[0] for p in pieces])
+
+    assert sum(first) * (2 * kv_heads + heads + 1) < 7_000 <= sum(rest) * (2 * kv_heads + heads + 1) and sum(rest) >= 16 * len(rest)   # the two preparation kernels
+    begun = run([p[:n] for p, n in zip(inputs, first)])
+    ended = run([p[n:] for p, n in zip(inputs, first)])
+    for a, b, expected in zip(begun, ended, want):
+        torch.testing.assert_close(torch.cat([a, b]), expected, rtol=3e-2, atol=3e-2)
 
 
 @pytest.mark.parametrize("what", ["value", "infinite value", "key", "query", "decay", "beta"])

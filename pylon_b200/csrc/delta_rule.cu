@@ -556,19 +556,28 @@ __global__ void __launch_bounds__(128) delta_chunk_matrices_kernel(const float* 
   __syncthreads();
   {
     const int t = tid >> 3, i0 = (tid & 7) * 2;
-    float sums[4] = {0.f, 0.f, 0.f, 0.f};   // k_t . k_i, q_t . k_i for i = i0, i0 + 1
+    // k_t . k_i, q_t . k_i for i = i0, i0 + 1, four chains of DIM / 4 each: with one of DIM the states of keys that are much alike were 2.6e-7
+    // from 64-bit ones, where token by token they are 1.5e-7.
+    float4 sums[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) sums[n] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
     for (int e = 0; e < DIM; e += 4) {
       const float4 kt = *reinterpret_cast<const float4*>(ks + t * ROW + e), qt = *reinterpret_cast<const float4*>(qs + t * ROW + e);
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const float4 ki = *reinterpret_cast<const float4*>(ks + (i0 + n) * ROW + e);
-        sums[n] = fmaf(kt.x, ki.x, fmaf(kt.y, ki.y, fmaf(kt.z, ki.z, fmaf(kt.w, ki.w, sums[n]))));
-        sums[2 + n] = fmaf(qt.x, ki.x, fmaf(qt.y, ki.y, fmaf(qt.z, ki.z, fmaf(qt.w, ki.w, sums[2 + n]))));
+        sums[n].x = fmaf(kt.x, ki.x, sums[n].x); sums[n].y = fmaf(kt.y, ki.y, sums[n].y);
+        sums[n].z = fmaf(kt.z, ki.z, sums[n].z); sums[n].w = fmaf(kt.w, ki.w, sums[n].w);
+        sums[2 + n].x = fmaf(qt.x, ki.x, sums[2 + n].x); sums[2 + n].y = fmaf(qt.y, ki.y, sums[2 + n].y);
+        sums[2 + n].z = fmaf(qt.z, ki.z, sums[2 + n].z); sums[2 + n].w = fmaf(qt.w, ki.w, sums[2 + n].w);
       }
     }
-    kk[t][i0] = sums[0]; kk[t][i0 + 1] = sums[1];
-    qk[t][i0] = sums[2]; qk[t][i0 + 1] = sums[3];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      kk[t][i0 + n] = (sums[n].x + sums[n].y) + (sums[n].z + sums[n].w);
+      qk[t][i0 + n] = (sums[2 + n].x + sums[2 + n].y) + (sums[2 + n].z + sums[2 + n].w);
+    }
   }
   const int group = heads / kv_heads;
   for (int h = kv * group; h < (kv + 1) * group; ++h) {

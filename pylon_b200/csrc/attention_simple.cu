@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(SIMPLE_THREADS) paged_attention_simple_kernel(
 // lanes (16 keys of the chunk at a time, float4 after float4 of the row); a warp per head turns the scores into weights; the four warps
 // take every fourth value row, whose columns lie across the lanes (NC float4 to a lane), and their sums meet in shared memory.  The order
 // of every sum is again a function of the token's position.  193 tokens of 32 heads over 8 of size 128: 148 us with the plain
-// kernel, under 31 with this one; 16 tokens over some 90 keys each: 36 and under 8.  What bounds it is the latency of a chunk's three phases at few tokens
+// kernel, under 31 inside a step with this one; 16 tokens over some 90 keys each: 36 and under 8.  What bounds it is the latency of a chunk's three phases at few tokens
 // and the traffic with L2 at many.
 // (Its inputs are not const __restrict__: what the kernel ahead writes must not be read through the non-coherent path, whose loads may be
 // moved ahead of the wait for that kernel.)

@@ -17,16 +17,20 @@
 // [heads, dim, vdim] followed by the last (taps - 1) inputs of the convolution [taps - 1, channels].
 // All of the recurrence is float32: unit norms, decay, beta, the state, the read-out and its norm.
 //
-// Four kernels:
+// The kernels:
 //   delta_prepare       one warp per (token, q/k/v head): convolution + silu (+ unit norm), and per
-//                       token the heads' decay and beta, into float32 buffers
+//                       token the heads' decay and beta, into float32 buffers; delta_prepare_wide is
+//                       the same for large prompt portions in bfloat16, eight tokens a warp
 //   delta_conv_advance  per (row, channel): the slot's convolution inputs move on by the row's tokens
 //   delta_recurrence    per (row, head, slice of vdim): walks the row's tokens in order; the columns
 //                       of S are independent of each other, so a block owns COLS of them, a column's
 //                       dim entries spread over P lanes that add up by shuffles
+//   delta_chunk_matrices, delta_chunk_walk   the walk 16 tokens at a time, for prompt portions of
+//                       bfloat16 models (heads of 128 keys)
 //   delta_gated_norm    one warp per (token, head): RMS norm of the read-out, weight, gate
-// The order of every sum depends on the sizes only, so a token's result does not depend on how the
-// step was cut or what else is in the batch.
+// In float32 the order of every sum depends on the sizes only, so a token's result does not depend on
+// how the step was cut or what else is in the batch.  In bfloat16 a large step's portions take other
+// kernels than a small one's, with the same float32 sums in another order: there results agree to rounding.
 #include "common.cuh"
 
 namespace pylon {

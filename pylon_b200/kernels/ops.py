@@ -667,15 +667,16 @@ def swiglu(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None, interleave
 # ---------------------------------------------------------------------------------------
 # matrix products: y = x @ w.T
 # ---------------------------------------------------------------------------------------
-SKINNY_MAX_ROWS = 8   # up to this many rows the weight-streaming kernel runs (it takes up to 64); above, the library
+SKINNY_MAX_ROWS = 8   # up to this many rows the weight-streaming kernel runs (it takes up to 64) where the TMA-fed one is not ahead of it
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, static_weights: bool = False) -> torch.Tensor:
     """``x [M, K] @ w [N, K].T`` with float32 accumulation.
 
     float32 operands use the plain-FMA kernels (true 32-bit, no tensor cores; a row's bits do not depend on the others).  bfloat16
-    operands with up to ``SKINNY_MAX_ROWS`` rows use the weight-streaming kernel; many rows
-    whose 128 x 256 tiles fill whole rounds over the SMs use our tcgen05 kernel; the rest go to
+    operands with up to ``SKINNY_MAX_ROWS`` rows use the weight-streaming kernel, or the TMA-fed one where there are many weight rows and k is
+    long; 9 to ``STREAM_MAX_ROWS`` rows the TMA-fed one over a long k (float32 results: :func:`_head_streams`); many rows
+    whose 128 x 256 tiles fill whole rounds over the SMs our tcgen05 kernel; the rest go to
     the library matrix product, as raun6k/Pylon's ``nn.Linear`` layers do
     (src/pylon/model/layers.py:17-23,95-106).  ``out_dtype=torch.float32`` keeps the 32-bit
     accumulator (used for logits).
@@ -869,7 +870,7 @@ def tcgen05_error_word(device: torch.device) -> torch.Tensor:
 
 def tcgen05_force_tile(columns: int = 0) -> None:
     """For measurements: later ``linear_tcgen05`` calls use ``128 x columns`` output tiles
-    (288, 256, 192, 160 or 128); 0 restores the choice by size."""
+    (288, 256, 192, 160 or 128; 1192: both row tiles of a gated product of 129 to 256 rows with 192 columns); 0 restores the choice by size."""
     _library("gemm_tcgen05.cu").pylon_gemm_tcgen05_force_tile(columns)
 
 

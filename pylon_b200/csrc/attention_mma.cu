@@ -29,6 +29,7 @@
 // element, rows of the output in a wider row; and its weights enter the weighted sum as two bfloat16 numbers, as the sigmoid ones do.
 #include "common.cuh"
 
+#include <algorithm>
 #include <cuda.h>
 
 #include <mutex>
@@ -610,6 +611,59 @@ __device__ __forceinline__ int decode_blocks_used(int total, int grid, int pairs
 __device__ __forceinline__ int run_begin(int block, int total, int used) { return (int)((long long)block * total / used); }
 __device__ __forceinline__ int run_of(int tile, int total, int used) { return (int)((((long long)tile + 1) * used - 1) / total); }   // a block takes at least this many tiles: below it the merging costs more than the walk
 
+// Adds up the `segments` partial results of a (row, KV head) pair, those of blocks first_block on, and writes the pair's output; by the whole block
+// that arrived last at the pair.
+__device__ __forceinline__ void combine_segments(const AttentionParams& p, int pair, int first_block, int segments, int q0, int packed_rows, int kv_head) {
+  const int G = p.group;
+  // One trip to L2: every thread asks for its four values of up to eight segments and for
+  // those segments' log-sum-exps at once, then weighs and adds them.  More segments go round
+  // again, the sum so far rescaled as in the attention loop itself.
+  constexpr int SLOT_VECTORS = SMALL_ROWS * D / 4;
+  const size_t slot0 = (size_t)pair + first_block;
+  const float4* partials = reinterpret_cast<const float4*>(p.decode_out + slot0 * SMALL_ROWS * D);
+  const float* lses = p.decode_lse + slot0 * SMALL_ROWS;
+  for (int v = threadIdx.x; v < packed_rows * (D / 4); v += ATT_THREADS) {
+    const int r = v / (D / 4), col = (v % (D / 4)) * 4;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    float run_max = -INFINITY, run_total = 0.f;
+    for (int s2 = 0; s2 < segments; s2 += 8) {
+      float4 part[8];
+      float lse[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int segment = min(s2 + j, segments - 1);
+        part[j] = __ldcg(partials + (size_t)segment * SLOT_VECTORS + v);
+        lse[j] = s2 + j < segments ? __ldcg(lses + (size_t)segment * SMALL_ROWS + r) : -INFINITY;
+      }
+      float new_max = run_max;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) new_max = fmaxf(new_max, lse[j]);
+      if (new_max == -INFINITY) continue;   // nothing visible in these segments
+      const float alpha = fast_exp2(run_max - new_max);   // 0 for the first round
+      sum.x *= alpha; sum.y *= alpha; sum.z *= alpha; sum.w *= alpha;
+      run_total *= alpha;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float weight = fast_exp2(lse[j] - new_max);   // 0 for -infinity
+        sum.x += weight * part[j].x; sum.y += weight * part[j].y; sum.z += weight * part[j].z; sum.w += weight * part[j].w;
+        run_total += weight;
+      }
+      run_max = new_max;
+    }
+    const size_t token = (size_t)q0 + r / G;
+    const int head = kv_head * G + r % G;
+    // with sigmoid weights every segment's log-sum-exp is written as 0: the parts have been added up with weights of one
+    const float inv = (SIGMOID ? 1.f : (run_total > 0.f ? 1.f / run_total : 0.f)) * head_factor(p.heads, token, head);
+    if (SPLIT && p.heads.gate_elements) {
+      sum.x *= element_factor(p.heads, token, head, col); sum.y *= element_factor(p.heads, token, head, col + 1);
+      sum.z *= element_factor(p.heads, token, head, col + 2); sum.w *= element_factor(p.heads, token, head, col + 3);
+    }
+    __nv_bfloat16* dst = p.out + token * p.out_stride + (size_t)head * D + col;
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(sum.x * inv, sum.y * inv), pack_bf16(sum.z * inv, sum.w * inv));
+  }
+  if (threadIdx.x == 0) p.counters[pair] = 0u;   // ready for the next launch
+}
+
 // Decoded rows.  All (row, KV head, tile) triples of the launch form one sequence, row-major,
 // and the blocks cut it into equal runs, so every block reads the same number of bytes however
 // the requests' lengths differ.  A run may end inside a (row, KV head) pair and go on into
@@ -825,64 +879,16 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
       const int pair = pending[entry][0], first_block = pending[entry][1], segments = pending[entry][2];
       const int q0 = pending[entry][3], packed_rows = pending[entry][4], kv_head = pending[entry][5];
       __threadfence();
-      // One trip to L2: every thread asks for its four values of up to eight segments and for
-      // those segments' log-sum-exps at once, then weighs and adds them.  More segments go round
-      // again, the sum so far rescaled as in the attention loop itself.
-      constexpr int SLOT_VECTORS = SMALL_ROWS * D / 4;
-      const size_t slot0 = (size_t)pair + first_block;
-      const float4* partials = reinterpret_cast<const float4*>(p.decode_out + slot0 * SMALL_ROWS * D);
-      const float* lses = p.decode_lse + slot0 * SMALL_ROWS;
-      for (int v = threadIdx.x; v < packed_rows * (D / 4); v += ATT_THREADS) {
-        const int r = v / (D / 4), col = (v % (D / 4)) * 4;
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        float run_max = -INFINITY, run_total = 0.f;
-        for (int s2 = 0; s2 < segments; s2 += 8) {
-          float4 part[8];
-          float lse[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int segment = min(s2 + j, segments - 1);
-            part[j] = __ldcg(partials + (size_t)segment * SLOT_VECTORS + v);
-            lse[j] = s2 + j < segments ? __ldcg(lses + (size_t)segment * SMALL_ROWS + r) : -INFINITY;
-          }
-          float new_max = run_max;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) new_max = fmaxf(new_max, lse[j]);
-          if (new_max == -INFINITY) continue;   // nothing visible in these segments
-          const float alpha = fast_exp2(run_max - new_max);   // 0 for the first round
-          sum.x *= alpha; sum.y *= alpha; sum.z *= alpha; sum.w *= alpha;
-          run_total *= alpha;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float weight = fast_exp2(lse[j] - new_max);   // 0 for -infinity
-            sum.x += weight * part[j].x; sum.y += weight * part[j].y; sum.z += weight * part[j].z; sum.w += weight * part[j].w;
-            run_total += weight;
-          }
-          run_max = new_max;
-        }
-        const size_t token = (size_t)q0 + r / G;
-        const int head = kv_head * G + r % G;
-        // with sigmoid weights every segment's log-sum-exp is written as 0: the parts have been added up with weights of one
-        const float inv = (SIGMOID ? 1.f : (run_total > 0.f ? 1.f / run_total : 0.f)) * head_factor(p.heads, token, head);
-        if (SPLIT && p.heads.gate_elements) {
-          sum.x *= element_factor(p.heads, token, head, col); sum.y *= element_factor(p.heads, token, head, col + 1);
-          sum.z *= element_factor(p.heads, token, head, col + 2); sum.w *= element_factor(p.heads, token, head, col + 3);
-        }
-        __nv_bfloat16* dst = p.out + token * p.out_stride + (size_t)head * D + col;
-        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(sum.x * inv, sum.y * inv), pack_bf16(sum.z * inv, sum.w * inv));
-      }
-      if (threadIdx.x == 0) p.counters[pair] = 0u;   // ready for the next launch
+      combine_segments(p, pair, first_block, segments, q0, packed_rows, kv_head);
     }
     pending_count = 0;
   };
 
-  Segment current, following;
+  Segment current;
   bool have = next_segment(current);
   const bool had_tiles = have;   // cluster form: this block has a share of the pair's tiles
   bool waited = false;       // for the kernel before this one (programmatic dependent launch)
-  bool prefetched = false;   // the segment's query and first tile were asked for while the one before it was merged
   while (have) {
-    const bool have_following = next_segment(following);
     const int kv_head = current.kv_head, tile_begin = current.tile_begin, tile_end = current.tile_end, pair = current.pair;
     const int first_block = current.first_block, segments = current.segments, q0 = current.q0, packed_rows = current.packed_rows;
     const int kv_len = current.kv_len, pos0 = current.pos0;
@@ -912,25 +918,23 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
       if (tile < tile_end) issue_tile(current, tile);
       if (!TMA) cp_async_commit();   // an empty group keeps the count of groups in step with the tiles
     };
-    if (!prefetched) {
-      if (!waited) {
-        // Tiles that end before the row's first new token hold nothing the kernel before this one writes: as many
-        // of them as the ring has stages are asked for before this kernel waits for that one.  The queries and the
-        // newest keys are its work.
-        if (TMA) {
-          while (issued_ahead < STAGES && tile_begin + issued_ahead < tile_end && (tile_begin + issued_ahead + 1) * BLOCK_N <= pos0) {
-            issue_tile(current, tile_begin + issued_ahead);
-            ++issued_ahead;
-          }
+    if (!waited) {
+      // Tiles that end before the row's first new token hold nothing the kernel before this one writes: as many
+      // of them as the ring has stages are asked for before this kernel waits for that one.  The queries and the
+      // newest keys are its work.
+      if (TMA) {
+        while (issued_ahead < STAGES && tile_begin + issued_ahead < tile_end && (tile_begin + issued_ahead + 1) * BLOCK_N <= pos0) {
+          issue_tile(current, tile_begin + issued_ahead);
+          ++issued_ahead;
         }
-        grid_dependency_wait();
-        allow_dependents();   // only now: a kernel that is itself still waiting must not pull the next one onto the SMs
-        waited = true;
       }
-      load_query(current);
-      if (TMA) cp_async_commit();   // otherwise the first tile's group carries the query
-      for (int s = issued_ahead; s < STAGES - 1; ++s) issue(tile_begin + s);   // the ring runs STAGES - 1 tiles ahead
+      grid_dependency_wait();
+      allow_dependents();   // only now: a kernel that is itself still waiting must not pull the next one onto the SMs
+      waited = true;
     }
+    load_query(current);
+    if (TMA) cp_async_commit();   // otherwise the first tile's group carries the query
+    for (int s = issued_ahead; s < STAGES - 1; ++s) issue(tile_begin + s);   // the ring runs STAGES - 1 tiles ahead
 
     const bool upper_rows_unused = packed_rows <= 8;
     // The query fragments stay in registers when the head is small enough to leave room.
@@ -938,15 +942,9 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     unsigned q_frag[Q_IN_REGISTERS ? D / 16 : 1][4];
     bool q_loaded = false;
 
-    bool tile_prefetched = false;   // the following segment's first tile is on its way
     for (int tile = tile_begin; tile < tile_end; ++tile) {
       if (tile + STAGES - 1 < tile_begin + issued_ahead) {
         // asked for before the wait
-      } else if (TMA && STAGES == 2 && tile + 1 == tile_end && have_following) {
-        // The ring has a free stage and this segment no tile for it: the following segment's
-        // first tile comes in while this one's last tile is multiplied and the warps are merged.
-        issue_tile(following, following.tile_begin);
-        tile_prefetched = true;
       } else {
         issue(tile + STAGES - 1);
       }
@@ -1093,17 +1091,6 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     }
     if (!TMA) cp_async_wait<0>();
 
-    // While this segment is merged and written out, the next one's query is on its way into the
-    // query tile, which every warp has read; its first tile went into the stage that is not the
-    // one read last (where the merge happens).
-    prefetched = false;
-    if (TMA && STAGES == 2 && have_following) {
-      load_query(following);
-      cp_async_commit();
-      if (!tile_prefetched) issue_tile(following, following.tile_begin);
-      prefetched = true;
-    }
-
     // Merge the four warps: each leaves its (max, sum, unnormalised output) in shared memory.
     __nv_bfloat16* idle_stage = stages + ((consumed + STAGES - 1) % STAGES) * Tiles::STAGE;   // the stage read last
     // [4][16][D]: exactly one stage of the TMA form; columns swizzled by row (merge_swizzle)
@@ -1207,8 +1194,7 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     }
     if (TMA) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // the merge buffers were written where TMA writes next
     __syncthreads();   // the query tile and the stages are free for the next segment
-    current = following;
-    have = have_following;
+    have = next_segment(current);
   }
   if (!CLUSTER) {
     if (!waited) grid_dependency_wait();   // a block without a segment: no grid ends before the grid ahead of it has
@@ -1261,6 +1247,469 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
       p.out[token * p.out_stride + (size_t)head * D + col] = __float2bfloat16_rn((SIGMOID ? sum : (total > 0.f ? sum / total : 0.f)) * head_factor(p.heads, token, head) *
                                                                                   element_factor(p.heads, token, head, col));
     }
+  }
+}
+
+// -----------------------------------------------------------------------------------------
+// Decoded rows without clusters, tiles by TMA: every warp walks a run of its own.
+//
+// Bound by the bytes of the cache.  All (row, KV head, tile of RUN_KEYS keys) triples of the launch form one sequence, row-major, that the
+// warps cut into equal runs, consecutive runs to the warps of a block.  A warp has a ring of stages of its own, which runs
+// ahead over the ends of rows, and keeps its scores, softmax and sums in registers: no warp waits for another before its run is done.
+// A (row, KV head) pair that lies in one run is written out by its warp.  The other pieces are left in shared memory (the
+// run's last one in the warp's own ring, which is idle by then, the first in a place of its own) and added up once, at the end of
+// the block; a pair that lies in several blocks goes through scratch slot (pair + block) as in the kernel above.
+// -----------------------------------------------------------------------------------------
+constexpr int RUN_KEYS = 16, RUN_WARPS = ATT_THREADS / 32;
+constexpr int RUN_MIN_TILES = 4;   // tiles a warp takes at least: below it, starting and merging cost more than the walk
+template <bool ROOMY>
+struct RunTiles {
+  static constexpr int TILE = RUN_KEYS * D;             // values in one tile of keys or of values: boxes of RUN_KEYS keys x 64 values
+  static constexpr int STAGE = 2 * TILE;                // keys then values
+  static constexpr int STAGE_BYTES = STAGE * (int)sizeof(__nv_bfloat16);
+  static constexpr int BLOCKS_PER_SM = D <= 128 ? 2 : 1;
+  // Stages of a block: 96 KB of two to an SM, 64 KB where pieces of many query rows need the room, 128 KB of a lone block.
+  static constexpr int STAGES = (BLOCKS_PER_SM == 1 ? 128 : ROOMY ? 96 : 64) * 1024 / RUN_WARPS / STAGE_BYTES;
+  static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
+  static_assert(RING_BYTES >= SMALL_ROWS * D * (int)sizeof(float), "a run's last piece is left in its ring");
+  // rings (1024-byte aligned for the swizzle), the runs' first pieces, the barriers of the stages
+  static constexpr size_t smem(int rows) { return 1024 + (size_t)RUN_WARPS * (RING_BYTES + (size_t)rows * D * sizeof(float) + STAGES * sizeof(uint64_t)); }
+  // with the static shared memory, the reserved KB of each block and their number
+  static constexpr bool fits(int rows) { return BLOCKS_PER_SM * (smem(rows) + 3072) <= 228 * 1024; }
+  static __device__ __forceinline__ int offset(int row, int chunk) { return (chunk >> 3) * (RUN_KEYS * 64) + row * 64 + (((chunk & 7) ^ (row & 7)) << 3); }
+};
+
+// As decode_row_tiles, in tiles of RUN_KEYS keys; and the position of the row's first new token.
+__device__ __forceinline__ int run_row_tiles(const AttentionParams& p, int row, int* first_tile, int* first_position) {
+  const int q_len = p.q_start[row + 1] - p.q_start[row], pos0 = p.kv_len[row] - q_len;
+  const int packed_rows = q_len * p.group;
+  *first_tile = 0;
+  *first_position = pos0;
+  if (packed_rows <= 0 || packed_rows > SMALL_ROWS) return 0;
+  const int hi = pos0 + q_len - 1;
+  const int lo = first_visible(p, pos0);
+  if (hi < lo) return 0;
+  *first_tile = lo / RUN_KEYS;
+  return hi / RUN_KEYS - lo / RUN_KEYS + 1;
+}
+
+// How many runs share `total` tiles.  Where it costs under a fifth of them, a number that makes the ends of equally long pairs fall on ends of
+// blocks, or at least of runs.
+__device__ __forceinline__ int runs_used(int total, int grid, int pairs) {
+  const int runs = max(1, min(grid, total / (RUN_WARPS * RUN_MIN_TILES))) * RUN_WARPS;
+  if (pairs <= 0) return min(runs, max(total, 1));
+  const int blocks_aligned = runs / (pairs * RUN_WARPS) * (pairs * RUN_WARPS), aligned = runs / pairs * pairs;
+  const int used = blocks_aligned * 5 >= runs * 4 ? blocks_aligned : aligned * 5 >= runs * 4 ? aligned : runs;
+  return min(used, max(total, 1));
+}
+
+template <bool ROOMY>
+__global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) paged_attention_runs_kernel(const AttentionParams p, const __grid_constant__ CUtensorMap map_k,
+                                                                                                          const __grid_constant__ CUtensorMap map_v) {
+  using Tiles = RunTiles<ROOMY>;
+  constexpr int STAGES = Tiles::STAGES, PIECES = 2 * RUN_WARPS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  unsigned char* smem_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  // The block's pieces, two places a warp: the pair (-1: none), its first block, how many blocks it lies in, q0 and packed rows of its row.
+  __shared__ __align__(16) int piece_pair[PIECES];
+  __shared__ int piece_first[PIECES], piece_blocks[PIECES], piece_q0[PIECES], piece_rows[PIECES];
+  __shared__ float piece_max[PIECES * SMALL_ROWS], piece_sum[PIECES * SMALL_ROWS];
+  __shared__ unsigned arrived_last;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+  const int G = p.group;
+  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(smem_base + (size_t)warp * Tiles::RING_BYTES);
+  float* first_pieces = reinterpret_cast<float*>(smem_base + (size_t)RUN_WARPS * Tiles::RING_BYTES);   // [RUN_WARPS][incoming_rows][D]
+  uint64_t* tile_full = reinterpret_cast<uint64_t*>(first_pieces + (size_t)RUN_WARPS * p.incoming_rows * D) + warp * STAGES;
+  // The tensor maps, and a row's page table each, on their way while the plan is made.
+  if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_k) : "memory");
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_v) : "memory");
+  }
+  if ((int)threadIdx.x * 32 < p.table_width)
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.block_table + (size_t)(blockIdx.x % p.num_rows) * p.table_width + threadIdx.x * 32));
+  if (lane < 2) piece_pair[2 * warp + lane] = -1;
+  if (lane == 0) {
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) att_mbar_init(&tile_full[s], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+
+  // The plan, made by every warp for itself: the rows' lengths were written long before the kernel ahead of this one started.
+  int unused;
+  const int first_chunk = lane < p.num_rows ? run_row_tiles(p, lane, &unused, &unused) : 0;
+  int total = first_chunk, with_tiles = first_chunk > 0;
+  for (int base = 32; base < p.num_rows; base += 32) {
+    const int tiles = base + lane < p.num_rows ? run_row_tiles(p, base + lane, &unused, &unused) : 0;
+    total += tiles;
+    with_tiles += tiles > 0;
+  }
+#pragma unroll
+  for (int offset = 16; offset; offset >>= 1) {
+    total += __shfl_xor_sync(0xffffffffu, total, offset);
+    with_tiles += __shfl_xor_sync(0xffffffffu, with_tiles, offset);
+  }
+  total *= p.nkv;
+  const int runs = runs_used(total, gridDim.x, with_tiles * p.nkv);
+  if ((int)blockIdx.x * RUN_WARPS >= runs || total == 0) {   // no run for this block
+    grid_dependency_wait();   // a grid must not end before the grid ahead of it has: the next kernel's wait sees only this one
+    return;
+  }
+  const int run = blockIdx.x * RUN_WARPS + warp;
+  // Run b begins at floor(b total / runs), in 32-bit arithmetic.
+  const int run_tiles = total / runs, rest = total - run_tiles * runs;
+  auto begin_of = [&](int b) { return b * run_tiles + b * rest / runs; };
+  auto block_of = [&](int tile) {   // of the run that holds the tile: a guess, at most one off
+    int b = min(runs - 1, (int)((float)tile * (float)runs / (float)total));
+    if (begin_of(b) > tile) --b;
+    else if (b + 1 < runs && begin_of(b + 1) <= tile) ++b;
+    return b / RUN_WARPS;
+  };
+  const int run_first = run < runs ? begin_of(run) : total, run_end = run < runs ? begin_of(run + 1) : total;
+
+  // A place in the sequence: the next tile, with its row and what is known of it.
+  struct Cursor { int position, row, row_tiles, first_tile, pos0, kv_head, tile; };   // tile counts from the row's first
+  Cursor at = {run_first, 0, 0, 0, 0, 0, 0};
+  if (run_first < run_end) {
+    int before = 0;
+    for (int base = 0; base < p.num_rows; base += 32) {
+      const int tiles = (base == 0 ? first_chunk : (base + lane < p.num_rows ? run_row_tiles(p, base + lane, &unused, &unused) : 0)) * p.nkv;
+      int inclusive = tiles;
+#pragma unroll
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, inclusive, offset);
+        if (lane >= offset) inclusive += below;
+      }
+      const int exclusive = before + inclusive - tiles;
+      const unsigned hit = __ballot_sync(0xffffffffu, tiles > 0 && exclusive <= run_first && run_first < exclusive + tiles);
+      if (hit) {
+        at.row = base + __ffs(hit) - 1;
+        const int within = run_first - __shfl_sync(0xffffffffu, exclusive, __ffs(hit) - 1);
+        at.row_tiles = run_row_tiles(p, at.row, &at.first_tile, &at.pos0);
+        at.kv_head = within / at.row_tiles;
+        at.tile = within % at.row_tiles;
+        break;
+      }
+      before += __shfl_sync(0xffffffffu, inclusive, 31);
+    }
+  }
+  auto next_row = [&](Cursor& c) {   // to the first tile of the next row that has any; there is one, since the run goes on
+    c.kv_head = c.tile = 0;
+    do {
+      ++c.row;
+      c.row_tiles = c.row < p.num_rows ? run_row_tiles(p, c.row, &c.first_tile, &c.pos0) : 1;
+    } while (c.row_tiles == 0);
+  };
+  auto next_pair = [&](Cursor& c) {
+    c.tile = 0;
+    if (++c.kv_head == p.nkv && c.position < run_end) next_row(c);
+  };
+
+  // Asks for tiles of the run, in order, stage after stage of the ring (lane 0; the others keep step).
+  Cursor ahead = at;
+  int issued = 0, page_end = -1, page_y = 0;   // keys below page_end lie in the page looked up last; key k of this head is TMA row page_y + k
+  auto issue_next = [&]() {
+    const int key0 = (ahead.first_tile + ahead.tile) * RUN_KEYS;
+    if (key0 >= page_end) {
+      // A tile lies in one page.  Without a page for it the row coordinate points past the pool and TMA fills the boxes with zeros.
+      const int place = key0 / p.page_size;
+      const int page = p.block_table[(size_t)ahead.row * p.table_width + place];
+      const bool page_ok = page >= 0 && page < p.num_pages;
+      if (lane == 0 && (page < -1 || page >= p.num_pages) && p.error) atomicExch(p.error, PYLON_ERROR_BAD_PAGE);   // a broken table; -1 is "no page"
+      page_end = page_ok ? (place + 1) * p.page_size : key0 + 1;
+      page_y = page_ok ? (page * p.nkv + ahead.kv_head) * p.page_size - place * p.page_size : p.num_pages * p.nkv * p.page_size - key0;
+    }
+    if (lane == 0) {
+      const int stage = issued % STAGES;
+      __nv_bfloat16* dst = ring + stage * Tiles::STAGE;
+      // A stage used before was read with ordinary loads (ldmatrix); TMA is another proxy, which a barrier alone does not order behind them.
+      if (issued >= STAGES) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      att_mbar_expect_tx(&tile_full[stage], Tiles::STAGE_BYTES);
+#pragma unroll
+      for (int box = 0; box < D / 64; ++box) {
+        att_tma_load(dst + box * (RUN_KEYS * 64), &map_k, &tile_full[stage], box * 64, page_y + key0);
+        att_tma_load(dst + Tiles::TILE + box * (RUN_KEYS * 64), &map_v, &tile_full[stage], box * 64, page_y + key0);
+      }
+    }
+    ++issued;
+    ++ahead.position;
+    if (++ahead.tile == ahead.row_tiles) { next_pair(ahead); page_end = -1; }
+  };
+  __syncwarp();
+  // Tiles that end before their row's first new token hold nothing the kernel ahead writes: as many as the ring has stages are asked
+  // for before this kernel waits for that one.  The queries and the newest keys are its work.
+  const int length = run_end - run_first;
+  while (issued < min(STAGES, length)) {
+    if ((ahead.first_tile + ahead.tile + 1) * RUN_KEYS > ahead.pos0) break;
+    issue_next();
+  }
+  grid_dependency_wait();
+  allow_dependents();   // only now: a kernel that is itself still waiting must not pull the next one onto the SMs
+  while (issued < min(STAGES, length)) issue_next();
+
+  const bool sloped = OPTIONS && p.heads.slopes != nullptr;   // the scores are brought to log2 units before the softmax
+  const float unit = sloped ? 1.f : p.scale_log2;
+  constexpr bool Q_IN_REGISTERS = D <= 128;   // else read again for every tile
+  int consumed = 0;
+  bool failed = false;
+  while (at.position < run_end && !failed) {
+    const int row = at.row, kv_head = at.kv_head, first_tile = at.first_tile, row_tiles = at.row_tiles, tile_begin = at.tile;
+    const int tile_end = min(row_tiles, tile_begin + run_end - at.position);
+    const int q0 = p.q_start[row], q_len = p.q_start[row + 1] - q0, packed_rows = q_len * G, pos0 = at.pos0, kv_len = pos0 + q_len;
+    const bool upper_rows_unused = packed_rows <= 8;
+    int row_pos[2], row_lo[2];
+    bool row_valid[2];
+    float row_bias[2], row_slope[2];
+    const __nv_bfloat16* row_q[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = g + 8 * h;
+      row_valid[h] = m < packed_rows;
+      const int head = kv_head * G + (row_valid[h] ? m % G : 0), token = row_valid[h] ? m / G : 0;
+      row_bias[h] = head_score_bias(p.heads, head);
+      row_slope[h] = head_slope(p.heads, head);
+      row_pos[h] = pos0 + token;
+      row_lo[h] = first_visible(p, row_pos[h]);
+      row_q[h] = p.q + (size_t)(q0 + token) * p.q_stride + (size_t)head * D + 2 * tq;
+    }
+    // The fragments of the queries come straight from memory.
+    unsigned q_frag[Q_IN_REGISTERS ? D / 16 : 1][4];
+    auto load_q = [&](unsigned (&a)[4], int kk) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = row_valid[i & 1] ? *reinterpret_cast<const unsigned*>(row_q[i & 1] + kk * 16 + 8 * (i >> 1)) : 0u;
+    };
+    if (Q_IN_REGISTERS) {
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) load_q(q_frag[Q_IN_REGISTERS ? kk : 0], kk);
+    }
+    float o[D / 8][4];
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+    float row_max[2] = {-INFINITY, -INFINITY}, row_sum[2] = {0.f, 0.f};
+
+    for (int tile = tile_begin; tile < tile_end; ++tile) {
+      const int stage = consumed % STAGES, key0 = (first_tile + tile) * RUN_KEYS;
+      const __nv_bfloat16* ks = ring + stage * Tiles::STAGE;
+      const __nv_bfloat16* vs = ks + Tiles::TILE;
+      if (!att_mbar_wait(&tile_full[stage], (consumed / STAGES) & 1)) failed = true;
+      if (__any_sync(0xffffffffu, failed)) { failed = true; break; }
+      ++consumed;
+      if (key0 + RUN_KEYS > kv_len) {
+        // Keys past the row's length are masked, but their values (whatever the page held) still meet a weight of zero in the product: make them zero.
+        for (int c = lane; c < RUN_KEYS * CHUNKS; c += 32)
+          if (key0 + c / CHUNKS >= kv_len) *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(vs) + Tiles::offset(c / CHUNKS, c % CHUNKS)) = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+      }
+      // Even and odd k-steps accumulate separately: four independent MMA chains instead of two.
+      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float s_odd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        unsigned a_loaded[4], b[4];
+        if (!Q_IN_REGISTERS) load_q(a_loaded, kk);
+        const unsigned (&a)[4] = Q_IN_REGISTERS ? q_frag[Q_IN_REGISTERS ? kk : 0] : a_loaded;
+        ldmatrix_x4(b, ks + Tiles::offset((lane & 7) + 8 * (lane >> 4), kk * 2 + ((lane >> 3) & 1)));
+        if (kk & 1) {
+          mma_bf16(s_odd[0], a, b[0], b[1]);
+          mma_bf16(s_odd[1], a, b[2], b[3]);
+        } else {
+          mma_bf16(s[0], a, b[0], b[1]);
+          mma_bf16(s[1], a, b[2], b[3]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          s[n][i] += s_odd[n][i];
+          if (p.cap_pre > 0.f) s[n][i] = soft_tanh(s[n][i] * p.cap_pre);
+          if (sloped) s[n][i] = fmaf(s[n][i], p.scale_log2, -row_slope[i >> 1] * (float)(row_pos[i >> 1] - (key0 + 2 * tq + n * 8 + (i & 1))));
+        }
+      // Tiles that end at or before the row's first new token, with no window, are visible whole.
+      if (p.window > 0 || p.chunk > 0 || key0 + RUN_KEYS - 1 > pos0) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int key = key0 + 2 * tq + n * 8 + (i & 1);
+            if (!row_valid[i >> 1] || key > row_pos[i >> 1] || key < row_lo[i >> 1]) s[n][i] = -INFINITY;
+          }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h == 1 && upper_rows_unused) continue;   // rows 8..15 hold zero queries, and nothing of them is stored
+        if (SIGMOID) {
+#pragma unroll
+          for (int n = 0; n < 2; ++n) {
+            s[n][2 * h] = sigmoid_exp2(fmaf(s[n][2 * h], p.scale_log2, row_bias[h]));
+            s[n][2 * h + 1] = sigmoid_exp2(fmaf(s[n][2 * h + 1], p.scale_log2, row_bias[h]));
+          }
+          continue;
+        }
+        float mx = fmaxf(fmaxf(s[0][2 * h], s[0][2 * h + 1]), fmaxf(s[1][2 * h], s[1][2 * h + 1]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float new_max = fmaxf(row_max[h], mx);
+        const float use_max = new_max == -INFINITY ? 0.f : new_max;
+        const float alpha = fast_exp2((row_max[h] - use_max) * unit);
+        const float shift = use_max * unit;
+        float sum = 0.f;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          s[n][2 * h] = fast_exp2(s[n][2 * h] * unit - shift);
+          s[n][2 * h + 1] = fast_exp2(s[n][2 * h + 1] * unit - shift);
+          sum += s[n][2 * h] + s[n][2 * h + 1];
+        }
+        row_sum[h] = row_sum[h] * alpha + sum;
+        row_max[h] = new_max;
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i) { o[i][2 * h] *= alpha; o[i][2 * h + 1] *= alpha; }
+      }
+      unsigned a[4] = {pack_bf16(s[0][0], s[0][1]), pack_bf16(s[0][2], s[0][3]), pack_bf16(s[1][0], s[1][1]), pack_bf16(s[1][2], s[1][3])};
+      unsigned dropped[4];
+      if (SPLIT) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) dropped[f] = pack_dropped(s[f >> 1][2 * (f & 1)], s[f >> 1][2 * (f & 1) + 1], a[f]);
+      }
+#pragma unroll
+      for (int d2 = 0; d2 < D / 16; ++d2) {
+        unsigned b[4];
+        ldmatrix_x4_trans(b, vs + Tiles::offset((lane & 7) + 8 * ((lane >> 3) & 1), d2 * 2 + (lane >> 4)));
+        mma_bf16(o[2 * d2], a, b[0], b[1]);
+        mma_bf16(o[2 * d2 + 1], a, b[2], b[3]);
+        if (SPLIT) {
+          mma_bf16(o[2 * d2], dropped, b[0], b[1]);
+          mma_bf16(o[2 * d2 + 1], dropped, b[2], b[3]);
+        }
+      }
+      __syncwarp();   // the stage has been read by all lanes
+      if (issued < length) issue_next();
+    }
+    at.position += tile_end - tile_begin;
+    at.tile = tile_end;
+
+    const bool whole = tile_begin == 0 && tile_end == row_tiles, last = at.position >= run_end;
+    const int place = 2 * warp + (last ? 1 : 0);
+    if (!whole && lane == 0) {
+      const int pair_first = at.position - tile_end, first_block = block_of(pair_first);
+      piece_pair[place] = row * p.nkv + kv_head;
+      piece_first[place] = first_block;
+      piece_blocks[place] = block_of(pair_first + row_tiles - 1) - first_block + 1;
+      piece_q0[place] = q0;
+      piece_rows[place] = packed_rows;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = g + 8 * h;
+      float sum = row_sum[h];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (whole) {
+        if (!row_valid[h]) continue;
+        const size_t token = (size_t)q0 + r / G;
+        const int head = kv_head * G + r % G;
+        float inv = 1.f;
+        if (!SIGMOID) {
+          float weight = 1.f;
+          if (OPTIONS && p.heads.sinks) {
+            const float sink = head_sink(p.heads, head) / unit, mx = fmaxf(row_max[h], sink);
+            weight = row_max[h] == -INFINITY ? 0.f : fast_exp2((row_max[h] - mx) * unit);
+            sum = weight * sum + fast_exp2((sink - mx) * unit);
+          }
+          inv = sum > 0.f ? weight / sum : 0.f;
+        }
+        if (SPLIT) inv *= head_factor(p.heads, token, head);
+        __nv_bfloat16* dst = p.out + token * p.out_stride + (size_t)head * D + 2 * tq;
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i) {
+          float x = o[i][2 * h] * inv, y = o[i][2 * h + 1] * inv;
+          if (SPLIT) { x *= element_factor(p.heads, token, head, i * 8 + 2 * tq); y *= element_factor(p.heads, token, head, i * 8 + 2 * tq + 1); }
+          *reinterpret_cast<unsigned*>(dst + i * 8) = pack_bf16(x, y);
+        }
+      } else if (r < packed_rows) {
+        if (tq == 0) { piece_max[place * SMALL_ROWS + r] = row_max[h]; piece_sum[place * SMALL_ROWS + r] = sum; }
+        float* dst = (last ? reinterpret_cast<float*>(ring) : first_pieces + (size_t)warp * p.incoming_rows * D) + r * D;
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i) *reinterpret_cast<float2*>(dst + ((i * 8 + 2 * tq) ^ merge_swizzle(r))) = make_float2(o[i][2 * h], o[i][2 * h + 1]);
+      }
+    }
+    if (!last && at.tile == row_tiles) next_pair(at);
+  }
+  if (failed) {
+    if (lane == 0 && p.error) atomicExch(p.error, 1);
+    for (; consumed < issued; ++consumed) att_mbar_wait(&tile_full[consumed % STAGES], (consumed / STAGES) & 1);   // no copy outlives the block
+  }
+  __syncthreads();
+
+  // The pieces of a pair lie side by side, in the order of the runs (with empty places between them): bit e of `begins` is set where a
+  // pair's first piece lies in place e.
+  unsigned begins = 0, shared = 0;   // shared: pairs that other blocks have pieces of as well
+  {
+    int pairs[PIECES], before = -1;
+#pragma unroll
+    for (int e = 0; e < PIECES; e += 4) *reinterpret_cast<int4*>(pairs + e) = *reinterpret_cast<const int4*>(piece_pair + e);
+#pragma unroll
+    for (int e = 0; e < PIECES; ++e) {
+      if (pairs[e] < 0) continue;
+      if (pairs[e] != before) begins |= 1u << e;
+      before = pairs[e];
+    }
+  }
+  for (unsigned left = begins; left; left &= left - 1) {
+    const int first = __ffs(left) - 1, end = left & (left - 1) ? __ffs(left & (left - 1)) - 1 : PIECES;
+    const int pair = piece_pair[first], kv_head = pair % p.nkv, q0 = piece_q0[first], packed_rows = piece_rows[first];
+    const bool alone = piece_blocks[first] == 1;
+    if (!alone) shared |= 1u << first;
+    const size_t slot = (size_t)pair + blockIdx.x;
+    for (int v = threadIdx.x; v < packed_rows * (D / 4); v += ATT_THREADS) {
+      const int r = v / (D / 4), col = (v % (D / 4)) * 4, head = kv_head * G + r % G;
+      float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+      float mx = -INFINITY, sum = 0.f;   // sigmoid weights: the pieces add up as they are
+      if (OPTIONS && p.heads.sinks && (int)blockIdx.x == piece_first[first]) {   // met in the pair's first block
+        mx = head_sink(p.heads, head) / unit;
+        sum = mx == -INFINITY ? 0.f : 1.f;
+      }
+      for (int e = first; e < end; ++e) {
+        if (piece_pair[e] < 0) continue;
+        const float* src = (e & 1) ? reinterpret_cast<const float*>(smem_base + (size_t)(e >> 1) * Tiles::RING_BYTES) : first_pieces + (size_t)(e >> 1) * p.incoming_rows * D;
+        const float4 part = *reinterpret_cast<const float4*>(src + r * D + (col ^ merge_swizzle(r)));
+        const float m = piece_max[e * SMALL_ROWS + r];
+        if (!SIGMOID && m == -INFINITY) continue;   // nothing visible
+        const float top = fmaxf(mx, m), alpha = SIGMOID ? 1.f : fast_exp2((mx - top) * unit), weight = SIGMOID ? 1.f : fast_exp2((m - top) * unit);
+        out.x = out.x * alpha + weight * part.x; out.y = out.y * alpha + weight * part.y;
+        out.z = out.z * alpha + weight * part.z; out.w = out.w * alpha + weight * part.w;
+        sum = sum * alpha + weight * piece_sum[e * SMALL_ROWS + r];
+        mx = top;
+      }
+      const float inv = SIGMOID ? 1.f : sum > 0.f ? 1.f / sum : 0.f;
+      out.x *= inv; out.y *= inv; out.z *= inv; out.w *= inv;
+      if (alone) {
+        const size_t token = (size_t)q0 + r / G;
+        if (SPLIT) {
+          const float factor = head_factor(p.heads, token, head);
+          out.x *= factor * element_factor(p.heads, token, head, col); out.y *= factor * element_factor(p.heads, token, head, col + 1);
+          out.z *= factor * element_factor(p.heads, token, head, col + 2); out.w *= factor * element_factor(p.heads, token, head, col + 3);
+        }
+        *reinterpret_cast<uint2*>(p.out + token * p.out_stride + (size_t)head * D + col) = make_uint2(pack_bf16(out.x, out.y), pack_bf16(out.z, out.w));
+      } else {
+        *reinterpret_cast<float4*>(p.decode_out + (slot * SMALL_ROWS + r) * D + col) = out;
+        if (col == 0) p.decode_lse[slot * SMALL_ROWS + r] = SIGMOID ? 0.f : sum > 0.f ? mx * unit + log2f(sum) : -INFINITY;
+      }
+    }
+  }
+  if (!shared) return;
+  __syncthreads();
+  if (warp == 0) {
+    __threadfence();   // what the block's threads wrote before the barrier, too
+    const bool last = (shared >> lane & 1) && atomicAdd(p.counters + piece_pair[lane % PIECES], 1u) == (unsigned)piece_blocks[lane % PIECES] - 1u;
+    const unsigned all = __ballot_sync(0xffffffffu, last);
+    if (lane == 0) arrived_last = all;
+    __threadfence();
+  }
+  __syncthreads();
+  for (unsigned left = arrived_last; left; left &= left - 1) {
+    const int e = __ffs(left) - 1;
+    combine_segments(p, piece_pair[e], piece_first[e], piece_blocks[e], piece_q0[e], piece_rows[e], piece_pair[e] % p.nkv);
   }
 }
 
@@ -1339,32 +1788,32 @@ static EncodeTiled encode_tiled() {
   return fn;
 }
 
-// Tensor map of a page pool [pages, KV heads, page size, D] seen as a matrix of rows of D values, boxes of 64 rows x 64
+// Tensor map of a page pool [pages, KV heads, page size, D] seen as a matrix of rows of D values, boxes of box_rows rows x 64
 // values in the 128-byte swizzle.  The last few maps are kept: a model asks for the same pools at every step.
-static bool page_pool_map(CUtensorMap* map, const void* pages, long long rows) {
-  struct Known { const void* pages; long long rows; CUtensorMap map; };
+static bool page_pool_map(CUtensorMap* map, const void* pages, long long rows, int box_rows) {
+  struct Known { const void* pages; long long rows; int box_rows; CUtensorMap map; };
   static Known known[64];
   static int count = 0, next = 0;
   static std::mutex mutex;
   std::lock_guard<std::mutex> guard(mutex);
   for (int i = 0; i < count; ++i)
-    if (known[i].pages == pages && known[i].rows == rows) { *map = known[i].map; return true; }
+    if (known[i].pages == pages && known[i].rows == rows && known[i].box_rows == box_rows) { *map = known[i].map; return true; }
   EncodeTiled encode = encode_tiled();
   if (!encode) return false;
   cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)D * sizeof(__nv_bfloat16)};
-  cuuint32_t box[2] = {64, (cuuint32_t)BLOCK_N};
+  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   cuuint32_t element_strides[2] = {1, 1};
   if (encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(pages), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
-  known[next].pages = pages; known[next].rows = rows; known[next].map = *map;
+  known[next].pages = pages; known[next].rows = rows; known[next].box_rows = box_rows; known[next].map = *map;
   next = (next + 1) % 64;
   if (count < 64) ++count;
   return true;
 }
 
-constexpr size_t DEC_SMEM_TMA = DecodeTiles<TMA_HEAD>::SMEM, DEC_SMEM_GATHER = DecodeTiles<false>::SMEM;
+constexpr size_t DEC_SMEM_GATHER = DecodeTiles<false>::SMEM;
 // The cluster form: its stages and query tile, then what the other blocks of the cluster send (partial results of
 // `rows` packed query rows in all, and every block's log-sum-exps).
 constexpr size_t DEC_SMEM_CLUSTER_BASE = DecodeTiles<TMA_HEAD, DEC_CLUSTER_STAGES>::SMEM;
@@ -1392,8 +1841,6 @@ static bool clusters_of_16() {
   }();
   return allowed;
 }
-constexpr size_t DEC_SMEM_MOST = DEC_SMEM_TMA > DEC_SMEM_GATHER ? DEC_SMEM_TMA : DEC_SMEM_GATHER;
-
 // Clusters of 16 blocks are beyond the portable size: the kernel has to opt in, and the device may refuse.
 static bool clusters_of_16();
 
@@ -1408,21 +1855,38 @@ static int decode_sm_count() {
   return count;
 }
 
-// Blocks of the decode kernel: as many as are resident at once, of the form that needs more
-// shared memory.
+// Blocks of the decode kernel that a caller may ask for: as many of the gathering form as are resident at once.
 extern "C" int pylon_attention_decode_blocks() {
   static int resident_on[pylon::MAX_DEVICES] = {};
   int& resident = resident_on[pylon::current_device_slot()];
   if (resident == 0) {
-    int device = 0, sm_count = 0, per_sm = 0, per_sm_tma = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return -1;
+    int per_sm = 0;
+    if (decode_sm_count() < 1) return -1;
     if (cudaFuncSetAttribute(paged_attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_GATHER) != cudaSuccess) return -1;
-    if (cudaFuncSetAttribute(paged_attention_decode_kernel<TMA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_TMA) != cudaSuccess) return -1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, paged_attention_decode_kernel<false>, ATT_THREADS, DEC_SMEM_GATHER) != cudaSuccess || per_sm < 1) return -1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tma, paged_attention_decode_kernel<TMA_HEAD>, ATT_THREADS, DEC_SMEM_TMA) != cudaSuccess || per_sm_tma < 1) return -1;
-    resident = (per_sm_tma < per_sm ? per_sm_tma : per_sm) * sm_count;
+    resident = per_sm * decode_sm_count();
   }
   return resident;
+}
+
+// The kernel of one run a warp, where a head's tiles come by TMA.
+template <bool TMA>
+static cudaError_t configure_runs() {
+  if constexpr (TMA) {
+    cudaError_t err = cudaFuncSetAttribute(paged_attention_runs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(paged_attention_runs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
+    return err;
+  }
+  return cudaSuccess;
+}
+template <bool TMA>
+static void launch_runs(const AttentionParams& p, int decode_blocks, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream) {
+  if constexpr (TMA) {
+    const bool roomy = RunTiles<true>::BLOCKS_PER_SM == 1 || RunTiles<true>::fits(p.incoming_rows);
+    const int blocks = std::min(decode_blocks, RunTiles<true>::BLOCKS_PER_SM * decode_sm_count());
+    launch_dependent(roomy ? paged_attention_runs_kernel<true> : paged_attention_runs_kernel<false>, dim3(blocks), dim3(ATT_THREADS),
+                     roomy ? RunTiles<true>::smem(p.incoming_rows) : RunTiles<false>::smem(p.incoming_rows), stream, p, map_k, map_v);
+  }
 }
 
 // Scratch floats a call needs: `num_splits` splits of the tiled kernel over `total_tokens`
@@ -1493,7 +1957,7 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
     if (err == cudaSuccess && WIDE_TILES)
       err = cudaFuncSetAttribute(paged_attention_mma_kernel<WIDE_TILES ? 2 : 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_SMEM_2);
     if (err == cudaSuccess) err = cudaFuncSetAttribute(paged_attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_GATHER);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(paged_attention_decode_kernel<TMA_HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_TMA);
+    if (err == cudaSuccess) err = configure_runs<TMA_HEAD>();
 #define PYLON_CLUSTER_CASE(N)                                                                                                   \
     if (err == cudaSuccess && TMA_HEAD)                                                                                         \
       err = cudaFuncSetAttribute(paged_attention_decode_kernel<TMA_HEAD, TMA_HEAD ? N : 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_CLUSTER);
@@ -1552,8 +2016,6 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
     const long long pool_rows = (long long)num_pages * nkv * page_size;
     const bool tma = TMA_HEAD && page_size % BLOCK_N == 0 && pool_rows < 2147483647LL - BLOCK_N;
     if (tma) {
-      if (!page_pool_map(&map_k, k_pages, pool_rows) || !page_pool_map(&map_v, v_pages, pool_rows))
-        PYLON_REFUSE("paged_attention_mma: the tensor maps of the page pools could not be made");
       // Few pairs of about equal length: a cluster of blocks for each (16 where the device places such clusters), as large as leaves two blocks to an SM (with three,
       // clusters measured slower than the runs: 3.23 against 2.97 ms a step at batch 8) and within the caller's blocks.
       const long long pairs = (long long)num_rows * nkv;
@@ -1563,6 +2025,9 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
         size = (room >= 16 && clusters_of_16()) ? 16 : room >= 8 ? 8 : room >= 6 ? 6 : room >= 4 ? 4 : room >= 3 ? 3 : room >= 2 ? 2 : 0;
         if (pairs * size > decode_blocks) size = 0;
       }
+      const int box_rows = size ? BLOCK_N : RUN_KEYS;
+      if (!page_pool_map(&map_k, k_pages, pool_rows, box_rows) || !page_pool_map(&map_v, v_pages, pool_rows, box_rows))
+        PYLON_REFUSE("paged_attention_mma: the tensor maps of the page pools could not be made");
 #define PYLON_CLUSTER_CASE(N)                                                                                                   \
       if (size == N) launch_dependent_cluster(paged_attention_decode_kernel<TMA_HEAD, TMA_HEAD ? N : 0>, dim3((unsigned)(pairs * N)), dim3(ATT_THREADS), dec_smem_cluster(p.incoming_rows, N), \
                                               stream, N, p, map_k, map_v);
@@ -1573,8 +2038,7 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
       }
       PYLON_CLUSTER_CASE(16) PYLON_CLUSTER_CASE(8) PYLON_CLUSTER_CASE(6) PYLON_CLUSTER_CASE(4) PYLON_CLUSTER_CASE(3) PYLON_CLUSTER_CASE(2)
 #undef PYLON_CLUSTER_CASE
-      if (size == 0)
-        launch_dependent(paged_attention_decode_kernel<TMA_HEAD>, dim3(decode_blocks), dim3(ATT_THREADS), DEC_SMEM_TMA, stream, p, map_k, map_v);
+      if (size == 0) launch_runs<TMA_HEAD>(p, decode_blocks, map_k, map_v, stream);
     } else {
       launch_dependent(paged_attention_decode_kernel<false>, dim3(decode_blocks), dim3(ATT_THREADS), DEC_SMEM_GATHER, stream, p, map_k, map_v);
     }

@@ -1,0 +1,353 @@
+// y = x W^T in bfloat16 for up to 256 rows of x on the fifth-generation tensor cores, with the weights on the wide side of the tile: 128 rows of
+// W are the M of a tcgen05.mma and the rows of x, rounded up to 16, its N.  For the steps between a few decoded rows and a long prompt.
+//
+// Bound by the bytes of W: every weight row is read once, whatever M is, and rows of x fill no more than the last 16 columns of the tile (with x on
+// the M side 33 rows cost what 128 do).  A block takes 128 rows of W and a slice of k; two blocks share an SM where N leaves
+// room, so that one's epilogue overlaps the other's loads.  Four warps: one lane of the first asks for boxes of W and x (TMA, 128-byte
+// swizzle) into a ring of stages - the boxes of W that nothing queued writes before it waits for the kernel ahead - one lane of the second issues the
+// products, and all four read the accumulator back, each its 32 lanes, a lane being a row of W: 32 neighbouring numbers of a row of y.
+//
+// The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k: k is cut into as many chains as
+// fit beside each other in 256 columns of tensor memory (256 / N, 512 k or more each), which the epilogue adds in float32.
+//
+// All waits on mbarriers are bounded: one that runs out sets an error word, the block waits for its own copies, frees its tensor memory and returns.
+// No TMA load here uses cluster multicast.
+//
+// Stands in for the library product behind raun6k/Pylon's nn.Linear (src/pylon/model/layers.py:26-27,126,138).
+#include "common.cuh"
+
+#include <cuda.h>
+
+#include <algorithm>
+#include <functional>
+#include <mutex>
+#include <unordered_map>
+
+namespace pylon {
+
+constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 128, GC_MOST_STAGES = 8, GC_CHAIN = 8;   // weight rows and k of a box; boxes of a chain at least
+constexpr int GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
+constexpr unsigned GC_WAIT_LIMIT = 1u << 22;                                                 // try_wait calls before a wait gives up
+enum GcForm { GC_PARTIAL = 0, GC_PRODUCT = 1, GC_GATED = 2 };
+
+__device__ __forceinline__ uint32_t gc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void gc_mbar_init(uint64_t* bar, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(gc_smem(bar)), "r"(count)); }
+__device__ __forceinline__ void gc_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(gc_smem(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool gc_wait(uint64_t* bar, uint32_t parity) {
+  for (unsigned tries = 0; tries < GC_WAIT_LIMIT; ++tries) {
+    uint32_t done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(gc_smem(bar)), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void gc_load(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+               ::"r"(gc_smem(dst)), "l"((uint64_t)map), "r"(gc_smem(bar)), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void gc_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(gc_smem(bar)) : "memory");
+}
+__device__ __forceinline__ void gc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// 16 consecutive float32 columns of this thread's lane of tensor memory; valid after gc_read_done().
+__device__ __forceinline__ void gc_read(uint32_t address, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                 "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(address));
+}
+__device__ __forceinline__ void gc_read_done() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void gc_cluster_barrier() { asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+// A K-major tile whose rows are 128 bytes in the 128-byte swizzle: start address, 1024 bytes between groups of 8 rows, version 1, swizzle 128B.
+__device__ __forceinline__ uint64_t gc_desc(const void* tile) {
+  return (uint64_t)((gc_smem(tile) & 0x3FFFF) >> 4) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ float gc_unit(float gate, float up, float limit, float alpha) {
+  float gain = 1.f;
+  if (limit > 0.f) {   // the clamped unit: min(gate, limit) * sigmoid(alpha * gate) * (clamp(up, -limit, limit) + 1)
+    gate = fminf(gate, limit);
+    up = fminf(fmaxf(up, -limit), limit) + 1.f;
+    gain = alpha;
+  }
+  return __fdividef(gate, 1.f + __expf(-gain * gate)) * up;   // approximate division: ample for bfloat16, no slow path
+}
+__device__ __forceinline__ uint32_t gc_pack(float a, float b) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
+struct GcArgs {
+  void* y;
+  long long ldy;
+  int M, N, K, columns, stages, tmem_columns;   // columns: M rounded up to 16
+  float unit_limit, unit_alpha;
+  int w_static;
+  int* error;   // 1: the copies, 2: the products, 3: the accumulator did not come in time
+};
+
+// Grid (slices of k, tiles of 128 weight rows).  With several slices the product and the gated unit run as clusters of them.
+template <int FORM>
+__global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GcArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full[GC_MOST_STAGES], empty[GC_MOST_STAGES], done;
+  __shared__ uint32_t tmem_slot;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int columns = a.columns, stages = a.stages, w_bytes = GC_ROWS * GC_BK * 2, x_bytes = columns * GC_BK * 2;
+  unsigned char* w_tiles = smem;
+  unsigned char* x_tiles = smem + stages * w_bytes;
+  const int boxes_of_k = (a.K + GC_BK - 1) / GC_BK, parts = gridDim.x;
+  const int box0 = (int)((long long)boxes_of_k * blockIdx.x / parts), boxes = (int)((long long)boxes_of_k * (blockIdx.x + 1) / parts) - box0;
+  const int row0 = blockIdx.y * GC_ROWS;
+  const int most_chains = max(1, a.tmem_columns / columns), chain = max(GC_CHAIN, (boxes + most_chains - 1) / most_chains), chains = (boxes + chain - 1) / chain;
+
+  const int ahead = a.w_static ? min(stages, boxes) : 0;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) { gc_mbar_init(&full[s], 1); gc_mbar_init(&empty[s], 1); }
+    gc_mbar_init(&done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    for (int s = 0; s < ahead; ++s) {
+      gc_expect(&full[s], w_bytes + x_bytes);
+      gc_load(w_tiles + s * w_bytes, &map_w, &full[s], (box0 + s) * GC_BK, row0);
+    }
+  }
+  if (warp == 1) {   // the whole warp allocates
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(gc_smem(&tmem_slot)), "r"(a.tmem_columns));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  grid_dependency_wait();
+  allow_dependents();
+
+  int issued = 0;   // boxes asked for (the first thread's)
+  if (warp == 0 && lane == 0) {
+    for (; issued < boxes; ++issued) {
+      const int s = issued % stages;
+      if (issued >= ahead) {
+        if (issued >= stages && !gc_wait(&empty[s], (issued / stages - 1) & 1)) { atomicExch(a.error, 1); break; }
+        gc_expect(&full[s], w_bytes + x_bytes);
+        gc_load(w_tiles + s * w_bytes, &map_w, &full[s], (box0 + issued) * GC_BK, row0);
+      }
+      gc_load(x_tiles + s * x_bytes, &map_x, &full[s], (box0 + issued) * GC_BK, 0);
+    }
+  } else if (warp == 1 && lane == 0) {
+    // Instruction descriptor of kind::f16: bfloat16 A and B, float32 D, both K-major.
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(GC_ROWS >> 4) << 24);
+    bool alive = true;
+    for (int box = 0; box < boxes; ++box) {
+      const int s = box % stages;
+      if (!gc_wait(&full[s], (box / stages) & 1)) { atomicExch(a.error, 2); alive = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint64_t w_desc = gc_desc(w_tiles + s * w_bytes), x_desc = gc_desc(x_tiles + s * x_bytes);
+      const int first = box % chain == 0;
+#pragma unroll
+      for (int k = 0; k < GC_BK / 16; ++k)   // 16 k are 32 bytes further along the swizzled row: +2 in 16-byte units
+        gc_mma(tmem + box / chain * columns, w_desc + 2 * k, x_desc + 2 * k, idesc, !(first && k == 0));
+      gc_commit(&empty[s]);
+    }
+    if (alive) gc_commit(&done);
+  }
+  __syncwarp();
+  const bool complete = gc_wait(&done, 0);
+  if (!complete && lane == 0) atomicExch(a.error, 3);
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+
+  // This thread's row of W; what it has of 16 rows of x from c0 on goes to y.
+  const int n = row0 + threadIdx.x;
+  auto write = [&](int c0, const float (&v)[16]) {
+    if (FORM == GC_PARTIAL) {
+      float* dst = reinterpret_cast<float*>(a.y) + ((size_t)blockIdx.x * a.M + c0) * a.N + n;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (n < a.N && c0 + j < a.M) dst[(size_t)j * a.N] = v[j];
+    } else if (FORM == GC_PRODUCT) {
+      // Neighbouring lanes exchange, so that each stores two neighbouring numbers: even lanes of the even rows of x, odd lanes of the odd ones.
+      const int odd = lane & 1;
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.y) + (size_t)(c0 + odd) * a.ldy + (n - odd);
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+        if (n < a.N && c0 + j + odd < a.M) *reinterpret_cast<uint32_t*>(dst + (size_t)j * a.ldy) = odd ? gc_pack(other, v[j + 1]) : gc_pack(v[j], other);
+      }
+    } else {
+      // Rows of gate and up alternate in groups of 8: lanes 8 apart exchange, the gate's lane then makes the even rows of x, the up's the odd ones.
+      const int is_up = (lane >> 3) & 1;
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.y) + (size_t)(c0 + is_up) * a.ldy + (n >> 4) * 8 + (n & 7);
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, is_up ? v[j] : v[j + 1], 8);
+        const float unit = is_up ? gc_unit(other, v[j + 1], a.unit_limit, a.unit_alpha) : gc_unit(v[j], other, a.unit_limit, a.unit_alpha);
+        if (n < a.N && c0 + j + is_up < a.M) dst[(size_t)j * a.ldy] = __float2bfloat16_rn(unit);
+      }
+    }
+  };
+  // The block's sums of 16 rows of x, its chains added up in order.
+  const uint32_t lane_address = tmem + ((uint32_t)(warp * 32) << 16);
+  auto sums = [&](int c0, float (&v)[16]) {
+    uint32_t raw[16];
+    gc_read(lane_address + c0, raw);
+    gc_read_done();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(raw[j]);
+    for (int c = 1; c < chains; ++c) {
+      gc_read(lane_address + c * columns + c0, raw);
+      gc_read_done();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(raw[j]);
+    }
+  };
+  float v[16];
+  if (FORM == GC_PARTIAL || parts == 1) {
+    for (int c0 = 0; complete && c0 < columns; c0 += 16) {
+      sums(c0, v);
+      write(c0, v);
+    }
+  } else {
+    // The slices of k are the blocks of a cluster: groups of 16 rows of x are dealt out to them, a block sends each other one the groups that it adds up.
+    const int rank = blockIdx.x, groups = columns / 16, most = (groups + parts - 1) / parts;
+    float* received = reinterpret_cast<float*>(smem);   // [slice][group][16][128], where the stages were
+    gc_cluster_barrier();   // every block's products have read their stages
+    for (int group = 0; group < groups; ++group) {
+      sums(group * 16, v);
+      uint32_t remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(gc_smem(received + (size_t)(rank * most + group / parts) * 16 * GC_ROWS + threadIdx.x)), "r"(group % parts));
+#pragma unroll
+      for (int j = 0; j < 16; ++j) asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote + j * GC_ROWS * 4), "f"(v[j]) : "memory");
+    }
+    gc_cluster_barrier();   // all that was sent is there
+    for (int group = rank; complete && group < groups; group += parts) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = 0.f;
+      for (int slice = 0; slice < parts; ++slice)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += received[((size_t)(slice * most + group / parts) * 16 + j) * GC_ROWS + threadIdx.x];
+      write(group * 16, v);
+    }
+  }
+  if (!complete && threadIdx.x == 0)   // no copy outlives the block
+    for (int box = max(0, issued - stages); box < issued; ++box) gc_wait(&full[box % stages], (box / stages) & 1);
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(a.tmem_columns));
+}
+
+// ---------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// Tensor map of a row-major bfloat16 matrix [rows, cols] (row stride ld elements) with boxes of box_rows x 64 columns in the 128-byte
+// swizzle.  Maps are kept by all their arguments (they are a function of them): a model multiplies by the same matrices at every step.
+static bool matrix_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows) {
+  struct Key {
+    const void* base; long long rows, cols, ld; int box_rows;
+    bool operator==(const Key& o) const { return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows; }
+  };
+  struct Hash {
+    size_t operator()(const Key& k) const { return std::hash<const void*>()(k.base) ^ (size_t)(k.rows * 1315423911LL) ^ (size_t)(k.cols * 2654435761LL) ^ (size_t)k.box_rows; }
+  };
+  static std::unordered_map<Key, CUtensorMap, Hash> known;
+  static std::mutex mutex;
+  static EncodeTiled encode = nullptr;
+  std::lock_guard<std::mutex> guard(mutex);
+  if (!encode) {
+    void* symbol = nullptr;
+    cudaDriverEntryPointQueryResult result;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &symbol, cudaEnableDefault, &result) != cudaSuccess || result != cudaDriverEntryPointSuccess) return false;
+    encode = (EncodeTiled)symbol;
+  }
+  const Key key{base, rows, cols, ld, box_rows};
+  auto found = known.find(key);
+  if (found != known.end()) { *map = found->second; return true; }
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {(cuuint32_t)GC_BK, (cuuint32_t)box_rows};
+  cuuint32_t element_strides[2] = {1, 1};
+  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return false;
+  if (known.size() >= 4096) known.clear();   // activations come and go; the weights' maps are made again on demand
+  known.emplace(key, *map);
+  return true;
+}
+
+constexpr int GC_SMEM_SHARED = 112 * 1024, GC_SMEM_ALONE = 224 * 1024;   // of one of two blocks on an SM, of a lone one
+
+template <int FORM>
+static int launch_columns(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts, int per_sm,
+                          float limit, float alpha, int w_static, int* error, cudaStream_t stream, const char* name) {
+  if (M <= 0 || N <= 0) return 0;
+  if (M > 256) PYLON_REFUSE("%s: M = %d is more than 256 rows", name, M);
+  if (K <= 0 || K % 8 || ldx % 8 || ldw % 8) PYLON_REFUSE("%s: K = %d and the row strides must be multiples of 8", name, K);
+  if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 4)) PYLON_REFUSE("%s: x and w must be 16-byte aligned", name);
+  if (ldx < K || ldw < K) PYLON_REFUSE("%s: a row stride is shorter than its row", name);
+  const int boxes = (K + GC_BK - 1) / GC_BK, tiles = (N + GC_ROWS - 1) / GC_ROWS;
+  if (parts < 1 || parts > boxes || parts > 65535 || tiles > 65535) PYLON_REFUSE("%s: %d parts over %d slices of k, %d tiles", name, parts, boxes, tiles);
+  if (FORM != GC_PARTIAL && parts > 8) PYLON_REFUSE("%s: %d slices of k, a cluster has 8 blocks at most", name, parts);
+  if (per_sm < 1 || per_sm > 2) PYLON_REFUSE("%s: %d blocks to an SM", name, per_sm);
+  if (!error) PYLON_REFUSE("%s: an error word is needed", name);
+  auto kernel = gemm_columns_kernel<FORM>;
+  static bool configured_on[MAX_DEVICES] = {};   // function attributes belong to a device
+  bool& configured = configured_on[current_device_slot()];
+  if (!configured) {
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM_ALONE);
+    if (err != cudaSuccess) PYLON_REFUSE("%s: %s", name, cudaGetErrorString(err));
+    configured = true;
+  }
+  GcArgs a;
+  a.y = y; a.ldy = ldy; a.M = M; a.N = N; a.K = K;
+  a.columns = (M + 15) / 16 * 16;
+  const int stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2, room = (per_sm == 2 ? GC_SMEM_SHARED : GC_SMEM_ALONE) - 1024, slice = (boxes + parts - 1) / parts;
+  a.stages = std::min({room / stage_bytes, GC_MOST_STAGES, slice});
+  const int wanted = std::min(a.columns * ((slice + GC_CHAIN - 1) / GC_CHAIN), GC_COLUMNS);
+  a.tmem_columns = 32;
+  while (a.tmem_columns < wanted) a.tmem_columns *= 2;
+  a.unit_limit = limit; a.unit_alpha = alpha; a.w_static = w_static; a.error = error;
+  CUtensorMap map_w, map_x;
+  if (!matrix_map(&map_w, w, N, K, ldw, GC_ROWS) || !matrix_map(&map_x, x, M, K, ldx, a.columns)) PYLON_REFUSE("%s: the tensor maps could not be made", name);
+  const size_t ring = (size_t)a.stages * stage_bytes, groups = a.columns / 16, received = (groups + parts - 1) / parts * parts * 16 * GC_ROWS * sizeof(float);
+  if (FORM == GC_PARTIAL || parts == 1)
+    launch_dependent<LAUNCH_GEMM>(kernel, dim3(parts, tiles), dim3(GC_THREADS), ring + 1024, stream, map_w, map_x, a);
+  else
+    launch_dependent_cluster<LAUNCH_GEMM>(kernel, dim3(parts, tiles), dim3(GC_THREADS), std::max(ring, received) + 1024, stream, (unsigned)parts, map_w, map_x, a);
+  PYLON_CHECK_LAUNCH(name);
+}
+
+}  // namespace pylon
+
+// x: bfloat16 [M, K] (row stride ldx), M <= 256; w: bfloat16 [N, K] (row stride ldw); y: float32 [parts, M, N] contiguous, whose sum over the
+// first dimension is x @ w.T.  K and the row strides multiples of 8, x and w 16-byte aligned, 1 <= parts <= number of 64-wide slices of
+// k; per_sm: 1 or 2 blocks to an SM.  error: one int in device memory that the kernel sets non-zero if one of its waits ran out (the
+// result is then void).  w_static: 1 where nothing queued on the stream writes w; its first boxes are then asked for while the kernel ahead is still running.
+extern "C" int pylon_gemm_columns_partial(const void* x, const void* w, float* y, int M, int N, int K, long long ldx, long long ldw, int parts, int per_sm,
+                                          int* error, int w_static, cudaStream_t stream) {
+  return pylon::launch_columns<pylon::GC_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, parts, per_sm, 0.f, 1.f, w_static, error, stream, "gemm_columns_partial");
+}
+
+// The product itself: y bfloat16 [M, N], row stride ldy; N and ldy even; up to 8 slices of k, added up in a cluster.
+extern "C" int pylon_gemm_columns_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts,
+                                       int per_sm, int* error, int w_static, cudaStream_t stream) {
+  if (ldy < N || N % 2 || ldy % 2) PYLON_REFUSE("gemm_columns_bf16: N = %d and the result's row stride must be even, the stride no shorter than a row", N);
+  return pylon::launch_columns<pylon::GC_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, parts, per_sm, 0.f, 1.f, w_static, error, stream, "gemm_columns_bf16");
+}
+
+// The gated unit of x gate^T and x up^T: w's rows are interleaved in groups of 8 (rows 16b..16b+7 gate rows 8b..8b+7, rows 16b+8..16b+15 the matching up
+// rows; N a multiple of 16); y bfloat16 [M, N / 2], row stride ldy.  limit 0: silu(gate) * up; limit > 0: the clamped unit,
+// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).  Slices of k as for the product.
+extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, float limit,
+                                        float alpha, int parts, int per_sm, int* error, int w_static, cudaStream_t stream) {
+  if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_columns_gated: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
+  if (limit < 0.f) PYLON_REFUSE("gemm_columns_gated: the limit must not be negative");
+  return pylon::launch_columns<pylon::GC_GATED>(x, w, y, M, N, K, ldx, ldw, ldy, parts, per_sm, limit, alpha, w_static, error, stream, "gemm_columns_gated");
+}

@@ -274,6 +274,12 @@ _SIGNATURES = {
         "pylon_gemm_stream_swiglu": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_int, c_void_p],
         "pylon_gemm_stream_glu_clamped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_int, c_void_p],
     },
+    "gemm_columns.cu": {
+        "pylon_gemm_columns_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p],
+        "pylon_gemm_columns_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p],
+        "pylon_gemm_columns_gated": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_int, c_int,
+                                     c_void_p, c_int, c_void_p],
+    },
     "gemm_tcgen05.cu": {
         "pylon_gemm_tcgen05_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
                                     c_void_p, c_int, c_int, c_void_p],
@@ -842,6 +848,33 @@ def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit:
         return y
     entry = library.pylon_gemm_stream_swiglu if swiglu else library.pylon_gemm_stream_bf16
     _check(library, entry(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), _ptr(stream_error_word(x.device)), int(static_weights), _stream()))
+    return y
+
+
+def linear_columns(x: torch.Tensor, w: torch.Tensor, form: str = "product", parts: int = 1, limit: Optional[float] = None, alpha: float = 1.0,
+                   static_weights: bool = False, per_sm: int = 2) -> torch.Tensor:
+    """bfloat16 ``x [M <= 256, K] @ w [N, K].T`` on the tcgen05 kernel whose tiles are 128 weight rows wide and as many rows of ``x`` deep as there are.
+    ``form``: ``"product"`` (bfloat16 ``[M, N]``), ``"partial"`` (float32 sums over ``parts`` slices of k, ``[parts, M, N]``) or ``"gated"`` (the rows of ``w``
+    interleaved by :func:`interleave_gate_up`, the unit of :func:`linear_stream`, ``[M, N / 2]``).  ``parts``: slices of k (up to 8 in the other two forms,
+    whose blocks add them up in a cluster); ``per_sm``: blocks that share an SM."""
+    _need_cuda(x, w)
+    _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16,
+          "linear_columns: bfloat16 x [M, K] and w [N, K]")
+    _need(x.stride(1) == 1 and w.stride(1) == 1, "linear_columns: the reduced dimension must be contiguous")
+    _need(form in ("product", "partial", "gated"), f"linear_columns: unknown form {form!r}")
+    m, k = x.shape
+    n = w.shape[0]
+    library, error, static = _library("gemm_columns.cu"), _ptr(stream_error_word(x.device)), int(static_weights)
+    if form == "partial":
+        y = torch.empty((parts, m, n), dtype=torch.float32, device=x.device)
+        _check(library, library.pylon_gemm_columns_partial(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), parts, per_sm, error, static, _stream()))
+        return y
+    y = torch.empty((m, n // 2 if form == "gated" else n), dtype=torch.bfloat16, device=x.device)
+    if form == "gated":
+        _check(library, library.pylon_gemm_columns_gated(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit or 0.0), float(alpha),
+                                                         parts, per_sm, error, static, _stream()))
+    else:
+        _check(library, library.pylon_gemm_columns_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), parts, per_sm, error, static, _stream()))
     return y
 
 

@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(128) delta_recurrence_exact_kernel(const float
 // kernel of its own makes them for all chunks at once; what is left of the walk is three small products a chunk.  (The chunked form of delta
 // rules: Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence Length", 2024.)  D is multiplied up and never
 // divided, so decays that vanish do no harm.  A row's chunks start at the first token it brings.
-constexpr int WALK_THREADS = 256, CHUNK = 16, CHUNK_MATRIX = 2 * CHUNK * CHUNK + 2 * CHUNK;   // T | B | G | D[last]
+constexpr int CHUNK = 16, CHUNK_MATRIX = 2 * CHUNK * CHUNK + 2 * CHUNK;   // T | B | G | D[last]
 
 // Chunk c of row r has the number q_start[r] / CHUNK + r + c: rows' numbers do not meet, and all lie below tokens / CHUNK + rows + 1.
 // grid (those numbers, kv_heads), 128 threads; matrices: float32 [numbers, heads, CHUNK_MATRIX].
@@ -622,41 +622,40 @@ __global__ void __launch_bounds__(128) delta_chunk_matrices_kernel(const float* 
   }
 }
 
-// sum + entries 0 .. t of a row of a lower triangular CHUNK x CHUNK matrix times a column's values of the tokens 0 .. t.  The row's
-// entries behind t are zeros, but what they would be multiplied by need not be finite: zeros take its place.  (A multiply-add under a condition
-// each, or sums of the warps' own lengths, took longer: 277 and 274 us for 2,048 tokens, all kernels, where this took 267.)
+// sum + entries 0 .. t of a row of a lower triangular CHUNK x CHUNK matrix times two columns' values of the tokens 0 .. t.  The row's
+// entries behind t are zeros, but what they would be multiplied by need not be finite: zeros take its place.  (2,048 tokens, all
+// kernels: 267 us, 259 without the zeros; a multiply-add under a condition each 277, the four warps' sums each of their own length 274.)
 template <int COLS>
-__device__ __forceinline__ float delta_lower_sum(const float* row, const float* column, int t, float sum) {
-  float x[CHUNK];
+__device__ __forceinline__ float2 delta_lower_sum(const float* row, const float* columns, int t, float2 sum) {
+  float2 x[CHUNK];
   float4 m[CHUNK / 4];
 #pragma unroll
-  for (int i = 0; i < CHUNK; ++i) x[i] = column[i * COLS];
+  for (int i = 0; i < CHUNK; ++i) x[i] = *reinterpret_cast<const float2*>(columns + i * COLS);
 #pragma unroll
   for (int i = 0; i < CHUNK / 4; ++i) m[i] = *reinterpret_cast<const float4*>(row + 4 * i);
 #pragma unroll
   for (int i = 0; i < CHUNK; ++i)
-    if (i > t) x[i] = 0.f;
+    if (i > t) x[i] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < CHUNK; i += 4) {
     const float each[4] = {m[i / 4].x, m[i / 4].y, m[i / 4].z, m[i / 4].w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sum = fmaf(each[j], x[i + j], sum);
+    for (int j = 0; j < 4; ++j) { sum.x = fmaf(each[j], x[i + j].x, sum.x); sum.y = fmaf(each[j], x[i + j].y, sum.y); }
   }
   return sum;
 }
 
-// The walk over the chunks: grid (slices of 16 columns, heads, rows), eight warps.  Every warp holds the slice of S whole, 64 numbers a
+// The walk over the chunks: grid (slices of 16 columns, heads, rows), 128 threads.  Every warp holds the slice of S whole, 64 numbers a
 // thread (16 entries of 4 columns), so that a read of a key or query serves 16 multiply-adds and S is never an operand in shared memory; the warps share
 // the 32 sums over S (16 keys, 16 queries) by rows and the update of S by entries, and give each other what they have updated through
 // shared memory.  Three barriers a chunk.  A lane's entries hang on its bits {0, 3, 4} and its columns on {1, 2}: 16-byte reads that differ in bits
-// {0, 1, 2} take twice as long.  Bound by the latencies of a chunk's dependent steps, of which two warps a scheduler hide some (four warps of twice the rows
-// and entries each: 3,000 cycles a chunk for 1,400 instructions a warp, 204 us for 2,048 tokens of 16 heads of 128 x 128 on 128 blocks; the
-// walk token by token 525).
+// {0, 1, 2} take twice as long.  2,048 tokens of 16 heads of 128 x 128, 128 blocks: 193 us (the walk token by token 525): 3,000 cycles a
+// chunk, 1,400 instructions of each of an SM's four warps, which nothing else hides the latencies of.
 template <int DIM>
-__global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const float* __restrict__ qkv, const float* __restrict__ matrices, float* __restrict__ state,
+__global__ void __launch_bounds__(128) delta_chunk_walk_kernel(const float* __restrict__ qkv, const float* __restrict__ matrices, float* __restrict__ state,
                                                                long long slot_floats, const int* __restrict__ q_start, const int* __restrict__ slots,
                                                                float* __restrict__ out, int heads, int kv_heads, int vdim) {
-  static_assert(DIM == 128 && WALK_THREADS == 256, "a warp updates an eighth of the entries, eight lanes' two each");
+  static_assert(DIM == 128, "a warp updates a fourth of the entries, eight lanes' four each");
   constexpr int COLS = 16, STAGE = 2 * CHUNK * DIM + CHUNK * COLS + CHUNK_MATRIX;   // keys | queries | values | matrices
   extern __shared__ __align__(16) float stages[];
   float* s_shared = stages + 2 * STAGE;        // [4][4][32 lanes' order][4]
@@ -683,7 +682,7 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const fl
       const int bytes = there ? 16 : 0;   // zeros for tokens that are not there
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from), "r"(bytes) : "memory");
     };
-    for (int x = tid; x < CHUNK * DIM / 4; x += WALK_THREADS) {
+    for (int x = tid; x < CHUNK * DIM / 4; x += 128) {
       const int t = x / (DIM / 4), e = (x % (DIM / 4)) * 4;
       const float* src = qkv + (long long)(first + min(t, count - 1)) * channels + e;
       copy(dst + t * DIM + e, src + k_col, t < count);
@@ -694,18 +693,17 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const fl
       copy(dst + 2 * CHUNK * DIM + t * COLS + e, qkv + (long long)(first + min(t, count - 1)) * channels + v_col + e, t < count);
     }
     const float* from = matrices + ((number0 + chunk) * heads + head) * CHUNK_MATRIX;
-    if (tid < CHUNK_MATRIX / 4) copy(dst + 2 * CHUNK * DIM + CHUNK * COLS + 4 * tid, from + 4 * tid, true);
+    for (int x = tid; x < CHUNK_MATRIX / 4; x += 128) copy(dst + 2 * CHUNK * DIM + CHUNK * COLS + 4 * x, from + 4 * x, true);
     delta_copy_commit();
   };
 
-  // s[n][j]: entry 4 (m 8 + dg) + j, columns 4 cg .. + 3, with m = (warp / 2 + n) % 4.  Of s[0] this warp updates the entries j = first_entry and + 1.
-  const int group = warp >> 1, first_entry = (warp & 1) * 2;
-  float4 s[4][4], own[2];
+  // s[n][j]: entry 4 (m 8 + dg) + j, columns 4 cg .. + 3, with m = (warp + n) % 4: s[0] is what this warp updates
+  float4 s[4][4];
   fetch(0, 0);
 #pragma unroll
   for (int n = 0; n < 4; ++n)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s[n][j] = *reinterpret_cast<const float4*>(mine + (long long)(4 * ((((group + n) & 3) << 3) + dg) + j) * vdim);
+    for (int j = 0; j < 4; ++j) s[n][j] = *reinterpret_cast<const float4*>(mine + (long long)(4 * ((((warp + n) & 3) << 3) + dg) + j) * vdim);
 
   const int chunks = (end - begin + CHUNK - 1) / CHUNK;
   for (int chunk = 0; chunk < chunks; ++chunk) {
@@ -720,20 +718,20 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const fl
     const float* behind = up_to + CHUNK;
     if (chunk > 0) {
 #pragma unroll
-      for (int n = 0; n < 4; ++n)
+      for (int n = 1; n < 4; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          s[n][j] = *reinterpret_cast<const float4*>(s_shared + (((((group + n) & 3) << 2) + j) * 32 + dg * 4 + cg) * 4);
+          s[n][j] = *reinterpret_cast<const float4*>(s_shared + (((((warp + n) & 3) << 2) + j) * 32 + dg * 4 + cg) * 4);
     }
-    // this warp's rows: keys 2 warp and + 1, then queries 2 warp and + 1
-    float4 part[4];
+    // this warp's rows: keys 4 warp .. + 3, then queries 4 warp .. + 3
+    float4 part[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) part[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < 8; ++i) part[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 x = *reinterpret_cast<const float4*>(keys + ((i >> 1) * CHUNK + 2 * warp + (i & 1)) * DIM + 4 * ((((group + n) & 3) << 3) + dg));
+      for (int i = 0; i < 8; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(keys + ((i >> 2) * CHUNK + 4 * warp + (i & 3)) * DIM + 4 * ((((warp + n) & 3) << 3) + dg));
         const float each[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -741,20 +739,24 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const fl
           part[i].z = fmaf(each[j], s[n][j].z, part[i].z); part[i].w = fmaf(each[j], s[n][j].w, part[i].w);
         }
       }
-    // over the eight lanes of a row: in two rounds a lane keeps half of its rows and hands on the others, in the third both lanes add
-    auto exchange = [&](float4 keep, float4 give, int bit) {
-      return make_float4(keep.x + __shfl_xor_sync(0xffffffffu, give.x, bit), keep.y + __shfl_xor_sync(0xffffffffu, give.y, bit),
-                         keep.z + __shfl_xor_sync(0xffffffffu, give.z, bit), keep.w + __shfl_xor_sync(0xffffffffu, give.w, bit));
+    // over the eight lanes of a row: each round a lane keeps half of its rows and hands on the others
+    auto halve = [&](auto& rows, int kept, int bit) {
+      const bool upper = lane & bit;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= kept) continue;
+        const float4 give = upper ? rows[i] : rows[i + kept], keep = upper ? rows[i + kept] : rows[i];
+        rows[i] = make_float4(keep.x + __shfl_xor_sync(0xffffffffu, give.x, bit), keep.y + __shfl_xor_sync(0xffffffffu, give.y, bit),
+                              keep.z + __shfl_xor_sync(0xffffffffu, give.z, bit), keep.w + __shfl_xor_sync(0xffffffffu, give.w, bit));
+      }
     };
-    const bool query = lane & 16, second = lane & 8;
-    part[0] = exchange(query ? part[2] : part[0], query ? part[0] : part[2], 16);
-    part[1] = exchange(query ? part[3] : part[1], query ? part[1] : part[3], 16);
-    part[0] = exchange(second ? part[1] : part[0], second ? part[0] : part[1], 8);
-    part[0] = exchange(part[0], part[0], 1);
-    if ((lane & 1) == 0) {
-      const int t = 2 * warp + (second ? 1 : 0);
+    halve(part, 4, 16);
+    halve(part, 2, 8);
+    halve(part, 1, 1);
+    {
+      const int t = 4 * warp + ((lane >> 2) & 2) + (lane & 1);
       const float g = up_to[t];
-      if (query) {
+      if (lane & 16) {
         *reinterpret_cast<float4*>(r + t * COLS + 4 * cg) = make_float4(g * part[0].x, g * part[0].y, g * part[0].z, g * part[0].w);
       } else {
         const float4 v = *reinterpret_cast<const float4*>(values + t * COLS + 4 * cg);
@@ -762,38 +764,40 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const fl
       }
     }
     __syncthreads();
-    const int t = tid >> 4, c = tid & 15;
+    const int t = tid >> 3, c = (tid & 7) * 2;
     {
-      const float sum = delta_lower_sum<COLS>(t_matrix + t * CHUNK, u + c, t, 0.f);
-      w[t * COLS + c] = sum;
-      wd[t * COLS + c] = behind[t] * sum;
+      const float2 sum = delta_lower_sum<COLS>(t_matrix + t * CHUNK, u + c, t, make_float2(0.f, 0.f));
+      const float d = behind[t];
+      *reinterpret_cast<float2*>(w + t * COLS + c) = sum;
+      *reinterpret_cast<float2*>(wd + t * COLS + c) = make_float2(d * sum.x, d * sum.y);
     }
     __syncthreads();
     {
       const float all = up_to[CHUNK - 1];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const float4 x = first_entry ? s[0][2 + j] : s[0][j];
-        own[j] = make_float4(all * x.x, all * x.y, all * x.z, all * x.w);
-      }
+      for (int j = 0; j < 4; ++j) { s[0][j].x *= all; s[0][j].y *= all; s[0][j].z *= all; s[0][j].w *= all; }
 #pragma unroll
       for (int i = 0; i < CHUNK; ++i) {
-        const float2 k = *reinterpret_cast<const float2*>(keys + i * DIM + 4 * ((group << 3) + dg) + first_entry);
+        const float4 k = *reinterpret_cast<const float4*>(keys + i * DIM + 4 * ((warp << 3) + dg));
         const float4 x = *reinterpret_cast<const float4*>(wd + i * COLS + 4 * cg);
-        own[0].x = fmaf(k.x, x.x, own[0].x); own[0].y = fmaf(k.x, x.y, own[0].y); own[0].z = fmaf(k.x, x.z, own[0].z); own[0].w = fmaf(k.x, x.w, own[0].w);
-        own[1].x = fmaf(k.y, x.x, own[1].x); own[1].y = fmaf(k.y, x.y, own[1].y); own[1].z = fmaf(k.y, x.z, own[1].z); own[1].w = fmaf(k.y, x.w, own[1].w);
+        const float each[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[0][j].x = fmaf(each[j], x.x, s[0][j].x); s[0][j].y = fmaf(each[j], x.y, s[0][j].y);
+          s[0][j].z = fmaf(each[j], x.z, s[0][j].z); s[0][j].w = fmaf(each[j], x.w, s[0][j].w);
+        }
       }
 #pragma unroll
-      for (int j = 0; j < 2; ++j) *reinterpret_cast<float4*>(s_shared + (((group << 2) + first_entry + j) * 32 + dg * 4 + cg) * 4) = own[j];
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(s_shared + (((warp << 2) + j) * 32 + dg * 4 + cg) * 4) = s[0][j];
     }
     {
-      const float sum = delta_lower_sum<COLS>(b_matrix + t * CHUNK, w + c, t, r[t * COLS + c]);
+      const float2 sum = delta_lower_sum<COLS>(b_matrix + t * CHUNK, w + c, t, *reinterpret_cast<const float2*>(r + t * COLS + c));
       const int token = begin + chunk * CHUNK + t;
-      if (token < end) out[((long long)token * heads + head) * vdim + col0 + c] = sum;
+      if (token < end) *reinterpret_cast<float2*>(out + ((long long)token * heads + head) * vdim + col0 + c) = sum;
     }
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j) *reinterpret_cast<float4*>(mine + (long long)(4 * ((group << 3) + dg) + first_entry + j) * vdim) = own[j];
+  for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(mine + (long long)(4 * ((warp << 3) + dg) + j) * vdim) = s[0][j];
 }
 
 // o: float32 [T, heads, vdim]; gate: columns of proj from col_gate, [heads, vdim], through silu - or, if given, the float32 tensor
@@ -885,7 +889,7 @@ static int launch_delta(const void* proj_v, long long ld, const float* conv_w, i
     }
     launch_dependent(delta_chunk_matrices_kernel<DIM>, dim3((unsigned)(num_tokens / CHUNK + num_rows + 1), kv_heads), dim3(128), 0, stream, (const float*)qkv,
                      (const float*)gates, matrices, q_start, num_rows, heads, kv_heads, vdim);
-    launch_dependent(delta_chunk_walk_kernel<DIM>, dim3(vdim / COLS, heads, num_rows), dim3(WALK_THREADS), alone ? HALF_SM : smem, stream, (const float*)qkv, (const float*)matrices, state,
+    launch_dependent(delta_chunk_walk_kernel<DIM>, dim3(vdim / COLS, heads, num_rows), dim3(128), alone ? HALF_SM : smem, stream, (const float*)qkv, (const float*)matrices, state,
                      slot_floats, q_start, slots, o, heads, kv_heads, vdim);
     walked = true;
   }

@@ -25,8 +25,8 @@
 
 namespace pylon {
 
-constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 128, GC_MOST_STAGES = 8, GC_CHAIN = 8;   // weight rows and k of a box; boxes of a chain at least
-constexpr int GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
+constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 128, GC_MOST_STAGES = 8;   // weight rows and k of a box
+constexpr int GC_MOST_CHAINS = 8, GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
 constexpr unsigned GC_WAIT_LIMIT = 1u << 22;                                                 // try_wait calls before a wait gives up
 enum GcForm { GC_PARTIAL = 0, GC_PRODUCT = 1, GC_GATED = 2 };
 
@@ -63,7 +63,6 @@ __device__ __forceinline__ void gc_read(uint32_t address, uint32_t (&r)[16]) {
                : "r"(address));
 }
 __device__ __forceinline__ void gc_read_done() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void gc_cluster_barrier() { asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 // A K-major tile whose rows are 128 bytes in the 128-byte swizzle: start address, 1024 bytes between groups of 8 rows, version 1, swizzle 128B.
 __device__ __forceinline__ uint64_t gc_desc(const void* tile) {
   return (uint64_t)((gc_smem(tile) & 0x3FFFF) >> 4) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
@@ -85,27 +84,36 @@ __device__ __forceinline__ uint32_t gc_pack(float a, float b) {
 struct GcArgs {
   void* y;
   long long ldy;
-  int M, N, K, columns, stages, tmem_columns;   // columns: M rounded up to 16
+  int M, N, K, columns, stages, chains, tmem_columns;   // columns: M rounded up to 16; chains: a power of two
+  int whole, slices;    // product and gated unit: tiles that one block takes, and blocks that share each of the others
+  float* scratch;       // their sums, [blocks of shared tiles][columns][128]
+  unsigned* counters;   // of shared tiles, zero between launches
   float unit_limit, unit_alpha;
   int w_static;
   int* error;   // 1: the copies, 2: the products, 3: the accumulator did not come in time
 };
 
-// Grid (slices of k, tiles of 128 weight rows).  With several slices the product and the gated unit run as clusters of them.
+// Partial sums: grid (slices of k, tiles of 128 weight rows).  Product and gated unit: a block for each of the first `whole` tiles, then `slices` for
+// each of the others; the one that arrives last at such a tile adds up what they all left in scratch memory, in the order of k.
 template <int FORM>
 __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GcArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[GC_MOST_STAGES], empty[GC_MOST_STAGES], done;
   __shared__ uint32_t tmem_slot;
+  __shared__ int arrived_last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int columns = a.columns, stages = a.stages, w_bytes = GC_ROWS * GC_BK * 2, x_bytes = columns * GC_BK * 2;
   unsigned char* w_tiles = smem;
   unsigned char* x_tiles = smem + stages * w_bytes;
-  const int boxes_of_k = (a.K + GC_BK - 1) / GC_BK, parts = gridDim.x;
-  const int box0 = (int)((long long)boxes_of_k * blockIdx.x / parts), boxes = (int)((long long)boxes_of_k * (blockIdx.x + 1) / parts) - box0;
-  const int row0 = blockIdx.y * GC_ROWS;
-  const int most_chains = max(1, a.tmem_columns / columns), chain = max(GC_CHAIN, (boxes + most_chains - 1) / most_chains), chains = (boxes + chain - 1) / chain;
+  const int boxes_of_k = (a.K + GC_BK - 1) / GC_BK;
+  const int extra = (int)blockIdx.x - a.whole;   // product and gated unit: number among the blocks that share tiles
+  const bool shared = FORM != GC_PARTIAL && extra >= 0 && a.slices > 1;
+  const int tile = FORM == GC_PARTIAL ? blockIdx.y : extra < 0 ? blockIdx.x : a.whole + extra / a.slices;
+  const int slices = FORM == GC_PARTIAL ? gridDim.x : shared ? a.slices : 1, slice = FORM == GC_PARTIAL ? blockIdx.x : shared ? extra % a.slices : 0;
+  const int box0 = (int)((long long)boxes_of_k * slice / slices), boxes = (int)((long long)boxes_of_k * (slice + 1) / slices) - box0;
+  const int row0 = tile * GC_ROWS;
+  const int chains = a.chains;
 
   const int ahead = a.w_static ? min(stages, boxes) : 0;
   if (threadIdx.x == 0) {
@@ -130,29 +138,32 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
 
   int issued = 0;   // boxes asked for (the first thread's)
   if (warp == 0 && lane == 0) {
-    for (; issued < boxes; ++issued) {
-      const int s = issued % stages;
+    for (int s = 0, round = 0; issued < boxes; ++issued) {
       if (issued >= ahead) {
-        if (issued >= stages && !gc_wait(&empty[s], (issued / stages - 1) & 1)) { atomicExch(a.error, 1); break; }
+        if (round > 0 && !gc_wait(&empty[s], (round - 1) & 1)) { atomicExch(a.error, 1); break; }
         gc_expect(&full[s], w_bytes + x_bytes);
         gc_load(w_tiles + s * w_bytes, &map_w, &full[s], (box0 + issued) * GC_BK, row0);
       }
       gc_load(x_tiles + s * x_bytes, &map_x, &full[s], (box0 + issued) * GC_BK, 0);
+      if (++s == stages) { s = 0; ++round; }
     }
   } else if (warp == 1 && lane == 0) {
     // Instruction descriptor of kind::f16: bfloat16 A and B, float32 D, both K-major.
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(GC_ROWS >> 4) << 24);
+    const uint64_t w_first = gc_desc(w_tiles), x_first = gc_desc(x_tiles);
     bool alive = true;
-    for (int box = 0; box < boxes; ++box) {
-      const int s = box % stages;
-      if (!gc_wait(&full[s], (box / stages) & 1)) { atomicExch(a.error, 2); alive = false; break; }
+    for (int box = 0, s = 0, phase = 0, offset = 0; box < boxes; ++box) {
+      if (!gc_wait(&full[s], phase)) { atomicExch(a.error, 2); alive = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint64_t w_desc = gc_desc(w_tiles + s * w_bytes), x_desc = gc_desc(x_tiles + s * x_bytes);
-      const int first = box % chain == 0;
+      const uint64_t w_desc = w_first + (uint64_t)(s * (w_bytes >> 4)), x_desc = x_first + (uint64_t)(s * (x_bytes >> 4));
 #pragma unroll
-      for (int k = 0; k < GC_BK / 16; ++k)   // 16 k are 32 bytes further along the swizzled row: +2 in 16-byte units
-        gc_mma(tmem + box / chain * columns, w_desc + 2 * k, x_desc + 2 * k, idesc, !(first && k == 0));
+      for (int k = 0; k < GC_BK / 16; ++k) {   // 16 k are 32 bytes further along the swizzled row: +2 in 16-byte units
+        gc_mma(tmem + offset, w_desc + 2 * k, x_desc + 2 * k, idesc, box * (GC_BK / 16) + k >= chains);
+        offset += columns;
+        if (offset == chains * columns) offset = 0;
+      }
       gc_commit(&empty[s]);
+      if (++s == stages) { s = 0; phase ^= 1; }
     }
     if (alive) gc_commit(&done);
   }
@@ -206,31 +217,35 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
     }
   };
   float v[16];
-  if (FORM == GC_PARTIAL || parts == 1) {
+  if (!shared) {
     for (int c0 = 0; complete && c0 < columns; c0 += 16) {
       sums(c0, v);
       write(c0, v);
     }
   } else {
-    // The slices of k are the blocks of a cluster: groups of 16 rows of x are dealt out to them, a block sends each other one the groups that it adds up.
-    const int rank = blockIdx.x, groups = columns / 16, most = (groups + parts - 1) / parts;
-    float* received = reinterpret_cast<float*>(smem);   // [slice][group][16][128], where the stages were
-    gc_cluster_barrier();   // every block's products have read their stages
-    for (int group = 0; group < groups; ++group) {
-      sums(group * 16, v);
-      uint32_t remote;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(gc_smem(received + (size_t)(rank * most + group / parts) * 16 * GC_ROWS + threadIdx.x)), "r"(group % parts));
+    float* mine = a.scratch + (size_t)extra * columns * GC_ROWS + threadIdx.x;
+    for (int c0 = 0; c0 < columns; c0 += 16) {
+      sums(c0, v);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote + j * GC_ROWS * 4), "f"(v[j]) : "memory");
+      for (int j = 0; j < 16; ++j) mine[(size_t)(c0 + j) * GC_ROWS] = v[j];
     }
-    gc_cluster_barrier();   // all that was sent is there
-    for (int group = rank; complete && group < groups; group += parts) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();   // what the block's threads wrote before the barrier, too
+      unsigned* counter = a.counters + (tile - a.whole);
+      arrived_last = atomicAdd(counter, 1u) == (unsigned)a.slices - 1u;
+      if (arrived_last) *counter = 0u;   // ready for the next launch
+      __threadfence();
+    }
+    __syncthreads();
+    const float* all = a.scratch + (size_t)(extra - slice) * columns * GC_ROWS + threadIdx.x;
+    for (int c0 = 0; arrived_last && complete && c0 < columns; c0 += 16) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = 0.f;
-      for (int slice = 0; slice < parts; ++slice)
+      for (int other = 0; other < a.slices; ++other)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] += received[((size_t)(slice * most + group / parts) * 16 + j) * GC_ROWS + threadIdx.x];
-      write(group * 16, v);
+        for (int j = 0; j < 16; ++j) v[j] += __ldcg(all + ((size_t)other * columns + c0 + j) * GC_ROWS);
+      write(c0, v);
     }
   }
   if (!complete && threadIdx.x == 0)   // no copy outlives the block
@@ -282,10 +297,11 @@ static bool matrix_map(CUtensorMap* map, const void* base, long long rows, long 
   return true;
 }
 
-constexpr int GC_SMEM_SHARED = 112 * 1024, GC_SMEM_ALONE = 224 * 1024;   // of one of two blocks on an SM, of a lone one
+constexpr int GC_SMEM = 112 * 1024;   // two blocks to an SM: the next kernel's move in beside the last of this one's and ask for their weights
 
 template <int FORM>
-static int launch_columns(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts, int per_sm,
+static int launch_columns(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int whole, int parts, float* scratch,
+                          unsigned* counters,
                           float limit, float alpha, int w_static, int* error, cudaStream_t stream, const char* name) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 256) PYLON_REFUSE("%s: M = %d is more than 256 rows", name, M);
@@ -293,61 +309,62 @@ static int launch_columns(const void* x, const void* w, void* y, int M, int N, i
   if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 4)) PYLON_REFUSE("%s: x and w must be 16-byte aligned", name);
   if (ldx < K || ldw < K) PYLON_REFUSE("%s: a row stride is shorter than its row", name);
   const int boxes = (K + GC_BK - 1) / GC_BK, tiles = (N + GC_ROWS - 1) / GC_ROWS;
-  if (parts < 1 || parts > boxes || parts > 65535 || tiles > 65535) PYLON_REFUSE("%s: %d parts over %d slices of k, %d tiles", name, parts, boxes, tiles);
-  if (FORM != GC_PARTIAL && parts > 8) PYLON_REFUSE("%s: %d slices of k, a cluster has 8 blocks at most", name, parts);
-  if (per_sm < 1 || per_sm > 2) PYLON_REFUSE("%s: %d blocks to an SM", name, per_sm);
+  if (parts < 1 || parts > boxes || parts > 65535 || tiles > 65535) PYLON_REFUSE("%s: %d slices of %d steps of k, %d tiles", name, parts, boxes, tiles);
+  if (FORM != GC_PARTIAL && (whole < 0 || whole > tiles || (whole < tiles && parts > 1 && (!scratch || !counters))))
+    PYLON_REFUSE("%s: %d of %d tiles whole, the others in %d slices need scratch memory and counters", name, whole, tiles, parts);
   if (!error) PYLON_REFUSE("%s: an error word is needed", name);
   auto kernel = gemm_columns_kernel<FORM>;
   static bool configured_on[MAX_DEVICES] = {};   // function attributes belong to a device
   bool& configured = configured_on[current_device_slot()];
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM_ALONE);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM);
     if (err != cudaSuccess) PYLON_REFUSE("%s: %s", name, cudaGetErrorString(err));
     configured = true;
   }
   GcArgs a;
   a.y = y; a.ldy = ldy; a.M = M; a.N = N; a.K = K;
   a.columns = (M + 15) / 16 * 16;
-  const int stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2, room = (per_sm == 2 ? GC_SMEM_SHARED : GC_SMEM_ALONE) - 1024, slice = (boxes + parts - 1) / parts;
-  a.stages = std::min({room / stage_bytes, GC_MOST_STAGES, slice});
-  const int wanted = std::min(a.columns * ((slice + GC_CHAIN - 1) / GC_CHAIN), GC_COLUMNS);
+  const int stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2, room = GC_SMEM - 1024;
+  a.stages = std::min({room / stage_bytes, GC_MOST_STAGES, boxes});
+  a.chains = 1;
+  while (a.chains < GC_MOST_CHAINS && 2 * a.chains * a.columns <= GC_COLUMNS && 2 * a.chains <= boxes / parts * (GC_BK / 16)) a.chains *= 2;
   a.tmem_columns = 32;
-  while (a.tmem_columns < wanted) a.tmem_columns *= 2;
+  while (a.tmem_columns < a.chains * a.columns) a.tmem_columns *= 2;
+  a.whole = FORM == GC_PARTIAL ? 0 : whole; a.slices = parts; a.scratch = scratch; a.counters = counters;
   a.unit_limit = limit; a.unit_alpha = alpha; a.w_static = w_static; a.error = error;
   CUtensorMap map_w, map_x;
   if (!matrix_map(&map_w, w, N, K, ldw, GC_ROWS) || !matrix_map(&map_x, x, M, K, ldx, a.columns)) PYLON_REFUSE("%s: the tensor maps could not be made", name);
-  const size_t ring = (size_t)a.stages * stage_bytes, groups = a.columns / 16, received = (groups + parts - 1) / parts * parts * 16 * GC_ROWS * sizeof(float);
-  if (FORM == GC_PARTIAL || parts == 1)
-    launch_dependent<LAUNCH_GEMM>(kernel, dim3(parts, tiles), dim3(GC_THREADS), ring + 1024, stream, map_w, map_x, a);
-  else
-    launch_dependent_cluster<LAUNCH_GEMM>(kernel, dim3(parts, tiles), dim3(GC_THREADS), std::max(ring, received) + 1024, stream, (unsigned)parts, map_w, map_x, a);
+  const dim3 grid = FORM == GC_PARTIAL ? dim3(parts, tiles) : dim3(whole + (tiles - whole) * parts);
+  launch_dependent<LAUNCH_GEMM>(kernel, grid, dim3(GC_THREADS), (size_t)a.stages * stage_bytes + 1024, stream, map_w, map_x, a);
   PYLON_CHECK_LAUNCH(name);
 }
 
 }  // namespace pylon
 
 // x: bfloat16 [M, K] (row stride ldx), M <= 256; w: bfloat16 [N, K] (row stride ldw); y: float32 [parts, M, N] contiguous, whose sum over the
-// first dimension is x @ w.T.  K and the row strides multiples of 8, x and w 16-byte aligned, 1 <= parts <= number of 64-wide slices of
-// k; per_sm: 1 or 2 blocks to an SM.  error: one int in device memory that the kernel sets non-zero if one of its waits ran out (the
+// first dimension is x @ w.T.  K and the row strides multiples of 8, x and w 16-byte aligned, 1 <= parts <= number of 64-wide steps of
+// k.  error: one int in device memory that the kernel sets non-zero if one of its waits ran out (the
 // result is then void).  w_static: 1 where nothing queued on the stream writes w; its first boxes are then asked for while the kernel ahead is still running.
-extern "C" int pylon_gemm_columns_partial(const void* x, const void* w, float* y, int M, int N, int K, long long ldx, long long ldw, int parts, int per_sm,
+extern "C" int pylon_gemm_columns_partial(const void* x, const void* w, float* y, int M, int N, int K, long long ldx, long long ldw, int parts,
                                           int* error, int w_static, cudaStream_t stream) {
-  return pylon::launch_columns<pylon::GC_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, parts, per_sm, 0.f, 1.f, w_static, error, stream, "gemm_columns_partial");
+  return pylon::launch_columns<pylon::GC_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, 0, parts, nullptr, nullptr, 0.f, 1.f, w_static, error, stream, "gemm_columns_partial");
 }
 
-// The product itself: y bfloat16 [M, N], row stride ldy; N and ldy even; up to 8 slices of k, added up in a cluster.
-extern "C" int pylon_gemm_columns_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts,
-                                       int per_sm, int* error, int w_static, cudaStream_t stream) {
+// The product itself: y bfloat16 [M, N], row stride ldy; N and ldy even.  The first `whole` tiles of 128 weight rows go to a block each, the others to
+// `slices` blocks each, which need scratch: float32, (tiles - whole) * slices * 128 * M rounded up to 16, contents arbitrary; counters: a zero for each of those
+// tiles (zero again after the call).
+extern "C" int pylon_gemm_columns_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int whole,
+                                       int slices, float* scratch, unsigned* counters, int* error, int w_static, cudaStream_t stream) {
   if (ldy < N || N % 2 || ldy % 2) PYLON_REFUSE("gemm_columns_bf16: N = %d and the result's row stride must be even, the stride no shorter than a row", N);
-  return pylon::launch_columns<pylon::GC_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, parts, per_sm, 0.f, 1.f, w_static, error, stream, "gemm_columns_bf16");
+  return pylon::launch_columns<pylon::GC_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, whole, slices, scratch, counters, 0.f, 1.f, w_static, error, stream, "gemm_columns_bf16");
 }
 
 // The gated unit of x gate^T and x up^T: w's rows are interleaved in groups of 8 (rows 16b..16b+7 gate rows 8b..8b+7, rows 16b+8..16b+15 the matching up
 // rows; N a multiple of 16); y bfloat16 [M, N / 2], row stride ldy.  limit 0: silu(gate) * up; limit > 0: the clamped unit,
-// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).  Slices of k as for the product.
+// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).  Tiles as for the product.
 extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, float limit,
-                                        float alpha, int parts, int per_sm, int* error, int w_static, cudaStream_t stream) {
+                                        float alpha, int whole, int slices, float* scratch, unsigned* counters, int* error, int w_static, cudaStream_t stream) {
   if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_columns_gated: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
   if (limit < 0.f) PYLON_REFUSE("gemm_columns_gated: the limit must not be negative");
-  return pylon::launch_columns<pylon::GC_GATED>(x, w, y, M, N, K, ldx, ldw, ldy, parts, per_sm, limit, alpha, w_static, error, stream, "gemm_columns_gated");
+  return pylon::launch_columns<pylon::GC_GATED>(x, w, y, M, N, K, ldx, ldw, ldy, whole, slices, scratch, counters, limit, alpha, w_static, error, stream, "gemm_columns_gated");
 }

@@ -275,10 +275,11 @@ _SIGNATURES = {
         "pylon_gemm_stream_glu_clamped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_int, c_void_p],
     },
     "gemm_columns.cu": {
-        "pylon_gemm_columns_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p],
-        "pylon_gemm_columns_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p],
+        "pylon_gemm_columns_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p],
+        "pylon_gemm_columns_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p, c_void_p,
+                                    c_void_p, c_int, c_void_p],
         "pylon_gemm_columns_gated": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_int, c_int,
-                                     c_void_p, c_int, c_void_p],
+                                     c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     },
     "gemm_tcgen05.cu": {
         "pylon_gemm_tcgen05_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
@@ -851,12 +852,25 @@ def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit:
     return y
 
 
-def linear_columns(x: torch.Tensor, w: torch.Tensor, form: str = "product", parts: int = 1, limit: Optional[float] = None, alpha: float = 1.0,
-                   static_weights: bool = False, per_sm: int = 2) -> torch.Tensor:
+_column_streams: dict[tuple[int, int], int] = {}
+
+
+def _column_counters(device: torch.device, count: int) -> torch.Tensor:
+    """``count`` zeroed counters that calls on other streams do not use at the same time: every stream has 1,024 of its own (the first 64 of a device)."""
+    streams = 64
+    buffer = _zeroed_counters(device, "columns", 1024 * streams)
+    _need(count <= 1024, f"linear_columns: {count} tiles of 128 weight rows are too many to share")
+    index = _column_streams.setdefault((_device_index(device), _stream()), len(_column_streams)) % streams
+    return buffer[1024 * index : 1024 * index + count]
+
+
+def linear_columns(x: torch.Tensor, w: torch.Tensor, form: str = "product", parts: Optional[int] = None, limit: Optional[float] = None, alpha: float = 1.0,
+                   static_weights: bool = False, whole: Optional[int] = None) -> torch.Tensor:
     """bfloat16 ``x [M <= 256, K] @ w [N, K].T`` on the tcgen05 kernel whose tiles are 128 weight rows wide and as many rows of ``x`` deep as there are.
     ``form``: ``"product"`` (bfloat16 ``[M, N]``), ``"partial"`` (float32 sums over ``parts`` slices of k, ``[parts, M, N]``) or ``"gated"`` (the rows of ``w``
-    interleaved by :func:`interleave_gate_up`, the unit of :func:`linear_stream`, ``[M, N / 2]``).  ``parts``: slices of k (up to 8 in the other two forms,
-    whose blocks add them up in a cluster); ``per_sm``: blocks that share an SM."""
+    interleaved by :func:`interleave_gate_up`, the unit of :func:`linear_stream`, ``[M, N / 2]``).  In the other two forms the first ``whole`` tiles go to a
+    block each and the others to ``parts`` blocks each, slices of k that the last of them adds up; by default as many tiles are whole as
+    fill whole rounds over the SMs."""
     _need_cuda(x, w)
     _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16,
           "linear_columns: bfloat16 x [M, K] and w [N, K]")
@@ -864,17 +878,28 @@ def linear_columns(x: torch.Tensor, w: torch.Tensor, form: str = "product", part
     _need(form in ("product", "partial", "gated"), f"linear_columns: unknown form {form!r}")
     m, k = x.shape
     n = w.shape[0]
+    sms, tiles, steps = _multiprocessors(x.device), -(-n // 128), -(-k // 64)
     library, error, static = _library("gemm_columns.cu"), _ptr(stream_error_word(x.device)), int(static_weights)
     if form == "partial":
+        if parts is None:
+            parts = max(1, min(steps, 2 * sms // tiles))
         y = torch.empty((parts, m, n), dtype=torch.float32, device=x.device)
-        _check(library, library.pylon_gemm_columns_partial(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), parts, per_sm, error, static, _stream()))
+        _check(library, library.pylon_gemm_columns_partial(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), parts, error, static, _stream()))
         return y
+    whole = tiles // sms * sms if whole is None else int(whole)
+    if parts is None:
+        parts = max(1, min(8, steps // 4, sms // (tiles - whole))) if whole < tiles else 1
+    scratch = counters = None
+    if whole < tiles and parts > 1:
+        scratch = torch.empty(((tiles - whole) * parts * 128 * (-(-m // 16) * 16),), dtype=torch.float32, device=x.device)
+        counters = _column_counters(x.device, tiles - whole)
     y = torch.empty((m, n // 2 if form == "gated" else n), dtype=torch.bfloat16, device=x.device)
     if form == "gated":
         _check(library, library.pylon_gemm_columns_gated(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit or 0.0), float(alpha),
-                                                         parts, per_sm, error, static, _stream()))
+                                                         whole, parts, _ptr(scratch), _ptr(counters), error, static, _stream()))
     else:
-        _check(library, library.pylon_gemm_columns_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), parts, per_sm, error, static, _stream()))
+        _check(library, library.pylon_gemm_columns_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), whole, parts, _ptr(scratch),
+                                                        _ptr(counters), error, static, _stream()))
     return y
 
 

@@ -7,8 +7,8 @@
 // swizzle) into a ring of stages - the boxes of W that nothing queued writes before it waits for the kernel ahead - one lane of the second issues the
 // products, and all four read the accumulator back, each its 32 lanes, a lane being a row of W: 32 neighbouring numbers of a row of y.
 //
-// The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k: k is cut into as many chains as
-// fit beside each other in 256 columns of tensor memory (256 / N, 512 k or more each), which the epilogue adds in float32.
+// The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k: the steps of 16 k take turns on as many
+// accumulators as fit beside each other in 256 columns of tensor memory (eight at most), which the epilogue adds in float32.
 //
 // All waits on mbarriers are bounded: one that runs out sets an error word, the block waits for its own copies, frees its tensor memory and returns.
 // No TMA load here uses cluster multicast.
@@ -85,34 +85,25 @@ struct GcArgs {
   void* y;
   long long ldy;
   int M, N, K, columns, stages, chains, tmem_columns;   // columns: M rounded up to 16; chains: a power of two
-  int whole, slices;    // product and gated unit: tiles that one block takes, and blocks that share each of the others
-  float* scratch;       // their sums, [blocks of shared tiles][columns][128]
-  unsigned* counters;   // of shared tiles, zero between launches
   float unit_limit, unit_alpha;
   int w_static;
   int* error;   // 1: the copies, 2: the products, 3: the accumulator did not come in time
 };
 
-// Partial sums: grid (slices of k, tiles of 128 weight rows).  Product and gated unit: a block for each of the first `whole` tiles, then `slices` for
-// each of the others; the one that arrives last at such a tile adds up what they all left in scratch memory, in the order of k.
+// Grid (slices of k, tiles of 128 weight rows).
 template <int FORM>
 __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GcArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[GC_MOST_STAGES], empty[GC_MOST_STAGES], done;
   __shared__ uint32_t tmem_slot;
-  __shared__ int arrived_last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int columns = a.columns, stages = a.stages, w_bytes = GC_ROWS * GC_BK * 2, x_bytes = columns * GC_BK * 2;
   unsigned char* w_tiles = smem;
   unsigned char* x_tiles = smem + stages * w_bytes;
   const int boxes_of_k = (a.K + GC_BK - 1) / GC_BK;
-  const int extra = (int)blockIdx.x - a.whole;   // product and gated unit: number among the blocks that share tiles
-  const bool shared = FORM != GC_PARTIAL && extra >= 0 && a.slices > 1;
-  const int tile = FORM == GC_PARTIAL ? blockIdx.y : extra < 0 ? blockIdx.x : a.whole + extra / a.slices;
-  const int slices = FORM == GC_PARTIAL ? gridDim.x : shared ? a.slices : 1, slice = FORM == GC_PARTIAL ? blockIdx.x : shared ? extra % a.slices : 0;
-  const int box0 = (int)((long long)boxes_of_k * slice / slices), boxes = (int)((long long)boxes_of_k * (slice + 1) / slices) - box0;
-  const int row0 = tile * GC_ROWS;
+  const int box0 = (int)((long long)boxes_of_k * blockIdx.x / gridDim.x), boxes = (int)((long long)boxes_of_k * (blockIdx.x + 1) / gridDim.x) - box0;
+  const int row0 = blockIdx.y * GC_ROWS;
   const int chains = a.chains;
 
   const int ahead = a.w_static ? min(stages, boxes) : 0;
@@ -216,37 +207,10 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
       for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(raw[j]);
     }
   };
-  float v[16];
-  if (!shared) {
-    for (int c0 = 0; complete && c0 < columns; c0 += 16) {
-      sums(c0, v);
-      write(c0, v);
-    }
-  } else {
-    float* mine = a.scratch + (size_t)extra * columns * GC_ROWS + threadIdx.x;
-    for (int c0 = 0; c0 < columns; c0 += 16) {
-      sums(c0, v);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) mine[(size_t)(c0 + j) * GC_ROWS] = v[j];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();   // what the block's threads wrote before the barrier, too
-      unsigned* counter = a.counters + (tile - a.whole);
-      arrived_last = atomicAdd(counter, 1u) == (unsigned)a.slices - 1u;
-      if (arrived_last) *counter = 0u;   // ready for the next launch
-      __threadfence();
-    }
-    __syncthreads();
-    const float* all = a.scratch + (size_t)(extra - slice) * columns * GC_ROWS + threadIdx.x;
-    for (int c0 = 0; arrived_last && complete && c0 < columns; c0 += 16) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = 0.f;
-      for (int other = 0; other < a.slices; ++other)
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] += __ldcg(all + ((size_t)other * columns + c0 + j) * GC_ROWS);
-      write(c0, v);
-    }
+  for (int c0 = 0; complete && c0 < columns; c0 += 16) {
+    float v[16];
+    sums(c0, v);
+    write(c0, v);
   }
   if (!complete && threadIdx.x == 0)   // no copy outlives the block
     for (int box = max(0, issued - stages); box < issued; ++box) gc_wait(&full[box % stages], (box / stages) & 1);
@@ -300,8 +264,7 @@ static bool matrix_map(CUtensorMap* map, const void* base, long long rows, long 
 constexpr int GC_SMEM = 112 * 1024;   // two blocks to an SM: the next kernel's move in beside the last of this one's and ask for their weights
 
 template <int FORM>
-static int launch_columns(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int whole, int parts, float* scratch,
-                          unsigned* counters,
+static int launch_columns(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts,
                           float limit, float alpha, int w_static, int* error, cudaStream_t stream, const char* name) {
   if (M <= 0 || N <= 0) return 0;
   if (M > 256) PYLON_REFUSE("%s: M = %d is more than 256 rows", name, M);
@@ -310,8 +273,6 @@ static int launch_columns(const void* x, const void* w, void* y, int M, int N, i
   if (ldx < K || ldw < K) PYLON_REFUSE("%s: a row stride is shorter than its row", name);
   const int boxes = (K + GC_BK - 1) / GC_BK, tiles = (N + GC_ROWS - 1) / GC_ROWS;
   if (parts < 1 || parts > boxes || parts > 65535 || tiles > 65535) PYLON_REFUSE("%s: %d slices of %d steps of k, %d tiles", name, parts, boxes, tiles);
-  if (FORM != GC_PARTIAL && (whole < 0 || whole > tiles || (whole < tiles && parts > 1 && (!scratch || !counters))))
-    PYLON_REFUSE("%s: %d of %d tiles whole, the others in %d slices need scratch memory and counters", name, whole, tiles, parts);
   if (!error) PYLON_REFUSE("%s: an error word is needed", name);
   auto kernel = gemm_columns_kernel<FORM>;
   static bool configured_on[MAX_DEVICES] = {};   // function attributes belong to a device
@@ -330,12 +291,10 @@ static int launch_columns(const void* x, const void* w, void* y, int M, int N, i
   while (a.chains < GC_MOST_CHAINS && 2 * a.chains * a.columns <= GC_COLUMNS && 2 * a.chains <= boxes / parts * (GC_BK / 16)) a.chains *= 2;
   a.tmem_columns = 32;
   while (a.tmem_columns < a.chains * a.columns) a.tmem_columns *= 2;
-  a.whole = FORM == GC_PARTIAL ? 0 : whole; a.slices = parts; a.scratch = scratch; a.counters = counters;
   a.unit_limit = limit; a.unit_alpha = alpha; a.w_static = w_static; a.error = error;
   CUtensorMap map_w, map_x;
   if (!matrix_map(&map_w, w, N, K, ldw, GC_ROWS) || !matrix_map(&map_x, x, M, K, ldx, a.columns)) PYLON_REFUSE("%s: the tensor maps could not be made", name);
-  const dim3 grid = FORM == GC_PARTIAL ? dim3(parts, tiles) : dim3(whole + (tiles - whole) * parts);
-  launch_dependent<LAUNCH_GEMM>(kernel, grid, dim3(GC_THREADS), (size_t)a.stages * stage_bytes + 1024, stream, map_w, map_x, a);
+  launch_dependent<LAUNCH_GEMM>(kernel, dim3(parts, tiles), dim3(GC_THREADS), (size_t)a.stages * stage_bytes + 1024, stream, map_w, map_x, a);
   PYLON_CHECK_LAUNCH(name);
 }
 
@@ -347,24 +306,22 @@ static int launch_columns(const void* x, const void* w, void* y, int M, int N, i
 // result is then void).  w_static: 1 where nothing queued on the stream writes w; its first boxes are then asked for while the kernel ahead is still running.
 extern "C" int pylon_gemm_columns_partial(const void* x, const void* w, float* y, int M, int N, int K, long long ldx, long long ldw, int parts,
                                           int* error, int w_static, cudaStream_t stream) {
-  return pylon::launch_columns<pylon::GC_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, 0, parts, nullptr, nullptr, 0.f, 1.f, w_static, error, stream, "gemm_columns_partial");
+  return pylon::launch_columns<pylon::GC_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, parts, 0.f, 1.f, w_static, error, stream, "gemm_columns_partial");
 }
 
-// The product itself: y bfloat16 [M, N], row stride ldy; N and ldy even.  The first `whole` tiles of 128 weight rows go to a block each, the others to
-// `slices` blocks each, which need scratch: float32, (tiles - whole) * slices * 128 * M rounded up to 16, contents arbitrary; counters: a zero for each of those
-// tiles (zero again after the call).
-extern "C" int pylon_gemm_columns_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int whole,
-                                       int slices, float* scratch, unsigned* counters, int* error, int w_static, cudaStream_t stream) {
+// The product itself: y bfloat16 [M, N], row stride ldy; N and ldy even.
+extern "C" int pylon_gemm_columns_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+                                       int* error, int w_static, cudaStream_t stream) {
   if (ldy < N || N % 2 || ldy % 2) PYLON_REFUSE("gemm_columns_bf16: N = %d and the result's row stride must be even, the stride no shorter than a row", N);
-  return pylon::launch_columns<pylon::GC_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, whole, slices, scratch, counters, 0.f, 1.f, w_static, error, stream, "gemm_columns_bf16");
+  return pylon::launch_columns<pylon::GC_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, 1, 0.f, 1.f, w_static, error, stream, "gemm_columns_bf16");
 }
 
 // The gated unit of x gate^T and x up^T: w's rows are interleaved in groups of 8 (rows 16b..16b+7 gate rows 8b..8b+7, rows 16b+8..16b+15 the matching up
 // rows; N a multiple of 16); y bfloat16 [M, N / 2], row stride ldy.  limit 0: silu(gate) * up; limit > 0: the clamped unit,
-// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).  Tiles as for the product.
+// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).
 extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, float limit,
-                                        float alpha, int whole, int slices, float* scratch, unsigned* counters, int* error, int w_static, cudaStream_t stream) {
+                                        float alpha, int* error, int w_static, cudaStream_t stream) {
   if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_columns_gated: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
   if (limit < 0.f) PYLON_REFUSE("gemm_columns_gated: the limit must not be negative");
-  return pylon::launch_columns<pylon::GC_GATED>(x, w, y, M, N, K, ldx, ldw, ldy, whole, slices, scratch, counters, limit, alpha, w_static, error, stream, "gemm_columns_gated");
+  return pylon::launch_columns<pylon::GC_GATED>(x, w, y, M, N, K, ldx, ldw, ldy, 1, limit, alpha, w_static, error, stream, "gemm_columns_gated");
 }

@@ -276,10 +276,8 @@ _SIGNATURES = {
     },
     "gemm_columns.cu": {
         "pylon_gemm_columns_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p],
-        "pylon_gemm_columns_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p, c_void_p,
-                                    c_void_p, c_int, c_void_p],
-        "pylon_gemm_columns_gated": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_int, c_int,
-                                     c_void_p, c_void_p, c_void_p, c_int, c_void_p],
+        "pylon_gemm_columns_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_int, c_void_p],
+        "pylon_gemm_columns_gated": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_int, c_void_p],
     },
     "gemm_tcgen05.cu": {
         "pylon_gemm_tcgen05_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
@@ -770,6 +768,15 @@ def _tcgen05_fills_the_sms(m: int, n: int, sms: int) -> bool:
 
 STREAM_MAX_ROWS = 32   # up to this many rows the TMA-fed kernel beats the library (it takes up to 64)
 STREAM_MAX_PARTS = 4
+COLUMNS_MAX_ROWS = 160
+
+
+def _columns_take(x: torch.Tensor, w: torch.Tensor, most_rows: int) -> bool:
+    """Whether :func:`linear_columns` takes this product: more rows than the TMA-fed kernel's, up to ``most_rows``, in bfloat16 and aligned for TMA."""
+    m, k = x.shape
+    return (STREAM_MAX_ROWS < m <= most_rows and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and k >= 1024 and k % 8 == 0
+            and w.shape[0] % 16 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.stride(0) >= k
+            and w.stride(0) >= k and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def linear_for_residual(x: torch.Tensor, w: torch.Tensor, static_weights: bool = False) -> torch.Tensor:
@@ -784,6 +791,8 @@ def linear_for_residual(x: torch.Tensor, w: torch.Tensor, static_weights: bool =
             and n % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         return linear_stream_partial(x, w, static_weights=static_weights)
+    if _columns_take(x, w, COLUMNS_MAX_ROWS):
+        return linear_columns(x, w, "partial", static_weights=static_weights)
     return linear(x, w, static_weights=static_weights)
 
 
@@ -798,7 +807,14 @@ def linear_for_rotation(x: torch.Tensor, w: torch.Tensor, head_dim: int, rotary_
             and head_dim in (64, 128, 256) and rotary_dim in (0, head_dim) and n % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
             and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         return linear_stream_partial(x, w, static_weights=static_weights)
+    if ROTATION_COLUMNS and head_dim in (64, 128, 256) and rotary_dim in (0, head_dim) and _columns_take(x, w, COLUMNS_MAX_ROWS):
+        return linear_columns(x, w, "partial", static_weights=static_weights)
     return linear(x, w, static_weights=static_weights)
+
+
+ROTATION_COLUMNS = True
+COLUMNS_MAX_PARTS = 14
+GATED_COLUMNS = ()
 
 
 def stream_error_word(device: torch.device) -> torch.Tensor:
@@ -852,54 +868,32 @@ def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit:
     return y
 
 
-_column_streams: dict[tuple[int, int], int] = {}
-
-
-def _column_counters(device: torch.device, count: int) -> torch.Tensor:
-    """``count`` zeroed counters that calls on other streams do not use at the same time: every stream has 1,024 of its own (the first 64 of a device)."""
-    streams = 64
-    buffer = _zeroed_counters(device, "columns", 1024 * streams)
-    _need(count <= 1024, f"linear_columns: {count} tiles of 128 weight rows are too many to share")
-    index = _column_streams.setdefault((_device_index(device), _stream()), len(_column_streams)) % streams
-    return buffer[1024 * index : 1024 * index + count]
-
-
 def linear_columns(x: torch.Tensor, w: torch.Tensor, form: str = "product", parts: Optional[int] = None, limit: Optional[float] = None, alpha: float = 1.0,
-                   static_weights: bool = False, whole: Optional[int] = None) -> torch.Tensor:
+                   static_weights: bool = False) -> torch.Tensor:
     """bfloat16 ``x [M <= 256, K] @ w [N, K].T`` on the tcgen05 kernel whose tiles are 128 weight rows wide and as many rows of ``x`` deep as there are.
-    ``form``: ``"product"`` (bfloat16 ``[M, N]``), ``"partial"`` (float32 sums over ``parts`` slices of k, ``[parts, M, N]``) or ``"gated"`` (the rows of ``w``
-    interleaved by :func:`interleave_gate_up`, the unit of :func:`linear_stream`, ``[M, N / 2]``).  In the other two forms the first ``whole`` tiles go to a
-    block each and the others to ``parts`` blocks each, slices of k that the last of them adds up; by default as many tiles are whole as
-    fill whole rounds over the SMs."""
+    ``form``: ``"product"`` (bfloat16 ``[M, N]``), ``"gated"`` (the rows of ``w`` interleaved by :func:`interleave_gate_up`, the unit of
+    :func:`linear_stream`, ``[M, N / 2]``) or ``"partial"`` (float32 sums over ``parts`` slices of k, ``[parts, M, N]``; by default as many as give every SM
+    two blocks, up to ``COLUMNS_MAX_PARTS``)."""
     _need_cuda(x, w)
     _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16,
           "linear_columns: bfloat16 x [M, K] and w [N, K]")
     _need(x.stride(1) == 1 and w.stride(1) == 1, "linear_columns: the reduced dimension must be contiguous")
-    _need(form in ("product", "partial", "gated"), f"linear_columns: unknown form {form!r}")
+    _need(form in ("product", "partial", "gated") and (form == "partial" or parts is None), f"linear_columns: form {form!r} with {parts} parts")
     m, k = x.shape
     n = w.shape[0]
-    sms, tiles, steps = _multiprocessors(x.device), -(-n // 128), -(-k // 64)
     library, error, static = _library("gemm_columns.cu"), _ptr(stream_error_word(x.device)), int(static_weights)
     if form == "partial":
         if parts is None:
-            parts = max(1, min(steps, 2 * sms // tiles))
+            parts = max(1, min(COLUMNS_MAX_PARTS, -(-k // 64), 2 * _multiprocessors(x.device) // -(-n // 128)))
         y = torch.empty((parts, m, n), dtype=torch.float32, device=x.device)
         _check(library, library.pylon_gemm_columns_partial(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), parts, error, static, _stream()))
         return y
-    whole = tiles // sms * sms if whole is None else int(whole)
-    if parts is None:
-        parts = max(1, min(8, steps // 4, sms // (tiles - whole))) if whole < tiles else 1
-    scratch = counters = None
-    if whole < tiles and parts > 1:
-        scratch = torch.empty(((tiles - whole) * parts * 128 * (-(-m // 16) * 16),), dtype=torch.float32, device=x.device)
-        counters = _column_counters(x.device, tiles - whole)
     y = torch.empty((m, n // 2 if form == "gated" else n), dtype=torch.bfloat16, device=x.device)
     if form == "gated":
         _check(library, library.pylon_gemm_columns_gated(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit or 0.0), float(alpha),
-                                                         whole, parts, _ptr(scratch), _ptr(counters), error, static, _stream()))
+                                                         error, static, _stream()))
     else:
-        _check(library, library.pylon_gemm_columns_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), whole, parts, _ptr(scratch),
-                                                        _ptr(counters), error, static, _stream()))
+        _check(library, library.pylon_gemm_columns_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), error, static, _stream()))
     return y
 
 
@@ -1041,7 +1035,9 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and m <= STREAM_MAX_ROWS and x.shape[1] == k
             and k % 8 == 0 and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0
             and w_interleaved.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
+        if GATED_COLUMNS and n >= GATED_COLUMNS[0] and m > 8: return linear_columns(x, w_interleaved, "gated", limit=limit, alpha=alpha, static_weights=static_weights)
         return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)
+    if GATED_COLUMNS and n >= GATED_COLUMNS[1] and m <= GATED_COLUMNS[2]: return linear_columns(x, w_interleaved, "gated", limit=limit, alpha=alpha, static_weights=static_weights)
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and m >= TCGEN05_MIN_ROWS and k % 8 == 0
             and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0 and w_interleaved.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):

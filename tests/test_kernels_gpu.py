@@ -661,6 +661,31 @@ def test_a_block_table_that_names_a_page_outside_the_pool_is_reported(dtype):
     ops.raise_on_kernel_errors(device)
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 100, 129, 160, 256])
+@pytest.mark.parametrize("n, k", [(128, 64), (144, 1_032), (400, 2_568), (2_048, 584)])
+def test_tcgen05_product_with_the_weights_on_the_wide_side(m, n, k):
+    """Around the edges of its tiles (16 rows of x, 128 weight rows, 64 k), few and many slices of k, every form; rows behind the last one stay as they were."""
+    from pylon_b200.kernels import ops
+
+    x = torch.randn(m, k + 8, device=DEVICE).to(torch.bfloat16)[:, :k]
+    w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
+    expected = x.double() @ w.double().T
+    steps = -(-k // 64)
+    for parts in sorted({1, min(3, steps), min(14, steps), steps}):
+        sums = ops.linear_columns(x, w, "partial", parts=parts)
+        assert sums.shape == (parts, m, n)
+        # numbers of order 1, cut off at 2^-24 of a partial sum for every 16 k of a chain and every chain: some k / 16 of them at most
+        torch.testing.assert_close(sums.double().sum(0), expected, rtol=0, atol=(k / 16 + 16) * 2.0**-22)
+    rounded = dict(rtol=2.0**-8, atol=1e-4)   # half an ulp of bfloat16, and the float32 sums' error where they cancel
+    torch.testing.assert_close(ops.linear_columns(x, w, static_weights=True).double(), expected, **rounded)
+    pairs = expected.view(m, n // 16, 2, 8)
+    gate, up = pairs[:, :, 0].reshape(m, -1), pairs[:, :, 1].reshape(m, -1)
+    torch.testing.assert_close(ops.linear_columns(x, w, "gated").double(), gate * torch.sigmoid(gate) * up, **rounded)
+    gate, up = gate.clamp(max=0.5), up.clamp(-0.5, 0.5)
+    torch.testing.assert_close(ops.linear_columns(x, w, "gated", limit=0.5, alpha=1.7).double(), gate * torch.sigmoid(1.7 * gate) * (up + 1), **rounded)
+    assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
+
+
 def test_skinny_gemm_refuses():
     from pylon_b200.kernels import ops
 
@@ -779,6 +804,30 @@ def test_paged_attention(case, mode):
     )
     torch.testing.assert_close(out.double(), expected, **(dict(rtol=1e-4, atol=1e-5) if dtype == torch.float32 else dict(rtol=2e-2, atol=2e-2)))
     assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0   # no wait for a TMA copy ran out
+
+
+@pytest.mark.parametrize("nq, nkv, d, page", [(4, 4, 64, 64), (10, 2, 128, 256), (16, 2, 128, 64), (32, 2, 64, 128), (3, 1, 192, 64), (8, 2, 256, 64)])
+@pytest.mark.parametrize("blocks", [None, 1, 2, 13])
+def test_decoded_rows_a_run_to_a_warp(nq, nkv, d, page, blocks):
+    """Lengths around the tiles of 16 keys, runs that end inside rows, in a block and between blocks, several tokens to a row, rows without a
+    group's places, a window; what lies behind a row's keys in its page is not finite."""
+    from pylon_b200.kernels import ops
+
+    group = nq // nkv
+    kv_lens = [1, 15, 16, 17, 33, 255, 256, 257, 700, 2, 64, 131]
+    q_lens = [1] * 8 + [min(16 // group, 4), 1, min(16 // group, 3), 1]
+    cache = Paged(kv_lens, q_lens, nkv, d, page, torch.bfloat16)
+    for r, kv in enumerate(kv_lens):
+        last = int(cache.table[r, (kv - 1) // page])
+        for pages in (cache.k_pages, cache.v_pages):
+            pages[last, :, (kv - 1) % page + 1 :] = float("nan")
+    fused = torch.randn(cache.tokens, (nq + 2 * nkv) * d, device=DEVICE).to(torch.bfloat16)
+    for window in (None, 40):
+        expected = attention_reference(fused[:, : nq * d].reshape(cache.tokens, nq, d), cache, nq, nkv, d, window, d**-0.5)
+        out = ops.paged_attention(fused, cache.k_pages, cache.v_pages, cache.positions, cache.token_row, cache.q_start, cache.kv_len, cache.table, nq,
+                                  max(q_lens), max(kv_lens), window=window, decode_blocks=blocks)
+        torch.testing.assert_close(out.double(), expected, rtol=2e-2, atol=2e-2)
+    assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0
 
 
 @pytest.mark.parametrize("nq, nkv, d, dv", [(4, 1, 64, 64), (6, 3, 20, 36), (3, 3, 128, 192), (8, 1, 132, 512), (5, 1, 8, 4)])

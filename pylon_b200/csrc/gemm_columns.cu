@@ -1,19 +1,23 @@
-// y = x W^T in bfloat16 for up to 256 rows of x on the fifth-generation tensor cores, with the weights on the wide side of the tile: 128 rows of
-// W are the M of a tcgen05.mma and the rows of x, rounded up to 16, its N.  For the steps between a few decoded rows and a long prompt.
+// The gated unit of a feed-forward in bfloat16 for a few rows of x on the fifth-generation tensor cores, with the weights on the wide side of the tile:
+// 128 interleaved rows of gate and up are the M of a tcgen05.mma and the rows of x, rounded up to 16, its N.
 //
-// Bound by the bytes of W: every weight row is read once, whatever M is, and rows of x fill no more than the last 16 columns of the tile (with x on
-// the M side 33 rows cost what 128 do).  A block takes 128 rows of W and a slice of k; two blocks share an SM where N leaves
-// room, so that one's epilogue overlaps the other's loads.  Four warps: one lane of the first asks for boxes of W and x (TMA, 128-byte
+// Bound by the bytes of W: 16 rows of [34816, 5120] 58 us behind a norm (356 MB: 6.1 TB/s), where the kernel that multiplies with mma.sync from
+// registers (gemm_stream.cu) takes 66 us, its warps busy with fragments; 32 rows 62 and 75 us.  A block takes 128 rows of W over the whole of k; two share an
+// SM, so that one's epilogue overlaps the other's loads.  Four warps: one lane of the first asks for boxes of W and x (TMA, 128-byte
 // swizzle) into a ring of stages - the boxes of W that nothing queued writes before it waits for the kernel ahead - one lane of the second issues the
-// products, and all four read the accumulator back, each its 32 lanes, a lane being a row of W: 32 neighbouring numbers of a row of y.
+// products, and all four read the accumulator back, each its 32 lanes, a lane being a row of W.
+//
+// Measured and dropped: partial sums over slices of k for the products into the stream and the rotation (33 to 200 rows: 6.4 us for the 4B shape's output
+// projection of 64 rows where the library takes 8.4, 10.6 and 14.9 for the down projection; but the norm that adds 14 parts up lost what they gained: steps of
+// 64 to 190 tokens 2 % faster to 10 % slower); slices added up in a cluster (2.5 to 4 us more than partial sums) or by the last block of a tile (9 to 60 us).
 //
 // The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k: the steps of 16 k take turns on as many
-// accumulators as fit beside each other in 256 columns of tensor memory (eight at most), which the epilogue adds in float32.
+// accumulators as fit beside each other in 256 columns of tensor memory (16 at most), which the epilogue adds in float32.
 //
 // All waits on mbarriers are bounded: one that runs out sets an error word, the block waits for its own copies, frees its tensor memory and returns.
 // No TMA load here uses cluster multicast.
 //
-// Stands in for the library product behind raun6k/Pylon's nn.Linear (src/pylon/model/layers.py:26-27,126,138).
+// Stands in for the first half of raun6k/Pylon's feed-forward (src/pylon/model/layers.py:13-27).
 #include "common.cuh"
 
 #include <cuda.h>
@@ -26,9 +30,8 @@
 namespace pylon {
 
 constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 128, GC_MOST_STAGES = 8;   // weight rows and k of a box
-constexpr int GC_MOST_CHAINS = 8, GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
+constexpr int GC_MOST_CHAINS = 16, GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
 constexpr unsigned GC_WAIT_LIMIT = 1u << 22;                                                 // try_wait calls before a wait gives up
-enum GcForm { GC_PARTIAL = 0, GC_PRODUCT = 1, GC_GATED = 2 };
 
 __device__ __forceinline__ uint32_t gc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void gc_mbar_init(uint64_t* bar, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(gc_smem(bar)), "r"(count)); }
@@ -76,13 +79,8 @@ __device__ __forceinline__ float gc_unit(float gate, float up, float limit, floa
   }
   return __fdividef(gate, 1.f + __expf(-gain * gate)) * up;   // approximate division: ample for bfloat16, no slow path
 }
-__device__ __forceinline__ uint32_t gc_pack(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
 struct GcArgs {
-  void* y;
+  __nv_bfloat16* y;
   long long ldy;
   int M, N, K, columns, stages, chains, tmem_columns;   // columns: M rounded up to 16; chains: a power of two
   float unit_limit, unit_alpha;
@@ -90,8 +88,7 @@ struct GcArgs {
   int* error;   // 1: the copies, 2: the products, 3: the accumulator did not come in time
 };
 
-// Grid (slices of k, tiles of 128 weight rows).
-template <int FORM>
+// Grid (tiles of 128 weight rows).
 __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GcArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -101,9 +98,7 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
   const int columns = a.columns, stages = a.stages, w_bytes = GC_ROWS * GC_BK * 2, x_bytes = columns * GC_BK * 2;
   unsigned char* w_tiles = smem;
   unsigned char* x_tiles = smem + stages * w_bytes;
-  const int boxes_of_k = (a.K + GC_BK - 1) / GC_BK;
-  const int box0 = (int)((long long)boxes_of_k * blockIdx.x / gridDim.x), boxes = (int)((long long)boxes_of_k * (blockIdx.x + 1) / gridDim.x) - box0;
-  const int row0 = blockIdx.y * GC_ROWS;
+  const int boxes = (a.K + GC_BK - 1) / GC_BK, row0 = blockIdx.x * GC_ROWS;
   const int chains = a.chains;
 
   const int ahead = a.w_static ? min(stages, boxes) : 0;
@@ -113,7 +108,7 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     for (int s = 0; s < ahead; ++s) {
       gc_expect(&full[s], w_bytes + x_bytes);
-      gc_load(w_tiles + s * w_bytes, &map_w, &full[s], (box0 + s) * GC_BK, row0);
+      gc_load(w_tiles + s * w_bytes, &map_w, &full[s], s * GC_BK, row0);
     }
   }
   if (warp == 1) {   // the whole warp allocates
@@ -133,9 +128,9 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
       if (issued >= ahead) {
         if (round > 0 && !gc_wait(&empty[s], (round - 1) & 1)) { atomicExch(a.error, 1); break; }
         gc_expect(&full[s], w_bytes + x_bytes);
-        gc_load(w_tiles + s * w_bytes, &map_w, &full[s], (box0 + issued) * GC_BK, row0);
+        gc_load(w_tiles + s * w_bytes, &map_w, &full[s], issued * GC_BK, row0);
       }
-      gc_load(x_tiles + s * x_bytes, &map_x, &full[s], (box0 + issued) * GC_BK, 0);
+      gc_load(x_tiles + s * x_bytes, &map_x, &full[s], issued * GC_BK, 0);
       if (++s == stages) { s = 0; ++round; }
     }
   } else if (warp == 1 && lane == 0) {
@@ -163,38 +158,12 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
   if (!complete && lane == 0) atomicExch(a.error, 3);
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 
-  // This thread's row of W; what it has of 16 rows of x from c0 on goes to y.
-  const int n = row0 + threadIdx.x;
-  auto write = [&](int c0, const float (&v)[16]) {
-    if (FORM == GC_PARTIAL) {
-      float* dst = reinterpret_cast<float*>(a.y) + ((size_t)blockIdx.x * a.M + c0) * a.N + n;
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (n < a.N && c0 + j < a.M) dst[(size_t)j * a.N] = v[j];
-    } else if (FORM == GC_PRODUCT) {
-      // Neighbouring lanes exchange, so that each stores two neighbouring numbers: even lanes of the even rows of x, odd lanes of the odd ones.
-      const int odd = lane & 1;
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.y) + (size_t)(c0 + odd) * a.ldy + (n - odd);
-#pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
-        if (n < a.N && c0 + j + odd < a.M) *reinterpret_cast<uint32_t*>(dst + (size_t)j * a.ldy) = odd ? gc_pack(other, v[j + 1]) : gc_pack(v[j], other);
-      }
-    } else {
-      // Rows of gate and up alternate in groups of 8: lanes 8 apart exchange, the gate's lane then makes the even rows of x, the up's the odd ones.
-      const int is_up = (lane >> 3) & 1;
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.y) + (size_t)(c0 + is_up) * a.ldy + (n >> 4) * 8 + (n & 7);
-#pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        const float other = __shfl_xor_sync(0xffffffffu, is_up ? v[j] : v[j + 1], 8);
-        const float unit = is_up ? gc_unit(other, v[j + 1], a.unit_limit, a.unit_alpha) : gc_unit(v[j], other, a.unit_limit, a.unit_alpha);
-        if (n < a.N && c0 + j + is_up < a.M) dst[(size_t)j * a.ldy] = __float2bfloat16_rn(unit);
-      }
-    }
-  };
-  // The block's sums of 16 rows of x, its chains added up in order.
+  // This thread's row of W and, 16 rows of x at a time, its sums: the chains' in order.  Rows of gate and up alternate in groups of 8: lanes 8 apart exchange,
+  // the gate's lane then makes the even rows of x, the up's the odd ones.
+  const int n = row0 + threadIdx.x, is_up = (lane >> 3) & 1;
   const uint32_t lane_address = tmem + ((uint32_t)(warp * 32) << 16);
-  auto sums = [&](int c0, float (&v)[16]) {
+  for (int c0 = 0; complete && c0 < columns; c0 += 16) {
+    float v[16];
     uint32_t raw[16];
     gc_read(lane_address + c0, raw);
     gc_read_done();
@@ -206,11 +175,13 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(raw[j]);
     }
-  };
-  for (int c0 = 0; complete && c0 < columns; c0 += 16) {
-    float v[16];
-    sums(c0, v);
-    write(c0, v);
+    __nv_bfloat16* dst = a.y + (size_t)(c0 + is_up) * a.ldy + (n >> 4) * 8 + (n & 7);
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      const float other = __shfl_xor_sync(0xffffffffu, is_up ? v[j] : v[j + 1], 8);
+      const float unit = is_up ? gc_unit(other, v[j + 1], a.unit_limit, a.unit_alpha) : gc_unit(v[j], other, a.unit_limit, a.unit_alpha);
+      if (n < a.N && c0 + j + is_up < a.M) dst[(size_t)j * a.ldy] = __float2bfloat16_rn(unit);
+    }
   }
   if (!complete && threadIdx.x == 0)   // no copy outlives the block
     for (int box = max(0, issued - stages); box < issued; ++box) gc_wait(&full[box % stages], (box / stages) & 1);
@@ -263,65 +234,44 @@ static bool matrix_map(CUtensorMap* map, const void* base, long long rows, long 
 
 constexpr int GC_SMEM = 112 * 1024;   // two blocks to an SM: the next kernel's move in beside the last of this one's and ask for their weights
 
-template <int FORM>
-static int launch_columns(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, int parts,
-                          float limit, float alpha, int w_static, int* error, cudaStream_t stream, const char* name) {
+}  // namespace pylon
+
+// The gated unit of x gate^T and x up^T: x bfloat16 [M, K] (row stride ldx), M <= 256; w bfloat16 [N, K] (row stride ldw), its rows interleaved in groups of
+// 8 (rows 16b..16b+7 gate rows 8b..8b+7, rows 16b+8..16b+15 the matching up rows; N a multiple of 16); y bfloat16 [M, N / 2], row stride ldy.  limit 0:
+// silu(gate) * up; limit > 0: the clamped unit, min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).  K and the
+// operands' row strides multiples of 8, x and w 16-byte aligned.  error: one int in device memory that the kernel sets non-zero if one of its waits ran
+// out (the result is then void).  w_static: 1 where nothing queued on the stream writes w; its first boxes are then asked for while the kernel ahead is
+// still running.
+extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, float limit,
+                                        float alpha, int* error, int w_static, cudaStream_t stream) {
+  using namespace pylon;
   if (M <= 0 || N <= 0) return 0;
-  if (M > 256) PYLON_REFUSE("%s: M = %d is more than 256 rows", name, M);
-  if (K <= 0 || K % 8 || ldx % 8 || ldw % 8) PYLON_REFUSE("%s: K = %d and the row strides must be multiples of 8", name, K);
-  if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 4)) PYLON_REFUSE("%s: x and w must be 16-byte aligned", name);
-  if (ldx < K || ldw < K) PYLON_REFUSE("%s: a row stride is shorter than its row", name);
-  const int boxes = (K + GC_BK - 1) / GC_BK, tiles = (N + GC_ROWS - 1) / GC_ROWS;
-  if (parts < 1 || parts > boxes || parts > 65535 || tiles > 65535) PYLON_REFUSE("%s: %d slices of %d steps of k, %d tiles", name, parts, boxes, tiles);
-  if (!error) PYLON_REFUSE("%s: an error word is needed", name);
-  auto kernel = gemm_columns_kernel<FORM>;
+  if (M > 256) PYLON_REFUSE("gemm_columns_gated: M = %d is more than 256 rows", M);
+  if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_columns_gated: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
+  if (limit < 0.f) PYLON_REFUSE("gemm_columns_gated: the limit must not be negative");
+  if (K <= 0 || K % 8 || ldx % 8 || ldw % 8) PYLON_REFUSE("gemm_columns_gated: K = %d and the row strides must be multiples of 8", K);
+  if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 2)) PYLON_REFUSE("gemm_columns_gated: x and w must be 16-byte aligned");
+  if (ldx < K || ldw < K) PYLON_REFUSE("gemm_columns_gated: a row stride is shorter than its row");
+  if (!error) PYLON_REFUSE("gemm_columns_gated: an error word is needed");
   static bool configured_on[MAX_DEVICES] = {};   // function attributes belong to a device
   bool& configured = configured_on[current_device_slot()];
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM);
-    if (err != cudaSuccess) PYLON_REFUSE("%s: %s", name, cudaGetErrorString(err));
+    cudaError_t err = cudaFuncSetAttribute(gemm_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM);
+    if (err != cudaSuccess) PYLON_REFUSE("gemm_columns_gated: %s", cudaGetErrorString(err));
     configured = true;
   }
   GcArgs a;
-  a.y = y; a.ldy = ldy; a.M = M; a.N = N; a.K = K;
+  a.y = (__nv_bfloat16*)y; a.ldy = ldy; a.M = M; a.N = N; a.K = K;
   a.columns = (M + 15) / 16 * 16;
-  const int stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2, room = GC_SMEM - 1024;
-  a.stages = std::min({room / stage_bytes, GC_MOST_STAGES, boxes});
+  const int boxes = (K + GC_BK - 1) / GC_BK, stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2;
+  a.stages = std::min({(GC_SMEM - 1024) / stage_bytes, GC_MOST_STAGES, boxes});
   a.chains = 1;
-  while (a.chains < GC_MOST_CHAINS && 2 * a.chains * a.columns <= GC_COLUMNS && 2 * a.chains <= boxes / parts * (GC_BK / 16)) a.chains *= 2;
+  while (a.chains < GC_MOST_CHAINS && 2 * a.chains * a.columns <= GC_COLUMNS && 2 * a.chains <= boxes * (GC_BK / 16)) a.chains *= 2;
   a.tmem_columns = 32;
   while (a.tmem_columns < a.chains * a.columns) a.tmem_columns *= 2;
   a.unit_limit = limit; a.unit_alpha = alpha; a.w_static = w_static; a.error = error;
   CUtensorMap map_w, map_x;
-  if (!matrix_map(&map_w, w, N, K, ldw, GC_ROWS) || !matrix_map(&map_x, x, M, K, ldx, a.columns)) PYLON_REFUSE("%s: the tensor maps could not be made", name);
-  launch_dependent<LAUNCH_GEMM>(kernel, dim3(parts, tiles), dim3(GC_THREADS), (size_t)a.stages * stage_bytes + 1024, stream, map_w, map_x, a);
-  PYLON_CHECK_LAUNCH(name);
-}
-
-}  // namespace pylon
-
-// x: bfloat16 [M, K] (row stride ldx), M <= 256; w: bfloat16 [N, K] (row stride ldw); y: float32 [parts, M, N] contiguous, whose sum over the
-// first dimension is x @ w.T.  K and the row strides multiples of 8, x and w 16-byte aligned, 1 <= parts <= number of 64-wide steps of
-// k.  error: one int in device memory that the kernel sets non-zero if one of its waits ran out (the
-// result is then void).  w_static: 1 where nothing queued on the stream writes w; its first boxes are then asked for while the kernel ahead is still running.
-extern "C" int pylon_gemm_columns_partial(const void* x, const void* w, float* y, int M, int N, int K, long long ldx, long long ldw, int parts,
-                                          int* error, int w_static, cudaStream_t stream) {
-  return pylon::launch_columns<pylon::GC_PARTIAL>(x, w, y, M, N, K, ldx, ldw, N, parts, 0.f, 1.f, w_static, error, stream, "gemm_columns_partial");
-}
-
-// The product itself: y bfloat16 [M, N], row stride ldy; N and ldy even.
-extern "C" int pylon_gemm_columns_bf16(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
-                                       int* error, int w_static, cudaStream_t stream) {
-  if (ldy < N || N % 2 || ldy % 2) PYLON_REFUSE("gemm_columns_bf16: N = %d and the result's row stride must be even, the stride no shorter than a row", N);
-  return pylon::launch_columns<pylon::GC_PRODUCT>(x, w, y, M, N, K, ldx, ldw, ldy, 1, 0.f, 1.f, w_static, error, stream, "gemm_columns_bf16");
-}
-
-// The gated unit of x gate^T and x up^T: w's rows are interleaved in groups of 8 (rows 16b..16b+7 gate rows 8b..8b+7, rows 16b+8..16b+15 the matching up
-// rows; N a multiple of 16); y bfloat16 [M, N / 2], row stride ldy.  limit 0: silu(gate) * up; limit > 0: the clamped unit,
-// min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1).
-extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, float limit,
-                                        float alpha, int* error, int w_static, cudaStream_t stream) {
-  if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_columns_gated: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
-  if (limit < 0.f) PYLON_REFUSE("gemm_columns_gated: the limit must not be negative");
-  return pylon::launch_columns<pylon::GC_GATED>(x, w, y, M, N, K, ldx, ldw, ldy, 1, limit, alpha, w_static, error, stream, "gemm_columns_gated");
+  if (!matrix_map(&map_w, w, N, K, ldw, GC_ROWS) || !matrix_map(&map_x, x, M, K, ldx, a.columns)) PYLON_REFUSE("gemm_columns_gated: the tensor maps could not be made");
+  launch_dependent<LAUNCH_GEMM>(gemm_columns_kernel, dim3((N + GC_ROWS - 1) / GC_ROWS), dim3(GC_THREADS), (size_t)a.stages * stage_bytes + 1024, stream, map_w, map_x, a);
+  PYLON_CHECK_LAUNCH("gemm_columns_gated");
 }

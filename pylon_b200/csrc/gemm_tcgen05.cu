@@ -181,7 +181,7 @@ struct RotateArgs {
   // the gated unit of a SWIGLU epilogue: limit 0 is silu(gate) * up; limit > 0 the clamped unit,
   // min(gate, limit) * sigmoid(alpha * min(gate, limit)) * (clamp(up, -limit, limit) + 1)
   float unit_limit = 0.f, unit_alpha = 1.f;
-  int w_static = 0;   // nothing queued on the stream writes the weights: with R = 2 their first boxes are asked for while the kernel ahead still runs
+  int w_static = 0;   // nothing queued on the stream writes the weights: with one tile of rows to a block's round (at most 128 rows, or R = 2) their first boxes are asked for while the kernel ahead still runs
   const float* unit_row_scale = nullptr;   // not null: a row's sums of gate and up are multiplied by its number before the unit (a row of the operand times it)
 };
 enum TcMode { TC_PLAIN = 0, TC_SWIGLU = 1, TC_ROTATE = 2 };
@@ -349,10 +349,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tcgen05_kernel(const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
-  // Barriers and tensor memory are set up while the kernel before this one finishes (dependent launch).  With R = 2, one round of tiles whose
+  // Barriers and tensor memory are set up while the kernel before this one finishes (dependent launch).  With one tile of rows in all, or R = 2, whose
   // weights come from memory, the first boxes of weights that nothing queued writes (w_static) are asked for as well; the activations' boxes
   // follow on the same barriers.  (Products of many rows gain nothing: 2,079 rows beside decoded ones 6.81 against 6.70 ms a step.)
-  const int ahead = R == 1 || !rot.w_static || (int)blockIdx.x >= total_tiles ? 0 : (k_blocks < stages ? k_blocks : stages);
+  const int ahead = (R == 1 && (tiles_m > 1 || tile_group)) || !rot.w_static || (int)blockIdx.x >= total_tiles ? 0 : (k_blocks < stages ? k_blocks : stages);
   if (warp == 0 && lane == 0) {
     for (int kb = 0; kb < ahead; ++kb) {
       mbar_expect_tx(&full[kb], a_bytes + S::B_BYTES);
@@ -637,16 +637,16 @@ static int gemm_tcgen05_entry(const void* x, const void* w, void* y, int M, int 
   __nv_bfloat16* out = (__nv_bfloat16*)y;
 #define PYLON_TC_CASE(BN_)                                                                                          \
   if (bn == BN_) {                                                                                                  \
-    if (swiglu) return launch_tcgen05<BN_, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale); \
-    return launch_tcgen05<BN_, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N);                          \
+    if (swiglu) return launch_tcgen05<BN_, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale, w_static); \
+    return launch_tcgen05<BN_, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N, nullptr, w_static);       \
   }
   if (row_tiles == 2) return launch_tcgen05<192, true, 2>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, nullptr, 0, nullptr, w_static);
   PYLON_TC_CASE(256) PYLON_TC_CASE(192)
 #undef PYLON_TC_CASE
-  if (bn == 288) return launch_tcgen05<288, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream);
-  if (bn == 160) return launch_tcgen05<160, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream);
-  if (swiglu) return launch_tcgen05<128, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale);
-  return launch_tcgen05<128, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N);
+  if (bn == 288) return launch_tcgen05<288, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, nullptr, 0, nullptr, w_static);
+  if (bn == 160) return launch_tcgen05<160, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, nullptr, 0, nullptr, w_static);
+  if (swiglu) return launch_tcgen05<128, true>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, unit_limit, unit_alpha, tile_group, N, unit_row_scale, w_static);
+  return launch_tcgen05<128, false>(map_a, map_b, out, M, N, K, ldy, error, sm_count, stream, 0.f, 1.f, tile_group, N, nullptr, w_static);
 }
 
 // The grouped form: w is [groups, N, K] (contiguous in its first dimension: group g's rows start at row g * N), and the 128 rows of

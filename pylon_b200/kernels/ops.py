@@ -275,8 +275,6 @@ _SIGNATURES = {
         "pylon_gemm_stream_glu_clamped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_int, c_void_p],
     },
     "gemm_columns.cu": {
-        "pylon_gemm_columns_partial": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_void_p, c_int, c_void_p],
-        "pylon_gemm_columns_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_int, c_void_p],
         "pylon_gemm_columns_gated": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_float, c_float, c_void_p, c_int, c_void_p],
     },
     "gemm_tcgen05.cu": {
@@ -768,15 +766,6 @@ def _tcgen05_fills_the_sms(m: int, n: int, sms: int) -> bool:
 
 STREAM_MAX_ROWS = 32   # up to this many rows the TMA-fed kernel beats the library (it takes up to 64)
 STREAM_MAX_PARTS = 4
-COLUMNS_MAX_ROWS = 160
-
-
-def _columns_take(x: torch.Tensor, w: torch.Tensor, most_rows: int) -> bool:
-    """Whether :func:`linear_columns` takes this product: more rows than the TMA-fed kernel's, up to ``most_rows``, in bfloat16 and aligned for TMA."""
-    m, k = x.shape
-    return (STREAM_MAX_ROWS < m <= most_rows and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and k >= 1024 and k % 8 == 0
-            and w.shape[0] % 16 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.stride(0) >= k
-            and w.stride(0) >= k and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def linear_for_residual(x: torch.Tensor, w: torch.Tensor, static_weights: bool = False) -> torch.Tensor:
@@ -791,8 +780,6 @@ def linear_for_residual(x: torch.Tensor, w: torch.Tensor, static_weights: bool =
             and n % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         return linear_stream_partial(x, w, static_weights=static_weights)
-    if _columns_take(x, w, COLUMNS_MAX_ROWS):
-        return linear_columns(x, w, "partial", static_weights=static_weights)
     return linear(x, w, static_weights=static_weights)
 
 
@@ -807,14 +794,7 @@ def linear_for_rotation(x: torch.Tensor, w: torch.Tensor, head_dim: int, rotary_
             and head_dim in (64, 128, 256) and rotary_dim in (0, head_dim) and n % 4 == 0 and x.stride(1) == 1 and w.stride(1) == 1
             and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         return linear_stream_partial(x, w, static_weights=static_weights)
-    if ROTATION_COLUMNS and head_dim in (64, 128, 256) and rotary_dim in (0, head_dim) and _columns_take(x, w, COLUMNS_MAX_ROWS):
-        return linear_columns(x, w, "partial", static_weights=static_weights)
     return linear(x, w, static_weights=static_weights)
-
-
-ROTATION_COLUMNS = True
-COLUMNS_MAX_PARTS = 14
-GATED_COLUMNS = ()
 
 
 def stream_error_word(device: torch.device) -> torch.Tensor:
@@ -868,33 +848,27 @@ def linear_stream(x: torch.Tensor, w: torch.Tensor, swiglu: bool = False, limit:
     return y
 
 
-def linear_columns(x: torch.Tensor, w: torch.Tensor, form: str = "product", parts: Optional[int] = None, limit: Optional[float] = None, alpha: float = 1.0,
-                   static_weights: bool = False) -> torch.Tensor:
-    """bfloat16 ``x [M <= 256, K] @ w [N, K].T`` on the tcgen05 kernel whose tiles are 128 weight rows wide and as many rows of ``x`` deep as there are.
-    ``form``: ``"product"`` (bfloat16 ``[M, N]``), ``"gated"`` (the rows of ``w`` interleaved by :func:`interleave_gate_up`, the unit of
-    :func:`linear_stream`, ``[M, N / 2]``) or ``"partial"`` (float32 sums over ``parts`` slices of k, ``[parts, M, N]``; by default as many as give every SM
-    two blocks, up to ``COLUMNS_MAX_PARTS``)."""
+def linear_gated_columns(x: torch.Tensor, w: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0, static_weights: bool = False) -> torch.Tensor:
+    """The gated unit of :func:`linear_stream` (the rows of ``w`` interleaved by :func:`interleave_gate_up`) for bfloat16 ``x [M <= 256, K]`` on the tcgen05
+    kernel whose tiles are 128 weight rows wide and as many rows of ``x`` deep as there are."""
     _need_cuda(x, w)
     _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16,
-          "linear_columns: bfloat16 x [M, K] and w [N, K]")
-    _need(x.stride(1) == 1 and w.stride(1) == 1, "linear_columns: the reduced dimension must be contiguous")
-    _need(form in ("product", "partial", "gated") and (form == "partial" or parts is None), f"linear_columns: form {form!r} with {parts} parts")
+          "linear_gated_columns: bfloat16 x [M, K] and w [N, K]")
+    _need(x.stride(1) == 1 and w.stride(1) == 1, "linear_gated_columns: the reduced dimension must be contiguous")
     m, k = x.shape
     n = w.shape[0]
-    library, error, static = _library("gemm_columns.cu"), _ptr(stream_error_word(x.device)), int(static_weights)
-    if form == "partial":
-        if parts is None:
-            parts = max(1, min(COLUMNS_MAX_PARTS, -(-k // 64), 2 * _multiprocessors(x.device) // -(-n // 128)))
-        y = torch.empty((parts, m, n), dtype=torch.float32, device=x.device)
-        _check(library, library.pylon_gemm_columns_partial(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), parts, error, static, _stream()))
-        return y
-    y = torch.empty((m, n // 2 if form == "gated" else n), dtype=torch.bfloat16, device=x.device)
-    if form == "gated":
-        _check(library, library.pylon_gemm_columns_gated(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit or 0.0), float(alpha),
-                                                         error, static, _stream()))
-    else:
-        _check(library, library.pylon_gemm_columns_bf16(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), error, static, _stream()))
+    y = torch.empty((m, n // 2), dtype=torch.bfloat16, device=x.device)
+    library = _library("gemm_columns.cu")
+    _check(library, library.pylon_gemm_columns_gated(_ptr(x), _ptr(w), _ptr(y), m, n, k, x.stride(0), w.stride(0), y.stride(0), float(limit or 0.0), float(alpha),
+                                                     _ptr(stream_error_word(x.device)), int(static_weights), _stream()))
     return y
+
+
+def _gated_columns_fill(m: int, n: int, sms: int) -> bool:
+    """Whether the gated product of 9 to 32 rows goes to :func:`linear_gated_columns`: where its blocks, two to an SM, are one round that is three
+    quarters full.  Behind a norm, 16 and 32 rows: [34816, 5120] 58 and 62 us, :func:`linear_stream` 66 and 75; [28672, 4096] 45 and 46, 47 and
+    51; but [24576, 4096] 40 and 42, 36 and 38, and [51200, 5120] 92 and 96, 80 and 85.  (A row's distance from 64-bit sums is half an ulp of bfloat16 in both.)"""
+    return SKINNY_MAX_ROWS < m <= STREAM_MAX_ROWS and 3 * sms <= 2 * -(-n // 128) <= 4 * sms
 
 
 def linear_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, static_weights: bool = False) -> torch.Tensor:
@@ -1024,6 +998,19 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return torch.stack((gate.reshape(inter // 8, 8, k), up.reshape(inter // 8, 8, k)), dim=1).reshape(2 * inter, k).contiguous()
 
 
+def _gated_tcgen05(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the gated product of more than ``STREAM_MAX_ROWS`` rows goes to the tcgen05 kernel rather than to the library and a kernel for the unit: always from
+    ``TCGEN05_MIN_ROWS`` rows on.  Fewer are one row tile that asks for its first weights behind the kernel ahead, and what they read is W: from 65 rows on
+    where 128 columns for every SM do not hold it (80 rows behind a norm: [19456, 2560] 24.6 us, the library 26.1; [24576, 4096] 43 and 47;
+    but [16384, 2048] 17.4 and 16.3), from 33 on at half as much again (48 rows of [34816, 5120] 63 and 67, of [24576, 4096] 42 and 41).  Rows that share memory
+    are the library's."""
+    m, k = x.shape
+    n, sms = w.shape[0], _multiprocessors(x.device)
+    if m >= TCGEN05_MIN_ROWS:
+        return True
+    return m > STREAM_MAX_ROWS and n >= (128 if m > 64 else 192) * sms and x.stride(0) >= k and w.stride(0) >= k
+
+
 def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0, static_weights: bool = False) -> torch.Tensor:
     """``silu(x @ gate.T) * (x @ up.T)`` for weights stacked by :func:`interleave_gate_up`:
     one kernel for few rows (the TMA-fed decode kernel) and for many (the tcgen05 kernel), the
@@ -1035,10 +1022,10 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and m <= STREAM_MAX_ROWS and x.shape[1] == k
             and k % 8 == 0 and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0
             and w_interleaved.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
-        if GATED_COLUMNS and n >= GATED_COLUMNS[0] and m > 8: return linear_columns(x, w_interleaved, "gated", limit=limit, alpha=alpha, static_weights=static_weights)
+        if _gated_columns_fill(m, n, _multiprocessors(x.device)):
+            return linear_gated_columns(x, w_interleaved, limit=limit, alpha=alpha, static_weights=static_weights)
         return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)
-    if GATED_COLUMNS and n >= GATED_COLUMNS[1] and m <= GATED_COLUMNS[2]: return linear_columns(x, w_interleaved, "gated", limit=limit, alpha=alpha, static_weights=static_weights)
-    if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and m >= TCGEN05_MIN_ROWS and k % 8 == 0
+    if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and _gated_tcgen05(x, w_interleaved) and k % 8 == 0
             and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0 and w_interleaved.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
         return linear_tcgen05(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)   # many rows: our tcgen05 kernel with the gated unit in its epilogue

@@ -661,29 +661,36 @@ def test_a_block_table_that_names_a_page_outside_the_pool_is_reported(dtype):
     ops.raise_on_kernel_errors(device)
 
 
-@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 100, 129, 160, 256])
+@pytest.mark.parametrize("m", [1, 9, 16, 17, 32, 33, 100, 256])
 @pytest.mark.parametrize("n, k", [(128, 64), (144, 1_032), (400, 2_568), (2_048, 584)])
-def test_tcgen05_product_with_the_weights_on_the_wide_side(m, n, k):
-    """Around the edges of its tiles (16 rows of x, 128 weight rows, 64 k), few and many slices of k, every form; rows behind the last one stay as they were."""
+def test_gated_product_with_the_weights_on_the_wide_side(m, n, k):
+    """Around the edges of its tiles (16 rows of x, 128 weight rows, 64 k), with few and many chains, the plain and the clamped unit."""
     from pylon_b200.kernels import ops
 
     x = torch.randn(m, k + 8, device=DEVICE).to(torch.bfloat16)[:, :k]
     w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
-    expected = x.double() @ w.double().T
-    steps = -(-k // 64)
-    for parts in sorted({1, min(3, steps), min(14, steps), steps}):
-        sums = ops.linear_columns(x, w, "partial", parts=parts)
-        assert sums.shape == (parts, m, n)
-        # numbers of order 1, cut off at 2^-24 of a partial sum for every 16 k of a chain and every chain: some k / 16 of them at most
-        torch.testing.assert_close(sums.double().sum(0), expected, rtol=0, atol=(k / 16 + 16) * 2.0**-22)
+    pairs = (x.double() @ w.double().T).view(m, n // 16, 2, 8)
     rounded = dict(rtol=2.0**-8, atol=1e-4)   # half an ulp of bfloat16, and the float32 sums' error where they cancel
-    torch.testing.assert_close(ops.linear_columns(x, w, static_weights=True).double(), expected, **rounded)
-    pairs = expected.view(m, n // 16, 2, 8)
     gate, up = pairs[:, :, 0].reshape(m, -1), pairs[:, :, 1].reshape(m, -1)
-    torch.testing.assert_close(ops.linear_columns(x, w, "gated").double(), gate * torch.sigmoid(gate) * up, **rounded)
+    for static in (False, True):
+        torch.testing.assert_close(ops.linear_gated_columns(x, w, static_weights=static).double(), gate * torch.sigmoid(gate) * up, **rounded)
     gate, up = gate.clamp(max=0.5), up.clamp(-0.5, 0.5)
-    torch.testing.assert_close(ops.linear_columns(x, w, "gated", limit=0.5, alpha=1.7).double(), gate * torch.sigmoid(1.7 * gate) * (up + 1), **rounded)
+    torch.testing.assert_close(ops.linear_gated_columns(x, w, limit=0.5, alpha=1.7).double(), gate * torch.sigmoid(1.7 * gate) * (up + 1), **rounded)
     assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
+
+
+@pytest.mark.parametrize("m, n, k", [(9, 28_672, 1_024), (32, 34_816, 256), (33, 34_816, 256), (64, 30_000, 512), (65, 19_456, 520), (100, 24_576, 1_024), (127, 19_456, 512)])
+def test_linear_swiglu_around_the_edges_of_its_dispatch(m, n, k):
+    """Rows and weight rows at which another kernel takes over; rows that share memory are still multiplied."""
+    from pylon_b200.kernels import ops
+
+    n -= n % 16
+    w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
+    storage = torch.randn(m * k, device=DEVICE).to(torch.bfloat16)
+    for x in (storage.view(m, k), *((torch.as_strided(storage, (m, k), (k - 8, 1)),) if m > 32 else ())):
+        pairs = (x.double() @ w.double().T).view(m, n // 16, 2, 8)
+        gate, up = pairs[:, :, 0].reshape(m, -1), pairs[:, :, 1].reshape(m, -1)
+        torch.testing.assert_close(ops.linear_swiglu(x, w, static_weights=True).double(), gate * torch.sigmoid(gate) * up, rtol=2e-2, atol=2e-2)
 
 
 def test_skinny_gemm_refuses():

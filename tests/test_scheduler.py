@@ -455,3 +455,19 @@ def test_running_ahead_a_request_that_ends_by_length_makes_room_when_its_last_to
     assert [request.request_id for request in scheduler.leaving] == ["c"] and cache.free_slots() == 1
     assert scheduler.abort("c") and not scheduler.leaving
     assert scheduler.run() == [] and not scheduler.has_work()
+
+
+@pytest.mark.parametrize("count", [1, 2, 33])
+def test_the_arrays_of_a_decode_step_are_those_of_any_step(count):
+    from types import SimpleNamespace
+
+    import numpy as np
+    from pylon_b200.engine.step import StepEntry, StepFunction, StepLayout
+
+    entries = [StepEntry(SimpleNamespace(request_id=row, length=7 * row, slot=count - row), [1_000 + row], (0,) * (row % 3 != 1), (None, row) if row % 2 else None)
+               for row in range(count)]
+    layout = StepLayout(tokens=count, rows=count, logits=count, table_widths=(2,))
+    arrays = [np.full(layout.total, -9, dtype=np.int32) for _ in range(2)]
+    longest = StepFunction._fill_rows(entries, layout.offsets, arrays[0])
+    assert (1, StepFunction._fill_ones(entries, layout.offsets, arrays[1])) == longest
+    assert np.array_equal(*arrays)

@@ -19,7 +19,8 @@
 //          operands) and by the reads from shared memory, which add to them.  256 threads take 16 TM x 16 TN results, each thread TM x TN
 //          of them with two accumulators apiece; pairs of neighbouring k are the packed operands, so both operands stay
 //          in shared memory the way they lie in memory.  Two blocks to an SM (7 x 5: only in clusters of four, whose parking place is one tile): with
-//          one of 8 x 8 results a thread, 740 us for [224, 2560] x [19456, 2560]; with 7 x 4 or 7 x 5, 626 us (36 TFLOP/s).  One multiply-add
+//          one of 8 x 8 results a thread, 740 us for [224, 2560] x [19456, 2560]; with 7 x 4 or 7 x 5, 626 us, and with stages of 32 k, which halve the
+//          barriers, 544 (41 TFLOP/s).  One multiply-add
 //          to an instruction: the same.
 //
 //   short  k up to 128 and more than a few rows: a start of microseconds, not the sums, is what is left, and neither a ring of copies nor a
@@ -74,13 +75,13 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 template <int PENDING>
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory"); }
 
-// Copies columns [k0, k0 + BK) of ROWS rows, from row0 on, into a stage whose rows lie ROW floats apart.  Rows past the last one
+// Copies columns [k0, k0 + COLUMNS) of ROWS rows, from row0 on, into a stage whose rows lie ROW floats apart.  Rows past the last one
 // are copies of it (what is computed from them is not written), columns past K zeros.  SWIZZLE: the 16-byte unit u of row r goes to
 // unit u ^ ((r / 2) % 4), so that eight neighbouring rows of 64 bytes give the same unit from all 32 banks.  A thread's copies
 // lie in one column of units, a fixed number of rows apart: one address computation each.
-template <int VEC, int ROWS, int THREADS, int ROW, bool SWIZZLE>
+template <int VEC, int ROWS, int THREADS, int ROW, bool SWIZZLE, int COLUMNS = BK>
 __device__ __forceinline__ void stage_copy(float* dst, const float* __restrict__ src, long long ld, int row0, int last, int k0, int K, int t) {
-  constexpr int UNITS = BK / VEC, APART = THREADS / UNITS;
+  constexpr int UNITS = COLUMNS / VEC, APART = THREADS / UNITS;
   const int r0 = t / UNITS, c = (t % UNITS) * VEC;
   const bool inside = k0 + c < K;
   src += inside ? k0 + c : 0;
@@ -235,10 +236,11 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
 // ---------------------------------------------------------------------------------------------
 template <int TM, int TN>
 struct TileShape {
-  static constexpr int BM = 16 * TM, BN = 16 * TN, STAGES = 3;
+  static constexpr int BM = 16 * TM, BN = 16 * TN;
+  static constexpr int BK = 32, STAGES = 2;                // a barrier every 32 k (193 rows of [19456, 2560] 543 us; every 16 k, three stages, 621)
   static constexpr int ROW = BK + 4;                       // floats from row to row of a stage: eight rows' units lie in all 32 banks
   static constexpr int STAGE = (BM + BN) * ROW;
-  static constexpr int PARK_ROW = BN + 8, PARK = BM * PARK_ROW;
+  static constexpr int PARK_ROW = BN + 4, PARK = BM * PARK_ROW;
   static constexpr size_t smem(int blocks) { return ((size_t)STAGES * STAGE + (size_t)(blocks == 4 ? 1 : 2) * PARK) * sizeof(float); }
 };
 
@@ -249,6 +251,7 @@ struct TileShape {
 template <int TM, int TN, int VEC>
 __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const GemmArgs a) {
   using Shape = TileShape<TM, TN>;
+  constexpr int BK = Shape::BK;
   extern __shared__ __align__(16) float smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int blocks = cluster.num_blocks(), rank = cluster.block_rank();
@@ -270,12 +273,12 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const GemmArgs a)
   if (!a.w_static) grid_dependency_wait();
 #pragma unroll
   for (int s = 0; s < Shape::STAGES - 1; ++s)
-    if (s < steps) stage_copy<VEC, Shape::BN, 256, Shape::ROW, false>(stages + s * Shape::STAGE + Shape::BM * Shape::ROW, w, a.ldw, n0, a.N - 1, k_begin + s * BK, a.K, threadIdx.x);
+    if (s < steps) stage_copy<VEC, Shape::BN, 256, Shape::ROW, false, BK>(stages + s * Shape::STAGE + Shape::BM * Shape::ROW, w, a.ldw, n0, a.N - 1, k_begin + s * BK, a.K, threadIdx.x);
   grid_dependency_wait();
   allow_dependents();
 #pragma unroll
   for (int s = 0; s < Shape::STAGES - 1; ++s) {
-    if (s < steps) stage_copy<VEC, Shape::BM, 256, Shape::ROW, false>(stages + s * Shape::STAGE, x, a.ldx, m0, a.M - 1, k_begin + s * BK, a.K, threadIdx.x);
+    if (s < steps) stage_copy<VEC, Shape::BM, 256, Shape::ROW, false, BK>(stages + s * Shape::STAGE, x, a.ldx, m0, a.M - 1, k_begin + s * BK, a.K, threadIdx.x);
     copies_commit();
   }
 
@@ -293,8 +296,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_tile_kernel(const GemmArgs a)
       const int ahead = step + Shape::STAGES - 1;
       if (ahead < steps) {
         float* dst = stages + (ahead % Shape::STAGES) * Shape::STAGE;
-        stage_copy<VEC, Shape::BM, 256, Shape::ROW, false>(dst, x, a.ldx, m0, a.M - 1, k_begin + ahead * BK, a.K, threadIdx.x);
-        stage_copy<VEC, Shape::BN, 256, Shape::ROW, false>(dst + Shape::BM * Shape::ROW, w, a.ldw, n0, a.N - 1, k_begin + ahead * BK, a.K, threadIdx.x);
+        stage_copy<VEC, Shape::BM, 256, Shape::ROW, false, BK>(dst, x, a.ldx, m0, a.M - 1, k_begin + ahead * BK, a.K, threadIdx.x);
+        stage_copy<VEC, Shape::BN, 256, Shape::ROW, false, BK>(dst + Shape::BM * Shape::ROW, w, a.ldw, n0, a.N - 1, k_begin + ahead * BK, a.K, threadIdx.x);
       }
       copies_commit();
     }

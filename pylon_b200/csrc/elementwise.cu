@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_vec_kernel(float* __
     x[k] = i < groups ? Vec4<float>::load(res + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (del) {
-    constexpr int AT_ONCE = sizeof(DT) == 4 ? 4 : 1;
+    constexpr int AT_ONCE = sizeof(DT) == 4 && sizeof(T) == 2 ? 4 : 1;   // float32 activations come whole
     for (int part0 = 0; part0 < delta_parts; part0 += AT_ONCE) {
       float4 d[AT_ONCE][ITEMS];
 #pragma unroll

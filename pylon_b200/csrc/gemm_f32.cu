@@ -14,7 +14,7 @@
 //          the reads of x from shared memory, which do not overlap on them.  A lane owns two rows of W, a warp one leaf
 //          or quarter of 64 rows, which it streams through a ring of its own with cp.async; no warp waits for another before
 //          its part is done.  The rows of x are read from shared memory as broadcasts.  W [19456, 2560]: 48 us for one row of x (199 MB:
-//          4.2 TB/s), 79 us for 16; W [151936, 2560]: 243 and 399 us (6.4 TB/s and 31 TFLOP/s).
+//          4.2 TB/s), 74 us for 16; W [151936, 2560]: 243 and 369 us (6.4 TB/s and 34 TFLOP/s).
 //   tile   more rows: bound by the FMA units (2.2 to 2.5 cycles an instruction and scheduler, whatever the order of the
 //          operands) and by the reads from shared memory, which add to them.  256 threads take 16 TM x 16 TN results, each thread TM x TN
 //          of them with two accumulators apiece; pairs of neighbouring k are the packed operands, so both operands stay
@@ -102,16 +102,16 @@ __device__ __forceinline__ void stage_copy(float* dst, const float* __restrict__
 // ---------------------------------------------------------------------------------------------
 // A stage is BK columns: NR * 32 rows of W, MT rows of x.  Rows are 64 bytes; the 16-byte unit u of row r lies at unit
 // u ^ ((r / 2) % 4), so that eight neighbouring rows read the same unit from all 32 banks.
-template <int MT, int NR>
+template <int MT, int NR, int STAGES_>
 struct RowsRing {
-  static constexpr int STAGES = 4, W_FLOATS = NR * 32 * BK, X_FLOATS = MT * BK, STAGE = W_FLOATS + X_FLOATS;
+  static constexpr int STAGES = STAGES_, W_FLOATS = NR * 32 * BK, X_FLOATS = MT * BK, STAGE = W_FLOATS + X_FLOATS;
 };
 
 // Grid (slabs of NR * 32 rows of W x cluster size, MT rows of x each, products); blocks of `warps` warps.  With 16 warps in a
 // cluster each takes a leaf, with 4 a quarter.
-template <int MT, int NR, int VEC>
+template <int MT, int NR, int VEC, int STAGES>
 __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a) {
-  using Ring = RowsRing<MT, NR>;
+  using Ring = RowsRing<MT, NR, STAGES>;
   constexpr int TILE = MT * NR * 32;
   extern __shared__ __align__(16) float smem[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -143,12 +143,19 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
     copies_commit();
   }
 
-  Pair acc[MT][NR];
+  // A lane's results.  Up to 8 rows of x: all of them, of rows lane, lane + 32 of W.  16 rows: a read of x serves all lanes alike but takes as long as one of W, so
+  // the lanes share them 4 x 8: rows tm + 4 i of x, tn + 8 j of W (12 reads for 64 multiply-adds instead of 18, and from the bits of the lane
+  // that take two passes): 16 rows of [2560, 9728] 53.0 to 49.6 us, of [151936, 2560] 378 to 369.
+  constexpr bool SHARED = MT == 16 && NR == 2;
+  constexpr int MI = SHARED ? 4 : MT, NJ = SHARED ? 8 : NR;
+  const int tm = SHARED ? (lane >> 1) & 3 : 0, tn = SHARED ? ((lane >> 2) & 6) + (lane & 1) : lane;
+  auto result = [&](int i, int j) { return SHARED ? (tm + 4 * i) * (NR * 32) + tn + 8 * j : (i * NR + j) * 32 + lane; };
+  Pair acc[MI][NJ];
 #pragma unroll
-  for (int m = 0; m < MT; ++m)
+  for (int m = 0; m < MI; ++m)
 #pragma unroll
-    for (int r = 0; r < NR; ++r) acc[m][r] = 0;
-  const int leaf_steps = leaf / BK, w_xor = (lane >> 1) & 3;
+    for (int r = 0; r < NJ; ++r) acc[m][r] = 0;
+  const int leaf_steps = leaf / BK, w_xor = (tn >> 1) & 3;
   bool first = true;   // the first leaf of a quarter is its sum so far
   int until_fold = leaf_steps;
   for (int step = 0; step < steps; ++step) {
@@ -166,32 +173,35 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
     const float* stage = ring + (step % Ring::STAGES) * Ring::STAGE;
 #pragma unroll
     for (int u = 0; u < BK / 4; ++u) {
-      ulonglong2 wv[NR];
+      constexpr int GROUP = MI < 4 ? MI : 4;   // rows whose chains take turns, so that no multiply-add waits for the one before it
+      ulonglong2 wv[NJ];
 #pragma unroll
-      for (int r = 0; r < NR; ++r) wv[r] = *reinterpret_cast<const ulonglong2*>(stage + (r * 32 + lane) * BK + ((u ^ w_xor) << 2));
-      constexpr int GROUP = MT < 4 ? MT : 4;   // rows whose chains take turns, so that no multiply-add waits for the one before it
+      for (int r = 0; r < NJ; ++r) wv[r] = *reinterpret_cast<const ulonglong2*>(stage + (r * (SHARED ? 8 : 32) + tn) * BK + ((u ^ w_xor) << 2));
 #pragma unroll
-      for (int g = 0; g < MT; g += GROUP) {
+      for (int g = 0; g < MI; g += GROUP) {
         ulonglong2 xv[GROUP];
 #pragma unroll
-        for (int m = 0; m < GROUP; ++m)
-          xv[m] = *reinterpret_cast<const ulonglong2*>(stage + Ring::W_FLOATS + (g + m) * BK + ((u ^ (((g + m) >> 1) & 3)) << 2));
+        for (int m = 0; m < GROUP; ++m) {
+          const int row = SHARED ? 4 * m : g + m;   // and tm; its swizzle is that of row + tm
+          const int unit = SHARED ? (u ^ (2 * (m & 1)) ^ (tm >> 1)) : u ^ ((row >> 1) & 3);
+          xv[m] = *reinterpret_cast<const ulonglong2*>(stage + Ring::W_FLOATS + (row + tm) * BK + (unit << 2));
+        }
 #pragma unroll
         for (int m = 0; m < GROUP; ++m)
 #pragma unroll
-          for (int r = 0; r < NR; ++r) fma_pair(acc[g + m][r], xv[m].x, wv[r].x);
+          for (int r = 0; r < NJ; ++r) fma_pair(acc[g + m][r], xv[m].x, wv[r].x);
 #pragma unroll
         for (int m = 0; m < GROUP; ++m)
 #pragma unroll
-          for (int r = 0; r < NR; ++r) fma_pair(acc[g + m][r], xv[m].y, wv[r].y);
+          for (int r = 0; r < NJ; ++r) fma_pair(acc[g + m][r], xv[m].y, wv[r].y);
       }
     }
     if (--until_fold == 0 && step != steps - 1) {   // a leaf of a quarter: a lone block's warp, which keeps the sum in its own place
 #pragma unroll
-      for (int m = 0; m < MT; ++m)
+      for (int m = 0; m < MI; ++m)
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          float* place = gathered + (size_t)unit * share + (m * NR + r) * 32 + lane;
+        for (int r = 0; r < NJ; ++r) {
+          float* place = gathered + (size_t)unit * share + result(m, r);
           const float value = add_pair(acc[m][r]);
           *place = first ? value : *place + value;
           acc[m][r] = 0;
@@ -204,10 +214,10 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
   if (blocks > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   if (steps > 0) {
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+    for (int m = 0; m < MI; ++m)
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        const int e = (m * NR + r) * 32 + lane;
+      for (int r = 0; r < NJ; ++r) {
+        const int e = result(m, r);
         float* place = gathered + (size_t)unit * share + e % share;
         if (blocks > 1) place = cluster.map_shared_rank(place, e / share);
         const float value = add_pair(acc[m][r]);
@@ -519,22 +529,21 @@ constexpr long long LONE_WORK = 4096;
 
 template <int MT, int NR, int VEC>
 static int launch_rows(const GemmArgs& a, int batch, int force, cudaStream_t stream) {
-  using Ring = RowsRing<MT, NR>;
-  GemmKernel kernel = gemm_f32_rows_kernel<MT, NR, VEC>;
-  static KernelState states[MAX_DEVICES];
-  KernelState& state = states[current_device_slot()];
+  constexpr int LONE_STAGES = MT == 16 ? 2 : 4;   // three blocks to an SM instead of two: 16 rows of [151936, 2560] 394 to 378 us
+  using Lone = RowsRing<MT, NR, LONE_STAGES>;
+  using Ring = RowsRing<MT, NR, 4>;
   const long long slabs = (a.N + NR * 32 - 1) / (NR * 32);
   const long long all = slabs * batch;
   const bool lone = force ? (force & 2) : a.K <= 64 || (a.K < 512 && all >= (a.K <= 256 ? 32 : 64)) || (a.M > 4 && all * a.M >= LONE_WORK);
-  const int blocks = lone ? 1 : 8, warps = lone ? 4 : 2, units = blocks * warps;
-  const auto bytes = [](int units_, int blocks_, int warps_) {
-    return ((size_t)units_ * (MT * NR * 32 / blocks_) + (size_t)warps_ * Ring::STAGES * Ring::STAGE) * sizeof(float);
-  };
-  const size_t most = bytes(4, 1, 4) > bytes(16, 8, 2) ? bytes(4, 1, 4) : bytes(16, 8, 2);
-  cudaError_t err = configure(kernel, state, most);
+  GemmKernel kernel = lone ? gemm_f32_rows_kernel<MT, NR, VEC, LONE_STAGES> : gemm_f32_rows_kernel<MT, NR, VEC, 4>;
+  static KernelState states[2][MAX_DEVICES];
+  KernelState& state = states[lone][current_device_slot()];
+  const int blocks = lone ? 1 : 8, warps = lone ? 4 : 2;
+  const size_t lone_bytes = ((size_t)4 * MT * NR * 32 + (size_t)4 * Lone::STAGES * Lone::STAGE) * sizeof(float);
+  const size_t cluster_bytes = ((size_t)2 * MT * NR * 32 + (size_t)2 * Ring::STAGES * Ring::STAGE) * sizeof(float), bytes = lone ? lone_bytes : cluster_bytes;
+  cudaError_t err = configure(kernel, state, std::max(lone_bytes, cluster_bytes));
   if (err != cudaSuccess) PYLON_REFUSE("gemm_f32: %s", cudaGetErrorString(err));
-  launch_dependent_cluster<LAUNCH_GEMM>(kernel, dim3((unsigned)(slabs * blocks), (a.M + MT - 1) / MT, batch), dim3(32 * warps), bytes(units, blocks, warps),
-                                        stream, (unsigned)blocks, a);
+  launch_dependent_cluster<LAUNCH_GEMM>(kernel, dim3((unsigned)(slabs * blocks), (a.M + MT - 1) / MT, batch), dim3(32 * warps), bytes, stream, (unsigned)blocks, a);
   PYLON_CHECK_LAUNCH("gemm_f32");
 }
 

@@ -11,9 +11,9 @@
 // chain over the whole of k (3.2e-7 against 1.8e-6 of the result at K = 9,728).
 //
 //   rows   up to 16 rows of x (decode steps, the head): bound by the bytes of W up to some 8 rows, above by the FMA units and
-//          the reads of x from shared memory, which do not overlap on them.  A lane owns two rows of W, a warp one leaf
+//          the reads of x from shared memory, which do not overlap on them.  A lane owns two rows of W (with 9 to 16 rows of x, eight rows of W and four of x), a warp one leaf
 //          or quarter of 64 rows, which it streams through a ring of its own with cp.async; no warp waits for another before
-//          its part is done.  The rows of x are read from shared memory as broadcasts.  W [19456, 2560]: 48 us for one row of x (199 MB:
+//          its part is done.  Lanes read the rows of x that they share from shared memory as broadcasts.  W [19456, 2560]: 48 us for one row of x (199 MB:
 //          4.2 TB/s), 74 us for 16; W [151936, 2560]: 243 and 369 us (6.4 TB/s and 34 TFLOP/s).
 //   tile   more rows: bound by the FMA units (2.2 to 2.5 cycles an instruction and scheduler, whatever the order of the
 //          operands) and by the reads from shared memory, which add to them.  256 threads take 16 TM x 16 TN results, each thread TM x TN

@@ -886,7 +886,7 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = tor
     return y
 
 
-TCGEN05_MIN_ROWS = 128   # from this many rows the gate/up product runs on our tcgen05 kernel, SwiGLU in its epilogue
+TCGEN05_MIN_ROWS = 128   # from this many rows every gate/up product runs on our tcgen05 kernel, SwiGLU in its epilogue
 
 def tcgen05_error_word(device: torch.device) -> torch.Tensor:
     """The int32 word the tcgen05 kernels set when one of their bounded waits ran out
@@ -1013,8 +1013,8 @@ def _gated_tcgen05(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0, static_weights: bool = False) -> torch.Tensor:
     """``silu(x @ gate.T) * (x @ up.T)`` for weights stacked by :func:`interleave_gate_up`:
-    one kernel for few rows (the TMA-fed decode kernel) and for many (the tcgen05 kernel), the
-    library product and the SwiGLU kernel in between.  With a ``limit`` the gated unit is the clamped
+    one kernel for few rows (the TMA-fed decode kernel, or :func:`linear_gated_columns`) and for many (the tcgen05 kernel,
+    see :func:`_gated_tcgen05`), the library product and the SwiGLU kernel in between.  With a ``limit`` the gated unit is the clamped
     one of :func:`swiglu`, in the same kernels."""
     _need_cuda(x, w_interleaved)
     n, k = w_interleaved.shape

@@ -97,6 +97,29 @@ __device__ __forceinline__ void stage_copy(float* dst, const float* __restrict__
   }
 }
 
+// stage_copy of a warp's lanes with the swizzle, 16 bytes at a time, with the lane's first row looked up once: a copy then costs an addition of
+// addresses instead of a product: 8 rows of [2560, 9728] 30.9 to 28.6 us, of [2560, 4096] 15.5 to 14.5.
+template <int ROWS>
+struct RowsCopy {
+  static constexpr int UNITS = BK / 4, APART = 32 / UNITS, COPIES = (ROWS + APART - 1) / APART;
+  static_assert(APART % 8 == 0, "the unit's place must be the same for all of a lane's rows");
+  const float* src;
+  __device__ __forceinline__ RowsCopy(const float* matrix, long long ld, int row0, int last, int lane) { src = matrix + (size_t)min(row0 + lane / UNITS, last) * ld; }
+  __device__ __forceinline__ void operator()(float* stage, long long ld, int row0, int last, int k0, int K, int lane) const {
+    const int r0 = lane / UNITS, c = (lane % UNITS) * 4;
+    const bool inside = k0 + c < K, all = row0 + ROWS - 1 <= last;
+    const float* from = src + (inside ? k0 + c : 0);
+    float* to = stage + r0 * BK + ((((c >> 2) ^ (r0 >> 1)) & 3) << 2);
+#pragma unroll
+    for (int i = 0; i < COPIES; ++i) {
+      const int r = r0 + i * APART;
+      if (ROWS % APART != 0 && r >= ROWS) continue;
+      const bool there = all || row0 + r <= last;   // else zeros, and what is computed from them is not written
+      copy_async<4>(to + i * APART * BK, there ? from + i * (APART * ld) : src, there && inside);
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------------------------
 // few rows
 // ---------------------------------------------------------------------------------------------
@@ -130,16 +153,26 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
   const int k_begin = unit * leaves * leaf, k_end = min(a.K, k_begin + leaves * leaf);
   const int steps = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
 
+  const RowsCopy<NR * 32> rows_of_w(w, a.ldw, n0, a.N - 1, lane);
+  const RowsCopy<MT> rows_of_x(x, a.ldx, m0, a.M - 1, lane);
+  auto copy_w = [&](float* dst, int k0) {
+    if (VEC == 4) rows_of_w(dst, a.ldw, n0, a.N - 1, k0, a.K, lane);
+    else stage_copy<VEC, NR * 32, 32, BK, true>(dst, w, a.ldw, n0, a.N - 1, k0, a.K, lane);
+  };
+  auto copy_x = [&](float* dst, int k0) {
+    if (VEC == 4) rows_of_x(dst, a.ldx, m0, a.M - 1, k0, a.K, lane);
+    else stage_copy<VEC, MT, 32, BK, true>(dst, x, a.ldx, m0, a.M - 1, k0, a.K, lane);
+  };
   if (!a.w_static) grid_dependency_wait();
 #pragma unroll
   for (int s = 0; s < Ring::STAGES - 1; ++s)
-    if (s < steps) stage_copy<VEC, NR * 32, 32, BK, true>(ring + s * Ring::STAGE, w, a.ldw, n0, a.N - 1, k_begin + s * BK, a.K, lane);
+    if (s < steps) copy_w(ring + s * Ring::STAGE, k_begin + s * BK);
   grid_dependency_wait();
   allow_dependents();
   if (blocks > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");   // this block runs: its shared memory may be written
 #pragma unroll
   for (int s = 0; s < Ring::STAGES - 1; ++s) {
-    if (s < steps) stage_copy<VEC, MT, 32, BK, true>(ring + s * Ring::STAGE + Ring::W_FLOATS, x, a.ldx, m0, a.M - 1, k_begin + s * BK, a.K, lane);
+    if (s < steps) copy_x(ring + s * Ring::STAGE + Ring::W_FLOATS, k_begin + s * BK);
     copies_commit();
   }
 
@@ -165,8 +198,8 @@ __global__ void __launch_bounds__(128, 3) gemm_f32_rows_kernel(const GemmArgs a)
       const int ahead = step + Ring::STAGES - 1;
       if (ahead < steps) {
         float* dst = ring + (ahead % Ring::STAGES) * Ring::STAGE;
-        stage_copy<VEC, NR * 32, 32, BK, true>(dst, w, a.ldw, n0, a.N - 1, k_begin + ahead * BK, a.K, lane);
-        stage_copy<VEC, MT, 32, BK, true>(dst + Ring::W_FLOATS, x, a.ldx, m0, a.M - 1, k_begin + ahead * BK, a.K, lane);
+        copy_w(dst, k_begin + ahead * BK);
+        copy_x(dst + Ring::W_FLOATS, k_begin + ahead * BK);
       }
       copies_commit();
     }

@@ -611,6 +611,11 @@ __device__ __forceinline__ int decode_blocks_used(int total, int grid, int pairs
 __device__ __forceinline__ int run_begin(int block, int total, int used) { return (int)((long long)block * total / used); }
 __device__ __forceinline__ int run_of(int tile, int total, int used) { return (int)((((long long)tile + 1) * used - 1) / total); }   // a block takes at least this many tiles: below it the merging costs more than the walk
 
+// The log-sum-exp (log2) a partial result is weighed by, from its running maximum in log2 units and the sum of its weights: -infinity where nothing was
+// visible, and +infinity where a visible score was not a number.  fmaxf passes such scores over, so the maximum may be -infinity all the same and only the sum tells; as
+// the largest log-sum-exp of its pair it makes every weight there 0 or NaN, however the pair was cut.
+__device__ __forceinline__ float partial_lse(float max_log2, float sum) { return sum > 0.f ? max_log2 + log2f(sum) : sum == 0.f ? -INFINITY : INFINITY; }
+
 // Adds up the `segments` partial results of a (row, KV head) pair, those of blocks first_block on, and writes the pair's output; by the whole block
 // that arrived last at the pair.
 __device__ __forceinline__ void combine_segments(const AttentionParams& p, int pair, int first_block, int segments, int q0, int packed_rows, int kv_head) {
@@ -1138,7 +1143,7 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
       const float inv = total > 0.f ? 1.f / total : 0.f;
 #pragma unroll
       for (int w = 0; w < 4; ++w) merge_max[w * SMALL_ROWS + r] = weight[w] * inv;   // from here on: the warp's share
-      row_lse[r] = total > 0.f ? mx * unit + log2f(total) : -INFINITY;     // the segment's log-sum-exp (log2)
+      row_lse[r] = partial_lse(mx * unit, total);     // the segment's log-sum-exp (log2)
     }
     __syncthreads();
     const size_t slot = (size_t)pair + blockIdx.x;
@@ -1244,7 +1249,7 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
       }
       const size_t token = (size_t)q0 + r / G;
       const int head = kv_head * G + r % G;
-      p.out[token * p.out_stride + (size_t)head * D + col] = __float2bfloat16_rn((SIGMOID ? sum : (total > 0.f ? sum / total : 0.f)) * head_factor(p.heads, token, head) *
+      p.out[token * p.out_stride + (size_t)head * D + col] = __float2bfloat16_rn((SIGMOID ? sum : (total == 0.f ? 0.f : sum / total)) * head_factor(p.heads, token, head) *
                                                                                   element_factor(p.heads, token, head, col));
     }
   }
@@ -1678,7 +1683,7 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
         const float* src = (e & 1) ? reinterpret_cast<const float*>(smem_base + (size_t)(e >> 1) * Tiles::RING_BYTES) : first_pieces + (size_t)(e >> 1) * p.incoming_rows * D;
         const float4 part = *reinterpret_cast<const float4*>(src + r * D + (col ^ merge_swizzle(r)));
         const float m = piece_max[e * SMALL_ROWS + r];
-        if (!SIGMOID && m == -INFINITY) continue;   // nothing visible
+        if (!SIGMOID && piece_sum[e * SMALL_ROWS + r] == 0.f) continue;   // nothing visible (a maximum of -infinity does not say so: fmaxf passes over scores that are NaN)
         const float top = fmaxf(mx, m), alpha = SIGMOID ? 1.f : fast_exp2((mx - top) * unit), weight = SIGMOID ? 1.f : fast_exp2((m - top) * unit);
         out.x = out.x * alpha + weight * part.x; out.y = out.y * alpha + weight * part.y;
         out.z = out.z * alpha + weight * part.z; out.w = out.w * alpha + weight * part.w;
@@ -1697,7 +1702,7 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
         *reinterpret_cast<uint2*>(p.out + token * p.out_stride + (size_t)head * D + col) = make_uint2(pack_bf16(out.x, out.y), pack_bf16(out.z, out.w));
       } else {
         *reinterpret_cast<float4*>(p.decode_out + (slot * SMALL_ROWS + r) * D + col) = out;
-        if (col == 0) p.decode_lse[slot * SMALL_ROWS + r] = SIGMOID ? 0.f : sum > 0.f ? mx * unit + log2f(sum) : -INFINITY;
+        if (col == 0) p.decode_lse[slot * SMALL_ROWS + r] = SIGMOID ? 0.f : partial_lse(mx * unit, sum);
       }
     }
   }

@@ -837,6 +837,36 @@ def test_decoded_rows_a_run_to_a_warp(nq, nkv, d, page, blocks):
     assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0
 
 
+@pytest.mark.parametrize("form, page, rows, kv_len, blocks", [
+    ("a pair in one run", 64, 12, 16, None), ("a block's warps", 64, 2, 700, 1), ("many blocks", 64, 1, 3_000, None), ("few blocks", 64, 3, 700, 5),
+    ("clusters", 64, 1, 2_000, None), ("clusters", 64, 3, 90, None), ("gathered", 48, 2, 700, 1), ("gathered", 48, 1, 3_000, 40)])
+@pytest.mark.parametrize("options", ["plain", "split weights", "sigmoid"])
+def test_a_query_or_keys_that_are_not_numbers_reach_the_decoded_rows(form, page, rows, kv_len, blocks, options):
+    """However a (row, KV head) pair is cut: by one query that is NaN, and by a stretch of keys of one KV head that is (whole partial results of it)."""
+    from pylon_b200.kernels import ops
+
+    nq, nkv, d = 8, 2, 128
+    for spoilt in ("query", "first keys", "last keys", "all keys"):
+        cache = Paged([kv_len] * rows, [1] * rows, nkv, d, page, torch.bfloat16)
+        fused = torch.randn(rows, (nq + 2 * nkv) * d, device=DEVICE).to(torch.bfloat16)
+        if spoilt == "query":
+            fused[rows - 1, 5 * d + 3] = float("nan")
+            lost = [(rows - 1, 5)]
+        else:
+            begin, end = {"first keys": (0, (kv_len + 1) // 2), "last keys": (kv_len // 2, kv_len), "all keys": (0, kv_len)}[spoilt]
+            for j in range(begin, end):
+                cache.k_pages[int(cache.table[rows - 1, j // page]), 1, j % page, 7] = float("nan")
+            lost = [(rows - 1, head) for head in range(nq // nkv, nq)]
+        chosen = {"plain": {}, "split weights": {"split_weights": True}, "sigmoid": {"weighting": "sigmoid"}}[options]
+        out = ops.paged_attention(fused, cache.k_pages, cache.v_pages, cache.positions, cache.token_row, cache.q_start, cache.kv_len, cache.table, nq, 1, kv_len,
+                                  decode_blocks=blocks, rows_alike=form == "clusters", **chosen).view(rows, nq, d)
+        expected = torch.zeros(rows, nq, dtype=torch.bool, device=DEVICE)
+        for row, head in lost:
+            expected[row, head] = True
+        assert torch.equal(out.isnan().all(-1), expected) and torch.equal(out.isnan().any(-1), expected), (spoilt, out.isnan().any(-1))
+    assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0
+
+
 @pytest.mark.parametrize("nq, nkv, d, dv", [(4, 1, 64, 64), (6, 3, 20, 36), (3, 3, 128, 192), (8, 1, 132, 512), (5, 1, 8, 4)])
 @pytest.mark.parametrize("options", ["plain", "window", "kept", "chunk", "softcap", "bias", "slopes", "sinks", "sigmoid", "gate", "elements"])
 def test_float32_attention_with_shared_reads(nq, nkv, d, dv, options):

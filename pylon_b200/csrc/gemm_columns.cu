@@ -248,7 +248,7 @@ extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, i
   if (M <= 0 || N <= 0) return 0;
   if (M > 256) PYLON_REFUSE("gemm_columns_gated: M = %d is more than 256 rows", M);
   if (N % 16 || ldy < N / 2) PYLON_REFUSE("gemm_columns_gated: N = %d must be a multiple of 16 and the result N / 2 columns wide", N);
-  if (limit < 0.f) PYLON_REFUSE("gemm_columns_gated: the limit must not be negative");
+  if (!(limit >= 0.f)) PYLON_REFUSE("gemm_columns_gated: the limit must be positive, or 0 for none");
   if (K <= 0 || K % 8 || ldx % 8 || ldw % 8) PYLON_REFUSE("gemm_columns_gated: K = %d and the row strides must be multiples of 8", K);
   if (((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 2)) PYLON_REFUSE("gemm_columns_gated: x and w must be 16-byte aligned");
   if (ldx < K || ldw < K) PYLON_REFUSE("gemm_columns_gated: a row stride is shorter than its row");

@@ -855,6 +855,7 @@ def linear_gated_columns(x: torch.Tensor, w: torch.Tensor, limit: Optional[float
     _need(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16,
           "linear_gated_columns: bfloat16 x [M, K] and w [N, K]")
     _need(x.stride(1) == 1 and w.stride(1) == 1, "linear_gated_columns: the reduced dimension must be contiguous")
+    _need(limit is None or limit > 0, "linear_gated_columns: a limit must be positive")
     m, k = x.shape
     n = w.shape[0]
     y = torch.empty((m, n // 2), dtype=torch.bfloat16, device=x.device)
@@ -1017,6 +1018,7 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
     see :func:`_gated_tcgen05`), the library product and the SwiGLU kernel in between.  With a ``limit`` the gated unit is the clamped
     one of :func:`swiglu`, in the same kernels."""
     _need_cuda(x, w_interleaved)
+    _need(limit is None or limit > 0, "linear_swiglu: a limit must be positive")
     n, k = w_interleaved.shape
     m = x.shape[0]
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and m <= STREAM_MAX_ROWS and x.shape[1] == k

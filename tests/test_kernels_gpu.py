@@ -693,6 +693,18 @@ def test_linear_swiglu_around_the_edges_of_its_dispatch(m, n, k):
         torch.testing.assert_close(ops.linear_swiglu(x, w, static_weights=True).double(), gate * torch.sigmoid(gate) * up, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("m", [1, 9, 16, 32, 33, 80, 128, 200])
+@pytest.mark.parametrize("n", [1_024, 34_816])
+@pytest.mark.parametrize("limit", [0.0, -1.0, float("nan")])
+def test_a_limit_that_is_not_positive_is_refused_by_every_gated_product(m, n, limit):
+    from pylon_b200.kernels import ops
+
+    x, w = torch.zeros(m, 128, dtype=torch.bfloat16, device=DEVICE), torch.zeros(n, 128, dtype=torch.bfloat16, device=DEVICE)
+    for product in (ops.linear_swiglu, ops.linear_gated_columns):
+        with pytest.raises(ops.KernelError, match="positive"):
+            product(x, w, limit=limit)
+
+
 def test_skinny_gemm_refuses():
     from pylon_b200.kernels import ops
 

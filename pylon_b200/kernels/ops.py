@@ -999,17 +999,14 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return torch.stack((gate.reshape(inter // 8, 8, k), up.reshape(inter // 8, 8, k)), dim=1).reshape(2 * inter, k).contiguous()
 
 
-def _gated_tcgen05(x: torch.Tensor, w: torch.Tensor) -> bool:
+def _gated_tcgen05(m: int, n: int, sms: int) -> bool:
     """Whether the gated product of more than ``STREAM_MAX_ROWS`` rows goes to the tcgen05 kernel rather than to the library and a kernel for the unit: always from
     ``TCGEN05_MIN_ROWS`` rows on.  Fewer are one row tile that asks for its first weights behind the kernel ahead, and what they read is W: from 65 rows on
     where 128 columns for every SM do not hold it (80 rows behind a norm: [19456, 2560] 24.6 us, the library 26.1; [24576, 4096] 43 and 47;
-    but [16384, 2048] 17.4 and 16.3), from 33 on at half as much again (48 rows of [34816, 5120] 63 and 67, of [24576, 4096] 42 and 41).  Rows that share memory
-    are the library's."""
-    m, k = x.shape
-    n, sms = w.shape[0], _multiprocessors(x.device)
+    but [16384, 2048] 17.4 and 16.3), from 33 on at half as much again (48 rows of [34816, 5120] 63 and 67, of [24576, 4096] 42 and 41)."""
     if m >= TCGEN05_MIN_ROWS:
         return True
-    return m > STREAM_MAX_ROWS and n >= (128 if m > 64 else 192) * sms and x.stride(0) >= k and w.stride(0) >= k
+    return m > STREAM_MAX_ROWS and n >= (128 if m > 64 else 192) * sms
 
 
 def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0, static_weights: bool = False) -> torch.Tensor:
@@ -1027,7 +1024,8 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
         if _gated_columns_fill(m, n, _multiprocessors(x.device)):
             return linear_gated_columns(x, w_interleaved, limit=limit, alpha=alpha, static_weights=static_weights)
         return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)
-    if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and _gated_tcgen05(x, w_interleaved) and k % 8 == 0
+    apart = m >= TCGEN05_MIN_ROWS or (k > 0 and x.stride(0) >= k and w_interleaved.stride(0) >= k)   # fewer rows that share memory, or none of k, are the library's
+    if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and apart and _gated_tcgen05(m, n, _multiprocessors(x.device)) and k % 8 == 0
             and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0 and w_interleaved.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
         return linear_tcgen05(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)   # many rows: our tcgen05 kernel with the gated unit in its epilogue

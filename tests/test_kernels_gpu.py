@@ -705,6 +705,21 @@ def test_a_limit_that_is_not_positive_is_refused_by_every_gated_product(m, n, li
             product(x, w, limit=limit)
 
 
+@pytest.mark.parametrize("m", [40, 100])
+def test_gated_products_of_33_rows_and_more_take_and_refuse_what_the_library_product_does(m):
+    """No columns of k (a result of zeros), rows of another dimension, rows of another length: as for a matrix of few rows."""
+    from pylon_b200.kernels import ops
+
+    wide, small = (torch.zeros(n, 64, dtype=torch.bfloat16, device=DEVICE) for n in (34_816, 1_024))
+    x = torch.ones(m, 64, dtype=torch.bfloat16, device=DEVICE)
+    for w in (wide, small):
+        out = ops.linear_swiglu(x[:, :0], w[:, :0])
+        assert out.shape == (m, w.shape[0] // 2) and not out.any()
+        for wrong in (x.view(m, 8, 8), x[:, :56]):
+            with pytest.raises(ops.KernelError):
+                ops.linear_swiglu(wrong, w)
+
+
 def test_skinny_gemm_refuses():
     from pylon_b200.kernels import ops
 

@@ -562,21 +562,24 @@ constexpr long long LONE_WORK = 4096;
 
 template <int MT, int NR, int VEC>
 static int launch_rows(const GemmArgs& a, int batch, int force, cudaStream_t stream) {
-  constexpr int LONE_STAGES = MT == 16 ? 2 : 4;   // three blocks to an SM instead of two: 16 rows of [151936, 2560] 394 to 378 us
-  using Lone = RowsRing<MT, NR, LONE_STAGES>;
-  using Ring = RowsRing<MT, NR, 4>;
+  // A third lone block fits an SM with two stages of 16 rows instead of four, which pays where there is one for it: 16 rows of [151936, 2560] 394 to 378 us, of
+  // [19456, 2560] 75 to 72; but [16384, 2560], two blocks an SM either way, 53 us with four stages and 70 with two.
+  constexpr int SHORT = MT == 16 ? 2 : 4;
   const long long slabs = (a.N + NR * 32 - 1) / (NR * 32);
   const long long all = slabs * batch;
   const bool lone = force ? (force & 2) : a.K <= 64 || (a.K < 512 && all >= (a.K <= 256 ? 32 : 64)) || (a.M > 4 && all * a.M >= LONE_WORK);
-  GemmKernel kernel = lone ? gemm_f32_rows_kernel<MT, NR, VEC, LONE_STAGES> : gemm_f32_rows_kernel<MT, NR, VEC, 4>;
+  const bool brief = lone && SHORT != 4 && all > 2LL * multiprocessors();
+  GemmKernel kernel = brief ? gemm_f32_rows_kernel<MT, NR, VEC, SHORT> : gemm_f32_rows_kernel<MT, NR, VEC, 4>;
   static KernelState states[2][MAX_DEVICES];
-  KernelState& state = states[lone][current_device_slot()];
+  KernelState& state = states[brief][current_device_slot()];
   const int blocks = lone ? 1 : 8, warps = lone ? 4 : 2;
-  const size_t lone_bytes = ((size_t)4 * MT * NR * 32 + (size_t)4 * Lone::STAGES * Lone::STAGE) * sizeof(float);
-  const size_t cluster_bytes = ((size_t)2 * MT * NR * 32 + (size_t)2 * Ring::STAGES * Ring::STAGE) * sizeof(float), bytes = lone ? lone_bytes : cluster_bytes;
-  cudaError_t err = configure(kernel, state, std::max(lone_bytes, cluster_bytes));
+  const auto bytes = [](int places, int warps_, int stage_floats) { return ((size_t)places * MT * NR * 32 + (size_t)warps_ * stage_floats) * sizeof(float); };
+  const int ring = RowsRing<MT, NR, 4>::STAGES * RowsRing<MT, NR, 4>::STAGE, brief_ring = RowsRing<MT, NR, SHORT>::STAGES * RowsRing<MT, NR, SHORT>::STAGE;
+  const size_t lone_bytes = bytes(4, 4, brief ? brief_ring : ring), cluster_bytes = bytes(2, 2, ring);
+  cudaError_t err = configure(kernel, state, brief ? lone_bytes : std::max(lone_bytes, cluster_bytes));
   if (err != cudaSuccess) PYLON_REFUSE("gemm_f32: %s", cudaGetErrorString(err));
-  launch_dependent_cluster<LAUNCH_GEMM>(kernel, dim3((unsigned)(slabs * blocks), (a.M + MT - 1) / MT, batch), dim3(32 * warps), bytes, stream, (unsigned)blocks, a);
+  launch_dependent_cluster<LAUNCH_GEMM>(kernel, dim3((unsigned)(slabs * blocks), (a.M + MT - 1) / MT, batch), dim3(32 * warps), lone ? lone_bytes : cluster_bytes, stream,
+                                        (unsigned)blocks, a);
   PYLON_CHECK_LAUNCH("gemm_f32");
 }
 

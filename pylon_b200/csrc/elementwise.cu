@@ -103,8 +103,9 @@ constexpr int NORM_THREADS = 256;
 
 // DT: type of the delta (the activation type, or float when the delta comes as `delta_parts`
 // float32 partial sums, each [all rows, width], `part_stride` elements apart).  With the few rows of a decode step bound by the trips to
-// L2, so a thread asks for its places of four parts together: a load at a time, 16 rows of 5,120 in four parts took 9.4 us in the step.
-template <typename T, typename DT, int ITEMS>
+// L2, so a thread asks for its places of AT_ONCE = 4 parts together: a load at a time, 16 rows of 5,120 in four parts took 9.4 us in the step.
+// A delta that comes whole (AT_ONCE = 1) needs no such places, which cost many rows the warps in flight: 2,048 rows of 5,120 with a float32 delta 19 us, with them 36.
+template <typename T, typename DT, int ITEMS, int AT_ONCE>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_vec_kernel(float* __restrict__ residual, const DT* __restrict__ delta,
                                                                        const float* __restrict__ weight, const int* __restrict__ rows,
                                                                        T* __restrict__ out, int width, float eps, int write_residual,
@@ -132,21 +133,22 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_vec_kernel(float* __
     x[k] = i < groups ? Vec4<float>::load(res + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (del) {
-    constexpr int AT_ONCE = sizeof(DT) == 4 && sizeof(T) == 2 ? 4 : 1;   // float32 activations come whole
-    for (int part0 = 0; part0 < delta_parts; part0 += AT_ONCE) {
+    // One part known as such: without the loop's condition, but where several loads of an activation follow each other (21 against 19.7 us for 2,048 rows of 5,120).
+    const int parts = AT_ONCE == 1 && (ITEMS == 1 || sizeof(DT) > sizeof(T)) ? 1 : delta_parts;
+    for (int part0 = 0; part0 < parts; part0 += AT_ONCE) {
       float4 d[AT_ONCE][ITEMS];
 #pragma unroll
       for (int j = 0; j < AT_ONCE; ++j)
 #pragma unroll
         for (int k = 0; k < ITEMS; ++k) {
           const int i = threadIdx.x + k * NORM_THREADS;
-          if (part0 + j < delta_parts && i < groups) d[j][k] = Vec4<DT>::load(del + (size_t)(part0 + j) * part_stride + 4 * i);
+          if (part0 + j < parts && i < groups) d[j][k] = Vec4<DT>::load(del + (size_t)(part0 + j) * part_stride + 4 * i);
         }
 #pragma unroll
       for (int j = 0; j < AT_ONCE; ++j)   // in order: the sum does not depend on who wrote which part first
 #pragma unroll
         for (int k = 0; k < ITEMS; ++k)
-          if (part0 + j < delta_parts && threadIdx.x + k * NORM_THREADS < groups) { x[k].x += d[j][k].x; x[k].y += d[j][k].y; x[k].z += d[j][k].z; x[k].w += d[j][k].w; }
+          if (part0 + j < parts && threadIdx.x + k * NORM_THREADS < groups) { x[k].x += d[j][k].x; x[k].y += d[j][k].y; x[k].z += d[j][k].z; x[k].w += d[j][k].w; }
     }
   }
   float sumsq = 0.f;
@@ -171,9 +173,11 @@ static bool launch_add_rmsnorm_vec(float* residual, const DT* delta, const float
   if (((uintptr_t)residual % 16) || ((uintptr_t)weight % 16) || ((uintptr_t)out % 8) || (delta && ((uintptr_t)delta % 16))) return false;
   if (part_stride % 4) return false;
   const int items = (width / 4 + NORM_THREADS - 1) / NORM_THREADS;
+  constexpr bool SUMS = sizeof(DT) > sizeof(T);   // float32 activations come whole
+  const bool sums = SUMS && delta_parts > 1;
 #define PYLON_NORM_CASE(N)                                                                                     \
   case N:                                                                                                      \
-    launch_dependent(add_rmsnorm_vec_kernel<T, DT, N>, dim3(n_rows), dim3(NORM_THREADS), 0, stream, residual, delta, weight, rows, out, width, eps, write_residual, delta_parts, part_stride); \
+    launch_dependent(sums ? add_rmsnorm_vec_kernel<T, DT, N, SUMS ? 4 : 1> : add_rmsnorm_vec_kernel<T, DT, N, 1>, dim3(n_rows), dim3(NORM_THREADS), 0, stream, residual, delta, weight, rows, out, width, eps, write_residual, delta_parts, part_stride); \
     return true;
   switch (items) {
     PYLON_NORM_CASE(1) PYLON_NORM_CASE(2) PYLON_NORM_CASE(3) PYLON_NORM_CASE(4)

@@ -419,13 +419,14 @@ __global__ void qk_norm_rope_kv_write_vec_kernel(
     if (head_begin + h >= heads) continue;
     if (qkv_parts) {
       HeadChunk<float, CHUNK>::load(qkv_parts + token_offset + (size_t)(head_begin + h) * d, x[h]);
-      for (int part0 = 1; part0 < parts; part0 += 3) {   // three at once, so that the usual four parts are one trip to L2
-        float more[3][CHUNK];
+      constexpr int AT_ONCE = CHUNK == 2 ? 1 : 3;   // three at once, so that the usual four parts are one trip to L2; heads of 64: 1.8 us one by one, 1.9 together
+      for (int part0 = 1; part0 < parts; part0 += AT_ONCE) {
+        float more[AT_ONCE][CHUNK];
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
+        for (int j = 0; j < AT_ONCE; ++j)
           if (part0 + j < parts) HeadChunk<float, CHUNK>::load(qkv_parts + (size_t)(part0 + j) * part_stride + token_offset + (size_t)(head_begin + h) * d, more[j]);
 #pragma unroll
-        for (int j = 0; j < 3; ++j)   // in order: the sum does not depend on who wrote which part first
+        for (int j = 0; j < AT_ONCE; ++j)   // in order: the sum does not depend on who wrote which part first
 #pragma unroll
           for (int i = 0; i < CHUNK; ++i)
             if (part0 + j < parts) x[h][i] += more[j][i];

@@ -865,11 +865,12 @@ def linear_gated_columns(x: torch.Tensor, w: torch.Tensor, limit: Optional[float
     return y
 
 
-def _gated_columns_fill(m: int, n: int, sms: int) -> bool:
-    """Whether the gated product of 9 to 32 rows goes to :func:`linear_gated_columns`: where its blocks, two to an SM, are one round that is three
-    quarters full.  Behind a norm, 16 and 32 rows: [34816, 5120] 58 and 62 us, :func:`linear_stream` 66 and 75; [28672, 4096] 45 and 46, 47 and
-    51; but [24576, 4096] 40 and 42, 36 and 38, and [51200, 5120] 92 and 96, 80 and 85.  (A row's distance from 64-bit sums is half an ulp of bfloat16 in both.)"""
-    return SKINNY_MAX_ROWS < m <= STREAM_MAX_ROWS and 3 * sms <= 2 * -(-n // 128) <= 4 * sms
+def _gated_columns_fill(m: int, n: int, k: int, sms: int) -> bool:
+    """Whether the gated product of 9 to 32 rows goes to :func:`linear_gated_columns`: where the blocks of :func:`linear_stream` (64 weight rows, three to an
+    SM) begin a second round and this kernel's (128, two to an SM) are still one, and k is long enough for the walk to count (its start and end are longer).
+    Behind a norm, 16 and 32 rows: [34816, 5120] 63 and 63 us, :func:`linear_stream` 67 and 78; [30720, 2560] 31 and 33, 35 and 38; but [28416, 5120] 52 and
+    54, 48 and 49, [44032, 5120] 90 and 94, 70 and 79, and [34816, 512] 12.7 and 14.0, 12.1 and 13.9.  [37888, 2048] 31.5 and 32.8, 30.7 and 35.7.  (Elements that differ from the rounded 64-bit result: 16 rows, k = 4,096: 2.6e-4 of them, :func:`linear_stream` 3.7e-4.)"""
+    return SKINNY_MAX_ROWS < m <= STREAM_MAX_ROWS and -(-n // 64) > 3 * sms and -(-n // 128) <= 2 * sms and k >= (2_560 if m <= 16 else 1_536)
 
 
 def linear_skinny(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, static_weights: bool = False) -> torch.Tensor:
@@ -1021,7 +1022,7 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
     if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and m <= STREAM_MAX_ROWS and x.shape[1] == k
             and k % 8 == 0 and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0
             and w_interleaved.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
-        if _gated_columns_fill(m, n, _multiprocessors(x.device)):
+        if _gated_columns_fill(m, n, k, _multiprocessors(x.device)):
             return linear_gated_columns(x, w_interleaved, limit=limit, alpha=alpha, static_weights=static_weights)
         return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)
     apart = m >= TCGEN05_MIN_ROWS or (k > 0 and x.stride(0) >= k and w_interleaved.stride(0) >= k)   # fewer rows that share memory, or none of k, are the library's

@@ -1000,14 +1000,28 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return torch.stack((gate.reshape(inter // 8, 8, k), up.reshape(inter // 8, 8, k)), dim=1).reshape(2 * inter, k).contiguous()
 
 
-def _gated_tcgen05(m: int, n: int, sms: int) -> bool:
+def _gated_tiles_filled(n: int, sms: int) -> float:
+    """How much of its rounds over the SMs the tcgen05 kernel fills with a gated product of one row tile: its widths, and their cost, as in csrc/gemm_tcgen05.cu."""
+    rounds = {width: -(-(-(-n // width)) // sms) for width in (256, 192, 128)}
+    width = min(rounds, key=lambda w: rounds[w] * (w + 213))
+    return n / (rounds[width] * width * sms)
+
+
+def _gated_tcgen05(m: int, n: int, k: int, sms: int) -> bool:
     """Whether the gated product of more than ``STREAM_MAX_ROWS`` rows goes to the tcgen05 kernel rather than to the library and a kernel for the unit: always from
-    ``TCGEN05_MIN_ROWS`` rows on.  Fewer are one row tile that asks for its first weights behind the kernel ahead, and what they read is W: from 65 rows on
-    where 128 columns for every SM do not hold it (80 rows behind a norm: [19456, 2560] 24.6 us, the library 26.1; [24576, 4096] 43 and 47;
-    but [16384, 2048] 17.4 and 16.3), from 33 on at half as much again (48 rows of [34816, 5120] 63 and 67, of [24576, 4096] 42 and 41)."""
+    ``TCGEN05_MIN_ROWS`` rows on.  Fewer are one row tile that asks for its first weights behind the kernel ahead, and what they read is W.
+
+    73 rows and more (the library then takes tiles of 128 rows): where 128 columns for every SM do not hold W (80 rows behind a norm: [19456, 2560] 0.91 of the library's time,
+    [24576, 4096] 0.87, [34816, 5120] 0.92; [16384, 2048] 17.4 and 16.3 us), but not with a long k where a second round of tiles has just begun ([38400, 4096] 1.07,
+    [40960, 8192] 1.08, [43008, 8192] 1.02).  33 to 72 rows: from half as much again on, where the tiles fill their rounds and k is long (33 and 64 rows of [28416, 2560]
+    0.95 and 0.93, of [34816, 5120] 0.94 and 0.93; but of [19456, 2560] 1.04 and 1.03, of [38400, 2560] 1.09 and 1.05, of [28416, 1024] 1.09 and 0.99)."""
     if m >= TCGEN05_MIN_ROWS:
         return True
-    return m > STREAM_MAX_ROWS and n >= (128 if m > 64 else 192) * sms
+    if m <= STREAM_MAX_ROWS:
+        return False
+    if m > 72:
+        return n >= 128 * sms and (n <= 256 * sms or k < 4_096 or _gated_tiles_filled(n, sms) >= 0.74)
+    return n >= 192 * sms and _gated_tiles_filled(n, sms) >= 0.82 and (k >= 2_048 or m > 64)
 
 
 def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[float] = None, alpha: float = 1.0, static_weights: bool = False) -> torch.Tensor:
@@ -1026,7 +1040,7 @@ def linear_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, limit: Optional[
             return linear_gated_columns(x, w_interleaved, limit=limit, alpha=alpha, static_weights=static_weights)
         return linear_stream(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)
     apart = m >= TCGEN05_MIN_ROWS or (k > 0 and x.stride(0) >= k and w_interleaved.stride(0) >= k)   # fewer rows that share memory, or none of k, are the library's
-    if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and apart and _gated_tcgen05(m, n, _multiprocessors(x.device)) and k % 8 == 0
+    if (x.dtype == torch.bfloat16 and w_interleaved.dtype == torch.bfloat16 and x.dim() == 2 and apart and _gated_tcgen05(m, n, k, _multiprocessors(x.device)) and k % 8 == 0
             and n % 16 == 0 and x.stride(1) == 1 and w_interleaved.stride(1) == 1 and x.stride(0) % 8 == 0 and w_interleaved.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and w_interleaved.data_ptr() % 16 == 0):
         return linear_tcgen05(x, w_interleaved, swiglu=True, limit=limit, alpha=alpha, static_weights=static_weights)   # many rows: our tcgen05 kernel with the gated unit in its epilogue

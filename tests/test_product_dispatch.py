@@ -35,6 +35,19 @@ def test_gated_products_of_9_to_32_rows(route, sms):
         assert route(sms, 16, n, 4_096) == "stream"
 
 
+@pytest.mark.parametrize("sms", [132, 148, 160])
+def test_gated_products_of_33_to_127_rows(route, sms):
+    for n in (192 * sms, 256 * sms, 384 * sms, 512 * sms):   # whole rounds of tiles
+        assert route(sms, 33, n, 2_048) == route(sms, 65, n, 64) == route(sms, 127, n, 8_192) == "tcgen05"
+        assert route(sms, 33, n, 2_040) == route(sms, 64, n, 64) == "library"
+    for m in (33, 64, 65, 72):
+        assert route(sms, m, 192 * sms - 16, 4_096) == "library"
+        assert route(sms, m, 256 * sms + 16, 4_096) == "library"   # a second round of tiles for hardly more rows
+    assert route(sms, 73, 128 * sms, 64) == route(sms, 127, 128 * sms, 8_192) == "tcgen05"
+    assert route(sms, 73, 128 * sms - 16, 64) == "library"
+    assert route(sms, 100, 256 * sms + 16, 4_096) == "library" and route(sms, 100, 256 * sms + 16, 4_088) == "tcgen05"
+
+
 def test_gated_products_that_only_the_library_takes(route):
     assert route(148, 80, 37_888, 2_048, row=2_040) == route(148, 80, 37_888, 2_048, row=0) == route(148, 80, 37_888, 0) == "library"   # rows that share memory; no k
     assert route(148, 128, 1_024, 64) == route(148, 4_096, 19_456, 2_560) == "tcgen05"

@@ -177,6 +177,26 @@ def test_gemm_f32_of_a_short_k(m, k):
         assert torch.equal(heads[:, h], ops.linear(x[:, h].contiguous(), w[h])), h
 
 
+@pytest.mark.parametrize("k", [36, 72, 80, 112, 144, 208, 240, 244, 260])
+def test_gemm_f32_tiles_whose_last_stage_is_half_empty(k):
+    """Stages multiplied by halves (up to k = 240 where at most 16 k are left for the last) and whole: the bits of the streaming kernel, in every tile and cluster size."""
+    from pylon_b200.kernels import ops
+
+    x, w = torch.randn(33, k, device=DEVICE), torch.randn(200, k, device=DEVICE)
+    library = ops._library("gemm_f32.cu")
+
+    def forced(rows, form):
+        y = torch.full((rows, 200), float("nan"), device=DEVICE)
+        ops._check(library, library.pylon_gemm_f32_nt_forced(ops._ptr(x), ops._ptr(w), ops._ptr(y), rows, 200, k, k, k, 200, form, ops._stream()))
+        return y
+
+    want = forced(16, -2)
+    # chains of at most k / 32 + 16 products: half an ulp a step
+    torch.testing.assert_close(want.double(), x[:16].double() @ w.double().T, rtol=1e-5, atol=2.0**-24 * k**0.5 * (k / 32 + 16))
+    for form in (281, 351, 362, 454, 468, 471, 552, 651, 741, 754):
+        assert torch.equal(forced(33, form)[:16], want), form
+
+
 @pytest.mark.parametrize("k, form", [(64, 991), (64, 753), (64, 441), (33, 281), (33, 448), (64, -9)])
 def test_gemm_f32_refuses_a_form_that_is_not_there(k, form):
     from pylon_b200.kernels import ops

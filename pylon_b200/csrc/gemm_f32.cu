@@ -558,12 +558,23 @@ static cudaError_t configure(GemmKernel kernel, KernelState& state, size_t smem)
 }
 
 // Rows kernel: 16 warps of a cluster (eight blocks of two) take a leaf each, so that 40 slabs (a matrix of 2,560 rows) are 640 warps.
-// From LONE_WORK results in groups of 64 on, four warps of a lone block take a quarter each: no cluster to place and no shared memory to
-// cross, and a warp's ring runs four times as long (16 rows of x, 304 slabs: 79 against 92 us; 2,374 slabs: 399 against 577 us; 96
-// slabs 34 against 36; 40 slabs 50 against 28).  The same with a short k, of which most of a cluster's warps have nothing (one row of
-// [2560, 64]: 2.9 against 3.9 us; 12 of [9728, 300] 16.6 against 27.8; but one of [512, 128] 3.7 against 3.4).  With four rows of x or fewer the loads bound it and more, smaller blocks keep more
-// of them in flight (one row, 2,374 slabs: 243 against 268 us).
+// With enough slabs, four warps of a lone block take a quarter each: no cluster to place and no shared memory to cross, and a warp's ring runs four
+// times as long.  With four rows of x or fewer the loads bound it and more, smaller blocks keep more of them in flight (one row, 2,374 slabs: 243
+// against 268 us).  With a short k most of a cluster's warps have nothing to do (one row of [2560, 64]: 2.9 us alone, 3.9 in clusters; 12 of [9728, 300] 15.2
+// and 26.7; but one of [512, 128] 3.7 and 3.4).  5 to 8 rows: from 96 slabs on up to a k of 2,560 (8 of [6144, 2560] 20.4 and 23.4 us, of [24576, 512] 17.6 and
+// 34.7; but of [5120, 2560] 20.6 and 17.4, of [19456, 4096] 77 and 70), whatever k is from LONE_WORK results in groups of 64 on.  9 to 16 rows: by an estimate of
+// both forms fitted to their times over 16 to 640 slabs and k of 512 to 9,728, within 6 % of the better one (9 rows alone and in clusters: [6144, 2560] 32
+// and 37 us, [19456, 2560] 72 and 87, [16384, 9728] 188 and 203; but [5120, 4096] 48.7 and 43.0, [19456, 9728] 253 and 218).
 constexpr long long LONE_WORK = 4096;
+
+static bool rows_alone(const GemmArgs& a, long long slabs) {
+  if (a.K <= 64 || (a.K < 512 && slabs >= (a.K <= 256 ? 32 : 64))) return true;
+  if (a.M <= 4 || a.K < 512) return false;
+  if (slabs * a.M >= LONE_WORK) return true;
+  if (a.M <= 8) return slabs >= 96 && a.K <= 2560;
+  const long long rounds = (slabs + multiprocessors() - 1) / multiprocessors();
+  return slabs >= 80 && 1.07 * (6.0 + a.K * (0.0018 + 0.0083 * rounds)) < 4.5 + 0.003 * a.K + slabs * (0.105 + 5.1e-5 * a.K);   // us
+}
 
 template <int MT, int NR, int VEC>
 static int launch_rows(const GemmArgs& a, int batch, int force, cudaStream_t stream) {
@@ -572,7 +583,7 @@ static int launch_rows(const GemmArgs& a, int batch, int force, cudaStream_t str
   constexpr int SHORT = MT == 16 ? 2 : 4;
   const long long slabs = (a.N + NR * 32 - 1) / (NR * 32);
   const long long all = slabs * batch;
-  const bool lone = force ? (force & 2) : a.K <= 64 || (a.K < 512 && all >= (a.K <= 256 ? 32 : 64)) || (a.M > 4 && all * a.M >= LONE_WORK);
+  const bool lone = force ? (force & 2) : rows_alone(a, all);
   const bool brief = lone && SHORT != 4 && all > 2LL * multiprocessors();
   GemmKernel kernel = brief ? gemm_f32_rows_kernel<MT, NR, VEC, SHORT> : gemm_f32_rows_kernel<MT, NR, VEC, 4>;
   static KernelState states[2][MAX_DEVICES];

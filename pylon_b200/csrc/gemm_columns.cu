@@ -1,18 +1,21 @@
 // The gated unit of a feed-forward in bfloat16 for a few rows of x on the fifth-generation tensor cores, with the weights on the wide side of the tile:
 // 128 interleaved rows of gate and up are the M of a tcgen05.mma and the rows of x, rounded up to 16, its N.
 //
-// Bound by the bytes of W: 16 rows of [34816, 5120] 58 us behind a norm (356 MB: 6.1 TB/s), where the kernel that multiplies with mma.sync from
-// registers (gemm_stream.cu) takes 66 us, its warps busy with fragments; 32 rows 62 and 75 us.  A block takes 128 rows of W over the whole of k; two share an
-// SM, so that one's epilogue overlaps the other's loads.  Four warps: one lane of the first asks for boxes of W and x (TMA, 128-byte
-// swizzle) into a ring of stages - the boxes of W that nothing queued writes before it waits for the kernel ahead - one lane of the second issues the
-// products, and all four read the accumulator back, each its 32 lanes, a lane being a row of W.
+// Bound by the bytes of W: 16 rows of [34816, 5120] and the norm ahead of them 62.6 us (356 MB: 5.7 TB/s and more), where the kernel that multiplies with mma.sync
+// from registers (gemm_stream.cu) takes 66.6 us, its warps busy with fragments; 32 rows 62.9 and 77.7 us.  The products' dispatch sends it 9 to 32 rows; it takes up to 256,
+// those above 32 with one set of accumulators.  A block takes 128 rows of W over the whole of k; two share an
+// SM, so that one's epilogue overlaps the other's loads.  Six warps: one lane of the fifth asks for boxes of W and x (TMA, 128-byte
+// swizzle) into a ring of stages - the boxes of W that nothing queued writes before it waits for the kernel ahead - one lane of the next issues the
+// products, and the first four read the accumulators back, each its 32 lanes, a lane being a row of W.
 //
 // Measured and dropped: partial sums over slices of k for the products into the stream and the rotation (33 to 200 rows: 6.4 us for the 4B shape's output
 // projection of 64 rows where the library takes 8.4, 10.6 and 14.9 for the down projection; but the norm that adds 14 parts up lost what they gained: steps of
 // 64 to 190 tokens 2 % faster to 10 % slower); slices added up in a cluster (2.5 to 4 us more than partial sums) or by the last block of a tile (9 to 60 us).
 //
-// The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k: the steps of 16 k take turns on as many
-// accumulators as fit beside each other in 256 columns of tensor memory (16 at most), which the epilogue adds in float32.
+// The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k.  The steps of 16 k take turns on several
+// accumulators beside each other in tensor memory, and up to 32 rows of x two sets of them take turns, 512 k each: while one is filled the readers add the
+// other up in float32, so that no chain is longer than eight steps whatever k is.  Elements that are not the rounded 64-bit result: 32 rows of [34816, 5120] 2.3e-4
+// of them, with one set of chains over the whole of k 7.1e-4, gemm_stream.cu 3.8e-4; 24 of [37888, 8192] 2.8e-4, 12.3e-4 and 3.8e-4.  (1 % of the time.)
 //
 // All waits on mbarriers are bounded: one that runs out sets an error word, the block waits for its own copies, frees its tensor memory and returns.
 // No TMA load here uses cluster multicast.
@@ -29,8 +32,9 @@
 
 namespace pylon {
 
-constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 128, GC_MOST_STAGES = 8;   // weight rows and k of a box
-constexpr int GC_MOST_CHAINS = 16, GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
+constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 192, GC_MOST_STAGES = 8;   // weight rows and k of a box
+constexpr int GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
+constexpr int GC_SETS_MOST = 32, GC_SEGMENT = 8;                                  // columns up to which two sets of accumulators take turns; boxes to a turn
 constexpr unsigned GC_WAIT_LIMIT = 1u << 22;                                                 // try_wait calls before a wait gives up
 
 __device__ __forceinline__ uint32_t gc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -38,6 +42,7 @@ __device__ __forceinline__ void gc_mbar_init(uint64_t* bar, int count) { asm vol
 __device__ __forceinline__ void gc_expect(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(gc_smem(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void gc_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(gc_smem(bar)) : "memory"); }
 __device__ __forceinline__ bool gc_wait(uint64_t* bar, uint32_t parity) {
   for (unsigned tries = 0; tries < GC_WAIT_LIMIT; ++tries) {
     uint32_t done;
@@ -82,7 +87,7 @@ __device__ __forceinline__ float gc_unit(float gate, float up, float limit, floa
 struct GcArgs {
   __nv_bfloat16* y;
   long long ldy;
-  int M, N, K, columns, stages, chains, tmem_columns;   // columns: M rounded up to 16; chains: a power of two
+  int M, N, K, columns, stages, chains, segment, tmem_columns;   // columns: M rounded up to 16; chains of a set: a power of two; segment: boxes to a set's turn
   float unit_limit, unit_alpha;
   int w_static;
   int* error;   // 1: the copies, 2: the products, 3: the accumulator did not come in time
@@ -92,26 +97,26 @@ struct GcArgs {
 __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GcArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full[GC_MOST_STAGES], empty[GC_MOST_STAGES], done;
+  __shared__ __align__(8) uint64_t full[GC_MOST_STAGES], empty[GC_MOST_STAGES], filled[2], freed[2];   // freed: a set has been read
   __shared__ uint32_t tmem_slot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int columns = a.columns, stages = a.stages, w_bytes = GC_ROWS * GC_BK * 2, x_bytes = columns * GC_BK * 2;
   unsigned char* w_tiles = smem;
   unsigned char* x_tiles = smem + stages * w_bytes;
   const int boxes = (a.K + GC_BK - 1) / GC_BK, row0 = blockIdx.x * GC_ROWS;
-  const int chains = a.chains;
+  const int chains = a.chains, segment = a.segment, segments = (boxes + segment - 1) / segment;   // more than one only where there are two sets
 
   const int ahead = a.w_static ? min(stages, boxes) : 0;
-  if (threadIdx.x == 0) {
+  if (warp == 4 && lane == 0) {
     for (int s = 0; s < stages; ++s) { gc_mbar_init(&full[s], 1); gc_mbar_init(&empty[s], 1); }
-    gc_mbar_init(&done, 1);
+    for (int set = 0; set < 2; ++set) { gc_mbar_init(&filled[set], 1); gc_mbar_init(&freed[set], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     for (int s = 0; s < ahead; ++s) {
       gc_expect(&full[s], w_bytes + x_bytes);
       gc_load(w_tiles + s * w_bytes, &map_w, &full[s], s * GC_BK, row0);
     }
   }
-  if (warp == 1) {   // the whole warp allocates
+  if (warp == 5) {   // the whole warp allocates
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(gc_smem(&tmem_slot)), "r"(a.tmem_columns));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
@@ -122,72 +127,106 @@ __global__ void __launch_bounds__(GC_THREADS) gemm_columns_kernel(const __grid_c
   grid_dependency_wait();
   allow_dependents();
 
-  int issued = 0;   // boxes asked for (the first thread's)
-  if (warp == 0 && lane == 0) {
-    for (int s = 0, round = 0; issued < boxes; ++issued) {
-      if (issued >= ahead) {
-        if (round > 0 && !gc_wait(&empty[s], (round - 1) & 1)) { atomicExch(a.error, 1); break; }
-        gc_expect(&full[s], w_bytes + x_bytes);
-        gc_load(w_tiles + s * w_bytes, &map_w, &full[s], issued * GC_BK, row0);
+  if (warp == 4) {
+    if (lane == 0) {
+      int issued = 0;   // boxes asked for
+      for (int s = 0, round = 0; issued < boxes; ++issued) {
+        if (issued >= ahead) {
+          if (round > 0 && !gc_wait(&empty[s], (round - 1) & 1)) { atomicExch(a.error, 1); break; }
+          gc_expect(&full[s], w_bytes + x_bytes);
+          gc_load(w_tiles + s * w_bytes, &map_w, &full[s], issued * GC_BK, row0);
+        }
+        gc_load(x_tiles + s * x_bytes, &map_x, &full[s], issued * GC_BK, 0);
+        if (++s == stages) { s = 0; ++round; }
       }
-      gc_load(x_tiles + s * x_bytes, &map_x, &full[s], issued * GC_BK, 0);
-      if (++s == stages) { s = 0; ++round; }
+      for (int box = max(0, issued - stages); box < issued; ++box) gc_wait(&full[box % stages], (box / stages) & 1);   // no copy outlives the block
     }
-  } else if (warp == 1 && lane == 0) {
-    // Instruction descriptor of kind::f16: bfloat16 A and B, float32 D, both K-major.
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(GC_ROWS >> 4) << 24);
-    const uint64_t w_first = gc_desc(w_tiles), x_first = gc_desc(x_tiles);
-    bool alive = true;
-    for (int box = 0, s = 0, phase = 0, offset = 0; box < boxes; ++box) {
-      if (!gc_wait(&full[s], phase)) { atomicExch(a.error, 2); alive = false; break; }
+    __syncwarp();
+  } else if (warp == 5) {
+    if (lane == 0) {
+      // Instruction descriptor of kind::f16: bfloat16 A and B, float32 D, both K-major.
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(columns >> 3) << 17) | ((uint32_t)(GC_ROWS >> 4) << 24);
+      const uint64_t w_first = gc_desc(w_tiles), x_first = gc_desc(x_tiles);
+      int s = 0, phase = 0, box = 0;
+      for (int turn = 0; turn < segments; ++turn) {
+        const int set = turn & 1, end = min(boxes, box + segment);
+        const uint32_t d = tmem + set * chains * columns;
+        if (turn >= 2 && !gc_wait(&freed[set], ((turn >> 1) - 1) & 1)) { atomicExch(a.error, 2); break; }
+        bool alive = true;
+        for (int step = 0, offset = 0; box < end; ++box) {
+          if (!gc_wait(&full[s], phase)) { atomicExch(a.error, 2); alive = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          const uint64_t w_desc = w_first + (uint64_t)(s * (w_bytes >> 4)), x_desc = x_first + (uint64_t)(s * (x_bytes >> 4));
+#pragma unroll
+          for (int k = 0; k < GC_BK / 16; ++k) {   // 16 k are 32 bytes further along the swizzled row: +2 in 16-byte units
+            gc_mma(d + offset, w_desc + 2 * k, x_desc + 2 * k, idesc, step >= chains);
+            ++step;
+            offset += columns;
+            if (offset == chains * columns) offset = 0;
+          }
+          gc_commit(&empty[s]);
+          if (++s == stages) { s = 0; phase ^= 1; }
+        }
+        if (!alive) break;
+        gc_commit(&filled[set]);
+      }
+    }
+    __syncwarp();
+  } else {
+    // This thread's row of W and, 16 rows of x at a time, its sums: the chains' in order.  Rows of gate and up alternate in groups of 8: lanes 8 apart exchange,
+    // the gate's lane then makes the even rows of x, the up's the odd ones.
+    const int n = row0 + threadIdx.x, is_up = (lane >> 3) & 1;
+    const uint32_t lane_address = tmem + ((uint32_t)(warp * 32) << 16);
+    auto add_up = [&](float (&v)[16], int turn, int c0) {
+      const int count = min(chains, 4 * min(segment, boxes - turn * segment));   // a last turn of few steps fills the first chains only
+      for (int c = 0; c < count; ++c) {
+        uint32_t raw[16];
+        gc_read(lane_address + ((turn & 1) * chains + c) * columns + c0, raw);
+        gc_read_done();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(raw[j]);
+      }
+    };
+    auto finish = [&](const float (&v)[16], int c0) {
+      __nv_bfloat16* dst = a.y + (size_t)(c0 + is_up) * a.ldy + (n >> 4) * 8 + (n & 7);
+#pragma unroll
+      for (int j = 0; j < 16; j += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, is_up ? v[j] : v[j + 1], 8);
+        const float unit = is_up ? gc_unit(other, v[j + 1], a.unit_limit, a.unit_alpha) : gc_unit(v[j], other, a.unit_limit, a.unit_alpha);
+        if (n < a.N && c0 + j + is_up < a.M) dst[(size_t)j * a.ldy] = __float2bfloat16_rn(unit);
+      }
+    };
+    bool complete = true;
+    if (columns <= GC_SETS_MOST) {
+      float sums[GC_SETS_MOST / 16][16] = {};
+      for (int turn = 0; complete && turn < segments; ++turn) {
+        complete = __all_sync(0xffffffffu, gc_wait(&filled[turn & 1], (turn >> 1) & 1));
+        if (!complete) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+        for (int t = 0; t < GC_SETS_MOST / 16; ++t)
+          if (16 * t < columns) add_up(sums[t], turn, 16 * t);
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) gc_arrive(&freed[turn & 1]);
+      }
+#pragma unroll
+      for (int t = 0; t < GC_SETS_MOST / 16; ++t)
+        if (complete && 16 * t < columns) finish(sums[t], 16 * t);
+    } else {
+      complete = __all_sync(0xffffffffu, gc_wait(&filled[0], 0));
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const uint64_t w_desc = w_first + (uint64_t)(s * (w_bytes >> 4)), x_desc = x_first + (uint64_t)(s * (x_bytes >> 4));
-#pragma unroll
-      for (int k = 0; k < GC_BK / 16; ++k) {   // 16 k are 32 bytes further along the swizzled row: +2 in 16-byte units
-        gc_mma(tmem + offset, w_desc + 2 * k, x_desc + 2 * k, idesc, box * (GC_BK / 16) + k >= chains);
-        offset += columns;
-        if (offset == chains * columns) offset = 0;
+      for (int c0 = 0; complete && c0 < columns; c0 += 16) {
+        float sums[16] = {};
+        add_up(sums, 0, c0);
+        finish(sums, c0);
       }
-      gc_commit(&empty[s]);
-      if (++s == stages) { s = 0; phase ^= 1; }
     }
-    if (alive) gc_commit(&done);
+    if (!complete && lane == 0) atomicExch(a.error, 3);
   }
-  __syncwarp();
-  const bool complete = gc_wait(&done, 0);
-  if (!complete && lane == 0) atomicExch(a.error, 3);
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-
-  // This thread's row of W and, 16 rows of x at a time, its sums: the chains' in order.  Rows of gate and up alternate in groups of 8: lanes 8 apart exchange,
-  // the gate's lane then makes the even rows of x, the up's the odd ones.
-  const int n = row0 + threadIdx.x, is_up = (lane >> 3) & 1;
-  const uint32_t lane_address = tmem + ((uint32_t)(warp * 32) << 16);
-  for (int c0 = 0; complete && c0 < columns; c0 += 16) {
-    float v[16];
-    uint32_t raw[16];
-    gc_read(lane_address + c0, raw);
-    gc_read_done();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(raw[j]);
-    for (int c = 1; c < chains; ++c) {
-      gc_read(lane_address + c * columns + c0, raw);
-      gc_read_done();
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(raw[j]);
-    }
-    __nv_bfloat16* dst = a.y + (size_t)(c0 + is_up) * a.ldy + (n >> 4) * 8 + (n & 7);
-#pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-      const float other = __shfl_xor_sync(0xffffffffu, is_up ? v[j] : v[j + 1], 8);
-      const float unit = is_up ? gc_unit(other, v[j + 1], a.unit_limit, a.unit_alpha) : gc_unit(v[j], other, a.unit_limit, a.unit_alpha);
-      if (n < a.N && c0 + j + is_up < a.M) dst[(size_t)j * a.ldy] = __float2bfloat16_rn(unit);
-    }
-  }
-  if (!complete && threadIdx.x == 0)   // no copy outlives the block
-    for (int box = max(0, issued - stages); box < issued; ++box) gc_wait(&full[box % stages], (box / stages) & 1);
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(a.tmem_columns));
+  if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(a.tmem_columns));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -265,10 +304,12 @@ extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, i
   a.columns = (M + 15) / 16 * 16;
   const int boxes = (K + GC_BK - 1) / GC_BK, stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2;
   a.stages = std::min({(GC_SMEM - 1024) / stage_bytes, GC_MOST_STAGES, boxes});
+  const int sets = a.columns <= GC_SETS_MOST ? 2 : 1;
+  a.segment = sets == 2 ? GC_SEGMENT : boxes;
   a.chains = 1;
-  while (a.chains < GC_MOST_CHAINS && 2 * a.chains * a.columns <= GC_COLUMNS && 2 * a.chains <= boxes * (GC_BK / 16)) a.chains *= 2;
+  while (2 * a.chains * sets * a.columns <= GC_COLUMNS && 2 * a.chains <= std::min(a.segment, boxes) * (GC_BK / 16)) a.chains *= 2;
   a.tmem_columns = 32;
-  while (a.tmem_columns < a.chains * a.columns) a.tmem_columns *= 2;
+  while (a.tmem_columns < sets * a.chains * a.columns) a.tmem_columns *= 2;
   a.unit_limit = limit; a.unit_alpha = alpha; a.w_static = w_static; a.error = error;
   CUtensorMap map_w, map_x;
   if (!matrix_map(&map_w, w, N, K, ldw, GC_ROWS) || !matrix_map(&map_x, x, M, K, ldx, a.columns)) PYLON_REFUSE("gemm_columns_gated: the tensor maps could not be made");

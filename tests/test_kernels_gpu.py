@@ -699,6 +699,34 @@ def test_gated_product_with_the_weights_on_the_wide_side(m, n, k):
     assert int(ops.stream_error_word(torch.device(DEVICE)).item()) == 0
 
 
+@pytest.mark.parametrize("m, n, k", [(9, 2_048, 520), (16, 8_192, 5_120), (17, 8_192, 4_104), (24, 8_192, 8_192), (32, 8_192, 10_240)])
+def test_gated_product_with_the_weights_on_the_wide_side_is_as_near_to_64_bits_as_the_streaming_kernel(m, n, k):
+    """Elements that are not the rounded 64-bit result: of some 1e5, 30 to 400; two counts of one size differ by a few of their roots."""
+    from pylon_b200.kernels import ops
+
+    x = torch.randn(m, k, device=DEVICE).to(torch.bfloat16)
+    w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
+    pairs = (x.double() @ w.double().T).view(m, n // 16, 2, 8)
+    gate, up = pairs[:, :, 0].reshape(m, -1), pairs[:, :, 1].reshape(m, -1)
+    rounded = (gate * torch.sigmoid(gate) * up).to(torch.bfloat16)
+    off, streamed = (int((product != rounded).sum()) for product in (ops.linear_gated_columns(x, w), ops.linear_stream(x, w, swiglu=True)))
+    assert off <= streamed + 4 * streamed**0.5 + 4, (off, streamed)
+
+
+@pytest.mark.parametrize("m", [33, 65, 127])
+def test_linear_swiglu_clamped_where_the_tcgen05_kernel_takes_fewer_rows_than_a_tile(m):
+    from pylon_b200.kernels import ops
+
+    n, k = 192 * torch.cuda.get_device_properties(0).multi_processor_count, 2_048
+    x = torch.randn(m, k, device=DEVICE).to(torch.bfloat16)
+    w = (torch.randn(n, k, device=DEVICE) * k**-0.5).to(torch.bfloat16)
+    assert ops._gated_tcgen05(m, n, k, n // 192)
+    pairs = (x.double() @ w.double().T).view(m, n // 16, 2, 8)
+    gate, up = pairs[:, :, 0].reshape(m, -1).clamp(max=0.5), pairs[:, :, 1].reshape(m, -1).clamp(-0.5, 0.5)
+    # half an ulp of bfloat16, and the float32 sums' error (1e-5 of their terms' size) where up + 1 or the gate cancel
+    torch.testing.assert_close(ops.linear_swiglu(x, w, limit=0.5, alpha=1.7).double(), gate * torch.sigmoid(1.7 * gate) * (up + 1), rtol=2.0**-8, atol=1e-4)
+
+
 @pytest.mark.parametrize("m, n, k", [(9, 28_672, 1_024), (32, 34_816, 256), (33, 34_816, 256), (64, 30_000, 512), (65, 19_456, 520), (100, 24_576, 1_024), (127, 19_456, 512)])
 def test_linear_swiglu_around_the_edges_of_its_dispatch(m, n, k):
     """Rows and weight rows at which another kernel takes over; rows that share memory are still multiplied."""

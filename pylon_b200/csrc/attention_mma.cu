@@ -545,7 +545,7 @@ __device__ __forceinline__ bool att_mbar_wait(uint64_t* bar, unsigned parity) {
   }
   return false;
 }
-// One box of 64 keys x 64 values; no cluster multicast.
+// One box of the map's keys x 64 values; no cluster multicast.
 __device__ __forceinline__ void att_tma_load(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                ::"r"(smem_address(dst)), "l"((unsigned long long)map), "r"(smem_address(bar)), "r"(x), "r"(y) : "memory");
@@ -889,11 +889,13 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     pending_count = 0;
   };
 
-  Segment current;
+  Segment current, following;
   bool have = next_segment(current);
   const bool had_tiles = have;   // cluster form: this block has a share of the pair's tiles
   bool waited = false;       // for the kernel before this one (programmatic dependent launch)
+  bool prefetched = false;   // the segment's query and first tile were asked for while the one before it was merged
   while (have) {
+    const bool have_following = next_segment(following);
     const int kv_head = current.kv_head, tile_begin = current.tile_begin, tile_end = current.tile_end, pair = current.pair;
     const int first_block = current.first_block, segments = current.segments, q0 = current.q0, packed_rows = current.packed_rows;
     const int kv_len = current.kv_len, pos0 = current.pos0;
@@ -923,23 +925,25 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
       if (tile < tile_end) issue_tile(current, tile);
       if (!TMA) cp_async_commit();   // an empty group keeps the count of groups in step with the tiles
     };
-    if (!waited) {
-      // Tiles that end before the row's first new token hold nothing the kernel before this one writes: as many
-      // of them as the ring has stages are asked for before this kernel waits for that one.  The queries and the
-      // newest keys are its work.
-      if (TMA) {
-        while (issued_ahead < STAGES && tile_begin + issued_ahead < tile_end && (tile_begin + issued_ahead + 1) * BLOCK_N <= pos0) {
-          issue_tile(current, tile_begin + issued_ahead);
-          ++issued_ahead;
+    if (!prefetched) {
+      if (!waited) {
+        // Tiles that end before the row's first new token hold nothing the kernel before this one writes: as many
+        // of them as the ring has stages are asked for before this kernel waits for that one.  The queries and the
+        // newest keys are its work.
+        if (TMA) {
+          while (issued_ahead < STAGES && tile_begin + issued_ahead < tile_end && (tile_begin + issued_ahead + 1) * BLOCK_N <= pos0) {
+            issue_tile(current, tile_begin + issued_ahead);
+            ++issued_ahead;
+          }
         }
+        grid_dependency_wait();
+        allow_dependents();   // only now: a kernel that is itself still waiting must not pull the next one onto the SMs
+        waited = true;
       }
-      grid_dependency_wait();
-      allow_dependents();   // only now: a kernel that is itself still waiting must not pull the next one onto the SMs
-      waited = true;
+      load_query(current);
+      if (TMA) cp_async_commit();   // otherwise the first tile's group carries the query
+      for (int s = issued_ahead; s < STAGES - 1; ++s) issue(tile_begin + s);   // the ring runs STAGES - 1 tiles ahead
     }
-    load_query(current);
-    if (TMA) cp_async_commit();   // otherwise the first tile's group carries the query
-    for (int s = issued_ahead; s < STAGES - 1; ++s) issue(tile_begin + s);   // the ring runs STAGES - 1 tiles ahead
 
     const bool upper_rows_unused = packed_rows <= 8;
     // The query fragments stay in registers when the head is small enough to leave room.
@@ -947,9 +951,15 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     unsigned q_frag[Q_IN_REGISTERS ? D / 16 : 1][4];
     bool q_loaded = false;
 
+    bool tile_prefetched = false;   // the following segment's first tile is on its way
     for (int tile = tile_begin; tile < tile_end; ++tile) {
       if (tile + STAGES - 1 < tile_begin + issued_ahead) {
         // asked for before the wait
+      } else if (TMA && STAGES == 2 && tile + 1 == tile_end && have_following) {
+        // The ring has a free stage and this segment no tile for it: the following segment's
+        // first tile comes in while this one's last tile is multiplied and the warps are merged.
+        issue_tile(following, following.tile_begin);
+        tile_prefetched = true;
       } else {
         issue(tile + STAGES - 1);
       }
@@ -1096,6 +1106,17 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     }
     if (!TMA) cp_async_wait<0>();
 
+    // While this segment is merged and written out, the next one's query is on its way into the
+    // query tile, which every warp has read; its first tile went into the stage that is not the
+    // one read last (where the merge happens).
+    prefetched = false;
+    if (TMA && STAGES == 2 && have_following) {
+      load_query(following);
+      cp_async_commit();
+      if (!tile_prefetched) issue_tile(following, following.tile_begin);
+      prefetched = true;
+    }
+
     // Merge the four warps: each leaves its (max, sum, unnormalised output) in shared memory.
     __nv_bfloat16* idle_stage = stages + ((consumed + STAGES - 1) % STAGES) * Tiles::STAGE;   // the stage read last
     // [4][16][D]: exactly one stage of the TMA form; columns swizzled by row (merge_swizzle)
@@ -1199,7 +1220,8 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
     }
     if (TMA) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // the merge buffers were written where TMA writes next
     __syncthreads();   // the query tile and the stages are free for the next segment
-    have = next_segment(current);
+    current = following;
+    have = have_following;
   }
   if (!CLUSTER) {
     if (!waited) grid_dependency_wait();   // a block without a segment: no grid ends before the grid ahead of it has
@@ -1271,14 +1293,14 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
 // -----------------------------------------------------------------------------------------
 constexpr int RUN_KEYS = 16, RUN_WARPS = ATT_THREADS / 32;
 constexpr int RUN_MIN_TILES = 4;   // tiles a warp takes at least: below it, starting and merging cost more than the walk
+constexpr bool RUNS_HEAD = TMA_HEAD && D <= 128;   // larger heads: two tiles and four warps to an SM are too few in flight (16 rows of 2,000 keys of 24 / 8 heads of 192: 54 us, shared tiles 43)
 template <bool ROOMY>
 struct RunTiles {
   static constexpr int TILE = RUN_KEYS * D;             // values in one tile of keys or of values: boxes of RUN_KEYS keys x 64 values
   static constexpr int STAGE = 2 * TILE;                // keys then values
   static constexpr int STAGE_BYTES = STAGE * (int)sizeof(__nv_bfloat16);
-  static constexpr int BLOCKS_PER_SM = D <= 128 ? 2 : 1;
-  // Stages of a block: 96 KB of two to an SM, 64 KB where pieces of many query rows need the room, 128 KB of a lone block.
-  static constexpr int STAGES = (BLOCKS_PER_SM == 1 ? 128 : ROOMY ? 96 : 64) * 1024 / RUN_WARPS / STAGE_BYTES;
+  static constexpr int BLOCKS_PER_SM = 2;
+  static constexpr int STAGES = (ROOMY ? 96 : 64) * 1024 / RUN_WARPS / STAGE_BYTES;   // of a warp; fewer where pieces of many query rows need the room
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
   static_assert(RING_BYTES >= SMALL_ROWS * D * (int)sizeof(float), "a run's last piece is left in its ring");
   // rings (1024-byte aligned for the swizzle), the runs' first pieces, the barriers of the stages
@@ -1458,7 +1480,6 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
 
   const bool sloped = OPTIONS && p.heads.slopes != nullptr;   // the scores are brought to log2 units before the softmax
   const float unit = sloped ? 1.f : p.scale_log2;
-  constexpr bool Q_IN_REGISTERS = D <= 128;   // else read again for every tile
   int consumed = 0;
   bool failed = false;
   while (at.position < run_end && !failed) {
@@ -1482,15 +1503,11 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
       row_q[h] = p.q + (size_t)(q0 + token) * p.q_stride + (size_t)head * D + 2 * tq;
     }
     // The fragments of the queries come straight from memory.
-    unsigned q_frag[Q_IN_REGISTERS ? D / 16 : 1][4];
-    auto load_q = [&](unsigned (&a)[4], int kk) {
+    unsigned q_frag[D / 16][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = row_valid[i & 1] ? *reinterpret_cast<const unsigned*>(row_q[i & 1] + kk * 16 + 8 * (i >> 1)) : 0u;
-    };
-    if (Q_IN_REGISTERS) {
+    for (int kk = 0; kk < D / 16; ++kk)
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) load_q(q_frag[Q_IN_REGISTERS ? kk : 0], kk);
-    }
+      for (int i = 0; i < 4; ++i) q_frag[kk][i] = row_valid[i & 1] ? *reinterpret_cast<const unsigned*>(row_q[i & 1] + kk * 16 + 8 * (i >> 1)) : 0u;
     float o[D / 8][4];
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
@@ -1514,9 +1531,8 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
       float s_odd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk) {
-        unsigned a_loaded[4], b[4];
-        if (!Q_IN_REGISTERS) load_q(a_loaded, kk);
-        const unsigned (&a)[4] = Q_IN_REGISTERS ? q_frag[Q_IN_REGISTERS ? kk : 0] : a_loaded;
+        unsigned b[4];
+        const unsigned (&a)[4] = q_frag[kk];
         ldmatrix_x4(b, ks + Tiles::offset((lane & 7) + 8 * (lane >> 4), kk * 2 + ((lane >> 3) & 1)));
         if (kk & 1) {
           mma_bf16(s_odd[0], a, b[0], b[1]);
@@ -1822,7 +1838,8 @@ static bool page_pool_map(CUtensorMap* map, const void* pages, long long rows, i
   return true;
 }
 
-constexpr size_t DEC_SMEM_GATHER = DecodeTiles<false>::SMEM;
+constexpr bool TMA_SHARED = TMA_HEAD && !RUNS_HEAD;   // whether the form whose blocks walk shared tiles is fed by TMA where the page size allows
+constexpr size_t DEC_SMEM_SHARED = DecodeTiles<TMA_SHARED>::SMEM, DEC_SMEM_GATHER = DecodeTiles<false>::SMEM;
 // The cluster form: its stages and query tile, then what the other blocks of the cluster send (partial results of
 // `rows` packed query rows in all, and every block's log-sum-exps).
 constexpr size_t DEC_SMEM_CLUSTER_BASE = DecodeTiles<TMA_HEAD, DEC_CLUSTER_STAGES>::SMEM;
@@ -1864,37 +1881,42 @@ static int decode_sm_count() {
   return count;
 }
 
-// Blocks of the decode kernel that a caller may ask for: as many of the gathering form as are resident at once.
+// Blocks of the decode kernel that a caller may ask for: as many as are resident at once of the forms whose blocks walk shared tiles.
 extern "C" int pylon_attention_decode_blocks() {
   static int resident_on[pylon::MAX_DEVICES] = {};
   int& resident = resident_on[pylon::current_device_slot()];
   if (resident == 0) {
-    int per_sm = 0;
+    int per_sm = 0, per_sm_shared = 0;
     if (decode_sm_count() < 1) return -1;
     if (cudaFuncSetAttribute(paged_attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_GATHER) != cudaSuccess) return -1;
+    if (cudaFuncSetAttribute(paged_attention_decode_kernel<TMA_SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_SHARED) != cudaSuccess) return -1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, paged_attention_decode_kernel<false>, ATT_THREADS, DEC_SMEM_GATHER) != cudaSuccess || per_sm < 1) return -1;
-    resident = per_sm * decode_sm_count();
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_shared, paged_attention_decode_kernel<TMA_SHARED>, ATT_THREADS, DEC_SMEM_SHARED) != cudaSuccess || per_sm_shared < 1) return -1;
+    resident = std::min(per_sm, per_sm_shared) * decode_sm_count();
   }
   return resident;
 }
 
-// The kernel of one run a warp, where a head's tiles come by TMA.
-template <bool TMA>
+// The kernel of one run a warp.
+template <bool RUNS>
 static cudaError_t configure_runs() {
-  if constexpr (TMA) {
+  if constexpr (RUNS) {
     cudaError_t err = cudaFuncSetAttribute(paged_attention_runs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
     if (err == cudaSuccess) err = cudaFuncSetAttribute(paged_attention_runs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
     return err;
   }
   return cudaSuccess;
 }
-template <bool TMA>
-static void launch_runs(const AttentionParams& p, int decode_blocks, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream) {
-  if constexpr (TMA) {
-    const bool roomy = RunTiles<true>::BLOCKS_PER_SM == 1 || RunTiles<true>::fits(p.incoming_rows);
+// Tiles by TMA without clusters: runs a warp, or for larger heads blocks over shared tiles.
+template <bool RUNS>
+static void launch_without_clusters(const AttentionParams& p, int decode_blocks, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream) {
+  if constexpr (RUNS) {
+    const bool roomy = RunTiles<true>::fits(p.incoming_rows);
     const int blocks = std::min(decode_blocks, RunTiles<true>::BLOCKS_PER_SM * decode_sm_count());
     launch_dependent(roomy ? paged_attention_runs_kernel<true> : paged_attention_runs_kernel<false>, dim3(blocks), dim3(ATT_THREADS),
                      roomy ? RunTiles<true>::smem(p.incoming_rows) : RunTiles<false>::smem(p.incoming_rows), stream, p, map_k, map_v);
+  } else {
+    launch_dependent(paged_attention_decode_kernel<TMA_SHARED>, dim3(decode_blocks), dim3(ATT_THREADS), DEC_SMEM_SHARED, stream, p, map_k, map_v);
   }
 }
 
@@ -1966,7 +1988,8 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
     if (err == cudaSuccess && WIDE_TILES)
       err = cudaFuncSetAttribute(paged_attention_mma_kernel<WIDE_TILES ? 2 : 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_SMEM_2);
     if (err == cudaSuccess) err = cudaFuncSetAttribute(paged_attention_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_GATHER);
-    if (err == cudaSuccess) err = configure_runs<TMA_HEAD>();
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(paged_attention_decode_kernel<TMA_SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_SHARED);
+    if (err == cudaSuccess) err = configure_runs<RUNS_HEAD>();
 #define PYLON_CLUSTER_CASE(N)                                                                                                   \
     if (err == cudaSuccess && TMA_HEAD)                                                                                         \
       err = cudaFuncSetAttribute(paged_attention_decode_kernel<TMA_HEAD, TMA_HEAD ? N : 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM_CLUSTER);
@@ -2034,7 +2057,7 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
         size = (room >= 16 && clusters_of_16()) ? 16 : room >= 8 ? 8 : room >= 6 ? 6 : room >= 4 ? 4 : room >= 3 ? 3 : room >= 2 ? 2 : 0;
         if (pairs * size > decode_blocks) size = 0;
       }
-      const int box_rows = size ? BLOCK_N : RUN_KEYS;
+      const int box_rows = RUNS_HEAD && size == 0 ? RUN_KEYS : BLOCK_N;
       if (!page_pool_map(&map_k, k_pages, pool_rows, box_rows) || !page_pool_map(&map_v, v_pages, pool_rows, box_rows))
         PYLON_REFUSE("paged_attention_mma: the tensor maps of the page pools could not be made");
 #define PYLON_CLUSTER_CASE(N)                                                                                                   \
@@ -2047,7 +2070,7 @@ static int attention_mma_entry(const void* q, long long q_stride, const void* k_
       }
       PYLON_CLUSTER_CASE(16) PYLON_CLUSTER_CASE(8) PYLON_CLUSTER_CASE(6) PYLON_CLUSTER_CASE(4) PYLON_CLUSTER_CASE(3) PYLON_CLUSTER_CASE(2)
 #undef PYLON_CLUSTER_CASE
-      if (size == 0) launch_runs<TMA_HEAD>(p, decode_blocks, map_k, map_v, stream);
+      if (size == 0) launch_without_clusters<RUNS_HEAD>(p, decode_blocks, map_k, map_v, stream);
     } else {
       launch_dependent(paged_attention_decode_kernel<false>, dim3(decode_blocks), dim3(ATT_THREADS), DEC_SMEM_GATHER, stream, p, map_k, map_v);
     }

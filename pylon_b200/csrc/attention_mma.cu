@@ -1291,8 +1291,8 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
 // behind the rotation: 34.3 us a layer with it, 27.6 now (100 MB of cache, 16 us of bytes); 31 of 64 to 1,500 keys 34 and 27; 16 of up to 3,700 37 and 35.
 // Inside, by the clock: 2 to 3 us for the plan and the first tiles' way, the walk at 6 TB/s, 2 to 3 us to add up, 3 to 8 through scratch memory.
 // -----------------------------------------------------------------------------------------
-constexpr int RUN_KEYS = 16, RUN_WARPS = ATT_THREADS / 32;
-constexpr int RUN_MIN_TILES = 4;   // tiles a warp takes at least: below it, starting and merging cost more than the walk
+constexpr int RUN_KEYS = D <= 64 ? 32 : 16, RUN_WARPS = ATT_THREADS / 32;   // 8 KB of keys and values a tile: a warp spends some 0.8 us on one, whatever it holds
+constexpr int RUN_MIN_TILES = 64 / RUN_KEYS;   // tiles a warp takes at least of equal runs: below it, starting and merging cost more than the walk
 constexpr bool RUNS_HEAD = TMA_HEAD && D <= 128;   // larger heads: two tiles and four warps to an SM are too few in flight (16 rows of 2,000 keys of 24 / 8 heads of 192: 54 us, shared tiles 43)
 template <bool ROOMY>
 struct RunTiles {
@@ -1324,21 +1324,45 @@ __device__ __forceinline__ int run_row_tiles(const AttentionParams& p, int row, 
   return hi / RUN_KEYS - lo / RUN_KEYS + 1;
 }
 
-// How many runs share `total` tiles.  Where it costs under a fifth of them, a number that makes the ends of equally long pairs fall on ends of
-// blocks, or at least of runs.
-__device__ __forceinline__ int runs_used(int total, int grid, int pairs) {
+// Quotients of the plan's numbers (a up to 2^20) without the integer division's long way.
+__device__ __forceinline__ int quotient(int a, int b) { return (int)__fdividef((float)a + 0.5f, (float)b); }
+
+// How many equal runs share `total` tiles.  Where it costs under a fifth of them, a multiple of the pairs' blocks, or at least of the pairs.
+__device__ __forceinline__ int equal_runs(int total, int grid, int pairs) {
   const int runs = max(1, min(grid, total / (RUN_WARPS * RUN_MIN_TILES))) * RUN_WARPS;
   if (pairs <= 0) return min(runs, max(total, 1));
-  const int blocks_aligned = runs / (pairs * RUN_WARPS) * (pairs * RUN_WARPS), aligned = runs / pairs * pairs;
+  const int blocks_aligned = quotient(runs, pairs * RUN_WARPS) * pairs * RUN_WARPS, aligned = quotient(runs, pairs) * pairs;
   const int used = blocks_aligned * 5 >= runs * 4 ? blocks_aligned : aligned * 5 >= runs * 4 ? aligned : runs;
   return min(used, max(total, 1));
+}
+
+// Into how many runs of its own every (row, KV head) pair is cut; 0: the tiles of all pairs are one sequence that `equal` equal runs share, wherever their ends fall.
+// Cut by pairs, few pairs or none lie in several blocks (3 to 8 us through scratch memory), but the longest pair's runs are longer than
+// an equal share.  A block's four warps for a pair, unless it is only a few tiles or the pairs are more than the blocks; several blocks for one where their walk
+// is five tiles shorter, two tiles to a warp at least (four beyond eight blocks of many packed rows, of which the merging is more).  Cut by pairs are rows of about equal lengths, short ones, and others
+// as long as the longest run exceeds the equal share by less than the way through scratch memory costs: some four tiles, more with many pairs.
+// A layer behind a norm, 32 query heads over 8 of 128, by pairs and in equal runs: eight rows of 100 keys 8.7 and 16.0 us, 16 of up to 1,000
+// 18.4 and 19.3, 48 of 4,000 123 and 133; but 16 of up to 4,000 40.5 and 36.2, 31 of up to 4,000 64.6 and 53.8.
+__device__ __forceinline__ int run_cut(int total, int longest, int grid, int pairs, int equal, int packed_rows) {
+  const int most = grid * RUN_WARPS;
+  if (pairs > most) return 0;
+  int cut = 1;
+  if (pairs > grid) {
+    if (longest >= 8 && 2 * pairs <= most) cut = 2;
+  } else if (longest > 4) {
+    cut = RUN_WARPS;
+    const int wide = min(min(quotient(most, pairs), packed_rows > 8 ? max(longest / 4, min(longest / 2, 32)) : longest / 2), 64) / RUN_WARPS * RUN_WARPS;
+    if (longest * (wide - RUN_WARPS) >= 5 * RUN_WARPS * wide) cut = wide;
+  }
+  if (longest < 8 || (float)longest * pairs <= 1.125f * total) return cut;
+  return (float)longest * equal <= (float)cut * (total + equal * (4.f + pairs / 48.f)) ? cut : 0;
 }
 
 template <bool ROOMY>
 __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) paged_attention_runs_kernel(const AttentionParams p, const __grid_constant__ CUtensorMap map_k,
                                                                                                           const __grid_constant__ CUtensorMap map_v) {
   using Tiles = RunTiles<ROOMY>;
-  constexpr int STAGES = Tiles::STAGES, PIECES = 2 * RUN_WARPS;
+  constexpr int STAGES = Tiles::STAGES, PIECES = 2 * RUN_WARPS, NB = RUN_KEYS / 8;   // NB: products of eight keys to a tile
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   // The block's pieces, two places a warp: the pair (-1: none), its first block, how many blocks it lies in, q0 and packed rows of its row.
@@ -1369,19 +1393,22 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
   // The plan, made by every warp for itself: the rows' lengths were written long before the kernel ahead of this one started.
   int unused;
   const int first_chunk = lane < p.num_rows ? run_row_tiles(p, lane, &unused, &unused) : 0;
-  int total = first_chunk, with_tiles = first_chunk > 0;
+  int total = first_chunk, with_tiles = first_chunk > 0, longest = first_chunk;
   for (int base = 32; base < p.num_rows; base += 32) {
     const int tiles = base + lane < p.num_rows ? run_row_tiles(p, base + lane, &unused, &unused) : 0;
     total += tiles;
     with_tiles += tiles > 0;
+    longest = max(longest, tiles);
   }
 #pragma unroll
   for (int offset = 16; offset; offset >>= 1) {
     total += __shfl_xor_sync(0xffffffffu, total, offset);
     with_tiles += __shfl_xor_sync(0xffffffffu, with_tiles, offset);
+    longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, offset));
   }
   total *= p.nkv;
-  const int runs = runs_used(total, gridDim.x, with_tiles * p.nkv);
+  const int pairs = with_tiles * p.nkv, equal = equal_runs(total, gridDim.x, pairs);
+  const int cut = run_cut(total, longest, gridDim.x, pairs, equal, p.incoming_rows), runs = cut ? pairs * cut : equal;
   if ((int)blockIdx.x * RUN_WARPS >= runs || total == 0) {   // no run for this block
     grid_dependency_wait();   // a grid must not end before the grid ahead of it has: the next kernel's wait sees only this one
     return;
@@ -1396,13 +1423,14 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
     else if (b + 1 < runs && begin_of(b + 1) <= tile) ++b;
     return b / RUN_WARPS;
   };
-  const int run_first = run < runs ? begin_of(run) : total, run_end = run < runs ? begin_of(run + 1) : total;
-
   // A place in the sequence: the next tile, with its row and what is known of it.
   struct Cursor { int position, row, row_tiles, first_tile, pos0, kv_head, tile; };   // tile counts from the row's first
-  Cursor at = {run_first, 0, 0, 0, 0, 0, 0};
-  if (run_first < run_end) {
-    int before = 0;
+  Cursor at = {0, 0, 0, 0, 0, 0, 0};
+  int run_first = 0, run_end = 0;   // empty: a warp without a run, or the end of a pair of fewer tiles than `cut`
+  if (run < runs) {
+    const int run_pair = cut ? quotient(run, cut) : 0, wanted_row = quotient(run_pair, p.nkv);   // among the rows that have tiles
+    if (!cut) { run_first = begin_of(run); run_end = begin_of(run + 1); }
+    int before = 0, rows_before = 0;
     for (int base = 0; base < p.num_rows; base += 32) {
       const int tiles = (base == 0 ? first_chunk : (base + lane < p.num_rows ? run_row_tiles(p, base + lane, &unused, &unused) : 0)) * p.nkv;
       int inclusive = tiles;
@@ -1412,17 +1440,29 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
         if (lane >= offset) inclusive += below;
       }
       const int exclusive = before + inclusive - tiles;
-      const unsigned hit = __ballot_sync(0xffffffffu, tiles > 0 && exclusive <= run_first && run_first < exclusive + tiles);
+      const unsigned filled = __ballot_sync(0xffffffffu, tiles > 0);
+      const bool here = tiles > 0 && (cut ? rows_before + __popc(filled & ((1u << lane) - 1u)) == wanted_row : exclusive <= run_first && run_first < exclusive + tiles);
+      const unsigned hit = __ballot_sync(0xffffffffu, here);
       if (hit) {
         at.row = base + __ffs(hit) - 1;
-        const int within = run_first - __shfl_sync(0xffffffffu, exclusive, __ffs(hit) - 1);
+        const int row_first = __shfl_sync(0xffffffffu, exclusive, __ffs(hit) - 1);
         at.row_tiles = run_row_tiles(p, at.row, &at.first_tile, &at.pos0);
-        at.kv_head = within / at.row_tiles;
-        at.tile = within % at.row_tiles;
+        if (cut) {
+          at.kv_head = run_pair - wanted_row * p.nkv;
+          const int part = run - run_pair * cut, parts = min(cut, at.row_tiles), pair_first = row_first + at.kv_head * at.row_tiles;
+          at.tile = part < parts ? part * at.row_tiles / parts : 0;
+          run_first = pair_first + at.tile;
+          run_end = part < parts ? pair_first + (part + 1) * at.row_tiles / parts : run_first;
+        } else {
+          at.kv_head = (run_first - row_first) / at.row_tiles;
+          at.tile = (run_first - row_first) % at.row_tiles;
+        }
         break;
       }
       before += __shfl_sync(0xffffffffu, inclusive, 31);
+      rows_before += __popc(filled);
     }
+    at.position = run_first;
   }
   auto next_row = [&](Cursor& c) {   // to the first tile of the next row that has any; there is one, since the run goes on
     c.kv_head = c.tile = 0;
@@ -1527,23 +1567,20 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
         __syncwarp();
       }
       // Even and odd k-steps accumulate separately: four independent MMA chains instead of two.
-      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      float s_odd[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float s[NB][4] = {}, s_odd[NB][4] = {};
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk) {
-        unsigned b[4];
         const unsigned (&a)[4] = q_frag[kk];
-        ldmatrix_x4(b, ks + Tiles::offset((lane & 7) + 8 * (lane >> 4), kk * 2 + ((lane >> 3) & 1)));
-        if (kk & 1) {
-          mma_bf16(s_odd[0], a, b[0], b[1]);
-          mma_bf16(s_odd[1], a, b[2], b[3]);
-        } else {
-          mma_bf16(s[0], a, b[0], b[1]);
-          mma_bf16(s[1], a, b[2], b[3]);
+#pragma unroll
+        for (int n = 0; n < NB; n += 2) {
+          unsigned b[4];
+          ldmatrix_x4(b, ks + Tiles::offset(8 * n + (lane & 7) + 8 * (lane >> 4), kk * 2 + ((lane >> 3) & 1)));
+          mma_bf16(kk & 1 ? s_odd[n] : s[n], a, b[0], b[1]);
+          mma_bf16(kk & 1 ? s_odd[n + 1] : s[n + 1], a, b[2], b[3]);
         }
       }
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < NB; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           s[n][i] += s_odd[n][i];
@@ -1553,7 +1590,7 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
       // Tiles that end at or before the row's first new token, with no window, are visible whole.
       if (p.window > 0 || p.chunk > 0 || key0 + RUN_KEYS - 1 > pos0) {
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < NB; ++n)
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int key = key0 + 2 * tq + n * 8 + (i & 1);
@@ -1565,13 +1602,15 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
         if (h == 1 && upper_rows_unused) continue;   // rows 8..15 hold zero queries, and nothing of them is stored
         if (SIGMOID) {
 #pragma unroll
-          for (int n = 0; n < 2; ++n) {
+          for (int n = 0; n < NB; ++n) {
             s[n][2 * h] = sigmoid_exp2(fmaf(s[n][2 * h], p.scale_log2, row_bias[h]));
             s[n][2 * h + 1] = sigmoid_exp2(fmaf(s[n][2 * h + 1], p.scale_log2, row_bias[h]));
           }
           continue;
         }
-        float mx = fmaxf(fmaxf(s[0][2 * h], s[0][2 * h + 1]), fmaxf(s[1][2 * h], s[1][2 * h + 1]));
+        float mx = fmaxf(s[0][2 * h], s[0][2 * h + 1]);
+#pragma unroll
+        for (int n = 1; n < NB; ++n) mx = fmaxf(mx, fmaxf(s[n][2 * h], s[n][2 * h + 1]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         const float new_max = fmaxf(row_max[h], mx);
@@ -1580,7 +1619,7 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
         const float shift = use_max * unit;
         float sum = 0.f;
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
+        for (int n = 0; n < NB; ++n) {
           s[n][2 * h] = fast_exp2(s[n][2 * h] * unit - shift);
           s[n][2 * h + 1] = fast_exp2(s[n][2 * h + 1] * unit - shift);
           sum += s[n][2 * h] + s[n][2 * h + 1];
@@ -1590,21 +1629,24 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
 #pragma unroll
         for (int i = 0; i < D / 8; ++i) { o[i][2 * h] *= alpha; o[i][2 * h + 1] *= alpha; }
       }
-      unsigned a[4] = {pack_bf16(s[0][0], s[0][1]), pack_bf16(s[0][2], s[0][3]), pack_bf16(s[1][0], s[1][1]), pack_bf16(s[1][2], s[1][3])};
-      unsigned dropped[4];
-      if (SPLIT) {
 #pragma unroll
-        for (int f = 0; f < 4; ++f) dropped[f] = pack_dropped(s[f >> 1][2 * (f & 1)], s[f >> 1][2 * (f & 1) + 1], a[f]);
-      }
-#pragma unroll
-      for (int d2 = 0; d2 < D / 16; ++d2) {
-        unsigned b[4];
-        ldmatrix_x4_trans(b, vs + Tiles::offset((lane & 7) + 8 * ((lane >> 3) & 1), d2 * 2 + (lane >> 4)));
-        mma_bf16(o[2 * d2], a, b[0], b[1]);
-        mma_bf16(o[2 * d2 + 1], a, b[2], b[3]);
+      for (int n = 0; n < NB; n += 2) {
+        unsigned a[4] = {pack_bf16(s[n][0], s[n][1]), pack_bf16(s[n][2], s[n][3]), pack_bf16(s[n + 1][0], s[n + 1][1]), pack_bf16(s[n + 1][2], s[n + 1][3])};
+        unsigned dropped[4];
         if (SPLIT) {
-          mma_bf16(o[2 * d2], dropped, b[0], b[1]);
-          mma_bf16(o[2 * d2 + 1], dropped, b[2], b[3]);
+#pragma unroll
+          for (int f = 0; f < 4; ++f) dropped[f] = pack_dropped(s[n + (f >> 1)][2 * (f & 1)], s[n + (f >> 1)][2 * (f & 1) + 1], a[f]);
+        }
+#pragma unroll
+        for (int d2 = 0; d2 < D / 16; ++d2) {
+          unsigned b[4];
+          ldmatrix_x4_trans(b, vs + Tiles::offset(8 * n + (lane & 7) + 8 * ((lane >> 3) & 1), d2 * 2 + (lane >> 4)));
+          mma_bf16(o[2 * d2], a, b[0], b[1]);
+          mma_bf16(o[2 * d2 + 1], a, b[2], b[3]);
+          if (SPLIT) {
+            mma_bf16(o[2 * d2], dropped, b[0], b[1]);
+            mma_bf16(o[2 * d2 + 1], dropped, b[2], b[3]);
+          }
         }
       }
       __syncwarp();   // the stage has been read by all lanes
@@ -1616,10 +1658,11 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
     const bool whole = tile_begin == 0 && tile_end == row_tiles, last = at.position >= run_end;
     const int place = 2 * warp + (last ? 1 : 0);
     if (!whole && lane == 0) {
-      const int pair_first = at.position - tile_end, first_block = block_of(pair_first);
+      const int pair_first = at.position - tile_end, pair_run = quotient(run, max(cut, 1)) * cut;   // cut: the pair's first run
+      const int first_block = cut ? pair_run / RUN_WARPS : block_of(pair_first);
       piece_pair[place] = row * p.nkv + kv_head;
       piece_first[place] = first_block;
-      piece_blocks[place] = block_of(pair_first + row_tiles - 1) - first_block + 1;
+      piece_blocks[place] = (cut ? (pair_run + min(cut, row_tiles) - 1) / RUN_WARPS : block_of(pair_first + row_tiles - 1)) - first_block + 1;
       piece_q0[place] = q0;
       piece_rows[place] = packed_rows;
     }

@@ -912,6 +912,28 @@ def test_decoded_rows_a_run_to_a_warp(nq, nkv, d, page, blocks):
     assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0
 
 
+@pytest.mark.parametrize("nq, nkv, d", [(8, 2, 64), (10, 2, 128), (4, 4, 128), (16, 1, 128)])
+@pytest.mark.parametrize("kv_lens, portion, blocks", [
+    ([40] * 3, None, None), ([64] * 40, None, None), ([65, 80, 97], None, None), ([600, 610, 590], None, None), ([2_500], None, None), ([2_500, 30, 900], None, None),
+    ([200] * 9, 5, None), ([300, 260, 280], 0, None), ([130] * 35, 33, 21), ([500] * 4, None, 9), ([500] * 4, None, 5), ([90, 1, 16, 17, 100, 33] * 7, 20, 30)])
+def test_decoded_rows_cut_by_pairs_or_in_equal_runs(nq, nkv, d, kv_lens, portion, blocks):
+    """Pairs cut into one, two, four and more runs and equal runs, more and fewer pairs than blocks, more rows than a warp has lanes, a prompt's row among them (which is not
+    walked here); page 64."""
+    from pylon_b200.kernels import ops
+
+    q_lens = [1] * len(kv_lens)
+    if portion is not None:
+        q_lens[portion] = min(kv_lens[portion], 40)
+    cache = Paged(kv_lens, q_lens, nkv, d, 64, torch.bfloat16)
+    fused = torch.randn(cache.tokens, (nq + 2 * nkv) * d, device=DEVICE).to(torch.bfloat16)
+    expected = attention_reference(fused[:, : nq * d].reshape(cache.tokens, nq, d), cache, nq, nkv, d, None, d**-0.5)
+    for _ in range(2):   # the counters are zero again
+        out = ops.paged_attention(fused, cache.k_pages, cache.v_pages, cache.positions, cache.token_row, cache.q_start, cache.kv_len, cache.table, nq,
+                                  max(q_lens), max(kv_lens), decode_blocks=blocks)
+        torch.testing.assert_close(out.double(), expected, rtol=2e-2, atol=2e-2)
+    assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0
+
+
 @pytest.mark.parametrize("form, page, rows, kv_len, blocks", [
     ("a pair in one run", 64, 12, 16, None), ("a block's warps", 64, 2, 700, 1), ("many blocks", 64, 1, 3_000, None), ("few blocks", 64, 3, 700, 5),
     ("clusters", 64, 1, 2_000, None), ("clusters", 64, 3, 90, None), ("gathered", 48, 2, 700, 1), ("gathered", 48, 1, 3_000, 40)])

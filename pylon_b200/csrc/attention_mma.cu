@@ -1633,20 +1633,16 @@ __global__ void __launch_bounds__(ATT_THREADS, RunTiles<ROOMY>::BLOCKS_PER_SM) p
       for (int n = 0; n < NB; n += 2) {
         unsigned a[4] = {pack_bf16(s[n][0], s[n][1]), pack_bf16(s[n][2], s[n][3]), pack_bf16(s[n + 1][0], s[n + 1][1]), pack_bf16(s[n + 1][2], s[n + 1][3])};
         unsigned dropped[4];
-        if (SPLIT) {
 #pragma unroll
-          for (int f = 0; f < 4; ++f) dropped[f] = pack_dropped(s[n + (f >> 1)][2 * (f & 1)], s[n + (f >> 1)][2 * (f & 1) + 1], a[f]);
-        }
+        for (int f = 0; f < 4; ++f) dropped[f] = pack_dropped(s[n + (f >> 1)][2 * (f & 1)], s[n + (f >> 1)][2 * (f & 1) + 1], a[f]);
 #pragma unroll
         for (int d2 = 0; d2 < D / 16; ++d2) {
           unsigned b[4];
           ldmatrix_x4_trans(b, vs + Tiles::offset(8 * n + (lane & 7) + 8 * ((lane >> 3) & 1), d2 * 2 + (lane >> 4)));
           mma_bf16(o[2 * d2], a, b[0], b[1]);
           mma_bf16(o[2 * d2 + 1], a, b[2], b[3]);
-          if (SPLIT) {
-            mma_bf16(o[2 * d2], dropped, b[0], b[1]);
-            mma_bf16(o[2 * d2 + 1], dropped, b[2], b[3]);
-          }
+          mma_bf16(o[2 * d2], dropped, b[0], b[1]);
+          mma_bf16(o[2 * d2 + 1], dropped, b[2], b[3]);
         }
       }
       __syncwarp();   // the stage has been read by all lanes

@@ -934,6 +934,21 @@ def test_decoded_rows_cut_by_pairs_or_in_equal_runs(nq, nkv, d, kv_lens, portion
     assert int(ops.attention_error_word(torch.device(DEVICE)).item()) == 0
 
 
+@pytest.mark.parametrize("nq, nkv, d", [(4, 2, 64), (32, 8, 128), (8, 8, 128)])
+@pytest.mark.parametrize("kv_lens", [[385] * 16, [64, 1_500, 333, 900, 120, 700, 48, 2_000], [100] * 12])
+def test_decoded_rows_are_as_near_to_64_bits_as_bfloat16_allows(nq, nkv, d, kv_lens):
+    """Weights of 16 bits: what is left is the result's own rounding, half an ulp at most and 1.66e-3 in the mean; weights of 8 bits add 1.1e-3 to 1.3e-3 (in
+    squares: a fifth to a quarter more)."""
+    from pylon_b200.kernels import ops
+
+    cache = Paged(kv_lens, [1] * len(kv_lens), nkv, d, 64, torch.bfloat16)
+    fused = torch.randn(cache.tokens, (nq + 2 * nkv) * d, device=DEVICE).to(torch.bfloat16)
+    expected = attention_reference(fused[:, : nq * d].reshape(cache.tokens, nq, d), cache, nq, nkv, d, None, d**-0.5)
+    out = ops.paged_attention(fused, cache.k_pages, cache.v_pages, cache.positions, cache.token_row, cache.q_start, cache.kv_len, cache.table, nq, 1, max(kv_lens))
+    rounded = (expected.to(torch.bfloat16).double() - expected).norm()
+    assert float((out.double() - expected).norm() / rounded) < 1.03
+
+
 @pytest.mark.parametrize("form, page, rows, kv_len, blocks", [
     ("a pair in one run", 64, 12, 16, None), ("a block's warps", 64, 2, 700, 1), ("many blocks", 64, 1, 3_000, None), ("few blocks", 64, 3, 700, 5),
     ("clusters", 64, 1, 2_000, None), ("clusters", 64, 3, 90, None), ("gathered", 48, 2, 700, 1), ("gathered", 48, 1, 3_000, 40)])

@@ -595,21 +595,22 @@ __device__ __forceinline__ int decode_row_tiles(const AttentionParams& p, int ro
   return hi / BLOCK_N - lo / BLOCK_N + 1;
 }
 
+constexpr bool RUNS_HEAD = TMA_HEAD && D <= 128;   // larger heads: two tiles and four warps to an SM are too few in flight (16 rows of 2,000 keys of 24 / 8 heads of 192: 54 us, shared tiles 43)
 constexpr int DEC_PENDING = 16;    // segments a block collects before it publishes them
 constexpr int DEC_MIN_TILES = 4;   // a block takes about this many tiles at least: below it, starting and merging cost more than the walk
 
-// The runs: `used` blocks share `total` tiles, block b takes [run_begin(b), run_begin(b + 1)), so the
+// Blocks over shared tiles (every head size where tiles are gathered, heads above 128 where TMA brings them).  The runs: `used` blocks share `total` tiles, block b takes [run_begin(b), run_begin(b + 1)), so the
 // runs differ by one tile at most; run_of(x) is the block whose run holds tile x.
 // `pairs`: (row, KV head) pairs with tiles.  When the rows are equally long, a number of blocks that is a
 // multiple of the pairs makes every run end where a pair ends, and no block has to merge and publish
-// twice (30 instead of 35 us at batch 8, context 4096); it is taken if it costs under a fifth of the blocks.
+// twice; it is taken if it costs under a fifth of the blocks.
 __device__ __forceinline__ int decode_blocks_used(int total, int grid, int pairs) {
   const int used = max(1, min(grid, total / DEC_MIN_TILES));
   const int aligned = pairs > 0 ? used / pairs * pairs : 0;
   return aligned * 5 >= used * 4 ? aligned : used;
 }
 __device__ __forceinline__ int run_begin(int block, int total, int used) { return (int)((long long)block * total / used); }
-__device__ __forceinline__ int run_of(int tile, int total, int used) { return (int)((((long long)tile + 1) * used - 1) / total); }   // a block takes at least this many tiles: below it the merging costs more than the walk
+__device__ __forceinline__ int run_of(int tile, int total, int used) { return (int)((((long long)tile + 1) * used - 1) / total); }
 
 // The log-sum-exp (log2) a partial result is weighed by, from its running maximum in log2 units and the sum of its weights: -infinity where nothing was
 // visible, and +infinity where a visible score was not a number.  fmaxf passes such scores over, so the maximum may be -infinity all the same and only the sum tells; as
@@ -691,6 +692,7 @@ __device__ __forceinline__ void combine_segments(const AttentionParams& p, int p
 template <bool TMA, int CLUSTER = 0, int CLUSTER_STAGES = DEC_CLUSTER_STAGES>
 __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ? 3 : 1) paged_attention_decode_kernel(const AttentionParams p, const __grid_constant__ CUtensorMap map_k,
                                                                               const __grid_constant__ CUtensorMap map_v) {
+  static_assert(!TMA || CLUSTER > 0 || !RUNS_HEAD, "without clusters, smaller heads' tiles come by TMA to runs of warps");
   constexpr int STAGES = CLUSTER ? CLUSTER_STAGES : DEC_STAGES;
   using Tiles = DecodeTiles<TMA, STAGES>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1281,19 +1283,23 @@ __global__ void __launch_bounds__(ATT_THREADS, D <= 128 && CLUSTER_STAGES <= 2 ?
 // Decoded rows without clusters, tiles by TMA: every warp walks a run of its own.
 //
 // Bound by the bytes of the cache.  All (row, KV head, tile of RUN_KEYS keys) triples of the launch form one sequence, row-major, that the
-// warps cut into equal runs, consecutive runs to the warps of a block.  A warp has a ring of stages of its own, which runs
+// warps cut into runs (run_cut), consecutive runs to the warps of a block.  A warp has a ring of stages of its own, which runs
 // ahead over the ends of rows, and keeps its scores, softmax and sums in registers: no warp waits for another before its run is done.
 // A (row, KV head) pair that lies in one run is written out by its warp.  The other pieces are left in shared memory (the
 // run's last one in the warp's own ring, which is idle by then, the first in a place of its own) and added up once, at the end of
 // the block; a pair that lies in several blocks goes through scratch slot (pair + block) as in the kernel above.
 //
-// Why so: the form above, fed by TMA, walked 64-key tiles with four warps in step and merged them behind every row.  64 requests of 400 keys of the Qwen3-4B shape
-// behind the rotation: 34.3 us a layer with it, 27.6 now (100 MB of cache, 16 us of bytes); 31 of 64 to 1,500 keys 34 and 27; 16 of up to 3,700 37 and 35.
+// Why so: the form above, fed by TMA, walks 64-key tiles with four warps in step and merges them behind every row.  32 query heads over 8 of 128, behind a norm: 64 requests of
+// 400 keys 37.5 us with it, 27.3 so (100 MB of cache, 16 us of bytes); 31 of 64 to 1,500 keys 36 and 31; 16 of up to 3,700 38 and 35; 16 of 100 15.0 and 9.4.  Slower, in 7
+// of 852 sizes by more than 5 %: pairs that are a little more than the blocks, and long (48 requests of 4,000 keys 126 and 134 us, of four tokens each over 3,000 keys 104 and 119).
 // Inside, by the clock: 2 to 3 us for the plan and the first tiles' way, the walk at 6 TB/s, 2 to 3 us to add up, 3 to 8 through scratch memory.
+//
+// A weight enters the weighted sum as two bfloat16 numbers, the rounded weight and what the rounding dropped, with any build: the largest weight of a warp is 1 and
+// rounds to itself, and with one or two warps to a pair instead of four there are fewer such weights.  Error against 64 bits over 131 sizes, of the result's norm:
+// 1.66e-3 (its own rounding), with weights of 8 bits 2.05e-3, the form above 2.01e-3.  It costs 4 % (tensor cores have the time in a walk bound by bytes).
 // -----------------------------------------------------------------------------------------
 constexpr int RUN_KEYS = D <= 64 ? 32 : 16, RUN_WARPS = ATT_THREADS / 32;   // 8 KB of keys and values a tile: a warp spends some 0.8 us on one, whatever it holds
 constexpr int RUN_MIN_TILES = 64 / RUN_KEYS;   // tiles a warp takes at least of equal runs: below it, starting and merging cost more than the walk
-constexpr bool RUNS_HEAD = TMA_HEAD && D <= 128;   // larger heads: two tiles and four warps to an SM are too few in flight (16 rows of 2,000 keys of 24 / 8 heads of 192: 54 us, shared tiles 43)
 template <bool ROOMY>
 struct RunTiles {
   static constexpr int TILE = RUN_KEYS * D;             // values in one tile of keys or of values: boxes of RUN_KEYS keys x 64 values
@@ -1341,7 +1347,7 @@ __device__ __forceinline__ int equal_runs(int total, int grid, int pairs) {
 // an equal share.  A block's four warps for a pair, unless it is only a few tiles or the pairs are more than the blocks; several blocks for one where their walk
 // is five tiles shorter, two tiles to a warp at least (four beyond eight blocks of many packed rows, of which the merging is more).  Cut by pairs are rows of about equal lengths, short ones, and others
 // as long as the longest run exceeds the equal share by less than the way through scratch memory costs: some four tiles, more with many pairs.
-// A layer behind a norm, 32 query heads over 8 of 128, by pairs and in equal runs: eight rows of 100 keys 8.7 and 16.0 us, 16 of up to 1,000
+// A layer behind a norm, 32 query heads over 8 of 128 (weights of 8 bits), by pairs and in equal runs: eight rows of 100 keys 8.7 and 16.0 us, 16 of up to 1,000
 // 18.4 and 19.3, 48 of 4,000 123 and 133; but 16 of up to 4,000 40.5 and 36.2, 31 of up to 4,000 64.6 and 53.8.
 __device__ __forceinline__ int run_cut(int total, int longest, int grid, int pairs, int equal, int packed_rows) {
   const int most = grid * RUN_WARPS;

@@ -560,11 +560,11 @@ static cudaError_t configure(GemmKernel kernel, KernelState& state, size_t smem)
 // Rows kernel: 16 warps of a cluster (eight blocks of two) take a leaf each, so that 40 slabs (a matrix of 2,560 rows) are 640 warps.
 // With enough slabs, four warps of a lone block take a quarter each: no cluster to place and no shared memory to cross, and a warp's ring runs four
 // times as long.  With four rows of x or fewer the loads bound it and more, smaller blocks keep more of them in flight (one row, 2,374 slabs: 243
-// against 268 us).  With a short k most of a cluster's warps have nothing to do (one row of [2560, 64]: 2.9 us alone, 3.9 in clusters; 12 of [9728, 300] 15.2
-// and 26.7; but one of [512, 128] 3.7 and 3.4).  5 to 8 rows: from 96 slabs on up to a k of 2,560 (8 of [6144, 2560] 20.4 and 23.4 us, of [24576, 512] 17.6 and
-// 34.7; but of [5120, 2560] 20.6 and 17.4, of [19456, 4096] 77 and 70), whatever k is from LONE_WORK results in groups of 64 on.  9 to 16 rows: by an estimate of
-// both forms fitted to their times over 16 to 640 slabs and k of 512 to 9,728, within 6 % of the better one (9 rows alone and in clusters: [6144, 2560] 32
-// and 37 us, [19456, 2560] 72 and 87, [16384, 9728] 188 and 203; but [5120, 4096] 48.7 and 43.0, [19456, 9728] 253 and 218).
+// against 268 us).  With a short k most of a cluster's warps have nothing to do (one row of [2560, 64]: 2.9 us alone, 3.9 in clusters; 12 of [9728, 300] 14.7
+// and 26.7; but one of [512, 128] 3.7 and 3.4).  5 to 8 rows: from 96 slabs on up to a k of 2,560 (8 of [6144, 2560] 20.9 and 22.1 us, of [24576, 512] 16 and
+// 33; but of [5120, 2560] 20.6 and 15.6, of [19456, 4096] 77 and 70), whatever k is from LONE_WORK results in groups of 64 on.  9 to 16 rows: by an estimate of
+// both forms fitted to their times over 16 to 640 slabs and k of 512 to 9,728, and where it is 7 % ahead (9 rows alone and in clusters: [6144, 2560] 32 and
+// 35 us, [16384, 2560] 50 and 72, [19456, 2560] 72 and 85; but [5120, 4096] 48.7 and 41, [19456, 9728] 253 and 225).
 constexpr long long LONE_WORK = 4096;
 
 static bool rows_alone(const GemmArgs& a, long long slabs) {
@@ -636,9 +636,10 @@ static int tile_kernel(const GemmArgs& a, int batch, int blocks, cudaStream_t st
   PYLON_CHECK_LAUNCH("gemm_f32");
 }
 
-// The estimate is a least-squares fit to 580 timed launches (32 to 320 rows of the four matrices of the Qwen3-4B shape, all tiles and
-// cluster sizes): within 6 % of them, and the tile it picks within 2 % of the fastest on average, 10 % at worst.  Over 1,663 other sizes (17 to
-// 2,048 rows, 64 to 32,000 weight rows, k from 16 to 2,561) the tile is 8 % behind the fastest on average.  What it weighs: results
+// The estimate is a least-squares fit to 580 launches of stages of 16 k (32 to 320 rows of the four matrices of the Qwen3-4B shape, all tiles and
+// cluster sizes).  With stages of 32 all tiles became faster alike: it is 14 % too long on average, but of 48 such sizes (17 to 320 rows, all tiles timed again)
+// the tile it picks is within 1.1 % of the fastest on average, 19 % at worst ([256, 9728] x [2560, 9728]), and of 160 others (17 to 2,048 rows, 64 to 32,000 weight rows,
+// k from 16 to 2,556) 7 % behind it on average.  A fit to all of these launches picks 1.5 % better on average and up to 40 % worse (960 rows of [249, 424]).  What it weighs: results
 // and reads per four k, rounds of blocks (a lone block in the last round runs faster than two that share an SM), the sum across blocks.
 typedef int (*TileEntry)(const GemmArgs&, int, int, cudaStream_t, double*);
 
@@ -685,8 +686,8 @@ static int gemm_f32(const GemmArgs& a, int batch, int force, cudaStream_t stream
     // Short k: always up to 64 (64 rows of [6144, 64] 5.7 us, tile kernel 6.2; 16 of [1000, 64] 4.9 and 5.7); up to 128 where 16-byte copies do not reach
     // (300 rows of [1000, 65] 6.3 and 6.9) or a grid of few rows is many blocks (64 rows of [2560, 128] level at 9.2, but of [512, 128] 9.2 and 6.7).
     if (!few && (a.K <= 64 || (a.K <= SHORT_MOST && (!aligned || (a.M <= 64 && slabs >= 64))))) return launch_short(a, batch, stream);
-    // 9 to 16 rows stream the weights where there are enough of them for lone blocks (12 rows of [9728, 256] 14.9 us, tile kernel 18.0) or a long
-    // k over a large matrix (12 of [2560, 2560] 20 and 28); else the tile kernel's clusters end sooner (16 of [1000, 512] 9.1 and 7.3).
+    // 9 to 16 rows stream the weights where there are enough of them for lone blocks (12 rows of [9728, 300] 15.2 us, tile kernel 19.7) or a long
+    // k over a large matrix (12 of [2560, 2560] 20.0 and 24.8); else the tile kernel's clusters end sooner (16 of [1000, 512] 9.0 and 6.5).
     const bool streams = a.M <= ROWS_MOST && (slabs * a.M >= LONE_WORK || (aligned && a.K < 512 && slabs >= 64) || (a.K >= 512 && slabs * 64 * a.K >= 1 << 20));
     if (!few && !streams) return launch_tile(a, batch, aligned, 0, stream);
   }

@@ -1110,7 +1110,8 @@ def paged_attention(
     """Causal attention of every token of a step over its request's pages.
 
     ``split_weights`` (softmax weights on the tensor cores): a weight enters the weighted sum as two bfloat16 numbers, the rounded
-    weight and what the rounding dropped, so that it counts with 16 bits instead of 8, at twice the products over the values.
+    weight and what the rounding dropped, so that it counts with 16 bits instead of 8, at twice the products over the values.  (Decoded rows of heads of 64
+    and 128 over pages of a multiple of 64 keys, without ``rows_alike``, count so in any case.)
 
     ``distance_slopes`` (float32 ``[nq]``, softmax weights): the scaled (and capped) score of the key ``p - j`` positions back loses
     ``distance_slopes[h] * (p - j)``.  Slopes, gated outputs, a factor and an ``out`` that is a slice of wider rows, and sinks with any of these or

@@ -1,7 +1,7 @@
 // The gated unit of a feed-forward in bfloat16 for a few rows of x on the fifth-generation tensor cores, with the weights on the wide side of the tile:
 // 128 interleaved rows of gate and up are the M of a tcgen05.mma and the rows of x, rounded up to 16, its N.
 //
-// Bound by the bytes of W: 16 rows of [34816, 5120] and the norm ahead of them 62.6 us (356 MB: 5.7 TB/s and more), where the kernel that multiplies with mma.sync
+// Bound by the bytes of W: 16 rows of [34816, 5120] and the norm ahead of them 62.2 us (356 MB: 5.7 TB/s and more), where the kernel that multiplies with mma.sync
 // from registers (gemm_stream.cu) takes 66.6 us, its warps busy with fragments; 32 rows 62.9 and 77.7 us.  The products' dispatch sends it 9 to 32 rows; it takes up to 256,
 // those above 32 with one set of accumulators.  A block takes 128 rows of W over the whole of k; two share an
 // SM, so that one's epilogue overlaps the other's loads.  Six warps: one lane of the fifth asks for boxes of W and x (TMA, 128-byte
@@ -13,9 +13,9 @@
 // 64 to 190 tokens 2 % faster to 10 % slower); slices added up in a cluster (2.5 to 4 us more than partial sums) or by the last block of a tile (9 to 60 us).
 //
 // The tensor core cuts off what a sum drops instead of rounding it, so a long chain's error grows with k.  The steps of 16 k take turns on several
-// accumulators beside each other in tensor memory, and up to 32 rows of x two sets of them take turns, 512 k each: while one is filled the readers add the
+// accumulators beside each other in tensor memory, and up to 32 rows of x two sets of them take turns, 512 k each (1,024 up to 16 rows): while one is filled the readers add the
 // other up in float32, so that no chain is longer than eight steps whatever k is.  Elements that are not the rounded 64-bit result: 32 rows of [34816, 5120] 2.3e-4
-// of them, with one set of chains over the whole of k 7.1e-4, gemm_stream.cu 3.8e-4; 24 of [37888, 8192] 2.8e-4, 12.3e-4 and 3.8e-4.  (1 % of the time.)
+// of them, with one set of chains over the whole of k 7.1e-4, gemm_stream.cu 3.8e-4; 24 of [37888, 8192] 2.8e-4, 12.3e-4 and 3.8e-4.  It costs 0.2 % of the time up to 16 rows, 1 % above.
 //
 // All waits on mbarriers are bounded: one that runs out sets an error word, the block waits for its own copies, frees its tensor memory and returns.
 // No TMA load here uses cluster multicast.
@@ -34,7 +34,7 @@ namespace pylon {
 
 constexpr int GC_ROWS = 128, GC_BK = 64, GC_THREADS = 192, GC_MOST_STAGES = 8;   // weight rows and k of a box
 constexpr int GC_COLUMNS = 256;                                                             // of tensor memory: two blocks to an SM
-constexpr int GC_SETS_MOST = 32, GC_SEGMENT = 8;                                  // columns up to which two sets of accumulators take turns; boxes to a turn
+constexpr int GC_SETS_MOST = 32, GC_SEGMENT = 8;                                  // columns up to which two sets of accumulators take turns; boxes to a turn of so many
 constexpr unsigned GC_WAIT_LIMIT = 1u << 22;                                                 // try_wait calls before a wait gives up
 
 __device__ __forceinline__ uint32_t gc_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -305,7 +305,7 @@ extern "C" int pylon_gemm_columns_gated(const void* x, const void* w, void* y, i
   const int boxes = (K + GC_BK - 1) / GC_BK, stage_bytes = (GC_ROWS + a.columns) * GC_BK * 2;
   a.stages = std::min({(GC_SMEM - 1024) / stage_bytes, GC_MOST_STAGES, boxes});
   const int sets = a.columns <= GC_SETS_MOST ? 2 : 1;
-  a.segment = sets == 2 ? GC_SEGMENT : boxes;
+  a.segment = sets == 2 ? GC_SEGMENT * (GC_SETS_MOST / a.columns) : boxes;
   a.chains = 1;
   while (2 * a.chains * sets * a.columns <= GC_COLUMNS && 2 * a.chains <= std::min(a.segment, boxes) * (GC_BK / 16)) a.chains *= 2;
   a.tmem_columns = 32;
